@@ -43,8 +43,7 @@ enum mhd_status {
                            at its next step, the batch's other solves go on */
   MHD_ERR_SOLVE = 6,    /* implicit solve did not converge */
   MHD_ERR_STATE = 7,    /* call out of order (e.g. step before prepare) */
-  MHD_ERR_TIMEOUT = 8   /* a tile's staged copies did not complete within the fluid
-                           kernel's bounded wait (TMA-staged variant): the solve stops */
+  MHD_ERR_TIMEOUT = 8   /* a wait inside a kernel ran into its bound: the solve stops */
 };
 
 /* Field identifiers: the reference's catalog names
@@ -486,17 +485,17 @@ int mhd_batch_set_constants(mhd_batch *batch, int slot, const mhd_constants *con
 int mhd_batch_sync(mhd_batch *batch, int slot, int group);
 int mhd_batch_prepare(mhd_batch *batch, int slot, double time, int64_t step);
 /* The fluid kernel's tile variants (Scheme_U_ + sources + update, the
- * step's largest pass): variant v tiles the owned cells in CTAs of 256
- * threads, shape[0] x shape[1] x shape[2] cells along k, j, i, compiled for
- * shape[3] resident CTAs per SM (its register cap).  A batch runs one
+ * step's largest pass): variant v tiles the owned cells in work items of 256
+ * cells, shape[0] x shape[1] x shape[2] along k, j, i, and shape[3] ranks its
+ * register budget (more resident work items, fewer registers each).  A batch runs one
  * (default 0); mhd_batch_time_fluid_tiles times each on the batch's active
  * solves (the fluid pass alone, `reps` launches after one untimed, writing
  * only the next-step state buffer, which the next step rewrites: the solves'
  * results do not change), mhd_batch_fluid_tile sets one (the step graphs are
  * captured anew).  The choice does not change results: every variant
  * computes each face flux and cell update with the same operations.
- * Variant 6 (16 x 4 x 4) stages each tile's cells with TMA tensor copies,
- * the next tile's while the current one is computed. */
+ * Variant 6 is variant 0's tile with more resident work items in mixed
+ * precision. */
 #define MHD_NUM_FLUID_TILES 7
 int mhd_fluid_tile_shape(int variant, int32_t shape[4]);
 int mhd_batch_fluid_tile(mhd_batch *batch, int variant);

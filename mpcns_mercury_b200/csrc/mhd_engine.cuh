@@ -15,12 +15,12 @@
 
 namespace mhd {
 
-// The fluid kernel's tile variants: cells along k, j, i of one 256-thread
-// CTA, and the resident CTAs per SM asked of the compiler (its register cap,
-// 65536 / (256 n)).  The batch runs one of them (mhd_batch_fluid_tile),
+// The fluid kernel's tile variants: cells along k, j, i of one work item (256
+// cells, two items per tile, one per ion species), and a rank of its register
+// budget (fluid_ctas).  The batch runs one of them (mhd_batch_fluid_tile),
 // picked by timing (mhd_batch_time_fluid_tiles); variant 0 is the default:
-// 16 x 4 x 4 wastes fewer lanes than 32 x 4 x 2 on k extents that are not
-// multiples of 32 and needs 6% fewer face fluxes per tile (912 vs 968).
+// 16 x 4 x 4 wastes fewer lanes than wider tiles on k extents that are not
+// multiples of 32.
 struct FluidTile {
   int k, j, i, min_ctas;
 };
@@ -29,20 +29,18 @@ __host__ __device__ constexpr FluidTile fluid_tile(int v) {
   return v == 1 ? FluidTile{8, 8, 4, 4} : v == 2 ? FluidTile{8, 8, 4, 3} : v == 3 ? FluidTile{16, 4, 4, 4}
          : v == 4 ? FluidTile{16, 4, 4, 2} : v == 5 ? FluidTile{8, 8, 4, 2} : FluidTile{16, 4, 4, 3};
 }
-// Variant 6 stages each tile's cell box (density and u, v, w, p of its
-// species) with TMA tensor copies issued by a producer warp up to two tiles
-// ahead of the compute threads (double-buffered, mbarrier-completed).  Its box: the 16 x 4 x 4
-// tile and one cell beyond each side, the k window widened to whole 16-byte
-// units from a 16-byte-aligned start.
-__host__ __device__ constexpr bool fluid_tma(int v) { return v == 6; }
-// Threads of a fluid CTA: 256 that compute (one per cell of the tile), and
-// for the staged variant a producer warp that issues the copies.
-__host__ __device__ constexpr int fluid_threads(int v) { return fluid_tma(v) ? 256 + 32 : 256; }
-constexpr int kTmaBoxJI = 6;  // j and i extents of the staged box
-__host__ __device__ constexpr int tma_box_k(int es) { return es == 4 ? 24 : 20; }
-// Components of a block's real-valued M region that its tensor map spans
-// (through the primitive variables of both species).
-constexpr int kTmaMComps = kComp.first[MHD_PV_NA] + 5 - kNumUComps;
+// Threads of a fluid CTA: one per column of the tile's cells along i.
+__host__ __device__ constexpr int fluid_threads(int v) { return fluid_tile(v).k * fluid_tile(v).j; }
+// Ion species that a thread advances together: both in FP32, where the metric
+// and the source fields are then loaded once, one in FP64, whose values take
+// two registers each.
+__host__ __device__ constexpr int fluid_species(int es) { return es == 8 ? 1 : 2; }
+// Resident CTAs per SM asked of the compiler.  The kernel waits on loads, and
+// registers (loads in flight per thread) are worth more to it than warps.
+__host__ __device__ constexpr int fluid_ctas(int v, int es) {
+  const int n = fluid_tile(v).min_ctas;
+  return es == 8 ? 6 + n : v == 6 ? 8 : 3 + n;
+}
 constexpr int kTileThreads = 256;
 constexpr bool fluid_tiles_ok() {
   for (int v = 0; v < kNumFluidTiles; ++v)
@@ -96,18 +94,12 @@ __host__ __device__ constexpr bool is_metric(int comp) { return comp >= kMetricF
 __host__ __device__ constexpr int rslot(int comp) {
   return comp - kNumUComps - (comp >= kMetricFirst + kNumMetric ? kNumMetric : 0);
 }
-static_assert(kTmaMComps == rslot(kComp.first[MHD_PV_NA] + 4) + 1 && kComp.first[MHD_PV_NA] < kMetricFirst,
-              "the primitive variables lie in the first kTmaMComps real-valued M components");
 
 // Per-block descriptor (device).  Block memory: U buffers of 10 real arrays
 // each; M = [10 metric double arrays | kNumRComps real arrays].
 struct DevBlock {
   void *U[2];         // U_H, U_Na components (10) of buffer 0 / 1
   char *M;
-  // TMA tensor maps of the block (U buffer 0, U buffer 1, the real-valued M
-  // components; 128 bytes each, 64-byte aligned), null where none could be
-  // encoded: the staged fluid variant then loads that block's boxes itself
-  const void *tmap;
   int64_t total, si, sj;
   int G, n[3];
   int solve;          // index of the owning solve in the directory
@@ -127,8 +119,24 @@ struct ConstsT {
   int nghost;
   int resistive;
   T bc[MHD_NUM_BC];  // values of the physical boundary operations (mhd_bc_const)
+  // combinations of the above that the sources (FluidRHS.cpp:206-527) and the
+  // ambipolar EMF form per cell, evaluated once on the host in the same order
+  T src_a4, src_a5, src_a1Na, src_a6;
+  T src_b1[2], src_b2[2];  // M / (M + M_Na) and M_Na / (M + M_Na) of H+, Na+
+  T pe_coeff;
 };
 using Consts = ConstsT<double>;
+inline void combine(Consts &c) {
+  c.src_a4 = c.L_ref / c.U_ref;
+  c.src_a5 = (3.0 * c.L_ref * c.k_Boltz * c.n_ref) / (c.rho_ref * c.U_ref * c.U_ref * c.U_ref);
+  c.src_a1Na = (c.L_ref / c.U_ref) * (c.m_Na / c.rho_ref) * 1e6;
+  c.src_a6 = (1.0e6 * c.L_ref * c.k_Boltz) / (c.rho_ref * c.U_ref * c.U_ref * c.U_ref * (c.gamma - 1.0));
+  c.src_b1[0] = c.M_H / (c.M_H + c.M_Na);
+  c.src_b1[1] = c.M_Na / (c.M_Na + c.M_Na);
+  c.src_b2[0] = c.M_Na / (c.M_H + c.M_Na);
+  c.src_b2[1] = c.M_Na / (c.M_Na + c.M_Na);
+  c.pe_coeff = (c.rho_ref * c.U_ref) / (c.q_e * c.L_ref * c.B_ref * c.n_ref);
+}
 inline ConstsT<float> to_float(const Consts &c) {
   ConstsT<float> f{(float)c.gamma, (float)c.M_H, (float)c.M_Na, (float)c.M_ref, (float)c.T_ref,
                    (float)c.L_ref, (float)c.U_ref, (float)c.B_ref, (float)c.n_ref, (float)c.rho_ref,
@@ -138,6 +146,15 @@ inline ConstsT<float> to_float(const Consts &c) {
                    (float)c.arti_eta_max, (float)c.arti_J_start, (float)c.arti_J_on, c.ambipolar,
                    c.local_arti, c.nghost, c.resistive, {}};
   for (int q = 0; q < MHD_NUM_BC; ++q) f.bc[q] = (float)c.bc[q];
+  f.src_a4 = (float)c.src_a4;
+  f.src_a5 = (float)c.src_a5;
+  f.src_a1Na = (float)c.src_a1Na;
+  f.src_a6 = (float)c.src_a6;
+  for (int q = 0; q < 2; ++q) {
+    f.src_b1[q] = (float)c.src_b1[q];
+    f.src_b2[q] = (float)c.src_b2[q];
+  }
+  f.pe_coeff = (float)c.pe_coeff;
   return f;
 }
 
@@ -301,7 +318,7 @@ __host__ __device__ inline RangeBox range_of(int kind, const int n[3], int g) {
   return r;
 }
 // Work items of a block: the fluid kinds use 3-D tiles of their variant's
-// shape (two work items per tile, one per species); every other range is
+// shape (two work items per tile, one per ion species); every other range is
 // cut into runs of kTileThreads consecutive positions of its box (k fastest),
 // so no lane idles at the end of short k rows.
 __host__ __device__ inline int tiles_of(const RangeBox &r, int kind) {

@@ -45,6 +45,7 @@ constexpr int cPEN = kComp.first[MHD_PE_NODE], cAMB = kComp.first[MHD_AMBI_COEF]
 constexpr int cUCK = kComp.first[MHD_UCON_COEF];
 constexpr int cIHX = kComp.first[MHD_HALL_IH_XI], cIHY = kComp.first[MHD_HALL_IH_ETA], cIHZ = kComp.first[MHD_HALL_IH_ZETA];
 constexpr int cFM = kComp.first[MHD_FLUX_METRIC];
+constexpr int cFT = kFirstInternal;  // re, c of H+, re, c of Na+
 constexpr int cJAC = kComp.first[MHD_JAC], cJDX = kComp.first[MHD_JDXI], cJDY = kComp.first[MHD_JDET],
               cJDZ = kComp.first[MHD_JDZE];
 constexpr int cAX = kComp.first[MHD_AREA_XI], cAY = kComp.first[MHD_AREA_ETA], cAZ = kComp.first[MHD_AREA_ZETA];
@@ -69,21 +70,32 @@ template <class R>
 __device__ __forceinline__ R dmin(R a, R b) { return (b < a) ? b : a; }
 
 // One block's fields for the current step: U = current buffer, M = metric
-// (double) then the other real-valued components (mhd_engine.cuh).
+// (double) then, at Mr, the other real-valued components (mhd_engine.cuh).
 // Element offsets inside a block are 32-bit (mhd_batch_add keeps every
 // block's component arrays below 2^31 elements in total).
 template <class R>
 struct V {
-  R *U, *Un;
-  char *M;
+  char *U, *Un, *M, *Mr;
+  uint32_t tb;  // bytes of one real-valued component array
   int total, si, sj;
   int G, n0, n1, n2;
   // real-valued component (U or M)
   __device__ __forceinline__ R *c(int comp) const {
-    return comp < kNumUComps ? U + comp * total : (R *)(M + (int64_t)kNumMetric * total * 8) + rslot(comp) * total;
+    return (R *)(comp < kNumUComps ? U + (uint64_t)comp * tb : Mr + (uint64_t)rslot(comp) * tb);
   }
+  __device__ __forceinline__ R *next(int comp) const { return (R *)(Un + (uint64_t)comp * tb); }  // U, the other buffer
   // metric component (JAC, JD*), double in every precision
-  __device__ __forceinline__ double *m(int comp) const { return (double *)M + (comp - kMetricFirst) * total; }
+  __device__ __forceinline__ double *m(int comp) const {
+    return (double *)(M + (uint64_t)(comp - kMetricFirst) * (tb * (8 / (uint32_t)sizeof(R))));
+  }
+  // Component `comp` at byte offset bo of its array (bo = off() times the
+  // element size), through the read-only path.  The array's address is
+  // warp-uniform (build_item) and bo is 32 bits, so no thread holds 64-bit
+  // addresses: without that k_fluid spilled 700 bytes at 80 registers.
+  __device__ __forceinline__ R ld(int comp, uint32_t bo) const { return __ldg((const R *)((const char *)c(comp) + bo)); }
+  __device__ __forceinline__ double ldm(int comp, uint32_t bo) const {
+    return __ldg((const double *)((const char *)m(comp) + bo));
+  }
   __device__ __forceinline__ int off(int i, int j, int k) const { return (i + G) * si + (j + G) * sj + (k + G); }
 };
 #define AT(cc, i, j, k) (B.c(cc)[B.off((i), (j), (k))])
@@ -98,10 +110,9 @@ struct V {
 struct Item {
   int s;       // solve
   int blk;     // block of the solve
-  int species; // kCells2 only
+  int species; // fluid ranges only
   int i, j, k;
   bool in;     // inside the kernel's range
-  int o[3];    // tile origin (i, j, k)
   int hi[3];   // range upper bounds (exclusive)
   int lo[3];   // range lower bounds
 };
@@ -132,18 +143,31 @@ __device__ __forceinline__ void lookup_item(const Dir &D, int w, int &s, int &b,
   t = lw - bp[blo];
 }
 
-// Origin (i, j, k) and species of tile t of a fluid range over range box r.
-template <int KIND>
-__device__ __forceinline__ void fluid_tile_origin(const RangeBox &r, int t, int o[3], int &species) {
-  constexpr FluidTile T = fluid_tile(fluid_variant(KIND));
-  species = t & 1;
-  t >>= 1;
-  const int tk = (r.hi[2] - r.lo[2] + T.k - 1) / T.k;
-  const int tj = (r.hi[1] - r.lo[1] + T.j - 1) / T.j;
-  const int bk = t % tk, bj = (t / tk) % tj, bi = t / (tk * tj);
-  o[0] = r.lo[0] + bi * T.i;
-  o[1] = r.lo[1] + bj * T.j;
-  o[2] = r.lo[2] + bk * T.k;
+// The view of block DB with U buffer `cur` current.
+template <class R>
+__device__ __forceinline__ void set_view(V<R> &B, const DevBlock &DB, int cur) {
+  B.U = (char *)DB.U[cur];
+  B.Un = (char *)DB.U[cur ^ 1];
+  B.M = DB.M;
+  B.total = (int)DB.total;
+  B.tb = (uint32_t)B.total * (uint32_t)sizeof(R);
+  B.Mr = DB.M + (int64_t)kNumMetric * DB.total * 8;
+  B.si = (int)DB.si;
+  B.sj = (int)DB.sj;
+  B.G = DB.G;
+  B.n0 = DB.n[0];
+  B.n1 = DB.n[1];
+  B.n2 = DB.n[2];
+}
+
+// A value that every lane of the (converged) warp holds, in a form the
+// compiler knows to be the same for the warp.
+__device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+template <class T>
+__device__ __forceinline__ T *uniform(T *p) {
+  const unsigned long long v = (unsigned long long)p;
+  const unsigned lo = __shfl_sync(0xffffffffu, (unsigned)v, 0), hi = __shfl_sync(0xffffffffu, (unsigned)(v >> 32), 0);
+  return (T *)(((unsigned long long)hi << 32) | lo);
 }
 
 // The work item (s, b, t) of range KIND as this thread sees it, and the
@@ -157,18 +181,19 @@ __device__ __forceinline__ void build_item(const Dir &D, int s, int b, int t, It
   if constexpr (KIND == kResK) r.hi[2] = DB.reskhi;
   it.s = s;
   it.blk = b;
-  it.species = 0;
   for (int a = 0; a < 3; ++a) {
     it.hi[a] = r.hi[a];
     it.lo[a] = r.lo[a];
   }
-  if constexpr (fluid_variant(KIND) >= 0) {  // a fluid tile, one species
+  if constexpr (fluid_variant(KIND) >= 0) {  // a fluid tile: one thread per column of cells along i
     constexpr FluidTile T = fluid_tile(fluid_variant(KIND));
-    fluid_tile_origin<KIND>(r, t, it.o, it.species);
-    it.k = it.o[2] + (tid % T.k);
-    it.j = it.o[1] + ((tid / T.k) % T.j);
-    it.i = it.o[0] + (tid / (T.k * T.j));
-    it.in = it.i < r.hi[0] && it.j < r.hi[1] && it.k < r.hi[2];
+    const int tk = (r.hi[2] - r.lo[2] + T.k - 1) / T.k, tj = (r.hi[1] - r.lo[1] + T.j - 1) / T.j;
+    const int q = t >> 1, rest = q / tk;
+    it.species = t & 1;
+    it.k = r.lo[2] + (q - rest * tk) * T.k + tid % T.k;
+    it.j = r.lo[1] + (rest % tj) * T.j + tid / T.k;
+    it.i = r.lo[0] + (rest / tj) * T.i;  // the column's first cell
+    it.in = it.j < r.hi[1] && it.k < r.hi[2];
   } else {  // a run of kTileThreads consecutive positions of the range box (k fastest)
     const int ek = r.hi[2] - r.lo[2], ej = r.hi[1] - r.lo[1];
     const int L = t * kTileThreads + tid;
@@ -177,19 +202,17 @@ __device__ __forceinline__ void build_item(const Dir &D, int s, int b, int t, It
     it.j = r.lo[1] + rest % ej;
     it.i = r.lo[0] + rest / ej;
     it.in = L < ek * ej * (r.hi[0] - r.lo[0]);
-    it.o[0] = it.o[1] = it.o[2] = 0;
   }
   const int cur = D.state[s].cur;
-  B.U = (R *)DB.U[cur];
-  B.Un = (R *)DB.U[cur ^ 1];
-  B.M = DB.M;
-  B.total = (int)DB.total;
-  B.si = (int)DB.si;
-  B.sj = (int)DB.sj;
-  B.G = DB.G;
-  B.n0 = DB.n[0];
-  B.n1 = DB.n[1];
-  B.n2 = DB.n[2];
+  set_view(B, DB, cur);
+  B.U = uniform(B.U);
+  B.Un = uniform(B.Un);
+  B.M = uniform(B.M);
+  B.Mr = uniform(B.Mr);
+  B.tb = uniform((int)B.tb);
+  B.total = uniform(B.total);
+  B.si = uniform(B.si);
+  B.sj = uniform(B.sj);
 }
 
 // Work-item loop: for every tile of range `KIND` of every active solve, call
@@ -212,168 +235,6 @@ __device__ __forceinline__ void for_items(const Dir &D, F &&f, E &&end = E{}) {
     build_item<R, KIND>(D, s, b, t, it, B);
     f(D.solves[s], B, it);
     end(w);
-  }
-}
-
-// ------------------------------------------------------------------ TMA staging
-__device__ __forceinline__ uint32_t smem_u32(const void *p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(done)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-// Waits for phase `parity` of the barrier to complete, at most about a
-// second: false when it did not (the caller records MHD_ERR_TIMEOUT).
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity) {
-  for (int n = 0; n < (1 << 24); ++n) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if (n >= 16) __nanosleep(64);
-  }
-  return false;
-}
-// One 4-D tiled tensor copy (no multicast) of the box at coordinates
-// (c0 .. c3) into this CTA's shared memory, completing on `bar`.
-__device__ __forceinline__ void tma_load_4d(void *dst, const void *map, int c0, int c1, int c2, int c3,
-                                            uint64_t *bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
-      "[%6];" ::"r"(smem_u32(dst)),
-      "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
-      : "memory");
-}
-
-// The staged variant's 256 compute threads synchronise among themselves
-// (named barrier 1; its producer warp takes no part).
-__device__ __forceinline__ void compute_bar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
-__device__ __forceinline__ bool compute_and(bool v) {
-  uint32_t r;
-  asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.and.pred q, 1, 256, p;\n selp.u32 %0, 1, 0, q;\n}"
-               : "=r"(r)
-               : "r"((uint32_t)v)
-               : "memory");
-  return r != 0;
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-// Work-item loop of the TMA-staged fluid variant, warp-specialised: the
-// CTA's 256 compute threads run f(S, B, item, box) for its items, while its
-// ninth warp (one lane) looks the items up and stages each one's box
-// (density, then u, v, w, p of its species; k window of
-// tma_box_k(sizeof(R)) from the 16-byte unit holding k = o - 1, j and i
-// windows of 6 from o - 1) with TMA tensor copies into one of two stages,
-// running up to two items ahead.  bars[0..1]: a stage is full (the item's
-// record, and its copies complete); bars[2..3]: the compute threads are done
-// reading it (f arrives once its face fluxes are built).  A block without
-// tensor maps has its box loaded by the compute threads instead.  A wait that
-// does not end within its bound records MHD_ERR_TIMEOUT on the solve of the
-// item waited for and ends the CTA's loop.
-template <class R, int KIND, class F>
-__device__ __forceinline__ void for_fluid_items_tma(const Dir &D, R *stage, uint64_t *bars, F &&f) {
-  constexpr int W = tma_box_k(sizeof(R)), BV = W * kTmaBoxJI * kTmaBoxJI;
-  constexpr int kAlign = 16 / (int)sizeof(R);
-  __shared__ int sh[2][4];  // per stage: solve, block, tile, copy state (0 inactive, 1 TMA, 2 by the threads)
-  const int total = D.solve_tile_prefix[KIND][D.nsolves];
-  const int tid = threadIdx.x;
-  // the box's coordinates in the block's arrays (k, j, i including the ghost offset)
-  auto box_at = [&](const DevBlock &DB, int s, int t, int c[3], int &species) {
-    const DevSolve &S = D.solves[s];
-    const RangeBox r = range_of(KIND, DB.n, S.c.nghost);
-    int o[3];
-    fluid_tile_origin<KIND>(r, t, o, species);
-    c[0] = (o[2] + DB.G - 1) & ~(kAlign - 1);
-    c[1] = o[1] - 1 + DB.G;
-    c[2] = o[0] - 1 + DB.G;
-  };
-  if (tid == 0) {
-    mbar_init(&bars[0], 1);
-    mbar_init(&bars[1], 1);
-    mbar_init(&bars[2], kTileThreads);
-    mbar_init(&bars[3], kTileThreads);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  if (tid >= kTileThreads) {  // the producer warp
-    if (tid != kTileThreads) return;
-    uint32_t n = 0;
-    for (int w = blockIdx.x; w < total; w += gridDim.x, ++n) {
-      const int st = n & 1;
-      int s, b, t;
-      lookup_item<KIND>(D, w, s, b, t);
-      if (n >= 2 && !mbar_wait_bounded(&bars[2 + st], ((n >> 1) - 1) & 1u)) {
-        atomicCAS(&D.state[s].status, 0, (int)MHD_ERR_TIMEOUT);
-        return;
-      }
-      sh[st][0] = s;
-      sh[st][1] = b;
-      sh[st][2] = t;
-      const DevBlock &DB = D.solves[s].blocks[b];
-      if (!solve_active(D, s) || !DB.tmap) {
-        sh[st][3] = solve_active(D, s) ? 2 : 0;
-        mbar_arrive(&bars[st]);
-        continue;
-      }
-      sh[st][3] = 1;
-      int c[3], species;
-      box_at(DB, s, t, c, species);
-      const char *maps = (const char *)DB.tmap;
-      R *dst = stage + st * 5 * BV;
-      const int cur = D.state[s].cur;
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the stage's earlier reads, then the copies
-      mbar_expect_tx(&bars[st], (uint32_t)(5 * BV * sizeof(R)));
-      tma_load_4d(dst, maps + 128 * cur, c[0], c[1], c[2], species ? 5 : 0, &bars[st]);
-      tma_load_4d(dst + BV, maps + 256, c[0], c[1], c[2], rslot(species ? cPVN : cPVH), &bars[st]);
-    }
-    return;
-  }
-  uint32_t n = 0;
-  for (int w = blockIdx.x; w < total; w += gridDim.x, ++n) {
-    const int st = n & 1;
-    const bool ok = mbar_wait_bounded(&bars[st], (n >> 1) & 1u);
-    if (!compute_and(ok)) {
-      if (tid == 0) atomicCAS(&D.state[sh[st][0]].status, 0, (int)MHD_ERR_TIMEOUT);
-      return;
-    }
-    const int s = sh[st][0], b = sh[st][1], t = sh[st][2], how = sh[st][3];
-    R *box = stage + st * 5 * BV;
-    if (how == 0) {  // inactive solve (every compute thread agrees)
-      mbar_arrive(&bars[2 + st]);
-      continue;
-    }
-    if (how == 2) {  // no tensor maps: the same box by plain loads (zeros outside the block's arrays)
-      const DevBlock &DB = D.solves[s].blocks[b];
-      int c[3], species;
-      box_at(DB, s, t, c, species);
-      const int cur = D.state[s].cur;
-      const R *u0p = (const R *)DB.U[cur] + (species ? 5 : 0) * DB.total;
-      const R *pvp = (const R *)(DB.M + (int64_t)kNumMetric * DB.total * 8) +
-                     (int64_t)rslot(species ? cPVN : cPVH) * DB.total;
-      const int ext1 = DB.n[1] + 1 + 2 * DB.G, ext0 = DB.n[0] + 1 + 2 * DB.G;
-      for (int q = tid; q < 5 * BV; q += kTileThreads) {
-        const int m = q / BV, e = q % BV;
-        const int x = c[0] + e % W, y = c[1] + (e / W) % kTmaBoxJI, z = c[2] + e / (W * kTmaBoxJI);
-        const R *src = m == 0 ? u0p : pvp + (int64_t)(m - 1) * DB.total;
-        box[q] = (x < DB.sj && y < ext1 && z < ext0) ? src[(int64_t)z * DB.si + (int64_t)y * DB.sj + x] : R(0.0);
-      }
-      compute_bar();
-    }
-    Item it;
-    V<R> B;
-    build_item<R, KIND>(D, s, b, t, it, B);
-    f(D.solves[s], B, it, (const R *)box);
   }
 }
 
@@ -580,7 +441,7 @@ __global__ void __launch_bounds__(kTileThreads) k_edge_emf(Dir D) {
     const ConstsT<R> &c = consts_of<R>(S);
     const int i = it.i, j = it.j, k = it.k;
     const R Cuct = R(0.5);
-    const R pc = (c.rho_ref * c.U_ref) / (c.q_e * c.L_ref * c.B_ref * c.n_ref);
+    const R pc = c.pe_coeff;
     if (i < B.n0) {
       const R Ec = R(0.25) * (AT(cEFY, i, j, k) + AT(cEFY, i, j, k - 1) + AT(cEFZ, i, j, k) + AT(cEFZ, i, j - 1, k));
       const R ae = max_abs_u4(B, 1, i, j, k, i, j - 1, k, i, j, k - 1, i, j - 1, k - 1);
@@ -712,318 +573,229 @@ __global__ void __launch_bounds__(kTileThreads) k_add_hall(Dir D) {
 }
 
 // ------------------------------------------------------------------ fluid update
-// Rusanov face flux of Scheme_U_ (Z4_Mercury/src/physics/MercurySolver_FluidRHS.cpp:36-104)
-// from the two cells' staged quantities (rho, u, v, w, p and
-// the per-cell terms re = p / (g - 1) + rho |u|^2 / 2, c = sqrt(g p / rho),
-// which Scheme_U_ evaluates per face with the same operations on the same
-// cell values, so staging them once per cell keeps the result bit for bit).
+// A cell's quantities in the Rusanov flux of Scheme_U_
+// (Z4_Mercury/src/physics/MercurySolver_FluidRHS.cpp:36-104): rho, u, v, w, p
+// and re = p / (g - 1) + rho |u|^2 / 2, c = sqrt(g p / rho), which Scheme_U_
+// evaluates per face with the same operations on the same cell values
+// (k_pv_uplus stores them per cell).
 template <class R>
-__device__ __forceinline__ void rusanov_staged(const R *L, const R *Rr, R k1, R k2, R k3, R sk, R out[5]) {
-  const R rhoL = L[0], uL = L[1], vL = L[2], wL = L[3], pL = L[4], reL = L[5], cL = L[6];
-  const R rhoR = Rr[0], uR = Rr[1], vR = Rr[2], wR = Rr[3], pR = Rr[4], reR = Rr[5], cR = Rr[6];
-  const R uvwL = k1 * uL + k2 * vL + k3 * wL, uvwR = k1 * uR + k2 * vR + k3 * wR;
-  const R rad = dmax(fabs(uvwL) + cL * sk, fabs(uvwR) + cR * sk);
-  out[0] = R(0.5) * (rhoL * uvwL + rhoR * uvwR) - R(0.5) * rad * (rhoR - rhoL);
-  out[1] = R(0.5) * ((rhoL * uvwL * uL + k1 * pL) + (rhoR * uvwR * uR + k1 * pR)) - R(0.5) * rad * (rhoR * uR - rhoL * uL);
-  out[2] = R(0.5) * ((rhoL * uvwL * vL + k2 * pL) + (rhoR * uvwR * vR + k2 * pR)) - R(0.5) * rad * (rhoR * vR - rhoL * vL);
-  out[3] = R(0.5) * ((rhoL * uvwL * wL + k3 * pL) + (rhoR * uvwR * wR + k3 * pR)) - R(0.5) * rad * (rhoR * wR - rhoL * wL);
-  out[4] = R(0.5) * (uvwL * (reL + pL) + uvwR * (reR + pR)) - R(0.5) * rad * (reR - reL);
+struct FluidCell {
+  R rho, u, v, w, p, re, c;
+};
+template <class R>
+__device__ __forceinline__ FluidCell<R> fluid_cell(const V<R> &B, int s, uint32_t o) {
+  const int pv0 = s ? cPVN : cPVH, t0 = cFT + 2 * s;
+  FluidCell<R> q;
+  q.rho = B.ld(s ? cUN : cUH, o);
+  q.u = B.ld(pv0, o);
+  q.v = B.ld(pv0 + 1, o);
+  q.w = B.ld(pv0 + 2, o);
+  q.p = B.ld(pv0 + 3, o);
+  q.re = B.ld(t0, o);
+  q.c = B.ld(t0 + 1, o);
+  return q;
+}
+// A face's JD and |JD|: FP32 reads the real-typed copy (k_face_normals), FP64
+// the metric itself (the same values).
+template <class R>
+struct FluidFace {
+  R k1, k2, k3, sk;
+};
+template <class R, int DIR>
+__device__ __forceinline__ FluidFace<R> fluid_face(const V<R> &B, uint32_t o) {
+  constexpr int cm = sizeof(R) == 4 ? cFM + 3 * DIR : DIR == 0 ? cJDX : DIR == 1 ? cJDY : cJDZ;
+  constexpr int cn = DIR == 0 ? cFNX : DIR == 1 ? cFNY : cFNZ;
+  FluidFace<R> f;
+  if constexpr (sizeof(R) == 4) {
+    f.k1 = B.ld(cm, o);
+    f.k2 = B.ld(cm + 1, o);
+    f.k3 = B.ld(cm + 2, o);
+  } else {
+    f.k1 = B.ldm(cm, o);
+    f.k2 = B.ldm(cm + 1, o);
+    f.k3 = B.ldm(cm + 2, o);
+  }
+  f.sk = B.ld(cn + 3, o);
+  return f;
+}
+template <class R>
+__device__ __forceinline__ void rusanov(const FluidCell<R> &L, const FluidCell<R> &Q, const FluidFace<R> &f, R out[5]) {
+  const R uvwL = f.k1 * L.u + f.k2 * L.v + f.k3 * L.w, uvwR = f.k1 * Q.u + f.k2 * Q.v + f.k3 * Q.w;
+  const R rad = dmax(fabs(uvwL) + L.c * f.sk, fabs(uvwR) + Q.c * f.sk);
+  out[0] = R(0.5) * (L.rho * uvwL + Q.rho * uvwR) - R(0.5) * rad * (Q.rho - L.rho);
+  out[1] = R(0.5) * ((L.rho * uvwL * L.u + f.k1 * L.p) + (Q.rho * uvwR * Q.u + f.k1 * Q.p)) -
+           R(0.5) * rad * (Q.rho * Q.u - L.rho * L.u);
+  out[2] = R(0.5) * ((L.rho * uvwL * L.v + f.k2 * L.p) + (Q.rho * uvwR * Q.v + f.k2 * Q.p)) -
+           R(0.5) * rad * (Q.rho * Q.v - L.rho * L.v);
+  out[3] = R(0.5) * ((L.rho * uvwL * L.w + f.k3 * L.p) + (Q.rho * uvwR * Q.w + f.k3 * Q.p)) -
+           R(0.5) * rad * (Q.rho * Q.w - L.rho * L.w);
+  out[4] = R(0.5) * (uvwL * (L.re + L.p) + uvwR * (Q.re + Q.p)) - R(0.5) * rad * (Q.re - L.re);
 }
 
-// A tile's faces per direction and in all (variant V).
-template <int VT>
-struct TileFaces {
-  static constexpr FluidTile T = fluid_tile(VT);
-  static constexpr int n0 = (T.i + 1) * T.j * T.k, n1 = T.i * (T.j + 1) * T.k, n2 = T.i * T.j * (T.k + 1);
-  static constexpr int all = n0 + n1 + n2;
-};
-
-// Shared memory of the fluid kernel's tile (variant VT): the staged
-// quantities of the tile's cells and their face neighbours (7 values per cell
-// of the tile padded by one layer) and the tile's face fluxes (5 per face).
-// The TMA-staged variant instead holds two stages of its box (5 components
-// each), re and c over the box, the face fluxes, and 128 bytes to align the
-// stages to 128 bytes.
-template <class R, int VT>
-struct FluidSmem {
-  static constexpr FluidTile T = fluid_tile(VT);
-  static constexpr int PK = T.k + 2, PJ = T.j + 2, PI = T.i + 2, cells = PK * PJ * PI;
-  static constexpr int BV = tma_box_k(sizeof(R)) * kTmaBoxJI * kTmaBoxJI;  // elements of one component's box
-  static constexpr size_t bytes =
-      fluid_tma(VT) ? 128 + sizeof(R) * (size_t)(2 * 5 * BV + 2 * BV + 5 * TileFaces<VT>::all)
-                    : sizeof(R) * (size_t)(7 * cells + 5 * TileFaces<VT>::all);
-  static_assert(!fluid_tma(VT) || (T.k == 16 && T.j == 4 && T.i == 4), "the staged box assumes a 16 x 4 x 4 tile");
-  static_assert((BV * sizeof(R)) % 128 == 0, "stages stay 128-byte aligned");
-};
-
-// ZeroRHS_ + Scheme_U_ + AddSourceToRHS_Fluid (FluidRHS.cpp:206-527) +
-// ApplyUpdate_Euler_ (Z4_Mercury/src/physics/MercurySolver_Advance.cpp:73-147)
-// for one tile of owned cells and one ion species; the state goes to the
-// other buffer.  Per direction, the tile's face fluxes are computed once into
-// shared memory (a face's flux has the same inputs and operation order for
-// both cells that share it), then every cell accumulates
-// r[m] -= (F+ - F-) / J, the per-component order of Scheme_U_'s divergence.
 // Minimum resident CTAs per SM asked of the compiler for the primitive pass
-// (caps registers at 65536 / (256 * n)); the fluid kernel's is its tile variant's.
+// (caps registers at 65536 / (256 * n)).
 #ifndef MHD_MIN_CTAS_PV
 #define MHD_MIN_CTAS_PV 4
 #endif
+
+// ZeroRHS_ + Scheme_U_ + AddSourceToRHS_Fluid (FluidRHS.cpp:206-527) +
+// ApplyUpdate_Euler_ (Z4_Mercury/src/physics/MercurySolver_Advance.cpp:73-147)
+// for one tile of owned cells and both ion species; the state goes to the
+// other buffer.  A thread takes a column of the tile's cells along i: the
+// flux through the face between two of them is computed once and carried
+// over, the fluxes of the cell's four other faces are computed by each of
+// the two cells that share one, from loads that hit L1 (no shared memory, no
+// barrier).  Every cell then takes its six faces' differences direction by
+// direction, r[m] -= (F+ - F-) / J, the per-component order of Scheme_U_'s
+// divergence.
+// Bound by the latency of its loads: 15 to 24 warps per SM at the register
+// budget that keeps most of a cell's loads in flight.  On the 96^3 mixed box
+// 0.086 ms (0.150 for the shared-memory tile of face fluxes this replaced: 84 M
+// warp instructions against 40 M), on 64 x 64 x 128 cells in FP64 0.112 ms
+// (0.178); 236 B per cell would take 0.032 and 472 B 0.038.
+// Columns are the tile's whole depth along i; when the tiles would not fill the
+// grid they are cut into single cells, which trades the carried flux for four
+// times the threads (32^3 in FP64: 0.025 ms in columns, 0.017 in cells; 64^3
+// mixed, where the tiles fill the grid: 0.040 and 0.041).
 template <class R, int VT>
-__global__ void __launch_bounds__(fluid_threads(VT), (sizeof(R) == 8 && fluid_tma(VT)) ? 2 : fluid_tile(VT).min_ctas)
-    k_fluid(Dir D) {
-  constexpr FluidTile T = fluid_tile(VT);
-  constexpr int kNF0 = TileFaces<VT>::n0, kNF1 = TileFaces<VT>::n1, kTileFaces = TileFaces<VT>::all;
-  constexpr int kTileK = T.k, kTileJ = T.j;
-  constexpr int PK = FluidSmem<R, VT>::PK, PJ = FluidSmem<R, VT>::PJ, NP = FluidSmem<R, VT>::cells;
-  constexpr bool kTma = fluid_tma(VT);
-  constexpr int W = tma_box_k(sizeof(R)), BV = FluidSmem<R, VT>::BV;
-  extern __shared__ __align__(16) unsigned char fluid_smem[];
-  unsigned char *sbase = fluid_smem;
-  if constexpr (kTma) sbase += (128 - (smem_u32(fluid_smem) & 127)) & 127;
-  // the staged variant: [2 stages][5][BV] | RC [2][BV] (re, c) | F
-  R *stage = reinterpret_cast<R *>(sbase);
-  R(*RC)[BV] = reinterpret_cast<R(*)[BV]>(sbase + sizeof(R) * 10 * BV);
-  R(*C)[NP] = reinterpret_cast<R(*)[NP]>(sbase);  // [7][NP]
-  R(*F)[kTileFaces] =
-      reinterpret_cast<R(*)[kTileFaces]>(sbase + sizeof(R) * (kTma ? 12 * BV : 7 * NP));  // [5][faces]
-  __shared__ uint64_t bars[4];
-  auto cta_sync = [] {
-    if constexpr (kTma) compute_bar();
-    else __syncthreads();
-  };
-  auto body = [&](const DevSolve &S, const V<R> &B, const Item &it, const R *box) {
+__global__ void __launch_bounds__(fluid_threads(VT), fluid_ctas(VT, sizeof(R))) k_fluid(Dir D) {
+  constexpr int KIND = fluid_kind(VT), NS = fluid_species(sizeof(R)), TI = fluid_tile(VT).i;
+  __shared__ int sh[3];
+  const int items = D.solve_tile_prefix[KIND][D.nsolves] / NS;
+  const int split = items < (int)gridDim.x ? TI : 1;
+  const int li = TI / split;
+  for (int q = blockIdx.x; q < items * split; q += gridDim.x) {
+    const int part = q % split;
+    if (threadIdx.x == 0) lookup_item<KIND>(D, q / split * NS, sh[0], sh[1], sh[2]);
+    __syncthreads();
+    const int is = sh[0], ib = sh[1], t = sh[2];
+    __syncthreads();
+    if (!solve_active(D, is)) continue;  // inactive solve (the whole CTA agrees)
+    Item it;
+    V<R> B;
+    build_item<R, KIND>(D, is, ib, t, it, B);
+    it.i += part;
+    const DevSolve &S = D.solves[is];
     const ConstsT<R> &c = consts_of<R>(S);
     const R dt = __longlong_as_double((long long)D.state[it.s].dt_bits);
     // the reference aborts; k_flip records the status (and a solve with a
     // non-finite cell is not advanced)
-    const bool dt_ok = (dt >= R(1e-7)) && isfinite(dt) && !D.state[it.s].nonfinite;
-    const int i = it.i, j = it.j, k = it.k, s = it.species;
-    const int u0 = s ? cUN : cUH, pv0 = s ? cPVN : cPVH;
-    const R g = c.gamma;
-    const int tid = threadIdx.x;
-    const int li = tid / (kTileK * kTileJ), lj = (tid / kTileK) % kTileJ, lk = tid % kTileK;
-    R r[5] = {R(0.0), R(0.0), R(0.0), R(0.0), R(0.0)};
-    // The cell values the source terms and the update read: cen(q) loads
-    // value q; in FP32 all of them are loaded before the flux passes into
-    // registers (their latency hides behind the passes), in FP64 at their use.
-    auto cen = [&](int q) -> R {
-      switch (q) {
-        case 0: case 1: case 2: return AT(cUP + q, i, j, k);
-        case 3: case 4: case 5: return AT(cBC + (q - 3), i, j, k);
-        case 6: case 7: case 8: return AT(cJC + (q - 6), i, j, k);
-        case 9: return AT(cUH, i, j, k);
-        case 10: return AT(cUN, i, j, k);
-        case 11: return AT(pv0 + 4, i, j, k);
-        case 12: case 13: case 14: case 15: case 16: return AT(u0 + (q - 12), i, j, k);
-        case 17: return AT(cPHOTO, i, j, k);
-        case 18: case 19: case 20: return AT(cCX + (q - 18), i, j, k);
-        default: return AT(pv0 + (q - 21), i, j, k);  // 21..23: u, v, w
-      }
-    };
-    constexpr int kCen = sizeof(R) == 4 ? 24 : 1;
-    R cvals[kCen];
-    if constexpr (sizeof(R) == 4) {
-      if (it.in && dt_ok) {
+    if (!(dt >= R(1e-7)) || !isfinite(dt) || D.state[it.s].nonfinite || !it.in || it.i >= it.hi[0]) continue;
+    const int j = it.j, k = it.k;
+    const int s0 = NS == 2 ? 0 : it.species;
+    {
+      const uint32_t di = (uint32_t)B.si * sizeof(R), dj = (uint32_t)B.sj * sizeof(R), dk = sizeof(R);
+      uint32_t o = (uint32_t)B.off(it.i, j, k) * sizeof(R);
+      FluidCell<R> C[NS], N[NS];
+      R Fm[NS][5];
+      {
+        const FluidFace<R> f = fluid_face<R, 0>(B, o);
 #pragma unroll
-        for (int q = 0; q < 24; ++q) cvals[q] = cen(q);
+        for (int q = 0; q < NS; ++q) {
+          const int s = s0 + q, u0 = s ? cUN : cUH, pv0 = s ? cPVN : cPVH;
+          const FluidCell<R> L = fluid_cell(B, s, o - di);
+          C[q] = fluid_cell(B, s, o);
+          rusanov(L, C[q], f, Fm[q]);
+        }
       }
-    }
-    auto CV = [&](int q) -> R {
-      if constexpr (sizeof(R) == 4) return cvals[q];
-      else return cen(q);
-    };
-    // 1/J of this cell (the same value every direction divides by)
-    R invJ = R(0.0);
-    if (it.in && dt_ok) {
-      if constexpr (sizeof(R) == 4) invJ = AT(cFM + 9, i, j, k);  // R(1) / R(Jac), from k_face_normals
-      else invJ = R(1.0) / R(ATM(cJAC, i, j, k));
-    }
-    // Stage the cells the tile's faces read (the tile and one layer beyond
-    // each of its six sides, inside the owned range widened by one): rho,
-    // u, v, w, p and the per-cell terms re and c.
-    // the staged variant: the box of this item holds the cells; re and c of
-    // the cells the faces read go to RC (box indexing, k shifted by koff)
-    const int koff = kTma ? (it.o[2] + B.G - 1) & (16 / (int)sizeof(R) - 1) : 0;
 #pragma unroll 1
-    for (int q = tid; q < NP; q += kTileThreads) {
-      const int ck = q % PK, cj = (q / PK) % PJ, ci = q / (PK * PJ);
-      const int x0 = it.o[0] - 1 + ci, x1 = it.o[1] - 1 + cj, x2 = it.o[2] - 1 + ck;
-      const int out = (ci == 0 || ci == T.i + 1) + (cj == 0 || cj == T.j + 1) + (ck == 0 || ck == T.k + 1);
-      if (!dt_ok || out > 1 || x0 < it.lo[0] - 1 || x0 > it.hi[0] || x1 < it.lo[1] - 1 || x1 > it.hi[1] ||
-          x2 < it.lo[2] - 1 || x2 > it.hi[2])
-        continue;
-      if constexpr (kTma) {
-        const int e = (ci * kTmaBoxJI + cj) * W + ck + koff;
-        const R rho = box[e], u = box[BV + e], v = box[2 * BV + e], w = box[3 * BV + e], p = box[4 * BV + e];
-        RC[0][e] = p / (g - R(1.0)) + R(0.5) * rho * (u * u + v * v + w * w);
-        RC[1][e] = sqrt(dmax(R(0.0), g * p / dmax(rho, R(1e-30))));
-        continue;
-      }
-      const R rho = AT(u0, x0, x1, x2), u = AT(pv0, x0, x1, x2), v = AT(pv0 + 1, x0, x1, x2),
-              w = AT(pv0 + 2, x0, x1, x2), p = AT(pv0 + 3, x0, x1, x2);
-      C[0][q] = rho;
-      C[1][q] = u;
-      C[2][q] = v;
-      C[3][q] = w;
-      C[4][q] = p;
-      C[5][q] = p / (g - R(1.0)) + R(0.5) * rho * (u * u + v * v + w * w);
-      C[6][q] = sqrt(dmax(R(0.0), g * p / dmax(rho, R(1e-30))));
-    }
-    cta_sync();
-    // one face of direction dir (index f among that direction's faces, the
-    // slot gf of the tile's face array): the direction is a compile-time
-    // constant in each of the three instantiations, so the face grid's
-    // extents divide as constants
-    auto face = [&](auto dirc, int f, int gf) {
-      constexpr int dir = decltype(dirc)::value;
-      constexpr int ej = kTileJ + (dir == 1), ek = kTileK + (dir == 2);
-      // the face's JD: FP32 reads the real-typed copy (k_face_normals), FP64
-      // the metric itself (the same values; faster there)
-      constexpr int cm = sizeof(R) == 4 ? cFM + 3 * dir : dir == 0 ? cJDX : dir == 1 ? cJDY : cJDZ;
-      constexpr int cn = dir == 0 ? cFNX : dir == 1 ? cFNY : cFNZ;
-      const int fk = f % ek, fj = (f / ek) % ej, fi = f / (ek * ej);
-      const int x[3] = {it.o[0] + fi, it.o[1] + fj, it.o[2] + fk};
-      bool need = dt_ok;
+      for (int i = it.i; i < min(it.i + li, it.hi[0]); ++i, o += di) {
+        const R invJ = B.ld(cFM + 9, o);  // R(1) / R(Jac), from k_face_normals
+        R r[NS][5];
+        {
+          const FluidFace<R> f = fluid_face<R, 0>(B, o + di);
 #pragma unroll
-      for (int a = 0; a < 3; ++a) need = need && x[a] >= it.lo[a] && x[a] < it.hi[a] + (a == dir);
-      if (!need) return;
-      R k1, k2, k3;
-      if constexpr (sizeof(R) == 4) {
-        k1 = AT(cm, x[0], x[1], x[2]);
-        k2 = AT(cm + 1, x[0], x[1], x[2]);
-        k3 = AT(cm + 2, x[0], x[1], x[2]);
-      } else {
-        k1 = ATM(cm, x[0], x[1], x[2]);
-        k2 = ATM(cm + 1, x[0], x[1], x[2]);
-        k3 = ATM(cm + 2, x[0], x[1], x[2]);
-      }
-      // the face's right cell is (fi, fj, fk) of the tile, its left one step back along dir
-      R Lv[7], Rv[7];
-      if constexpr (kTma) {
-        const int er = ((fi + 1) * kTmaBoxJI + (fj + 1)) * W + (fk + 1) + koff;
-        const int el = er - (dir == 0 ? kTmaBoxJI * W : dir == 1 ? W : 1);
+          for (int q = 0; q < NS; ++q) {
+            const int s = s0 + q, u0 = s ? cUN : cUH, pv0 = s ? cPVN : cPVH;
+            N[q] = fluid_cell(B, s, o + di);
+            R F[5];
+            rusanov(C[q], N[q], f, F);
 #pragma unroll
-        for (int m = 0; m < 5; ++m) {
-          Lv[m] = box[m * BV + el];
-          Rv[m] = box[m * BV + er];
+            for (int m = 0; m < 5; ++m) {
+              r[q][m] = R(0.0) - (F[m] - Fm[q][m]) * invJ;
+              Fm[q][m] = F[m];
+            }
+          }
         }
+        auto across = [&](auto dirc, uint32_t d) {  // the faces below and above along j or k
+          constexpr int dir = decltype(dirc)::value;
+          const FluidFace<R> fl = fluid_face<R, dir>(B, o), fh = fluid_face<R, dir>(B, o + d);
 #pragma unroll
-        for (int m = 0; m < 2; ++m) {
-          Lv[5 + m] = RC[m][el];
-          Rv[5 + m] = RC[m][er];
+          for (int q = 0; q < NS; ++q) {
+            const int s = s0 + q, u0 = s ? cUN : cUH, pv0 = s ? cPVN : cPVH;
+            R Fl[5], Fh[5];
+            rusanov(fluid_cell(B, s, o - d), C[q], fl, Fl);
+            rusanov(C[q], fluid_cell(B, s, o + d), fh, Fh);
+#pragma unroll
+            for (int m = 0; m < 5; ++m) r[q][m] -= (Fh[m] - Fl[m]) * invJ;
+          }
+        };
+        across(std::integral_constant<int, 1>{}, dj);
+        across(std::integral_constant<int, 2>{}, dk);
+        // sources (FluidRHS.cpp:206-527)
+        auto at = [&](int comp) -> R { return B.ld(comp, o); };
+        const R Tn0 = R(1000.0), sk1 = R(5.0e-5), sk2 = R(1.0e-5);
+        const R a4 = c.src_a4, a5 = c.src_a5;
+        const R upx = at(cUP), upy = at(cUP + 1), upz = at(cUP + 2);
+        const R Bx = at(cBC), By = at(cBC + 1), Bz = at(cBC + 2);
+        const R Jx = at(cJC), Jy = at(cJC + 1), Jz = at(cJC + 2);
+        const R sjbx = Jy * Bz - Jz * By, sjby = Jz * Bx - Jx * Bz, sjbz = Jx * By - Jy * Bx;
+        const Num<R> num = num_limiter(c, at(cUH), at(cUN));
+        R dpex = R(0.0), dpey = R(0.0), dpez = R(0.0);
+        if (c.ambipolar) {  // grad p_e term, once per cell (k_face_emf)
+          dpex = at(cDPE);
+          dpey = at(cDPE + 1);
+          dpez = at(cDPE + 2);
         }
-      } else {
-        const int qr = ((fi + 1) * PJ + (fj + 1)) * PK + (fk + 1);
-        const int ql = qr - (dir == 0 ? PJ * PK : dir == 1 ? PK : 1);
+        const R x = at(cCX), y = at(cCX + 1), z = at(cCX + 2);
+        const R rho_cyl = sqrt(y * y + z * z);
+        const R vst = (x < R(0.0) && rho_cyl < R(1.0)) ? sk2 : sk1;
 #pragma unroll
-        for (int m = 0; m < 7; ++m) {
-          Lv[m] = C[m][ql];
-          Rv[m] = C[m][qr];
+        for (int q = 0; q < NS; ++q) {
+          const int s = s0 + q, u0 = s ? cUN : cUH, pv0 = s ? cPVN : cPVH;
+          const R nS = s ? num.nNa : num.nH;
+          const R chi = s ? num.wNa : num.wH;
+          const R rho = dmax(C[q].rho, R(0.0));
+          const R u = C[q].u, v = C[q].v, w = C[q].w;
+          const R u2 = u * u + v * v + w * w;
+          const R subx = (v - upy) * Bz - (w - upz) * By;
+          const R suby = (w - upz) * Bx - (u - upx) * Bz;
+          const R subz = (u - upx) * By - (v - upy) * Bx;
+          const R subu = subx * u + suby * v + subz * w;
+          const R sjbu = sjbx * u + sjby * v + sjbz * w;
+          const R dpeu = dpex * u + dpey * v + dpez * w;
+          const R Ts0 = at(pv0 + 4) * c.T_ref;
+          const R b1 = vst * (Tn0 - Ts0) * c.src_b1[s], b2 = c.src_b2[s] * vst;
+          R *rr = r[q];
+          rr[1] += c.momentum_induce_coeff * nS * subx + c.momentum_hall_coeff * chi * sjbx;
+          rr[2] += c.momentum_induce_coeff * nS * suby + c.momentum_hall_coeff * chi * sjby;
+          rr[3] += c.momentum_induce_coeff * nS * subz + c.momentum_hall_coeff * chi * sjbz;
+          rr[4] += c.momentum_induce_coeff * nS * subu + c.momentum_hall_coeff * chi * sjbu;
+          if (c.ambipolar) {
+            rr[1] -= chi * dpex;
+            rr[2] -= chi * dpey;
+            rr[3] -= chi * dpez;
+            rr[4] -= chi * dpeu;
+          }
+          if (s) {
+            const R sss = at(cPHOTO);
+            rr[0] += c.src_a1Na * sss;
+            rr[4] += c.src_a6 * sss * Tn0;
+          }
+          rr[1] -= a4 * rho * u * vst;
+          rr[2] -= a4 * rho * v * vst;
+          rr[3] -= a4 * rho * w * vst;
+          rr[4] -= a4 * rho * u2 * vst;
+          rr[4] += a5 * nS * b1;
+          rr[4] += a4 * rho * u2 * b2;
+          auto put = [&](int m, R v) { *(R *)((char *)B.next(u0 + m) + o) = v; };
+          put(0, C[q].rho + dt * rr[0]);
+#pragma unroll
+          for (int m = 1; m < 5; ++m) put(m, at(u0 + m) + dt * rr[m]);
+          C[q] = N[q];
         }
       }
-      R Fl[5];
-      rusanov_staged(Lv, Rv, k1, k2, k3, AT(cn + 3, x[0], x[1], x[2]), Fl);
-#pragma unroll
-      for (int m = 0; m < 5; ++m) F[m][gf] = Fl[m];
-    };
-    // The tile's face fluxes of all three directions in one pass, dealt
-    // round-robin over the threads (912 faces of a 16 x 4 x 4 tile take four
-    // rounds of 256; a warp straddles a direction change at most twice), then
-    // every cell takes its six faces' differences direction by direction, in
-    // Scheme_U_'s order.
-#pragma unroll 1
-    for (int gf = tid; gf < kTileFaces; gf += kTileThreads) {
-      if (gf < kNF0) face(std::integral_constant<int, 0>{}, gf, gf);
-      else if (gf < kNF0 + kNF1) face(std::integral_constant<int, 1>{}, gf - kNF0, gf);
-      else face(std::integral_constant<int, 2>{}, gf - kNF0 - kNF1, gf);
     }
-    cta_sync();
-    if constexpr (kTma) mbar_arrive(&bars[2 + (box == stage ? 0 : 1)]);  // this stage's box is no longer read
-    if (it.in && dt_ok) {
-      auto take = [&](auto dirc) {
-        constexpr int dir = decltype(dirc)::value;
-        constexpr int base = dir == 0 ? 0 : dir == 1 ? kNF0 : kNF0 + kNF1;
-        constexpr int ej = kTileJ + (dir == 1), ek = kTileK + (dir == 2);
-        const int fm = base + (li * ej + lj) * ek + lk;
-        const int fp = fm + (dir == 0 ? ej * ek : dir == 1 ? ek : 1);
-#pragma unroll
-        for (int m = 0; m < 5; ++m) r[m] -= (F[m][fp] - F[m][fm]) * invJ;
-      };
-      take(std::integral_constant<int, 0>{});
-      take(std::integral_constant<int, 1>{});
-      take(std::integral_constant<int, 2>{});
-    }
-    cta_sync();  // F is rewritten by the next tile
-    if (!it.in || !dt_ok) return;
-    // sources (FluidRHS.cpp:206-527)
-    const R Tn0 = R(1000.0), sk1 = R(5.0e-5), sk2 = R(1.0e-5);
-    const R a4 = (c.L_ref / c.U_ref);
-    const R a5 = (R(3.0) * c.L_ref * c.k_Boltz * c.n_ref) / (c.rho_ref * c.U_ref * c.U_ref * c.U_ref);
-    const R upx = CV(0), upy = CV(1), upz = CV(2);
-    const R Bx = CV(3), By = CV(4), Bz = CV(5);
-    const R Jx = CV(6), Jy = CV(7), Jz = CV(8);
-    const R sjbx = Jy * Bz - Jz * By, sjby = Jz * Bx - Jx * Bz, sjbz = Jx * By - Jy * Bx;
-    const Num<R> num = num_limiter(c, CV(9), CV(10));
-    R dpex = R(0.0), dpey = R(0.0), dpez = R(0.0);
-    if (c.ambipolar) {  // grad p_e term, once per cell (k_face_emf)
-      dpex = AT(cDPE, i, j, k);
-      dpey = AT(cDPE + 1, i, j, k);
-      dpez = AT(cDPE + 2, i, j, k);
-    }
-    const R x = CV(18), y = CV(19), z = CV(20);
-    const R rho_cyl = sqrt(y * y + z * z);
-    const R vst = (x < R(0.0) && rho_cyl < R(1.0)) ? sk2 : sk1;
-    const R nS = s ? num.nNa : num.nH;
-    const R chi = s ? num.wNa : num.wH;
-    const R rho = dmax(CV(12), R(0.0));
-    const R u = CV(21), v = CV(22), w = CV(23);
-    const R u2 = u * u + v * v + w * w;
-    const R subx = (v - upy) * Bz - (w - upz) * By;
-    const R suby = (w - upz) * Bx - (u - upx) * Bz;
-    const R subz = (u - upx) * By - (v - upy) * Bx;
-    const R subu = subx * u + suby * v + subz * w;
-    const R sjbu = sjbx * u + sjby * v + sjbz * w;
-    const R dpeu = dpex * u + dpey * v + dpez * w;
-    const R Ts0 = CV(11) * c.T_ref;
-    R b1, b2;
-    if (!s) {
-      b1 = vst * (Tn0 - Ts0) * (c.M_H / (c.M_H + c.M_Na));
-      b2 = (c.M_Na / (c.M_H + c.M_Na)) * vst;
-    } else {
-      b1 = vst * (Tn0 - Ts0) * (c.M_Na / (c.M_Na + c.M_Na));
-      b2 = (c.M_Na / (c.M_Na + c.M_Na)) * vst;
-    }
-    r[1] += c.momentum_induce_coeff * nS * subx + c.momentum_hall_coeff * chi * sjbx;
-    r[2] += c.momentum_induce_coeff * nS * suby + c.momentum_hall_coeff * chi * sjby;
-    r[3] += c.momentum_induce_coeff * nS * subz + c.momentum_hall_coeff * chi * sjbz;
-    r[4] += c.momentum_induce_coeff * nS * subu + c.momentum_hall_coeff * chi * sjbu;
-    if (c.ambipolar) {
-      r[1] -= chi * dpex;
-      r[2] -= chi * dpey;
-      r[3] -= chi * dpez;
-      r[4] -= chi * dpeu;
-    }
-    if (s) {
-      const R a1_Na = (c.L_ref / c.U_ref) * (c.m_Na / c.rho_ref) * R(1e6);
-      const R a6 = (R(1.0e6) * c.L_ref * c.k_Boltz) / (c.rho_ref * c.U_ref * c.U_ref * c.U_ref * (c.gamma - R(1.0)));
-      const R sss = CV(17);
-      r[0] += a1_Na * sss;
-      r[4] += a6 * sss * Tn0;
-    }
-    r[1] -= a4 * rho * u * vst;
-    r[2] -= a4 * rho * v * vst;
-    r[3] -= a4 * rho * w * vst;
-    r[4] -= a4 * rho * u2 * vst;
-    r[4] += a5 * nS * b1;
-    r[4] += a4 * rho * u2 * b2;
-    const int o = B.off(i, j, k);
-#pragma unroll
-    for (int m = 0; m < 5; ++m) B.Un[(u0 + m) * B.total + o] = CV(12 + m) + dt * r[m];
-  };
-  if constexpr (kTma) {
-    for_fluid_items_tma<R, fluid_kind(VT)>(D, stage, bars, body);
-  } else {
-    for_items<R, fluid_kind(VT)>(D, [&](const DevSolve &S, const V<R> &B, const Item &it) { body(S, B, it, nullptr); });
   }
 }
 
@@ -1795,6 +1567,9 @@ __global__ void __launch_bounds__(kTileThreads, MHD_MIN_CTAS_PV) k_pv_uplus(Dir 
         pr = dmax(pr, R(1e-12));
         const R T = pr / (rho * coeff);
         const int o = B.off(i, j, k);
+        // the Rusanov flux's terms of the cell (fluid_cell)
+        B.c(cFT + 2 * s)[o] = pr / (c.gamma - R(1.0)) + R(0.5) * r0 * (u * u + v * v + w * w);
+        B.c(cFT + 2 * s + 1)[o] = sqrt(dmax(R(0.0), c.gamma * pr / dmax(r0, R(1e-30))));
         B.c(pv0)[o] = u;
         B.c(pv0 + 1)[o] = v;
         B.c(pv0 + 2)[o] = w;
@@ -1946,16 +1721,7 @@ __device__ __forceinline__ V<R> block_view(const Dir &D, int s, int b) {
   const DevBlock &DB = D.solves[s].blocks[b];
   V<R> B;
   const int cur = D.state[s].cur;
-  B.U = (R *)DB.U[cur];
-  B.Un = (R *)DB.U[cur ^ 1];
-  B.M = DB.M;
-  B.total = (int)DB.total;
-  B.si = (int)DB.si;
-  B.sj = (int)DB.sj;
-  B.G = DB.G;
-  B.n0 = DB.n[0];
-  B.n1 = DB.n[1];
-  B.n2 = DB.n[2];
+  set_view(B, DB, cur);
   return B;
 }
 
@@ -2295,31 +2061,12 @@ static const void *fluid_fn(int v) {
     default: return (const void *)k_fluid<R, 0>;
   }
 }
-static_assert(kNumFluidTiles == 7, "fluid_fn and launch_fluid list every variant");
-template <class R>
-static size_t fluid_smem(int v) {
-  switch (v) {
-    case 1: return FluidSmem<R, 1>::bytes;
-    case 2: return FluidSmem<R, 2>::bytes;
-    case 3: return FluidSmem<R, 3>::bytes;
-    case 4: return FluidSmem<R, 4>::bytes;
-    case 5: return FluidSmem<R, 5>::bytes;
-    case 6: return FluidSmem<R, 6>::bytes;
-    default: return FluidSmem<R, 0>::bytes;
-  }
-}
+static_assert(kNumFluidTiles == 7, "fluid_fn lists every variant");
 template <class R>
 static void launch_fluid(int v, const Dir &D, cudaStream_t st) {
-  const int G = g_grid_fluid[(v >= 0 && v < kNumFluidTiles) ? v : 0];
-  switch (v) {
-    case 1: k_fluid<R, 1><<<G, kTileThreads, FluidSmem<R, 1>::bytes, st>>>(D); break;
-    case 2: k_fluid<R, 2><<<G, kTileThreads, FluidSmem<R, 2>::bytes, st>>>(D); break;
-    case 3: k_fluid<R, 3><<<G, kTileThreads, FluidSmem<R, 3>::bytes, st>>>(D); break;
-    case 4: k_fluid<R, 4><<<G, kTileThreads, FluidSmem<R, 4>::bytes, st>>>(D); break;
-    case 5: k_fluid<R, 5><<<G, kTileThreads, FluidSmem<R, 5>::bytes, st>>>(D); break;
-    case 6: k_fluid<R, 6><<<G, fluid_threads(6), FluidSmem<R, 6>::bytes, st>>>(D); break;
-    default: k_fluid<R, 0><<<G, kTileThreads, FluidSmem<R, 0>::bytes, st>>>(D); break;
-  }
+  v = (v >= 0 && v < kNumFluidTiles) ? v : 0;
+  void *args[] = {(void *)&D};
+  cudaLaunchKernel(fluid_fn<R>(v), dim3(g_grid_fluid[v]), dim3(fluid_threads(v)), args, 0, st);
 }
 
 template <class R>
@@ -2372,17 +2119,13 @@ static void grids_init() {
     g_grid_kernel[k] = sms * (per_sm < 8 ? per_sm : 8);
   }
   for (int v = 0; v < kNumFluidTiles; ++v) {
-    int per_sm = 8;
-    // the staged cells and face fluxes are dynamic shared memory (above the
-    // 48 KB default in FP64)
-    cudaFuncSetAttribute(fluid_fn<R>(v), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fluid_smem<R>(v));
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fluid_fn<R>(v), fluid_threads(v), fluid_smem<R>(v)) !=
-            cudaSuccess ||
+    int per_sm = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fluid_fn<R>(v), fluid_threads(v), 0) != cudaSuccess ||
         per_sm < 1) {
       cudaGetLastError();
       per_sm = 1;
     }
-    g_grid_fluid[v] = sms * (per_sm < 8 ? per_sm : 8);
+    g_grid_fluid[v] = sms * per_sm;
   }
   g_grid_tiles = sms * 8;
 }
@@ -2466,15 +2209,7 @@ __global__ void __launch_bounds__(kTileThreads) k_res_cross(Dir D, int op) {
       S.companion_state->dt_bits = D.state[it.s].dt_bits;
     }
     V<double> C;
-    C.U = C.Un = nullptr;
-    C.M = CB.M;
-    C.total = (int)CB.total;
-    C.si = (int)CB.si;
-    C.sj = (int)CB.sj;
-    C.G = CB.G;
-    C.n0 = CB.n[0];
-    C.n1 = CB.n[1];
-    C.n2 = CB.n[2];
+    set_view(C, CB, 0);
     const int o = B.off(it.i, it.j, it.k), oc = C.off(it.i, it.j, it.k);
     for (int a = 0; a < 3; ++a) {
       switch (op) {

@@ -56,13 +56,20 @@ constexpr FieldSpec kFieldSpec[MHD_NUM_FIELDS] = {
 // Stagger: 1 where the location is node-like (n + 1 owned DOFs) along an axis.
 constexpr int kStagger[8][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {0, 1, 1}, {1, 0, 1}, {1, 1, 0}, {1, 1, 1}};
 
+// Components outside the public fields: per ion species and cell the terms of
+// the Rusanov flux that depend on the cell alone, p / (gamma - 1) + rho |u|^2 / 2
+// and sqrt(gamma p / rho), refreshed with the primitive variables (k_pv_uplus).
+constexpr int kNumInternal = 4;  // re and c of H+, re and c of Na+
+
 // First component index of each field in the component numbering
-// (U_H, U_Na occupy 0..9; everything else follows).
+// (U_H, U_Na occupy 0..9; everything else follows, the internal components
+// ahead of the implicit substep's work arrays).
 struct CompTable {
   int first[MHD_NUM_FIELDS + 1];
   constexpr CompTable() : first() {
     int c = 0;
     for (int f = 0; f < MHD_NUM_FIELDS; ++f) {
+      if (f == MHD_RES_W) c += kNumInternal;
       first[f] = c;
       c += kFieldSpec[f].ncomp;
     }
@@ -70,6 +77,7 @@ struct CompTable {
   }
 };
 constexpr CompTable kComp{};
+constexpr int kFirstInternal = kComp.first[MHD_RES_W] - kNumInternal;
 constexpr int kNumComps = kComp.first[MHD_NUM_FIELDS];
 
 // One block's box geometry.
