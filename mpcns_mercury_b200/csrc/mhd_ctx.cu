@@ -1991,7 +1991,7 @@ static int add_solve(mhd_batch *b, const mhd_desc *desc, bool periodic, int *slo
     m += ((int64_t)kNumMetric * 8 + (int64_t)(kNumRComps - (desc->constants.resistive ? 0 : kNumResComps)) * S->es) *
          bx.total;
     for (int r = 0; r < kNumRanges; ++r)
-      prefix[r].push_back(prefix[r].back() + tiles_of(range_of(r, n, desc->nghost), r));
+      prefix[r].push_back(prefix[r].back() + tiles_of(range_of(r, n, desc->nghost), r, desc->nghost + 1, S->es));
   }
   S->ubuf = u;
   S->main_off = 2 * u;
@@ -2379,7 +2379,7 @@ static int apply_res_range(mhd_batch *b, Solve *S, const std::vector<int> &hi) {
     CUDA_TRY(cudaMemcpyAsync(&S->dblocks[bi].reskhi, &hi[bi], sizeof(int), cudaMemcpyHostToDevice, st));
     RangeBox r = range_of(kResK, S->boxes[bi].n, S->nghost);
     r.hi[2] = hi[bi];
-    prefix.push_back(prefix.back() + tiles_of(r, kResK));
+    prefix.push_back(prefix.back() + tiles_of(r, kResK, S->nghost + 1, S->es));
   }
   if (!whole) {
     int rc = dev_upload(S->pool, prefix, &S->dres_prefix, st);

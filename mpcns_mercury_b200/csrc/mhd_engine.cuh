@@ -3,8 +3,8 @@
 //
 // Every step kernel is a persistent, grid-stride loop over work items of one
 // "range kind" (cells, faces+edges, the extended face range of the ideal EMF,
-// the allocated cell range).  A work item is a 32 (k) x 4 (j) x 2 (i) tile of
-// one block of one solve; the directory maps the global item index to
+// the allocated cell range).  A work item is a tile of one block of one
+// solve; the directory maps the global item index to
 // (solve, block, tile) through per-range prefix sums.  Grid sizes depend only
 // on the SM count, so one CUDA graph captured once runs any set of solves:
 // membership changes only rewrite the directory in device memory.
@@ -42,6 +42,7 @@ __host__ __device__ constexpr int fluid_ctas(int v, int es) {
   return es == 8 ? 6 + n : v == 6 ? 8 : 3 + n;
 }
 constexpr int kTileThreads = 256;
+constexpr int kVecThreads = 128;  // threads of a tile of the vector ranges
 constexpr bool fluid_tiles_ok() {
   for (int v = 0; v < kNumFluidTiles; ++v)
     if (fluid_tile(v).k * fluid_tile(v).j * fluid_tile(v).i != kTileThreads) return false;
@@ -124,6 +125,8 @@ struct ConstsT {
   T src_a4, src_a5, src_a1Na, src_a6;
   T src_b1[2], src_b2[2];  // M / (M + M_Na) and M_Na / (M + M_Na) of H+, Na+
   T pe_coeff;
+  // reciprocals that the FP32 path multiplies by
+  T n_of_rho[2], inv_coeff[2], inv_g1;  // M_ref / M, 1 / state_coeff of H+, Na+; 1 / (gamma - 1)
 };
 using Consts = ConstsT<double>;
 inline void combine(Consts &c) {
@@ -136,6 +139,11 @@ inline void combine(Consts &c) {
   c.src_b2[0] = c.M_Na / (c.M_H + c.M_Na);
   c.src_b2[1] = c.M_Na / (c.M_Na + c.M_Na);
   c.pe_coeff = (c.rho_ref * c.U_ref) / (c.q_e * c.L_ref * c.B_ref * c.n_ref);
+  c.n_of_rho[0] = c.M_ref / c.M_H;
+  c.n_of_rho[1] = c.M_ref / c.M_Na;
+  c.inv_coeff[0] = 1.0 / c.state_coeff_H;
+  c.inv_coeff[1] = 1.0 / c.state_coeff_Na;
+  c.inv_g1 = 1.0 / (c.gamma - 1.0);
 }
 inline ConstsT<float> to_float(const Consts &c) {
   ConstsT<float> f{(float)c.gamma, (float)c.M_H, (float)c.M_Na, (float)c.M_ref, (float)c.T_ref,
@@ -153,7 +161,10 @@ inline ConstsT<float> to_float(const Consts &c) {
   for (int q = 0; q < 2; ++q) {
     f.src_b1[q] = (float)c.src_b1[q];
     f.src_b2[q] = (float)c.src_b2[q];
+    f.n_of_rho[q] = (float)c.n_of_rho[q];
+    f.inv_coeff[q] = (float)c.inv_coeff[q];
   }
+  f.inv_g1 = (float)c.inv_g1;
   f.pe_coeff = (float)c.pe_coeff;
   return f;
 }
@@ -317,11 +328,26 @@ __host__ __device__ inline RangeBox range_of(int kind, const int n[3], int g) {
   }
   return r;
 }
+// The vector ranges: their passes take 16-byte groups of consecutive k
+// positions (mhd_kernels.cu, Vec).
+__host__ __device__ constexpr bool vector_kind(int kind) {
+  return kind == kCells || kind == kBox || kind == kExt || kind == kAlloc;
+}
+// The aligned 16-byte groups of a row that hold positions of the range.
+struct RowGroups {
+  int first, count;
+};
+__host__ __device__ inline RowGroups row_groups(const RangeBox &r, int G, int es) {
+  const int n = 16 / es, first = (r.lo[2] + G) / n;
+  return RowGroups{first, (r.hi[2] - 1 + G) / n - first + 1};
+}
 // Work items of a block: the fluid kinds use 3-D tiles of their variant's
-// shape (two work items per tile, one per ion species); every other range is
-// cut into runs of kTileThreads consecutive positions of its box (k fastest),
-// so no lane idles at the end of short k rows.
-__host__ __device__ inline int tiles_of(const RangeBox &r, int kind) {
+// shape (two work items per tile, one per ion species); the vector ranges are
+// cut into runs of kVecThreads groups (row after row), the others into runs
+// of kTileThreads consecutive positions of their box (k fastest), so no lane
+// idles at the end of short k rows.  G: the block's ghost width, es: bytes
+// per real.
+__host__ __device__ inline int tiles_of(const RangeBox &r, int kind, int G, int es) {
   const int v = fluid_variant(kind);
   if (v >= 0) {
     const FluidTile T = fluid_tile(v);
@@ -329,6 +355,10 @@ __host__ __device__ inline int tiles_of(const RangeBox &r, int kind) {
     const int tj = (r.hi[1] - r.lo[1] + T.j - 1) / T.j;
     const int ti = (r.hi[0] - r.lo[0] + T.i - 1) / T.i;
     return tk * tj * ti * 2;
+  }
+  if (vector_kind(kind)) {
+    const int64_t groups = (int64_t)(r.hi[0] - r.lo[0]) * (r.hi[1] - r.lo[1]) * row_groups(r, G, es).count;
+    return (int)((groups + kVecThreads - 1) / kVecThreads);
   }
   const int64_t vol = (int64_t)(r.hi[0] - r.lo[0]) * (r.hi[1] - r.lo[1]) * (r.hi[2] - r.lo[2]);
   return (int)((vol + kTileThreads - 1) / kTileThreads);

@@ -59,7 +59,7 @@ constexpr int cWB = kComp.first[MHD_BCELL_W], cWJ = kComp.first[MHD_JCELL_W];
 static_assert(cBFY == cBFX + 1 && cBFZ == cBFX + 2 && cALY == cALX + 1 && cALZ == cALX + 2, "xi, eta, zeta consecutive");
 constexpr int cBAX = kComp.first[MHD_BADD_XI], cBAY = kComp.first[MHD_BADD_ETA], cBAZ = kComp.first[MHD_BADD_ZETA];
 constexpr int cPHOTO = kComp.first[MHD_PHOTO], cCX = kComp.first[MHD_CELL_X];  // CELL_Y, CELL_Z follow
-constexpr int cTPX = kComp.first[MHD_TAPER_XI], cTPY = kComp.first[MHD_TAPER_ETA], cTPZ = kComp.first[MHD_TAPER_ZETA];
+constexpr int cTPX = kComp.first[MHD_TAPER_XI];  // TAPER_ETA, TAPER_ZETA follow
 constexpr int cTPC = kComp.first[MHD_TAPER_CELL];
 constexpr int cLEX = kComp.first[MHD_LOCAL_ETA_XI];  // LOCAL_ETA_ETA, LOCAL_ETA_ZETA follow
 
@@ -100,12 +100,6 @@ struct V {
 };
 #define AT(cc, i, j, k) (B.c(cc)[B.off((i), (j), (k))])
 #define ATM(cc, i, j, k) (B.m(cc)[B.off((i), (j), (k))])
-// Reads of an array the kernel does not write, through the read-only path:
-// the compiler may then move them ahead of the kernel's stores (it cannot
-// prove that plain loads and stores into one arena do not alias).  Used by
-// the primitive-variable pass, where it measured faster; elsewhere it did not.
-#define LD(cc, i, j, k) __ldg(B.c(cc) + B.off((i), (j), (k)))
-#define LDM(cc, i, j, k) __ldg(B.m(cc) + B.off((i), (j), (k)))
 
 struct Item {
   int s;       // solve
@@ -238,6 +232,215 @@ __device__ __forceinline__ void for_items(const Dir &D, F &&f, E &&end = E{}) {
   }
 }
 
+// ------------------------------------------------------------------ vector items
+// The step's stencil passes take 16 bytes of consecutive k positions (4 FP32 or
+// 2 FP64 values, aligned: block rows start on 64-byte boundaries) per thread and
+// array, element by element with the operations of the scalar form.
+template <class R>
+struct alignas(16) Vec {
+  static constexpr int N = 16 / (int)sizeof(R);
+  R v[N];
+};
+template <class R, class F>
+__device__ __forceinline__ Vec<R> vmap(F &&f) {
+  Vec<R> r;
+#pragma unroll
+  for (int e = 0; e < Vec<R>::N; ++e) r.v[e] = f(e);
+  return r;
+}
+#define MHD_VEC_OP(op)                                                                                                \
+  template <class R>                                                                                                  \
+  __device__ __forceinline__ Vec<R> operator op(const Vec<R> &a, const Vec<R> &b) {                                  \
+    return vmap<R>([&](int e) { return a.v[e] op b.v[e]; });                                                          \
+  }                                                                                                                   \
+  template <class R>                                                                                                  \
+  __device__ __forceinline__ Vec<R> operator op(R a, const Vec<R> &b) {                                              \
+    return vmap<R>([&](int e) { return a op b.v[e]; });                                                               \
+  }                                                                                                                   \
+  template <class R>                                                                                                  \
+  __device__ __forceinline__ Vec<R> operator op(const Vec<R> &a, R b) {                                              \
+    return vmap<R>([&](int e) { return a.v[e] op b; });                                                               \
+  }
+MHD_VEC_OP(+)
+MHD_VEC_OP(-)
+MHD_VEC_OP(*)
+MHD_VEC_OP(/)
+#undef MHD_VEC_OP
+template <class R>
+__device__ __forceinline__ Vec<R> operator-(const Vec<R> &a) {
+  return vmap<R>([&](int e) { return -a.v[e]; });
+}
+template <class R>
+__device__ __forceinline__ Vec<R> vset(R x) {
+  return vmap<R>([&](int) { return x; });
+}
+template <class R>
+__device__ __forceinline__ Vec<R> vabs(const Vec<R> &a) {
+  return vmap<R>([&](int e) { return fabs(a.v[e]); });
+}
+template <class R>
+__device__ __forceinline__ Vec<R> vsqrt(const Vec<R> &a) {
+  return vmap<R>([&](int e) { return sqrt(a.v[e]); });
+}
+template <class R>
+__device__ __forceinline__ Vec<R> vmax(const Vec<R> &a, const Vec<R> &b) {
+  return vmap<R>([&](int e) { return dmax(a.v[e], b.v[e]); });
+}
+template <class R>
+__device__ __forceinline__ Vec<R> vmax(const Vec<R> &a, R b) {
+  return vmap<R>([&](int e) { return dmax(a.v[e], b); });
+}
+// The values one k lower (the lowest from `prev`), one k higher (the highest from `next`).
+template <class R>
+__device__ __forceinline__ Vec<R> vdown(const Vec<R> &a, R prev) {
+  return vmap<R>([&](int e) { return e == 0 ? prev : a.v[e > 0 ? e - 1 : 0]; });
+}
+template <class R>
+__device__ __forceinline__ Vec<R> vup(const Vec<R> &a, R next) {
+  constexpr int N = Vec<R>::N;
+  return vmap<R>([&](int e) { return e == N - 1 ? next : a.v[e < N - 1 ? e + 1 : e]; });
+}
+
+// One thread's part of a vector item: positions k .. k + N - 1 of row (i, j),
+// of which [klo, khi) are in the range.
+struct VItem {
+  int s, blk, i, j, k;
+  bool in;
+  uint32_t o;  // byte offset of position (i, j, k) in a real-valued component array
+  int klo, khi;
+  __device__ __forceinline__ bool has(int e) const { return k + e >= klo && k + e < khi; }
+};
+template <class R>
+struct VV : V<R> {
+  static constexpr int N = Vec<R>::N;
+  using V<R>::c;
+  using V<R>::m;
+  uint32_t di, dj;  // bytes to the neighbour along i and j (k: sizeof(R))
+  __device__ __forceinline__ Vec<R> lv(int comp, uint32_t o) const {
+    Vec<R> r;
+    const char *p = (const char *)c(comp) + o;
+    if constexpr (sizeof(R) == 4) *(float4 *)r.v = __ldg((const float4 *)p);
+    else *(double2 *)r.v = __ldg((const double2 *)p);
+    return r;
+  }
+  // the values one k lower / higher than lv(comp, o), of which v holds the shared ones
+  __device__ __forceinline__ Vec<R> lower(const Vec<R> &v, int comp, uint32_t o) const {
+    return vdown(v, this->ld(comp, o - (uint32_t)sizeof(R)));
+  }
+  __device__ __forceinline__ Vec<R> upper(const Vec<R> &v, int comp, uint32_t o) const {
+    return vup(v, this->ld(comp, o + 16u));
+  }
+  // values that the kernel itself updates (this thread's positions only)
+  __device__ __forceinline__ Vec<R> own(int comp, uint32_t o) const {
+    Vec<R> r;
+    const char *p = (const char *)c(comp) + o;
+    if constexpr (sizeof(R) == 4) *(float4 *)r.v = *(const float4 *)p;
+    else *(double2 *)r.v = *(const double2 *)p;
+    return r;
+  }
+  // metric values (double) at the item's positions
+  __device__ __forceinline__ Vec<R> lm(int comp, uint32_t o) const {
+    const char *p = (const char *)m(comp) + (uint64_t)o * (8 / sizeof(R));
+    Vec<R> r;
+    if constexpr (sizeof(R) == 4) {
+      const double2 a = __ldg((const double2 *)p), b = __ldg((const double2 *)p + 1);
+      r.v[0] = (R)a.x;
+      r.v[1] = (R)a.y;
+      r.v[2] = (R)b.x;
+      r.v[3] = (R)b.y;
+    } else {
+      *(double2 *)r.v = __ldg((const double2 *)p);
+    }
+    return r;
+  }
+  // writes the positions k + e in [lo, hi) where the item is in the range and `cond`
+  __device__ __forceinline__ void st(int comp, const VItem &it, const Vec<R> &v, int lo, int hi, bool cond = true) const {
+    char *p = (char *)c(comp) + it.o;
+    const bool w = it.in && cond, all = w && it.k >= lo && it.k + N <= hi;
+    if (all) {
+      if constexpr (sizeof(R) == 4) *(float4 *)p = *(const float4 *)v.v;
+      else *(double2 *)p = *(const double2 *)v.v;
+    }
+#pragma unroll
+    for (int e = 0; e < N; ++e)
+      if (w && !all && it.k + e >= lo && it.k + e < hi) ((R *)p)[e] = v.v[e];
+  }
+};
+
+template <class R, int KIND>
+__device__ __forceinline__ void build_vec_item(const Dir &D, int s, int b, int t, VItem &it, VV<R> &B) {
+  const DevSolve &S = D.solves[s];
+  const DevBlock &DB = S.blocks[b];
+  const RangeBox r = range_of(KIND, DB.n, S.c.nghost);
+  set_view(B, DB, D.state[s].cur);
+  B.U = uniform(B.U);
+  B.Un = uniform(B.Un);
+  B.M = uniform(B.M);
+  B.Mr = uniform(B.Mr);
+  B.tb = uniform((int)B.tb);
+  B.di = uniform((int)((uint32_t)B.si * (uint32_t)sizeof(R)));
+  B.dj = uniform((int)((uint32_t)B.sj * (uint32_t)sizeof(R)));
+  B.G = uniform(B.G);
+  B.n0 = uniform(B.n0);
+  B.n1 = uniform(B.n1);
+  B.n2 = uniform(B.n2);
+  const RowGroups g = row_groups(r, B.G, sizeof(R));
+  const int ej = r.hi[1] - r.lo[1];
+  const int L = t * kVecThreads + (int)threadIdx.x;
+  const int row = L / g.count, ri = row / ej;
+  it.s = s;
+  it.blk = b;
+  it.k = (g.first + (L - row * g.count)) * Vec<R>::N - B.G;
+  it.j = r.lo[1] + (row - ri * ej);
+  it.i = r.lo[0] + ri;
+  it.in = it.i < r.hi[0];
+  if (!it.in) {  // past the last row: work on the first one and write nothing (no divergence)
+    it.i = r.lo[0];
+    it.j = r.lo[1];
+    it.k = g.first * Vec<R>::N - B.G;
+  }
+  it.klo = r.lo[2];
+  it.khi = r.hi[2];
+  it.o = (uint32_t)B.off(it.i, it.j, it.k) * (uint32_t)sizeof(R);
+}
+
+// Work-item loop over the vector ranges: f(S, B, item) for every tile of
+// range KIND of every active solve.  Thread 0 looks the next tile up while the
+// CTA works on the current one (one barrier per tile).
+template <class R, int KIND, class F>
+__device__ __forceinline__ void for_vec_items(const Dir &D, F &&f) {
+  __shared__ int sh[2][3];
+  const int total = D.solve_tile_prefix[KIND][D.nsolves];
+  int w = blockIdx.x, p = 0;
+  if (threadIdx.x == 0 && w < total) lookup_item<KIND>(D, w, sh[0][0], sh[0][1], sh[0][2]);
+  __syncthreads();
+  for (; w < total; w += gridDim.x, p ^= 1) {
+    const int s = uniform(sh[p][0]), b = uniform(sh[p][1]), t = uniform(sh[p][2]);
+    if (threadIdx.x == 0 && w + (int)gridDim.x < total)
+      lookup_item<KIND>(D, w + gridDim.x, sh[p ^ 1][0], sh[p ^ 1][1], sh[p ^ 1][2]);
+    __syncwarp();
+    if (uniform((int)solve_active(D, s))) {
+      VItem it;
+      VV<R> B;
+      build_vec_item<R, KIND>(D, s, b, t, it, B);
+      f(D.solves[s], B, it);
+    }
+    __syncthreads();
+  }
+}
+// The same, position by position: f(S, B, pos) (passes that run once per solve).
+struct Pos {
+  int s, blk, i, j, k;
+};
+template <class R, int KIND, class F>
+__device__ __forceinline__ void for_positions(const Dir &D, F &&f) {
+  for_vec_items<R, KIND>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
+#pragma unroll 1
+    for (int e = 0; e < Vec<R>::N; ++e)
+      if (it.in && it.has(e)) f(S, B, Pos{it.s, it.blk, it.i, it.j, it.k + e});
+  });
+}
+
 template <class R>
 struct Num {
   R nH, nNa, ne_eff, chiH, chiNa, wH, wNa;
@@ -248,10 +451,24 @@ template <class R>
 __device__ __forceinline__ Num<R> num_limiter(const ConstsT<R> &c, R rhoH, R rhoNa) {
   Num<R> d;
   const R rH = dmax(rhoH, R(0.0)), rN = dmax(rhoNa, R(0.0));
-  d.nH = rH / c.M_H * c.M_ref;
-  d.nNa = rN / c.M_Na * c.M_ref;
+  if constexpr (sizeof(R) == 4) {  // one reciprocal per divisor
+    d.nH = rH * c.n_of_rho[0];
+    d.nNa = rN * c.n_of_rho[1];
+  } else {
+    d.nH = rH / c.M_H * c.M_ref;
+    d.nNa = rN / c.M_Na * c.M_ref;
+  }
   const R ne_true = d.nH + d.nNa;
   d.ne_eff = sqrt(ne_true * ne_true + c.ne_hall_floor * c.ne_hall_floor);
+  if constexpr (sizeof(R) == 4) {
+    const R it = R(1.0) / ne_true, ie = R(1.0) / d.ne_eff;
+    const bool some = ne_true > R(0.0);
+    d.chiH = some ? d.nH * it : R(1.0);
+    d.chiNa = some ? d.nNa * it : R(0.0);
+    d.wH = d.nH * ie;
+    d.wNa = d.nNa * ie;
+    return d;
+  }
   if ((double)ne_true > 1.0e-300) {
     d.chiH = d.nH / ne_true;
     d.chiNa = d.nNa / ne_true;
@@ -271,235 +488,211 @@ __device__ __forceinline__ void shift1(int axis, int &i, int &j, int &k, int s) 
 }
 
 // ------------------------------------------------------------------ ideal EMF
-__device__ __forceinline__ int bcomp(int axis) { return axis == 0 ? cBX : axis == 1 ? cBY : cBZ; }
-__device__ __forceinline__ int bacomp(int axis) { return axis == 0 ? cBAX : axis == 1 ? cBAY : cBAZ; }
-template <class R>
-__device__ __forceinline__ R face_tot(const V<R> &B, int axis, int i, int j, int k) {
-  return AT(bcomp(axis), i, j, k) + AT(bacomp(axis), i, j, k);
-}
-template <class R>
-__device__ __forceinline__ R cell_beta_ind(const V<R> &B, int axis, int i, int j, int k) {
-  int ip = i, jp = j, kp = k;
-  shift1(axis, ip, jp, kp, 1);
-  return R(0.5) * (AT(bcomp(axis), i, j, k) + AT(bcomp(axis), ip, jp, kp));
-}
-template <class R>
-__device__ __forceinline__ R cell_beta_tot(const V<R> &B, int axis, int i, int j, int k) {
-  int ip = i, jp = j, kp = k;
-  shift1(axis, ip, jp, kp, 1);
-  return R(0.5) * (face_tot(B, axis, i, j, k) + face_tot(B, axis, ip, jp, kp));
-}
-template <class R>
-__device__ __forceinline__ R ucon(const V<R> &B, int axis, int i, int j, int k) { return AT(cUC + axis, i, j, k); }
-
-// flux() of AssembleOneDirectionEMF_ (Ideal.cpp:517-536).  The right cell's
-// cell-averaged total and induced B (btR[ba], biR[ba]) and contravariant
-// velocities (uR[a]) are evaluated once per cell by the caller: every face
-// family of the cell shares that cell.
-template <class R>
-__device__ __forceinline__ R emf_flux(const V<R> &B, int ba, int fa, int iL, int jL, int kL, const R btR[3],
-                                      const R biR[3], const R uR[3], R bff) {
-  const R btL = cell_beta_tot(B, ba, iL, jL, kL);
-  const R biL = cell_beta_ind(B, ba, iL, jL, kL);
-  const R ufL = ucon(B, fa, iL, jL, kL), ufR = uR[fa];
-  const R ubL = ucon(B, ba, iL, jL, kL), ubR = uR[ba];
-  const R GL = ufL * btL - ubL * bff, GR = ufR * btR[ba] - ubR * bff;
-  const R r = dmax(fabs(ufL), fabs(ufR));
-  return R(0.5) * (GL + GR) - R(0.5) * r * (biR[ba] - biL);
-}
-
-// Electron pressure at node (i, j, k): the mean of p_H + p_Na over the 8
-// cells around it, summed in the order of AddAmbipolarEdgeEMF_
-// (Z4_Mercury/src/physics/MercurySolver_MagExplicit_Ambipo.cpp:3-143).
-template <class R>
-__device__ __forceinline__ R pe_node(const V<R> &B, int i, int j, int k) {
-  R sum = R(0.0);
-  for (int di = -1; di <= 0; ++di)
-    for (int dj = -1; dj <= 0; ++dj)
-      for (int dk = -1; dk <= 0; ++dk)
-        sum += AT(cPVH + 3, i + di, j + dj, k + dk) + AT(cPVN + 3, i + di, j + dj, k + dk);
-  return R(0.125) * sum;
-}
-
 // AssembleOneDirectionEMF_ (Ideal.cpp:433-594) for all three face families on
 // [-1, inner_hi + 1) (the one locally evaluated ghost layer, Ideal.cpp:548-555),
 // and, with the ambipolar term on, the node electron pressure on [0, n + 1)
 // that the edge EMFs of the owned edges read (each node is shared by six
 // edges) and the grad p_e source term of the owned cells that the fluid
-// update of both species reads.
+// update of both species reads.  A cell is the right cell of its three faces:
+// its cell-averaged total and induced B and its contravariant velocities are
+// evaluated once.
 template <class R>
-__global__ void __launch_bounds__(kTileThreads) k_face_emf(Dir D) {
-  for_items<R, kExt>(D, [&](const DevSolve &S, const V<R> &B, const Item &it) {
-    if (!it.in) return;
-    const int i = it.i, j = it.j, k = it.k;
-    const int q[3] = {i, j, k}, n[3] = {B.n0, B.n1, B.n2};
-    if (consts_of<R>(S).ambipolar && i >= 0 && j >= 0 && k >= 0 && i <= n[0] && j <= n[1] && k <= n[2]) {
-      AT(cPEN, i, j, k) = pe_node(B, i, j, k);
-      if (i < n[0] && j < n[1] && k < n[2]) {
+__global__ void __launch_bounds__(kVecThreads, sizeof(R) == 8 ? 2 : 3) k_face_emf(Dir D) {
+  for_vec_items<R, kExt>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
+    const int i = it.i, j = it.j;
+    const uint32_t o = it.o, di = B.di, dj = B.dj;
+    if (uniform(consts_of<R>(S).ambipolar)) {
+      auto pe = [&](uint32_t q) { return B.lv(cPVH + 3, q) + B.lv(cPVN + 3, q); };
+      auto pe1 = [&](uint32_t q) { return B.ld(cPVH + 3, q) + B.ld(cPVN + 3, q); };
+      constexpr uint32_t es = sizeof(R);
+      const Vec<R> p0 = pe(o), pim = pe(o - di), pjm = pe(o - dj), pijm = pe(o - di - dj);
+      const Vec<R> pkm = vdown(p0, pe1(o - es));
+      // the mean of p_H + p_Na over the 8 cells around the node, summed in the
+      // order of AddAmbipolarEdgeEMF_ (MercurySolver_MagExplicit_Ambipo.cpp:3-143)
+      Vec<R> sum = R(0.0) + vdown(pijm, pe1(o - di - dj - es));
+      sum = sum + pijm;
+      sum = sum + vdown(pim, pe1(o - di - es));
+      sum = sum + pim;
+      sum = sum + vdown(pjm, pe1(o - dj - es));
+      sum = sum + pjm;
+      sum = sum + pkm;
+      sum = sum + p0;
+      B.st(cPEN, it, R(0.125) * sum, 0, B.n2 + 1, i >= 0 && j >= 0 && i <= B.n0 && j <= B.n1);
+      {
         // grad p_e term of the ion momentum sources of an owned cell, the
         // same for both species (AddSourceToRHS_Fluid, FluidRHS.cpp:206-527)
-        const R pip = AT(cPVH + 3, i + 1, j, k) + AT(cPVN + 3, i + 1, j, k);
-        const R pim = AT(cPVH + 3, i - 1, j, k) + AT(cPVN + 3, i - 1, j, k);
-        const R pjp = AT(cPVH + 3, i, j + 1, k) + AT(cPVN + 3, i, j + 1, k);
-        const R pjm = AT(cPVH + 3, i, j - 1, k) + AT(cPVN + 3, i, j - 1, k);
-        const R pkp = AT(cPVH + 3, i, j, k + 1) + AT(cPVN + 3, i, j, k + 1);
-        const R pkm = AT(cPVH + 3, i, j, k - 1) + AT(cPVN + 3, i, j, k - 1);
-        const R ax = AT(cAMB, i, j, k), ay = AT(cAMB + 1, i, j, k), az = AT(cAMB + 2, i, j, k);
-        const R bx = AT(cAMB + 3, i, j, k), by = AT(cAMB + 4, i, j, k), bz = AT(cAMB + 5, i, j, k);
-        const R cxm = AT(cAMB + 6, i, j, k), cym = AT(cAMB + 7, i, j, k), czm = AT(cAMB + 8, i, j, k);
-        AT(cDPE, i, j, k) = R(0.5) * (ax * (pip - pim) + bx * (pjp - pjm) + cxm * (pkp - pkm));
-        AT(cDPE + 1, i, j, k) = R(0.5) * (ay * (pip - pim) + by * (pjp - pjm) + cym * (pkp - pkm));
-        AT(cDPE + 2, i, j, k) = R(0.5) * (az * (pip - pim) + bz * (pjp - pjm) + czm * (pkp - pkm));
-      }
-    }
-    // this cell is the right cell of its three faces
-    R btR[3], biR[3], uR[3];
+        const Vec<R> gi = pe(o + di) - pim, gj = pe(o + dj) - pjm, gk = vup(p0, pe1(o + 16u)) - pkm;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      btR[a] = cell_beta_tot(B, a, i, j, k);
-      biR[a] = cell_beta_ind(B, a, i, j, k);
-      uR[a] = ucon(B, a, i, j, k);
-    }
-#pragma unroll 1
-    for (int fa = 0; fa < 3; ++fa) {
-      bool in = true;
-      for (int a = 0; a < 3; ++a) in = in && q[a] < n[a] + (a == fa ? 1 : 0) + 1;
-      if (!in) continue;
-      int iL = i, jL = j, kL = k;
-      shift1(fa, iL, jL, kL, -1);
-      const R bff = face_tot(B, fa, i, j, k);
-      R e0 = R(0.0), e1 = R(0.0), e2 = R(0.0);
-      if (fa == 0) {
-        const R Ge = emf_flux(B, 1, 0, iL, jL, kL, btR, biR, uR, bff);
-        const R Gz = emf_flux(B, 2, 0, iL, jL, kL, btR, biR, uR, bff);
-        e1 = Gz;
-        e2 = -Ge;
-      } else if (fa == 1) {
-        const R Gx = emf_flux(B, 0, 1, iL, jL, kL, btR, biR, uR, bff);
-        const R Gz = emf_flux(B, 2, 1, iL, jL, kL, btR, biR, uR, bff);
-        e0 = -Gz;
-        e2 = Gx;
-      } else {
-        const R Gx = emf_flux(B, 0, 2, iL, jL, kL, btR, biR, uR, bff);
-        const R Ge = emf_flux(B, 1, 2, iL, jL, kL, btR, biR, uR, bff);
-        e0 = Ge;
-        e1 = -Gx;
+        for (int q = 0; q < 3; ++q)
+          B.st(cDPE + q, it, R(0.5) * (B.lv(cAMB + q, o) * gi + B.lv(cAMB + 3 + q, o) * gj + B.lv(cAMB + 6 + q, o) * gk), 0,
+               B.n2, i >= 0 && j >= 0 && i < B.n0 && j < B.n1);
       }
-      const int ce = fa == 0 ? cEFX : fa == 1 ? cEFY : cEFZ;
-      const int o = B.off(i, j, k);
-      B.c(ce)[o] = e0;
-      B.c(ce + 1)[o] = e1;
-      B.c(ce + 2)[o] = e2;
+    }
+    // induced and total B averaged to the cells (cell_beta_ind, cell_beta_tot)
+    auto ind = [&](int a, uint32_t q, uint32_t d) { return R(0.5) * (B.lv(cBX + a, q) + B.lv(cBX + a, q + d)); };
+    auto tot = [&](int a, uint32_t q, uint32_t d) {
+      return R(0.5) * ((B.lv(cBX + a, q) + B.lv(cBAX + a, q)) + (B.lv(cBX + a, q + d) + B.lv(cBAX + a, q + d)));
+    };
+    auto ind_k = [&](uint32_t q) {  // along k: the cell's upper face is the next position
+      const Vec<R> b = B.lv(cBZ, q);
+      return R(0.5) * (b + B.upper(b, cBZ, q));
+    };
+    auto tot_k = [&](uint32_t q) {
+      const Vec<R> b = B.lv(cBZ, q) + B.lv(cBAZ, q);
+      return R(0.5) * (b + vup(b, B.ld(cBZ, q + 16u) + B.ld(cBAZ, q + 16u)));
+    };
+    const Vec<R> bt[3] = {tot(0, o, di), tot(1, o, dj), tot_k(o)};
+    const Vec<R> bi[3] = {ind(0, o, di), ind(1, o, dj), ind_k(o)};
+    const Vec<R> u[3] = {B.lv(cUC, o), B.lv(cUC + 1, o), B.lv(cUC + 2, o)};
+    // flux() of AssembleOneDirectionEMF_ (Ideal.cpp:517-536) of component a of B
+    // through the face family f, from the left cell's values
+    auto flux = [&](int a, int f, const Vec<R> &btL, const Vec<R> &biL, const Vec<R> &ufL, const Vec<R> &ubL,
+                    const Vec<R> &bff) {
+      const Vec<R> GL = ufL * btL - ubL * bff, GR = u[f] * bt[a] - u[a] * bff;
+      const Vec<R> r = vmax(vabs(ufL), vabs(u[f]));
+      return R(0.5) * (GL + GR) - R(0.5) * r * (bi[a] - biL);
+    };
+    const bool ri = i < B.n0 + 1, rj = j < B.n1 + 1;  // in the range of the other families
+    const int k1 = B.n2 + 1;
+    {
+      const Vec<R> bff = B.lv(cBX, o) + B.lv(cBAX, o);
+      const uint32_t q = o - di;
+      const Vec<R> ufL = B.lv(cUC, q);
+      const Vec<R> Ge = flux(1, 0, tot(1, q, dj), ind(1, q, dj), ufL, B.lv(cUC + 1, q), bff);
+      const Vec<R> Gz = flux(2, 0, tot_k(q), ind_k(q), ufL, B.lv(cUC + 2, q), bff);
+      B.st(cEFX, it, vset(R(0.0)), -1, k1, rj);
+      B.st(cEFX + 1, it, Gz, -1, k1, rj);
+      B.st(cEFX + 2, it, -Ge, -1, k1, rj);
+    }
+    {
+      const Vec<R> bff = B.lv(cBY, o) + B.lv(cBAY, o);
+      const uint32_t q = o - dj;
+      const Vec<R> ufL = B.lv(cUC + 1, q);
+      const Vec<R> Gx = flux(0, 1, tot(0, q, di), ind(0, q, di), ufL, B.lv(cUC, q), bff);
+      const Vec<R> Gz = flux(2, 1, tot_k(q), ind_k(q), ufL, B.lv(cUC + 2, q), bff);
+      B.st(cEFY, it, -Gz, -1, k1, ri);
+      B.st(cEFY + 1, it, vset(R(0.0)), -1, k1, ri);
+      B.st(cEFY + 2, it, Gx, -1, k1, ri);
+    }
+    {
+      const Vec<R> bff = B.lv(cBZ, o) + B.lv(cBAZ, o);
+      const uint32_t q = o - (uint32_t)sizeof(R);  // the cell one k lower: its values from this thread's, and one more
+      auto totL = [&](int a, uint32_t d) {
+        return vdown(bt[a], R(0.5) * ((B.ld(cBX + a, q) + B.ld(cBAX + a, q)) + (B.ld(cBX + a, q + d) + B.ld(cBAX + a, q + d))));
+      };
+      auto indL = [&](int a, uint32_t d) { return vdown(bi[a], R(0.5) * (B.ld(cBX + a, q) + B.ld(cBX + a, q + d))); };
+      const Vec<R> ufL = vdown(u[2], B.ld(cUC + 2, q));
+      const Vec<R> Gx = flux(0, 2, totL(0, di), indL(0, di), ufL, vdown(u[0], B.ld(cUC, q)), bff);
+      const Vec<R> Ge = flux(1, 2, totL(1, dj), indL(1, dj), ufL, vdown(u[1], B.ld(cUC + 1, q)), bff);
+      B.st(cEFZ, it, Ge, -1, k1 + 1, ri && rj);
+      B.st(cEFZ + 1, it, -Gx, -1, k1 + 1, ri && rj);
+      B.st(cEFZ + 2, it, vset(R(0.0)), -1, k1 + 1, ri && rj);
     }
   });
 }
 
-template <class R>
-__device__ __forceinline__ R max_abs_u4(const V<R> &B, int axis, int i0, int j0, int k0, int i1, int j1, int k1,
-                                             int i2, int j2, int k2, int i3, int j3, int k3) {
-  R a = R(0.0);
-  a = dmax(a, fabs(ucon(B, axis, i0, j0, k0)));
-  a = dmax(a, fabs(ucon(B, axis, i1, j1, k1)));
-  a = dmax(a, fabs(ucon(B, axis, i2, j2, k2)));
-  a = dmax(a, fabs(ucon(B, axis, i3, j3, k3)));
-  return a;
-}
-
 // AddArtificialResistivityToEdgeEMF_ and AddLocalArtificialResistivityToEdgeEMF_
-// (Z4_Mercury/src/physics/MercurySolver_MagExplicit_Resis.cpp:6-64, 66-185) on one owned edge of
+// (Z4_Mercury/src/physics/MercurySolver_MagExplicit_Resis.cpp:6-64, 66-185) on owned edges of
 // family `axis`: E += eta_art(|J| / |dr|) J, then E += eta_local J.
 template <class R>
-__device__ __forceinline__ R add_artificial(const V<R> &B, const ConstsT<R> &c, int axis, int i, int j, int k, R e) {
-  const int cj = axis == 0 ? cJX : axis == 1 ? cJY : cJZ;
-  if (c.arti_eta_max > R(0.0)) {
+__device__ __forceinline__ Vec<R> add_artificial(const VV<R> &B, const ConstsT<R> &c, int axis, uint32_t o, Vec<R> e) {
+  const int cj = cJX + axis;
+  if (uniform((int)(c.arti_eta_max > R(0.0)))) {
     const int cd = axis == 0 ? cDRX : axis == 1 ? cDRY : cDRZ;
-    const R J1 = AT(cj, i, j, k);
-    const R dx = AT(cd, i, j, k), dy = AT(cd + 1, i, j, k), dz = AT(cd + 2, i, j, k);
-    const R dr_len = sqrt(dx * dx + dy * dy + dz * dz);
-    const R Jmag = fabs(J1) / dmax(dr_len, R(1.0e-30));
-    R eta;
-    if (c.arti_J_on <= c.arti_J_start) {
-      eta = (Jmag > c.arti_J_start) ? c.arti_eta_max : R(0.0);
-    } else {
-      R q = (Jmag - c.arti_J_start) / (c.arti_J_on - c.arti_J_start);
-      q = dmax(R(0.0), dmin(R(1.0), q));
-      const R S = q * q * (R(3.0) - R(2.0) * q);
-      eta = c.arti_eta_max * S;
+    const Vec<R> J = B.lv(cj, o), dx = B.lv(cd, o), dy = B.lv(cd + 1, o), dz = B.lv(cd + 2, o);
+#pragma unroll
+    for (int q = 0; q < Vec<R>::N; ++q) {
+      const R dr_len = sqrt(dx.v[q] * dx.v[q] + dy.v[q] * dy.v[q] + dz.v[q] * dz.v[q]);
+      const R Jmag = fabs(J.v[q]) / dmax(dr_len, R(1.0e-30));
+      R eta;
+      if (c.arti_J_on <= c.arti_J_start) {
+        eta = (Jmag > c.arti_J_start) ? c.arti_eta_max : R(0.0);
+      } else {
+        R x = (Jmag - c.arti_J_start) / (c.arti_J_on - c.arti_J_start);
+        x = dmax(R(0.0), dmin(R(1.0), x));
+        const R S = x * x * (R(3.0) - R(2.0) * x);
+        eta = c.arti_eta_max * S;
+      }
+      e.v[q] += eta * J.v[q];
     }
-    e += eta * J1;
   }
-  if (c.local_arti) e += AT(cLEX + axis, i, j, k) * AT(cj, i, j, k);
+  if (uniform(c.local_arti)) e = e + B.lv(cLEX + axis, o) * B.lv(cj, o);
   return e;
 }
 
 // AssembleEdgeEMF_FromFaceE_Ideal_ (Ideal.cpp:138-372) + AddAmbipolarEdgeEMF_
 // (Z4_Mercury/src/physics/MercurySolver_MagExplicit_Ambipo.cpp:3-143) on the owned edges.
 template <class R>
-__global__ void __launch_bounds__(kTileThreads) k_edge_emf(Dir D) {
-  for_items<R, kBox>(D, [&](const DevSolve &S, const V<R> &B, const Item &it) {
-    if (!it.in) return;
+__global__ void __launch_bounds__(kVecThreads, 4) k_edge_emf(Dir D) {
+  for_vec_items<R, kBox>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
     const ConstsT<R> &c = consts_of<R>(S);
-    const int i = it.i, j = it.j, k = it.k;
+    const uint32_t o = it.o, di = B.di, dj = B.dj;
     const R Cuct = R(0.5);
     const R pc = c.pe_coeff;
-    if (i < B.n0) {
-      const R Ec = R(0.25) * (AT(cEFY, i, j, k) + AT(cEFY, i, j, k - 1) + AT(cEFZ, i, j, k) + AT(cEFZ, i, j - 1, k));
-      const R ae = max_abs_u4(B, 1, i, j, k, i, j - 1, k, i, j, k - 1, i, j - 1, k - 1);
-      const R az = max_abs_u4(B, 2, i, j, k, i, j - 1, k, i, j, k - 1, i, j - 1, k - 1);
-      const R d1 = AT(cBZ, i, j, k) - AT(cBZ, i, j - 1, k);
-      const R d2 = AT(cBY, i, j, k) - AT(cBY, i, j, k - 1);
-      R e = Ec + Cuct * (R(0.5) * ae * d1 - R(0.5) * az * d2);
-      if (c.ambipolar) {
-        const R p0 = AT(cPEN, i, j, k), p1 = AT(cPEN, i + 1, j, k);
-        R rH = R(0.0), rN = R(0.0);
-        for (int dj = -1; dj <= 0; ++dj)
-          for (int dk = -1; dk <= 0; ++dk) {
-            rH += AT(cUH, i, j + dj, k + dk);
-            rN += AT(cUN, i, j + dj, k + dk);
-          }
-        e -= pc * (p1 - p0) / num_limiter(c, R(0.25) * rH, R(0.25) * rN).ne_eff;
-      }
-      AT(cEX, i, j, k) = add_artificial(B, c, 0, i, j, k, e);
+    auto lowk = [&](const Vec<R> &v, int comp, uint32_t q) { return B.lower(v, comp, q); };
+    // max |u^a| over the four cells at an edge: this row, the row below along
+    // d, and, for the edges that are not along k, both one k lower
+    auto umax_k = [&](int a, uint32_t d) {
+      const Vec<R> x = B.lv(cUC + a, o), y = B.lv(cUC + a, o - d);
+      Vec<R> r = vmax(vset(R(0.0)), vabs(x));
+      r = vmax(r, vabs(y));
+      r = vmax(r, vabs(lowk(x, cUC + a, o)));
+      return vmax(r, vabs(lowk(y, cUC + a, o - d)));
+    };
+    auto umax_ij = [&](int a) {
+      Vec<R> r = vmax(vset(R(0.0)), vabs(B.lv(cUC + a, o)));
+      r = vmax(r, vabs(B.lv(cUC + a, o - di)));
+      r = vmax(r, vabs(B.lv(cUC + a, o - dj)));
+      return vmax(r, vabs(B.lv(cUC + a, o - di - dj)));
+    };
+    // ne_eff of the densities averaged over the four cells
+    auto ne_of = [&](const Vec<R> &rH, const Vec<R> &rN) {
+      return vmap<R>([&](int e) { return num_limiter(c, R(0.25) * rH.v[e], R(0.25) * rN.v[e]).ne_eff; });
+    };
+    auto rho_k = [&](int comp, uint32_t d) {  // the row below along d first, k - 1 before k
+      const Vec<R> y = B.lv(comp, o - d), x = B.lv(comp, o);
+      Vec<R> r = R(0.0) + lowk(y, comp, o - d);
+      r = r + y;
+      r = r + lowk(x, comp, o);
+      return r + x;
+    };
+    auto rho_ij = [&](int comp) {
+      Vec<R> r = R(0.0) + B.lv(comp, o - di - dj);
+      r = r + B.lv(comp, o - di);
+      r = r + B.lv(comp, o - dj);
+      return r + B.lv(comp, o);
+    };
+    const int ambi = uniform(c.ambipolar);
+    const Vec<R> pn = ambi ? B.lv(cPEN, o) : vset(R(0.0));
+    {
+      const Vec<R> fy = B.lv(cEFY, o), by = B.lv(cBY, o);
+      const Vec<R> Ec = R(0.25) * (fy + lowk(fy, cEFY, o) + B.lv(cEFZ, o) + B.lv(cEFZ, o - dj));
+      const Vec<R> ae = umax_k(1, dj), az = umax_k(2, dj);
+      const Vec<R> d1 = B.lv(cBZ, o) - B.lv(cBZ, o - dj);
+      const Vec<R> d2 = by - lowk(by, cBY, o);
+      Vec<R> e = Ec + Cuct * (R(0.5) * ae * d1 - R(0.5) * az * d2);
+      if (ambi) e = e - pc * (B.lv(cPEN, o + di) - pn) / ne_of(rho_k(cUH, dj), rho_k(cUN, dj));
+      B.st(cEX, it, add_artificial(B, c, 0, o, e), 0, B.n2 + 1, it.i < B.n0);
     }
-    if (j < B.n1) {
-      const R Ec = R(0.25) * (AT(cEFX + 1, i, j, k) + AT(cEFX + 1, i, j, k - 1) + AT(cEFZ + 1, i, j, k) +
-                                AT(cEFZ + 1, i - 1, j, k));
-      const R az = max_abs_u4(B, 2, i, j, k, i - 1, j, k, i, j, k - 1, i - 1, j, k - 1);
-      const R ax = max_abs_u4(B, 0, i, j, k, i - 1, j, k, i, j, k - 1, i - 1, j, k - 1);
-      const R d1 = AT(cBX, i, j, k) - AT(cBX, i, j, k - 1);
-      const R d2 = AT(cBZ, i, j, k) - AT(cBZ, i - 1, j, k);
-      R e = Ec + Cuct * (R(0.5) * az * d1 - R(0.5) * ax * d2);
-      if (c.ambipolar) {
-        const R p0 = AT(cPEN, i, j, k), p1 = AT(cPEN, i, j + 1, k);
-        R rH = R(0.0), rN = R(0.0);
-        for (int di = -1; di <= 0; ++di)
-          for (int dk = -1; dk <= 0; ++dk) {
-            rH += AT(cUH, i + di, j, k + dk);
-            rN += AT(cUN, i + di, j, k + dk);
-          }
-        e -= pc * (p1 - p0) / num_limiter(c, R(0.25) * rH, R(0.25) * rN).ne_eff;
-      }
-      AT(cEY, i, j, k) = add_artificial(B, c, 1, i, j, k, e);
+    {
+      const Vec<R> fx = B.lv(cEFX + 1, o), bx = B.lv(cBX, o);
+      const Vec<R> Ec = R(0.25) * (fx + lowk(fx, cEFX + 1, o) + B.lv(cEFZ + 1, o) + B.lv(cEFZ + 1, o - di));
+      const Vec<R> az = umax_k(2, di), ax = umax_k(0, di);
+      const Vec<R> d1 = bx - lowk(bx, cBX, o);
+      const Vec<R> d2 = B.lv(cBZ, o) - B.lv(cBZ, o - di);
+      Vec<R> e = Ec + Cuct * (R(0.5) * az * d1 - R(0.5) * ax * d2);
+      if (ambi) e = e - pc * (B.lv(cPEN, o + dj) - pn) / ne_of(rho_k(cUH, di), rho_k(cUN, di));
+      B.st(cEY, it, add_artificial(B, c, 1, o, e), 0, B.n2 + 1, it.j < B.n1);
     }
-    if (k < B.n2) {
-      const R Ec = R(0.25) * (AT(cEFX + 2, i, j, k) + AT(cEFX + 2, i, j - 1, k) + AT(cEFY + 2, i, j, k) +
-                                AT(cEFY + 2, i - 1, j, k));
-      const R ax = max_abs_u4(B, 0, i, j, k, i - 1, j, k, i, j - 1, k, i - 1, j - 1, k);
-      const R ae = max_abs_u4(B, 1, i, j, k, i - 1, j, k, i, j - 1, k, i - 1, j - 1, k);
-      const R d1 = AT(cBY, i, j, k) - AT(cBY, i - 1, j, k);
-      const R d2 = AT(cBX, i, j, k) - AT(cBX, i, j - 1, k);
-      R e = Ec + Cuct * (R(0.5) * ax * d1 - R(0.5) * ae * d2);
-      if (c.ambipolar) {
-        const R p0 = AT(cPEN, i, j, k), p1 = AT(cPEN, i, j, k + 1);
-        R rH = R(0.0), rN = R(0.0);
-        for (int di = -1; di <= 0; ++di)
-          for (int dj = -1; dj <= 0; ++dj) {
-            rH += AT(cUH, i + di, j + dj, k);
-            rN += AT(cUN, i + di, j + dj, k);
-          }
-        e -= pc * (p1 - p0) / num_limiter(c, R(0.25) * rH, R(0.25) * rN).ne_eff;
-      }
-      AT(cEZ, i, j, k) = add_artificial(B, c, 2, i, j, k, e);
+    {
+      const Vec<R> Ec =
+          R(0.25) * (B.lv(cEFX + 2, o) + B.lv(cEFX + 2, o - dj) + B.lv(cEFY + 2, o) + B.lv(cEFY + 2, o - di));
+      const Vec<R> ax = umax_ij(0), ae = umax_ij(1);
+      const Vec<R> d1 = B.lv(cBY, o) - B.lv(cBY, o - di);
+      const Vec<R> d2 = B.lv(cBX, o) - B.lv(cBX, o - dj);
+      Vec<R> e = Ec + Cuct * (R(0.5) * ax * d1 - R(0.5) * ae * d2);
+      if (ambi) e = e - pc * (B.upper(pn, cPEN, o) - pn) / ne_of(rho_ij(cUH), rho_ij(cUN));
+      B.st(cEZ, it, add_artificial(B, c, 2, o, e), 0, B.n2);
     }
   });
 }
@@ -507,68 +700,61 @@ __global__ void __launch_bounds__(kTileThreads) k_edge_emf(Dir D) {
 // ------------------------------------------------------------------ Hall EMF
 // BuildHallFaceEMF_Rusanov_diff_ steps 2-4 (Hall.cpp:148-400).
 template <class R>
-__global__ void __launch_bounds__(kTileThreads) k_hall_edge(Dir D) {
-  for_items<R, kBox>(D, [&](const DevSolve &S, const V<R> &B, const Item &it) {
-    if (!it.in) return;
-    const int i = it.i, j = it.j, k = it.k;
+__global__ void __launch_bounds__(kVecThreads, 3) k_hall_edge(Dir D) {
+  for_vec_items<R, kBox>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
+    const uint32_t o = it.o, di = B.di, dj = B.dj;
     const R Cwh = R(0.1);
-    if (i < B.n0) {
-      R Ec[3];
-      for (int q = 0; q < 3; ++q)
-        Ec[q] = R(0.25) * (AT(cEHC + q, i, j - 1, k - 1) + AT(cEHC + q, i, j - 1, k) + AT(cEHC + q, i, j, k - 1) +
-                        AT(cEHC + q, i, j, k));
-      const R Ecen = Ec[0] * AT(cDRX, i, j, k) + Ec[1] * AT(cDRX + 1, i, j, k) + Ec[2] * AT(cDRX + 2, i, j, k);
-      const R be =
-          dmax(dmax(AT(cHB, i, j - 1, k - 1), AT(cHB, i, j - 1, k)), dmax(AT(cHB, i, j, k - 1), AT(cHB, i, j, k)));
-      const R ihe = AT(cIHX, i, j, k), ihz = AT(cIHX + 1, i, j, k);
-      const R mue = Cwh * be * ihe * ihe;
-      const R muz = Cwh * be * ihz * ihz;
-      const R d1 = AT(cBZ, i, j, k) - AT(cBZ, i, j - 1, k);
-      const R d2 = AT(cBY, i, j, k) - AT(cBY, i, j, k - 1);
-      AT(cHX, i, j, k) = AT(cTPX, i, j, k) * (Ecen + R(0.5) * mue * d1 - R(0.5) * muz * d2);
+    // over the four cells at an edge, in the reference's order: lower row and
+    // lower k first
+    auto mean_k = [&](int comp, uint32_t d) {
+      const Vec<R> y = B.lv(comp, o - d), x = B.lv(comp, o);
+      return R(0.25) * (B.lower(y, comp, o - d) + y + B.lower(x, comp, o) + x);
+    };
+    auto max_k = [&](int comp, uint32_t d) {
+      const Vec<R> y = B.lv(comp, o - d), x = B.lv(comp, o);
+      return vmax(vmax(B.lower(y, comp, o - d), y), vmax(B.lower(x, comp, o), x));
+    };
+    auto mean_ij = [&](int comp) {
+      return R(0.25) * (B.lv(comp, o - di - dj) + B.lv(comp, o - di) + B.lv(comp, o - dj) + B.lv(comp, o));
+    };
+    auto tail = [&](int ax, const Vec<R> &Ecen, const Vec<R> &be, const Vec<R> &d1, const Vec<R> &d2) {
+      const int ci = ax == 0 ? cIHX : ax == 1 ? cIHY : cIHZ;
+      const Vec<R> ih1 = B.lv(ci, o), ih2 = B.lv(ci + 1, o);
+      const Vec<R> mu1 = Cwh * be * ih1 * ih1;
+      const Vec<R> mu2 = Cwh * be * ih2 * ih2;
+      return B.lv(cTPX + ax, o) * (Ecen + R(0.5) * mu1 * d1 - R(0.5) * mu2 * d2);
+    };
+    {
+      const Vec<R> Ecen = mean_k(cEHC, dj) * B.lv(cDRX, o) + mean_k(cEHC + 1, dj) * B.lv(cDRX + 1, o) +
+                          mean_k(cEHC + 2, dj) * B.lv(cDRX + 2, o);
+      const Vec<R> by = B.lv(cBY, o);
+      B.st(cHX, it, tail(0, Ecen, max_k(cHB, dj), B.lv(cBZ, o) - B.lv(cBZ, o - dj), by - B.lower(by, cBY, o)), 0,
+           B.n2 + 1, it.i < B.n0);
     }
-    if (j < B.n1) {
-      R Ec[3];
-      for (int q = 0; q < 3; ++q)
-        Ec[q] = R(0.25) * (AT(cEHC + q, i - 1, j, k - 1) + AT(cEHC + q, i - 1, j, k) + AT(cEHC + q, i, j, k - 1) +
-                        AT(cEHC + q, i, j, k));
-      const R Ecen = Ec[0] * AT(cDRY, i, j, k) + Ec[1] * AT(cDRY + 1, i, j, k) + Ec[2] * AT(cDRY + 2, i, j, k);
-      const R be =
-          dmax(dmax(AT(cHB, i - 1, j, k - 1), AT(cHB, i - 1, j, k)), dmax(AT(cHB, i, j, k - 1), AT(cHB, i, j, k)));
-      const R ihz = AT(cIHY, i, j, k), ihx = AT(cIHY + 1, i, j, k);
-      const R muz = Cwh * be * ihz * ihz;
-      const R mux = Cwh * be * ihx * ihx;
-      const R d1 = AT(cBX, i, j, k) - AT(cBX, i, j, k - 1);
-      const R d2 = AT(cBZ, i, j, k) - AT(cBZ, i - 1, j, k);
-      AT(cHY, i, j, k) = AT(cTPY, i, j, k) * (Ecen + R(0.5) * muz * d1 - R(0.5) * mux * d2);
+    {
+      const Vec<R> Ecen = mean_k(cEHC, di) * B.lv(cDRY, o) + mean_k(cEHC + 1, di) * B.lv(cDRY + 1, o) +
+                          mean_k(cEHC + 2, di) * B.lv(cDRY + 2, o);
+      const Vec<R> bx = B.lv(cBX, o);
+      B.st(cHY, it, tail(1, Ecen, max_k(cHB, di), bx - B.lower(bx, cBX, o), B.lv(cBZ, o) - B.lv(cBZ, o - di)), 0,
+           B.n2 + 1, it.j < B.n1);
     }
-    if (k < B.n2) {
-      R Ec[3];
-      for (int q = 0; q < 3; ++q)
-        Ec[q] = R(0.25) * (AT(cEHC + q, i - 1, j - 1, k) + AT(cEHC + q, i - 1, j, k) + AT(cEHC + q, i, j - 1, k) +
-                        AT(cEHC + q, i, j, k));
-      const R Ecen = Ec[0] * AT(cDRZ, i, j, k) + Ec[1] * AT(cDRZ + 1, i, j, k) + Ec[2] * AT(cDRZ + 2, i, j, k);
-      const R be =
-          dmax(dmax(AT(cHB, i - 1, j - 1, k), AT(cHB, i - 1, j, k)), dmax(AT(cHB, i, j - 1, k), AT(cHB, i, j, k)));
-      const R ihx = AT(cIHZ, i, j, k), ihe = AT(cIHZ + 1, i, j, k);
-      const R mux = Cwh * be * ihx * ihx;
-      const R mue = Cwh * be * ihe * ihe;
-      const R d1 = AT(cBY, i, j, k) - AT(cBY, i - 1, j, k);
-      const R d2 = AT(cBX, i, j, k) - AT(cBX, i, j - 1, k);
-      AT(cHZ, i, j, k) = AT(cTPZ, i, j, k) * (Ecen + R(0.5) * mux * d1 - R(0.5) * mue * d2);
+    {
+      const Vec<R> Ecen =
+          mean_ij(cEHC) * B.lv(cDRZ, o) + mean_ij(cEHC + 1) * B.lv(cDRZ + 1, o) + mean_ij(cEHC + 2) * B.lv(cDRZ + 2, o);
+      const Vec<R> be = vmax(vmax(B.lv(cHB, o - di - dj), B.lv(cHB, o - di)), vmax(B.lv(cHB, o - dj), B.lv(cHB, o)));
+      B.st(cHZ, it, tail(2, Ecen, be, B.lv(cBY, o) - B.lv(cBY, o - di), B.lv(cBX, o) - B.lv(cBX, o - dj)), 0, B.n2);
     }
   });
 }
 
 // E += Ehall on owned edges (Z4_Mercury/src/physics/MercurySolver_MagneticRHS.cpp:135-147).
 template <class R>
-__global__ void __launch_bounds__(kTileThreads) k_add_hall(Dir D) {
-  for_items<R, kBox>(D, [&](const DevSolve &S, const V<R> &B, const Item &it) {
-    if (!it.in) return;
-    const int o = B.off(it.i, it.j, it.k);
-    if (it.i < B.n0) B.c(cEX)[o] += B.c(cHX)[o];
-    if (it.j < B.n1) B.c(cEY)[o] += B.c(cHY)[o];
-    if (it.k < B.n2) B.c(cEZ)[o] += B.c(cHZ)[o];
+__global__ void __launch_bounds__(kVecThreads) k_add_hall(Dir D) {
+  for_vec_items<R, kBox>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
+    // each thread reads and writes its own positions only
+    B.st(cEX, it, B.own(cEX, it.o) + B.lv(cHX, it.o), 0, B.n2 + 1, it.i < B.n0);
+    B.st(cEY, it, B.own(cEY, it.o) + B.lv(cHY, it.o), 0, B.n2 + 1, it.j < B.n1);
+    B.st(cEZ, it, B.own(cEZ, it.o) + B.lv(cHZ, it.o), 0, B.n2);
   });
 }
 
@@ -631,12 +817,6 @@ __device__ __forceinline__ void rusanov(const FluidCell<R> &L, const FluidCell<R
            R(0.5) * rad * (Q.rho * Q.w - L.rho * L.w);
   out[4] = R(0.5) * (uvwL * (L.re + L.p) + uvwR * (Q.re + Q.p)) - R(0.5) * rad * (Q.re - L.re);
 }
-
-// Minimum resident CTAs per SM asked of the compiler for the primitive pass
-// (caps registers at 65536 / (256 * n)).
-#ifndef MHD_MIN_CTAS_PV
-#define MHD_MIN_CTAS_PV 4
-#endif
 
 // ZeroRHS_ + Scheme_U_ + AddSourceToRHS_Fluid (FluidRHS.cpp:206-527) +
 // ApplyUpdate_Euler_ (Z4_Mercury/src/physics/MercurySolver_Advance.cpp:73-147)
@@ -706,7 +886,7 @@ __global__ void __launch_bounds__(fluid_threads(VT), fluid_ctas(VT, sizeof(R))) 
           const FluidFace<R> f = fluid_face<R, 0>(B, o + di);
 #pragma unroll
           for (int q = 0; q < NS; ++q) {
-            const int s = s0 + q, u0 = s ? cUN : cUH, pv0 = s ? cPVN : cPVH;
+            const int s = s0 + q;
             N[q] = fluid_cell(B, s, o + di);
             R F[5];
             rusanov(C[q], N[q], f, F);
@@ -722,7 +902,7 @@ __global__ void __launch_bounds__(fluid_threads(VT), fluid_ctas(VT, sizeof(R))) 
           const FluidFace<R> fl = fluid_face<R, dir>(B, o), fh = fluid_face<R, dir>(B, o + d);
 #pragma unroll
           for (int q = 0; q < NS; ++q) {
-            const int s = s0 + q, u0 = s ? cUN : cUH, pv0 = s ? cPVN : cPVH;
+            const int s = s0 + q;
             R Fl[5], Fh[5];
             rusanov(fluid_cell(B, s, o - d), C[q], fl, Fl);
             rusanov(C[q], fluid_cell(B, s, o + d), fh, Fh);
@@ -801,23 +981,24 @@ __global__ void __launch_bounds__(fluid_threads(VT), fluid_ctas(VT, sizeof(R))) 
 
 // B_face += dt * (-curl E) on the owned faces (CTOperators.cpp:6-56 with multiplier -1).
 template <class R>
-__global__ void __launch_bounds__(kTileThreads) k_bface(Dir D) {
-  for_items<R, kBox>(D, [&](const DevSolve &S, const V<R> &B, const Item &it) {
-    if (!it.in) return;
+__global__ void __launch_bounds__(kVecThreads) k_bface(Dir D) {
+  for_vec_items<R, kBox>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
     const R dt = __longlong_as_double((long long)D.state[it.s].dt_bits);
-    if (!(dt >= R(1e-7)) || !isfinite(dt) || D.state[it.s].nonfinite) return;  // k_flip records the status
-    const int i = it.i, j = it.j, k = it.k;
-    if (j < B.n1 && k < B.n2) {
-      const R rb = -R(1.0) * ((AT(cEY, i, j, k) - AT(cEY, i, j, k + 1)) + (AT(cEZ, i, j + 1, k) - AT(cEZ, i, j, k)));
-      AT(cBX, i, j, k) += dt * rb;
+    if (uniform((int)(!(dt >= R(1e-7)) || !isfinite(dt) || D.state[it.s].nonfinite))) return;  // k_flip records the status
+    const uint32_t o = it.o, di = B.di, dj = B.dj;
+    const bool ic = it.i < B.n0, jc = it.j < B.n1;
+    const Vec<R> ex = B.lv(cEX, o), ey = B.lv(cEY, o), ez = B.lv(cEZ, o);
+    {
+      const Vec<R> rb = -R(1.0) * ((ey - B.upper(ey, cEY, o)) + (B.lv(cEZ, o + dj) - ez));
+      B.st(cBX, it, B.own(cBX, o) + dt * rb, 0, B.n2, jc);
     }
-    if (i < B.n0 && k < B.n2) {
-      const R rb = -R(1.0) * ((AT(cEX, i, j, k + 1) - AT(cEX, i, j, k)) + (AT(cEZ, i, j, k) - AT(cEZ, i + 1, j, k)));
-      AT(cBY, i, j, k) += dt * rb;
+    {
+      const Vec<R> rb = -R(1.0) * ((B.upper(ex, cEX, o) - ex) + (ez - B.lv(cEZ, o + di)));
+      B.st(cBY, it, B.own(cBY, o) + dt * rb, 0, B.n2, ic);
     }
-    if (i < B.n0 && j < B.n1) {
-      const R rb = -R(1.0) * ((AT(cEX, i, j, k) - AT(cEX, i, j + 1, k)) + (AT(cEY, i + 1, j, k) - AT(cEY, i, j, k)));
-      AT(cBZ, i, j, k) += dt * rb;
+    {
+      const Vec<R> rb = -R(1.0) * ((ex - B.lv(cEX, o + dj)) + (B.lv(cEY, o + di) - ey));
+      B.st(cBZ, it, B.own(cBZ, o) + dt * rb, 0, B.n2 + 1, ic && jc);
     }
   });
 }
@@ -827,79 +1008,116 @@ __global__ void __launch_bounds__(kTileThreads) k_bface(Dir D) {
 // CurlAdjFaceToEdge + alpha scaling of Calc_J_Edge (CTOperators.cpp:59-110,
 // Z4_Mercury/src/physics/MercurySolver_Current.cpp:140-190) on owned edges.
 template <class R>
-__global__ void __launch_bounds__(kTileThreads) k_bcell_jedge(Dir D) {
-  for_items<R, kBox>(D, [&](const DevSolve &S, const V<R> &B, const Item &it) {
-    if (!it.in) return;
-    const int i = it.i, j = it.j, k = it.k;
-    if (i < B.n0 && j < B.n1 && k < B.n2) {
-      const R pt[6] = {-AT(cBX, i, j, k) - AT(cBAX, i, j, k), AT(cBX, i + 1, j, k) + AT(cBAX, i + 1, j, k),
-                            -AT(cBY, i, j, k) - AT(cBAY, i, j, k), AT(cBY, i, j + 1, k) + AT(cBAY, i, j + 1, k),
-                            -AT(cBZ, i, j, k) - AT(cBAZ, i, j, k), AT(cBZ, i, j, k + 1) + AT(cBAZ, i, j, k + 1)};
-      const R pi_[6] = {-AT(cBX, i, j, k), AT(cBX, i + 1, j, k), -AT(cBY, i, j, k),
-                             AT(cBY, i, j + 1, k), -AT(cBZ, i, j, k), AT(cBZ, i, j, k + 1)};
-      R bxt = 0, byt = 0, bzt = 0, bxi = 0, byi = 0, bzi = 0;
+__global__ void __launch_bounds__(kVecThreads, 3) k_bcell_jedge(Dir D) {
+  for_vec_items<R, kBox>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
+    const uint32_t o = it.o, di = B.di, dj = B.dj;
+    const bool ic = it.i < B.n0, jc = it.j < B.n1;
+    const Vec<R> bx = B.lv(cBX, o), by = B.lv(cBY, o), bz = B.lv(cBZ, o);
+    {
+      const Vec<R> ax = B.lv(cBAX, o), ay = B.lv(cBAY, o), az = B.lv(cBAZ, o);
+      const Vec<R> bxp = B.lv(cBX, o + di), byp = B.lv(cBY, o + dj), bzp = B.upper(bz, cBZ, o);
+      Vec<R> t[3] = {vset(R(0.0)), vset(R(0.0)), vset(R(0.0))}, in[3] = {t[0], t[0], t[0]};
+      auto add = [&](int q, const Vec<R> &total, const Vec<R> &induced) {  // face q of the cell
 #pragma unroll
-      for (int q = 0; q < 6; ++q) {
-        const R wx = AT(cWB + q, i, j, k), wy = AT(cWB + 6 + q, i, j, k), wz = AT(cWB + 12 + q, i, j, k);
-        bxt += wx * pt[q];
-        byt += wy * pt[q];
-        bzt += wz * pt[q];
-        bxi += wx * pi_[q];
-        byi += wy * pi_[q];
-        bzi += wz * pi_[q];
+        for (int x = 0; x < 3; ++x) {
+          const Vec<R> w = B.lv(cWB + 6 * x + q, o);
+          t[x] = t[x] + w * total;
+          in[x] = in[x] + w * induced;
+        }
+      };
+      add(0, -bx - ax, -bx);
+      add(1, bxp + B.lv(cBAX, o + di), bxp);
+      add(2, -by - ay, -by);
+      add(3, byp + B.lv(cBAY, o + dj), byp);
+      add(4, -bz - az, -bz);
+      add(5, bzp + B.upper(az, cBAZ, o), bzp);
+#pragma unroll
+      for (int x = 0; x < 3; ++x) {
+        B.st(cBC + x, it, t[x], 0, B.n2, ic && jc);
+        B.st(cBIC + x, it, in[x], 0, B.n2, ic && jc);
       }
-      const int o = B.off(i, j, k);
-      B.c(cBC)[o] = bxt;
-      B.c(cBC + 1)[o] = byt;
-      B.c(cBC + 2)[o] = bzt;
-      B.c(cBIC)[o] = bxi;
-      B.c(cBIC + 1)[o] = byi;
-      B.c(cBIC + 2)[o] = bzi;
     }
-    if (i < B.n0) {
-      const R v = ((AT(cBFY, i, j, k - 1) * AT(cBY, i, j, k - 1) - AT(cBFY, i, j, k) * AT(cBY, i, j, k)) +
-                        (AT(cBFZ, i, j, k) * AT(cBZ, i, j, k) - AT(cBFZ, i, j - 1, k) * AT(cBZ, i, j - 1, k))) * R(1.0);
-      AT(cJX, i, j, k) = v * AT(cALX, i, j, k);
+    // beta B on this position's faces and the lower neighbours'
+    const Vec<R> fx = B.lv(cBFX, o) * bx, fy = B.lv(cBFY, o) * by, fz = B.lv(cBFZ, o) * bz;
+    auto below = [&](int a, uint32_t d) { return B.lv(cBFX + a, o - d) * B.lv(cBX + a, o - d); };
+    constexpr uint32_t es = sizeof(R);
+    {
+      const Vec<R> v = ((vdown(fy, B.ld(cBFY, o - es) * B.ld(cBY, o - es)) - fy) + (fz - below(2, dj))) * R(1.0);
+      B.st(cJX, it, v * B.lv(cALX, o), 0, B.n2 + 1, ic);
     }
-    if (j < B.n1) {
-      const R v = ((AT(cBFX, i, j, k) * AT(cBX, i, j, k) - AT(cBFX, i, j, k - 1) * AT(cBX, i, j, k - 1)) +
-                        (AT(cBFZ, i - 1, j, k) * AT(cBZ, i - 1, j, k) - AT(cBFZ, i, j, k) * AT(cBZ, i, j, k))) * R(1.0);
-      AT(cJY, i, j, k) = v * AT(cALY, i, j, k);
+    {
+      const Vec<R> v = ((fx - vdown(fx, B.ld(cBFX, o - es) * B.ld(cBX, o - es))) + (below(2, di) - fz)) * R(1.0);
+      B.st(cJY, it, v * B.lv(cALY, o), 0, B.n2 + 1, jc);
     }
-    if (k < B.n2) {
-      const R v = ((AT(cBFX, i, j - 1, k) * AT(cBX, i, j - 1, k) - AT(cBFX, i, j, k) * AT(cBX, i, j, k)) +
-                        (AT(cBFY, i, j, k) * AT(cBY, i, j, k) - AT(cBFY, i - 1, j, k) * AT(cBY, i - 1, j, k))) * R(1.0);
-      AT(cJZ, i, j, k) = v * AT(cALZ, i, j, k);
+    {
+      const Vec<R> v = ((below(0, dj) - fx) + (fy - below(1, di))) * R(1.0);
+      B.st(cJZ, it, v * B.lv(cALZ, o), 0, B.n2);
     }
   });
 }
 
 // calc_Jcell (Current.cpp:203-243), owned cells.
 template <class R>
-__global__ void __launch_bounds__(kTileThreads) k_jcell(Dir D) {
-  for_items<R, kCells>(D, [&](const DevSolve &S, const V<R> &B, const Item &it) {
-    if (!it.in) return;
-    const int i = it.i, j = it.j, k = it.k;
-    const R s[12] = {AT(cJX, i, j, k),         AT(cJX, i, j + 1, k),     AT(cJX, i, j, k + 1),
-                          AT(cJX, i, j + 1, k + 1), AT(cJY, i, j, k),         AT(cJY, i + 1, j, k),
-                          AT(cJY, i, j, k + 1),     AT(cJY, i + 1, j, k + 1), AT(cJZ, i, j, k),
-                          AT(cJZ, i + 1, j, k),     AT(cJZ, i, j + 1, k),     AT(cJZ, i + 1, j + 1, k)};
-    R jx = 0, jy = 0, jz = 0;
+__global__ void __launch_bounds__(kVecThreads, 3) k_jcell(Dir D) {
+  for_vec_items<R, kCells>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
+    const uint32_t o = it.o, di = B.di, dj = B.dj;
+    Vec<R> j[3] = {vset(R(0.0)), vset(R(0.0)), vset(R(0.0))};
+    auto add = [&](int q, const Vec<R> &s) {  // edge q of the cell, the summation order of calc_Jcell
 #pragma unroll
-    for (int q = 0; q < 12; ++q) {
-      jx += AT(cWJ + q, i, j, k) * s[q];
-      jy += AT(cWJ + 12 + q, i, j, k) * s[q];
-      jz += AT(cWJ + 24 + q, i, j, k) * s[q];
+      for (int x = 0; x < 3; ++x) j[x] = j[x] + B.lv(cWJ + 12 * x + q, o) * s;
+    };
+    {
+      const Vec<R> a = B.lv(cJX, o), b = B.lv(cJX, o + dj);
+      add(0, a);
+      add(1, b);
+      add(2, B.upper(a, cJX, o));
+      add(3, B.upper(b, cJX, o + dj));
     }
-    const int o = B.off(i, j, k);
-    B.c(cJC)[o] = jx;
-    B.c(cJC + 1)[o] = jy;
-    B.c(cJC + 2)[o] = jz;
+    {
+      const Vec<R> a = B.lv(cJY, o), b = B.lv(cJY, o + di);
+      add(4, a);
+      add(5, b);
+      add(6, B.upper(a, cJY, o));
+      add(7, B.upper(b, cJY, o + di));
+    }
+    add(8, B.lv(cJZ, o));
+    add(9, B.lv(cJZ, o + di));
+    add(10, B.lv(cJZ, o + dj));
+    add(11, B.lv(cJZ, o + di + dj));
+#pragma unroll
+    for (int x = 0; x < 3; ++x) B.st(cJC + x, it, j[x], 0, B.n2);
   });
 }
 
-// CFL time step of one cell and both species (Compute_Timestep,
-// Z4_Mercury/src/physics/MercurySolver_Timestep.cpp:8-141).
+// Quotients by one divisor b > 0.  FP32: by its reciprocal.  FP64: the quotient
+// that IEEE division rounds to, from the correctly rounded reciprocal y = RN(1/b)
+// and one residual, q = RN(a y), RN(q + RN(a - b q) y) (Markstein, "Computation
+// of elementary functions on the IBM RISC System/6000 processor", 1990): exact
+// while nothing under- or overflows, so values outside [1e-280, 1e280] are
+// divided (a zero keeps its sign).
+template <class R>
+struct Divisor {
+  R b, y;
+  __device__ __forceinline__ explicit Divisor(R d) : b(d) {
+    if constexpr (sizeof(R) == 4) y = R(1.0) / d;
+    else y = __drcp_rn(d);
+  }
+  __device__ __forceinline__ Divisor(R d, R recip) : b(d), y(recip) {}
+  __device__ __forceinline__ R operator()(R a) const {
+    if constexpr (sizeof(R) == 4) return a * y;
+    else {
+      const R q = a * y, m = fabs(a);
+      if (m >= R(1e-280) && m <= R(1e280)) return fma(fma(-b, q, a), y, q);
+      return a == R(0.0) ? q : a / b;
+    }
+  }
+};
+
+// CFL time step of a thread's cells and both species (Compute_Timestep,
+// Z4_Mercury/src/physics/MercurySolver_Timestep.cpp:8-141): the smallest over
+// the cells.  (nx, ny, nz, An) are a face's precomputed a / |a| and |a|
+// (k_face_normals: the same operations as the reference evaluates per face);
+// vA2 = inver_MA2 * B2 / rho is the same for all faces of a cell and species.
 template <class R>
 __device__ __forceinline__ R fast_cf(R cs2, R vA2, R vAn2) {
   const R term = cs2 + vA2;
@@ -907,90 +1125,66 @@ __device__ __forceinline__ R fast_cf(R cs2, R vA2, R vAn2) {
   if (disc < R(0.0)) disc = R(0.0);
   return sqrt(R(0.5) * (term + sqrt(disc)));
 }
-// One face's term of the CFL denominator.  (nx, ny, nz, An) are the face's
-// precomputed a / |a| and |a| (k_face_normals: the same operations as the
-// reference evaluates per face); vA2 = inver_MA2 * B2 / rho is the same for
-// all faces of a cell and species.
 template <class R>
-__device__ __forceinline__ R face_term(const ConstsT<R> &c, R nx, R ny, R nz, R An,
-                                            bool outward_plus, R ux, R uy, R uz, R Bx, R By,
-                                            R Bz, R vA2, R rho, R cs2) {
-  if (An <= R(0.0)) return R(0.0);
-  if (!outward_plus) {
-    nx = -nx;
-    ny = -ny;
-    nz = -nz;
-  }
-  const R un = ux * nx + uy * ny + uz * nz;
-  const R Bn = Bx * nx + By * ny + Bz * nz;
-  const R vAn2 = c.inver_MA2 * (Bn * Bn) / rho;
-  return (fabs(un) + fast_cf(cs2, vA2, vAn2)) * An;
-}
-template <class R>
-__device__ __forceinline__ R cell_dt(const V<R> &B, const ConstsT<R> &c, int i, int j, int k) {
-  R dtl = R(1e100);
-  const R Vol = fabs(R(LDM(cJAC, i, j, k)));
-  if (!(Vol > R(0.0))) return dtl;
-  const R Bx = LD(cBC, i, j, k), By = LD(cBC + 1, i, j, k), Bz = LD(cBC + 2, i, j, k);
-  const R B2 = Bx * Bx + By * By + Bz * Bz;
-  if constexpr (sizeof(R) == 4) {
-    // FP32: the six faces' unit normals and |a| and both species' states are
-    // loaded once, up front (xi-, xi+, eta-, eta+, zeta-, zeta+: the
-    // reference's summation order)
-    R fn[6][4];
+__device__ __forceinline__ R cells_dt(const VV<R> &B, const ConstsT<R> &c, const VItem &it, bool own, const Vec<R> &Bx,
+                                      const Vec<R> &By, const Vec<R> &Bz, bool &bad) {
+  constexpr int N = Vec<R>::N;
+  const uint32_t o = it.o;
+  const Vec<R> Vol = vabs(B.lm(cJAC, o));
+  const Vec<R> B2 = Bx * Bx + By * By + Bz * Bz;
+  Vec<R> d = vset(R(1e100));
+#pragma unroll 1
+  for (int s = 0; s < 2; ++s) {
+    const int u0 = s ? cUN : cUH;
+    const Vec<R> rho0 = B.lv(u0, o), m1 = B.lv(u0 + 1, o), m2 = B.lv(u0 + 2, o), m3 = B.lv(u0 + 3, o), E = B.lv(u0 + 4, o);
+    Vec<R> ux, uy, uz, cs2, vA2, den = vset(R(0.0)), rho, y;
 #pragma unroll
-    for (int f = 0; f < 6; ++f) {
-      const int a = f >> 1, up = f & 1;
-      const int cn = a == 0 ? cFNX : a == 1 ? cFNY : cFNZ;
-      int fi = i, fj = j, fk = k;
-      shift1(a, fi, fj, fk, up);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) fn[f][q] = LD(cn + q, fi, fj, fk);
+    for (int e = 0; e < N; ++e) {
+      rho.v[e] = dmax(rho0.v[e], R(1e-2));
+      const Divisor<R> by(rho.v[e]);
+      y.v[e] = by.y;
+      const R u = by(m1.v[e]), v = by(m2.v[e]), w = by(m3.v[e]);
+      const R ke = R(0.5) * rho.v[e] * (u * u + v * v + w * w);
+      const R pr = (c.gamma - R(1.0)) * (E.v[e] - ke);
+      cs2.v[e] = by(c.gamma * pr);
+      vA2.v[e] = by(c.inver_MA2 * B2.v[e]);
+      ux.v[e] = u;
+      uy.v[e] = v;
+      uz.v[e] = w;
     }
-    R Us[2][5];
+    // faces xi-, xi+, eta-, eta+, zeta-, zeta+ (the reference's summation order)
+    auto face = [&](const Vec<R> &px, const Vec<R> &py, const Vec<R> &pz, const Vec<R> &An, bool up) {
 #pragma unroll
-    for (int s = 0; s < 2; ++s)
-#pragma unroll
-      for (int q = 0; q < 5; ++q) Us[s][q] = LD((s ? cUN : cUH) + q, i, j, k);
-#pragma unroll 1
-    for (int s = 0; s < 2; ++s) {
-      const R rho = dmax(Us[s][0], R(1e-2));
-      const R ux = Us[s][1] / rho, uy = Us[s][2] / rho, uz = Us[s][3] / rho;
-      const R E = Us[s][4];
-      const R ke = R(0.5) * rho * (ux * ux + uy * uy + uz * uz);
-      const R pr = (c.gamma - R(1.0)) * (E - ke);
-      const R cs2 = c.gamma * pr / rho;
-      const R vA2 = c.inver_MA2 * B2 / rho;
-      R den = R(0.0);
-#pragma unroll
-      for (int f = 0; f < 6; ++f)
-        den += face_term(c, fn[f][0], fn[f][1], fn[f][2], fn[f][3], (f & 1) != 0, ux, uy, uz, Bx, By, Bz, vA2, rho, cs2);
-      if (den > R(0.0)) dtl = dmin(dtl, c.CFL * Vol / den);
-    }
-  } else {
-#pragma unroll 1
-    for (int s = 0; s < 2; ++s) {
-      const int u0 = s ? cUN : cUH;
-      const R rho = dmax(LD(u0, i, j, k), R(1e-2));
-      const R ux = LD(u0 + 1, i, j, k) / rho, uy = LD(u0 + 2, i, j, k) / rho, uz = LD(u0 + 3, i, j, k) / rho;
-      const R E = LD(u0 + 4, i, j, k);
-      const R ke = R(0.5) * rho * (ux * ux + uy * uy + uz * uz);
-      const R pr = (c.gamma - R(1.0)) * (E - ke);
-      const R cs2 = c.gamma * pr / rho;
-      const R vA2 = c.inver_MA2 * B2 / rho;
-      R den = R(0.0);
-      // faces xi-, xi+, eta-, eta+, zeta-, zeta+ (the reference's summation order)
-#pragma unroll 1
-      for (int f = 0; f < 6; ++f) {
-        const int a = f >> 1, up = f & 1;
-        const int cn = a == 0 ? cFNX : a == 1 ? cFNY : cFNZ;
-        int fi = i, fj = j, fk = k;
-        shift1(a, fi, fj, fk, up);
-        den += face_term(c, LD(cn, fi, fj, fk), LD(cn + 1, fi, fj, fk), LD(cn + 2, fi, fj, fk), LD(cn + 3, fi, fj, fk),
-                         up != 0, ux, uy, uz, Bx, By, Bz, vA2, rho, cs2);
+      for (int e = 0; e < N; ++e) {
+        const R nx = up ? px.v[e] : -px.v[e], ny = up ? py.v[e] : -py.v[e], nz = up ? pz.v[e] : -pz.v[e];
+        const R un = ux.v[e] * nx + uy.v[e] * ny + uz.v[e] * nz;
+        const R Bn = Bx.v[e] * nx + By.v[e] * ny + Bz.v[e] * nz;
+        const Divisor<R> by(rho.v[e], y.v[e]);
+        const R vAn2 = by(c.inver_MA2 * (Bn * Bn));
+        if (!(An.v[e] <= R(0.0))) den.v[e] += (fabs(un) + fast_cf(cs2.v[e], vA2.v[e], vAn2)) * An.v[e];
       }
-      if (den > R(0.0)) dtl = dmin(dtl, c.CFL * Vol / den);
+    };
+#pragma unroll 1
+    for (int a = 0; a < 2; ++a) {  // rolled: two axes' face loads in flight at once spill
+      const int cn = cFNX + 4 * a;
+      const uint32_t q = o + (a == 0 ? B.di : B.dj);
+      face(B.lv(cn, o), B.lv(cn + 1, o), B.lv(cn + 2, o), B.lv(cn + 3, o), false);
+      face(B.lv(cn, q), B.lv(cn + 1, q), B.lv(cn + 2, q), B.lv(cn + 3, q), true);
     }
+    const Vec<R> zx = B.lv(cFNZ, o), zy = B.lv(cFNZ + 1, o), zz = B.lv(cFNZ + 2, o), zA = B.lv(cFNZ + 3, o);
+    face(zx, zy, zz, zA, false);
+    face(B.upper(zx, cFNZ, o), B.upper(zy, cFNZ + 1, o), B.upper(zz, cFNZ + 2, o), B.upper(zA, cFNZ + 3, o), true);
+#pragma unroll
+    for (int e = 0; e < N; ++e)
+      if (Vol.v[e] > R(0.0) && den.v[e] > R(0.0)) d.v[e] = dmin(d.v[e], c.CFL * Vol.v[e] / den.v[e]);
+  }
+  R dtl = R(1e100);
+#pragma unroll
+  for (int e = 0; e < N; ++e) {
+    if (!own || it.k + e < 0 || it.k + e >= B.n2) continue;
+    // a NaN drops out of the minimum: record it instead
+    bad = bad || !isfinite(d.v[e]);
+    dtl = dmin(dtl, d.v[e]);
   }
   return dtl;
 }
@@ -998,19 +1192,24 @@ __device__ __forceinline__ R cell_dt(const V<R> &B, const ConstsT<R> &c, int i, 
 // calc_divB (Z4_Mercury/src/physics/MercurySolver_MagneticCell.cpp:186-193) on the owned cells,
 // and max |div B| per solve (atomicMax on the bits of the non-negative double).
 template <class R>
-__global__ void __launch_bounds__(kTileThreads) k_div_b(Dir D) {
-  for_items<R, kCells>(D, [&](const DevSolve &S, const V<R> &B, const Item &it) {
-    R v = R(0.0);
-    if (it.in) {
-      const int i = it.i, j = it.j, k = it.k;
-      v = (AT(cBX, i + 1, j, k) - AT(cBX, i, j, k) + AT(cBY, i, j + 1, k) - AT(cBY, i, j, k) + AT(cBZ, i, j, k + 1) -
-           AT(cBZ, i, j, k)) /
-          R(ATM(cJAC, i, j, k));
-      AT(cDIVB, i, j, k) = v;
+__global__ void __launch_bounds__(kVecThreads) k_div_b(Dir D) {
+  for_vec_items<R, kCells>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
+    double a = 0.0;
+    {
+      const uint32_t o = it.o;
+      const Vec<R> bz = B.lv(cBZ, o);
+      const Vec<R> v = (B.lv(cBX, o + B.di) - B.lv(cBX, o) + B.lv(cBY, o + B.dj) - B.lv(cBY, o) + B.upper(bz, cBZ, o) - bz) /
+                       B.lm(cJAC, o);
+      B.st(cDIVB, it, v, 0, B.n2);
+#pragma unroll
+      for (int e = 0; e < Vec<R>::N; ++e) {
+        if (!it.in || !it.has(e)) continue;
+        double x = fabs((double)v.v[e]);
+        if (!(x == x)) x = __longlong_as_double(0x7ff0000000000000LL);  // NaN counts as infinite
+        a = fmax(a, x);
+      }
     }
-    double a = fabs((double)v);
-    if (!(a == a)) a = __longlong_as_double(0x7ff0000000000000LL);  // NaN counts as infinite
-    for (int o = 16; o > 0; o >>= 1) a = fmax(a, __shfl_xor_sync(0xffffffffu, a, o));
+    for (int w = 16; w > 0; w >>= 1) a = fmax(a, __shfl_xor_sync(0xffffffffu, a, w));
     if ((threadIdx.x & 31) == 0) atomicMax(&D.state[it.s].divb_bits, (unsigned long long)__double_as_longlong(a));
   });
 }
@@ -1032,9 +1231,8 @@ __device__ __forceinline__ bool edge_owned(int a, int i, int j, int k, int n0, i
 // run in mark mode then zeros its destinations, the non-owner aliases, so
 // an edge still at 1 is its own unknown.
 template <class R>
-__global__ void __launch_bounds__(kTileThreads) k_res_seed(Dir D) {
-  for_items<R, kBox>(D, [&](const DevSolve &S, const V<R> &B, const Item &it) {
-    if (!it.in) return;
+__global__ void __launch_bounds__(kVecThreads) k_res_seed(Dir D) {
+  for_positions<R, kBox>(D, [&](const DevSolve &S, const VV<R> &B, const Pos &it) {
     const int o = B.off(it.i, it.j, it.k);
     for (int a = 0; a < 3; ++a) B.c(cEX + a)[o] = R(1.0);
   });
@@ -1043,9 +1241,8 @@ __global__ void __launch_bounds__(kTileThreads) k_res_seed(Dir D) {
 // W = 1 / (eta alpha) on the unknowns (owned, not a non-owner alias, eta > 0,
 // alpha > 0: BuildImplicitResistiveEdgeDofMap_, Mercury_ImplicitResistive.cpp:168-226), 0 elsewhere.
 template <class R>
-__global__ void __launch_bounds__(kTileThreads) k_res_w(Dir D) {
-  for_items<R, kBox>(D, [&](const DevSolve &S, const V<R> &B, const Item &it) {
-    if (!it.in) return;
+__global__ void __launch_bounds__(kVecThreads) k_res_w(Dir D) {
+  for_positions<R, kBox>(D, [&](const DevSolve &S, const VV<R> &B, const Pos &it) {
     const int o = B.off(it.i, it.j, it.k);
     for (int a = 0; a < 3; ++a) {
       R w = R(0.0);
@@ -1063,11 +1260,14 @@ __global__ void __launch_bounds__(kTileThreads) k_res_w(Dir D) {
 // the faces below the unknowns' top layer read E_res one layer up, the
 // current on the unknowns reads those faces.
 template <class R>
-__global__ void __launch_bounds__(kTileThreads) k_res_kmax(Dir D, int *out) {
-  for_items<R, kBox>(D, [&](const DevSolve &S, const V<R> &B, const Item &it) {
-    const int o = it.in ? B.off(it.i, it.j, it.k) : 0;
-    const bool dof = it.in && (B.c(cRW)[o] > R(0.0) || B.c(cRW + 1)[o] > R(0.0) || B.c(cRW + 2)[o] > R(0.0));
-    int k = dof ? it.k : -1;
+__global__ void __launch_bounds__(kVecThreads) k_res_kmax(Dir D, int *out) {
+  for_vec_items<R, kBox>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
+    int k = -1;
+    for (int e = 0; e < Vec<R>::N; ++e) {
+      if (!it.in || !it.has(e)) continue;
+      const int o = B.off(it.i, it.j, it.k + e);
+      if (B.c(cRW)[o] > R(0.0) || B.c(cRW + 1)[o] > R(0.0) || B.c(cRW + 2)[o] > R(0.0)) k = it.k + e;
+    }
     for (int of = 16; of > 0; of >>= 1) k = max(k, __shfl_xor_sync(0xffffffffu, k, of));
     if ((threadIdx.x & 31) == 0 && k >= 0) atomicMax(out + it.blk, k);
   });
@@ -1437,9 +1637,8 @@ __global__ void __launch_bounds__(kTileThreads) k_res_bupdate(Dir D) {
 // cells k_pv_uplus refreshes), the Hall diffusion ratios (owned edges) and
 // the fluid fluxes' face JD and 1 / Jac in the real type.
 template <class R>
-__global__ void __launch_bounds__(kTileThreads) k_face_normals(Dir D) {
-  for_items<R, kAlloc>(D, [&](const DevSolve &S, const V<R> &B, const Item &it) {
-    if (!it.in) return;
+__global__ void __launch_bounds__(kVecThreads) k_face_normals(Dir D) {
+  for_positions<R, kAlloc>(D, [&](const DevSolve &S, const VV<R> &B, const Pos &it) {
     {
       // Coefficients of the contravariant velocities (calc_Uplus,
       // Tools.cpp:159-301) on the cells k_pv_uplus refreshes them on: the
@@ -1539,88 +1738,112 @@ __global__ void __launch_bounds__(kTileThreads) k_face_normals(Dir D) {
 }
 
 // calc_PV + calc_Uplus (Z4_Mercury/src/physics/MercurySolver_Tools.cpp:159-301) on the allocated
-// cell range the step keeps, the contravariant velocities UCON and the next
-// step's Hall cell field there, and the next step's CFL dt on owned cells (warp min, one atomicMin per warp on
-// the bit pattern of the positive double).
+// cell range the step keeps, the fluid fluxes' cell terms, the contravariant
+// velocities UCON and the next step's Hall cell field there, and the next
+// step's CFL dt on owned cells (warp min, one atomicMin per warp on the bit
+// pattern of the positive double).
 template <class R>
-__global__ void __launch_bounds__(kTileThreads, MHD_MIN_CTAS_PV) k_pv_uplus(Dir D) {
-  for_items<R, kAlloc>(D, [&](const DevSolve &S, const V<R> &B, const Item &it) {
+__global__ void __launch_bounds__(kVecThreads, 4) k_pv_uplus(Dir D) {
+  for_vec_items<R, kAlloc>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
+    constexpr int N = Vec<R>::N;
     const ConstsT<R> &c = consts_of<R>(S);
-    const int i = it.i, j = it.j, k = it.k;
     R dtl = R(1e100);
     bool bad = false;
-    if (it.in) {
-      R vel[2][3];
-      R chk = R(0.0);  // sum of the conserved components: non-finite if any of them is
+    {
+      const uint32_t o = it.o;
+      auto put = [&](int comp, const Vec<R> &v) { B.st(comp, it, v, it.klo, it.khi); };
+      Vec<R> rho[2], vel[2][3];
+      Vec<R> chk = vset(R(0.0));  // sum of the conserved components: non-finite if any of them is
+#pragma unroll
       for (int s = 0; s < 2; ++s) {
-        const int u0 = s ? cUN : cUH, pv0 = s ? cPVN : cPVH;
+        const int pv0 = s ? cPVN : cPVH, u0 = s ? cUN : cUH;
         const R coeff = s ? c.state_coeff_Na : c.state_coeff_H;
-        const R r0 = LD(u0, i, j, k), m1 = LD(u0 + 1, i, j, k), m2 = LD(u0 + 2, i, j, k), m3 = LD(u0 + 3, i, j, k);
-        const R rho = dmax(r0, R(1e-12));
-        const R u = m1 / rho, v = m2 / rho, w = m3 / rho;
-        const R E = LD(u0 + 4, i, j, k);
-        chk += ((r0 + m1) + (m2 + m3)) + E;
-        const R ke = R(0.5) * rho * (u * u + v * v + w * w);
-        R eint = E - ke;
-        if (eint < R(0.0)) eint = R(0.0);
-        R pr = (c.gamma - R(1.0)) * eint;
-        pr = dmax(pr, R(1e-12));
-        const R T = pr / (rho * coeff);
-        const int o = B.off(i, j, k);
-        // the Rusanov flux's terms of the cell (fluid_cell)
-        B.c(cFT + 2 * s)[o] = pr / (c.gamma - R(1.0)) + R(0.5) * r0 * (u * u + v * v + w * w);
-        B.c(cFT + 2 * s + 1)[o] = sqrt(dmax(R(0.0), c.gamma * pr / dmax(r0, R(1e-30))));
-        B.c(pv0)[o] = u;
-        B.c(pv0 + 1)[o] = v;
-        B.c(pv0 + 2)[o] = w;
-        B.c(pv0 + 3)[o] = pr;
-        B.c(pv0 + 4)[o] = T;
-        vel[s][0] = u;
-        vel[s][1] = v;
-        vel[s][2] = w;
+        const Vec<R> r0 = B.lv(u0, o), m1 = B.lv(u0 + 1, o), m2 = B.lv(u0 + 2, o), m3 = B.lv(u0 + 3, o), E = B.lv(u0 + 4, o);
+        rho[s] = r0;
+        chk = chk + (((r0 + m1) + (m2 + m3)) + E);
+        Vec<R> pr, T, re, cs;
+#pragma unroll
+        for (int e = 0; e < N; ++e) {
+          const R rh = dmax(r0.v[e], R(1e-12));
+          const Divisor<R> by(rh);
+          const R u = by(m1.v[e]), v = by(m2.v[e]), w = by(m3.v[e]);
+          const R u2 = u * u + v * v + w * w;
+          const R ke = R(0.5) * rh * u2;
+          R eint = E.v[e] - ke;
+          if (eint < R(0.0)) eint = R(0.0);
+          const R p = dmax((c.gamma - R(1.0)) * eint, R(1e-12));
+          pr.v[e] = p;
+          // the Rusanov flux's terms of the cell (fluid_cell)
+          if constexpr (sizeof(R) == 4) {
+            T.v[e] = by(p) * c.inv_coeff[s];
+            re.v[e] = p * c.inv_g1 + R(0.5) * r0.v[e] * u2;
+          } else {
+            T.v[e] = p / (rh * coeff);
+            re.v[e] = p / (c.gamma - R(1.0)) + R(0.5) * r0.v[e] * u2;
+          }
+          cs.v[e] = sqrt(dmax(R(0.0), c.gamma * p / dmax(r0.v[e], R(1e-30))));
+          vel[s][0].v[e] = u;
+          vel[s][1].v[e] = v;
+          vel[s][2].v[e] = w;
+        }
+        put(pv0, vel[s][0]);
+        put(pv0 + 1, vel[s][1]);
+        put(pv0 + 2, vel[s][2]);
+        put(pv0 + 3, pr);
+        put(pv0 + 4, T);
+        put(cFT + 2 * s, re);
+        put(cFT + 2 * s + 1, cs);
       }
-      const R rH = dmax(LD(cUH, i, j, k), R(0.0)), rN = dmax(LD(cUN, i, j, k), R(0.0));
-      const Num<R> d = num_limiter(c, rH, rN);
+      const Vec<R> Bx = B.lv(cBC, o), By = B.lv(cBC + 1, o), Bz = B.lv(cBC + 2, o);
+      Vec<R> alpha, up[3];
+#pragma unroll
+      for (int e = 0; e < N; ++e) {
+        const R rH = dmax(rho[0].v[e], R(0.0)), rN = dmax(rho[1].v[e], R(0.0));
+        const Num<R> d = num_limiter(c, rH, rN);
+        alpha.v[e] = c.hall_coef / d.ne_eff;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          const R uH = rH > R(1e-20) ? vel[0][q].v[e] : R(0.0);
+          const R uN = rN > R(1e-20) ? vel[1][q].v[e] : R(0.0);
+          up[q].v[e] = d.chiH * uH + d.chiNa * uN;
+        }
+      }
       {
         // the next step's Hall cell field, BuildHallFaceEMF_Rusanov_diff_ step 1
         // (Z4_Mercury/src/physics/MercurySolver_MagExplicit_Hall.cpp:110-146): its inputs (J_cell,
         // B_cell, the densities) are final here (num_limiter clamps the
-        // densities at zero itself, so d is the limiter of the raw densities)
-        const R alpha = c.hall_coef / d.ne_eff;
-        const R Jx = LD(cJC, i, j, k), Jy = LD(cJC + 1, i, j, k), Jz = LD(cJC + 2, i, j, k);
-        const R Bx = LD(cBC, i, j, k), By = LD(cBC + 1, i, j, k), Bz = LD(cBC + 2, i, j, k);
-        AT(cEHC, i, j, k) = alpha * (Jy * Bz - Jz * By);
-        AT(cEHC + 1, i, j, k) = alpha * (Jz * Bx - Jx * Bz);
-        AT(cEHC + 2, i, j, k) = alpha * (Jx * By - Jy * Bx);
-        AT(cHB, i, j, k) = fabs(alpha) * sqrt(Bx * Bx + By * By + Bz * Bz);
+        // densities at zero itself, so it is the limiter of the raw densities)
+        const Vec<R> Jx = B.lv(cJC, o), Jy = B.lv(cJC + 1, o), Jz = B.lv(cJC + 2, o);
+        put(cEHC, alpha * (Jy * Bz - Jz * By));
+        put(cEHC + 1, alpha * (Jz * Bx - Jx * Bz));
+        put(cEHC + 2, alpha * (Jx * By - Jy * Bx));
+        put(cHB, vabs(alpha) * vsqrt(Bx * Bx + By * By + Bz * Bz));
       }
-      R up[3];
-      for (int q = 0; q < 3; ++q) {
-        const R uH = rH > R(1e-20) ? vel[0][q] : R(0.0);
-        const R uN = rN > R(1e-20) ? vel[1][q] : R(0.0);
-        up[q] = d.chiH * uH + d.chiNa * uN;
-        AT(cUP + q, i, j, k) = up[q];
-      }
-      const int gm = min(c.nghost - 1, kStepGhost);
-      if (i >= -gm && i < B.n0 + gm && j >= -gm && j < B.n1 + gm && k >= -gm && k < B.n2 + gm) {
-        // coefficients (cell-averaged JD, 1 / (|Jac| + 1e-30)) from k_face_normals
-        const R inv_jac = LD(cUCK + 9, i, j, k);
 #pragma unroll
-        for (int axis = 0; axis < 3; ++axis) {
-          const R kx = LD(cUCK + 3 * axis, i, j, k), ky = LD(cUCK + 3 * axis + 1, i, j, k),
-                  kz = LD(cUCK + 3 * axis + 2, i, j, k);
-          AT(cUC + axis, i, j, k) = (kx * up[0] + ky * up[1] + kz * up[2]) * inv_jac;
-        }
+      for (int q = 0; q < 3; ++q) put(cUP + q, up[q]);
+      const int gm = min(c.nghost - 1, kStepGhost);
+      const bool near = it.i >= -gm && it.i < B.n0 + gm && it.j >= -gm && it.j < B.n1 + gm;
+      {
+        // coefficients (cell-averaged JD, 1 / (|Jac| + 1e-30)) from k_face_normals
+        const Vec<R> inv_jac = B.lv(cUCK + 9, o);
+#pragma unroll
+        for (int axis = 0; axis < 3; ++axis)
+          B.st(cUC + axis, it,
+               (B.lv(cUCK + 3 * axis, o) * up[0] + B.lv(cUCK + 3 * axis + 1, o) * up[1] +
+                B.lv(cUCK + 3 * axis + 2, o) * up[2]) *
+                   inv_jac,
+               max(it.klo, -gm), min(it.khi, B.n2 + gm), near);
       }
-      if (i >= 0 && i < B.n0 && j >= 0 && j < B.n1 && k >= 0 && k < B.n2) {
-        dtl = cell_dt(B, c, i, j, k);
-        // a NaN drops out of the minimum below (and the pressure floors can
-        // hide a non-finite energy from it): record it instead
-        bad = !isfinite(dtl) || !isfinite(chk);
+      const bool own = it.in && it.i >= 0 && it.i < B.n0 && it.j >= 0 && it.j < B.n1;
+      if (__any_sync(0xffffffffu, own)) {
+        dtl = cells_dt(B, c, it, own, Bx, By, Bz, bad);
+        // the pressure floors can hide a non-finite energy from the dt
+#pragma unroll
+        for (int e = 0; e < N; ++e) bad = bad || (own && it.k + e >= 0 && it.k + e < B.n2 && !isfinite(chk.v[e]));
       }
     }
     // warp minimum, one atomicMin per warp (min is exact in any order)
-    for (int o = 16; o > 0; o >>= 1) dtl = dmin(dtl, __shfl_xor_sync(0xffffffffu, dtl, o));
+    for (int w = 16; w > 0; w >>= 1) dtl = dmin(dtl, __shfl_xor_sync(0xffffffffu, dtl, w));
     if ((threadIdx.x & 31) == 0 && dtl < R(1e100))
       atomicMin(&D.state[it.s].dt_bits, (unsigned long long)__double_as_longlong(dtl));
     if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicExch(&D.state[it.s].nonfinite, 1);
@@ -1628,8 +1851,7 @@ __global__ void __launch_bounds__(kTileThreads, MHD_MIN_CTAS_PV) k_pv_uplus(Dir 
 }
 
 #undef AT
-#undef LD
-#undef LDM
+#undef ATM
 
 // ------------------------------------------------------------------ sync, alias, bookkeeping
 __device__ __forceinline__ int find_solve(const int *prefix, int nsolves, int e) {
@@ -2042,7 +2264,7 @@ __global__ void k_retire(Dir D) {
 
 // ------------------------------------------------------------------ launchers
 // Every range kernel is persistent (grid-stride over tiles): its grid is the
-// SM count times the CTAs of it that fit on one SM (at most 8), so all CTAs
+// SM count times the CTAs of it that fit on one SM, so all CTAs
 // are resident at once and none starts in a late partial wave.  The
 // residual-dot kernel keeps a fixed grid: its partial sums are indexed by CTA.
 static int g_grid_tiles = 0;
@@ -2101,6 +2323,16 @@ static const void *kernel_fn(StepKernel k) {
   }
 }
 
+// Threads of a kernel's CTAs.
+static int kernel_threads(StepKernel k) {
+  switch (k) {
+    case SK_FACE_EMF: case SK_EDGE_EMF: case SK_HALL_EDGE: case SK_ADD_HALL: case SK_BFACE: case SK_BCELL_JEDGE:
+    case SK_JCELL: case SK_PV_UPLUS: case SK_FACE_NORMALS: case SK_DIVB: case SK_RES_SEED: case SK_RES_W:
+      return kVecThreads;
+    default: return kTileThreads;
+  }
+}
+
 static std::once_flag g_grids_once;
 
 template <class R>
@@ -2111,12 +2343,12 @@ static void grids_init() {
   for (int k = 0; k < SK_COUNT; ++k) {
     int per_sm = 8;
     const void *fn = kernel_fn<R>((StepKernel)k);
-    if (fn && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kTileThreads, 0) != cudaSuccess ||
+    if (fn && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kernel_threads((StepKernel)k), 0) != cudaSuccess ||
                per_sm < 1)) {
       cudaGetLastError();
       per_sm = 1;
     }
-    g_grid_kernel[k] = sms * (per_sm < 8 ? per_sm : 8);
+    g_grid_kernel[k] = sms * per_sm;
   }
   for (int v = 0; v < kNumFluidTiles; ++v) {
     int per_sm = 1;
@@ -2140,20 +2372,20 @@ static void launch_as(StepKernel k, const Dir &D, cudaStream_t st, const SyncOps
                       ResScratch rs) {
   const int G = g_grid_kernel[k];
   switch (k) {
-    case SK_FACE_EMF: k_face_emf<R><<<G, kTileThreads, 0, st>>>(D); break;
-    case SK_EDGE_EMF: k_edge_emf<R><<<G, kTileThreads, 0, st>>>(D); break;
-    case SK_HALL_EDGE: k_hall_edge<R><<<G, kTileThreads, 0, st>>>(D); break;
-    case SK_ADD_HALL: k_add_hall<R><<<G, kTileThreads, 0, st>>>(D); break;
+    case SK_FACE_EMF: k_face_emf<R><<<G, kVecThreads, 0, st>>>(D); break;
+    case SK_EDGE_EMF: k_edge_emf<R><<<G, kVecThreads, 0, st>>>(D); break;
+    case SK_HALL_EDGE: k_hall_edge<R><<<G, kVecThreads, 0, st>>>(D); break;
+    case SK_ADD_HALL: k_add_hall<R><<<G, kVecThreads, 0, st>>>(D); break;
     case SK_FLUID: launch_fluid<R>(iarg, D, st); break;  // iarg: the tile variant
-    case SK_BFACE: k_bface<R><<<G, kTileThreads, 0, st>>>(D); break;
-    case SK_BCELL_JEDGE: k_bcell_jedge<R><<<G, kTileThreads, 0, st>>>(D); break;
-    case SK_JCELL: k_jcell<R><<<G, kTileThreads, 0, st>>>(D); break;
-    case SK_PV_UPLUS: k_pv_uplus<R><<<G, kTileThreads, 0, st>>>(D); break;
+    case SK_BFACE: k_bface<R><<<G, kVecThreads, 0, st>>>(D); break;
+    case SK_BCELL_JEDGE: k_bcell_jedge<R><<<G, kVecThreads, 0, st>>>(D); break;
+    case SK_JCELL: k_jcell<R><<<G, kVecThreads, 0, st>>>(D); break;
+    case SK_PV_UPLUS: k_pv_uplus<R><<<G, kVecThreads, 0, st>>>(D); break;
     case SK_SYNC: k_sync<R><<<G, kTileThreads, 0, st>>>(D, *ops); break;
-    case SK_FACE_NORMALS: k_face_normals<R><<<G, kTileThreads, 0, st>>>(D); break;
-    case SK_DIVB: k_div_b<R><<<G, kTileThreads, 0, st>>>(D); break;
-    case SK_RES_SEED: k_res_seed<R><<<G, kTileThreads, 0, st>>>(D); break;
-    case SK_RES_W: k_res_w<R><<<G, kTileThreads, 0, st>>>(D); break;
+    case SK_FACE_NORMALS: k_face_normals<R><<<G, kVecThreads, 0, st>>>(D); break;
+    case SK_DIVB: k_div_b<R><<<G, kVecThreads, 0, st>>>(D); break;
+    case SK_RES_SEED: k_res_seed<R><<<G, kVecThreads, 0, st>>>(D); break;
+    case SK_RES_W: k_res_w<R><<<G, kVecThreads, 0, st>>>(D); break;
     case SK_RES_VEC: k_res_vec<R><<<G, kTileThreads, 0, st>>>(D, iarg); break;
     case SK_RES_DB: k_res_db<R><<<G, kTileThreads, 0, st>>>(D); break;
     case SK_RES_DJ: k_res_dj<R><<<G, kTileThreads, 0, st>>>(D); break;
@@ -2244,7 +2476,7 @@ void init_launch_grids_f32() { grids<float>(); }
 
 void launch_res_kmax_f32(const Dir &D, int *out, cudaStream_t st) {
   grids<float>();
-  k_res_kmax<float><<<g_grid_tiles, kTileThreads, 0, st>>>(D, out);
+  k_res_kmax<float><<<g_grid_tiles, kVecThreads, 0, st>>>(D, out);
 }
 #else
 void launch_res_kmax_f32(const Dir &D, int *out, cudaStream_t st);
@@ -2254,7 +2486,7 @@ void launch_res_kmax(const Dir &D, int precision, int *out, cudaStream_t st) {
     launch_res_kmax_f32(D, out, st);
   } else {
     grids<double>();
-    k_res_kmax<double><<<g_grid_tiles, kTileThreads, 0, st>>>(D, out);
+    k_res_kmax<double><<<g_grid_tiles, kVecThreads, 0, st>>>(D, out);
   }
 }
 
