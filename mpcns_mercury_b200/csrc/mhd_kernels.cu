@@ -75,7 +75,7 @@ __device__ __forceinline__ R dmin(R a, R b) { return (b < a) ? b : a; }
 // block's component arrays below 2^31 elements in total).
 template <class R>
 struct V {
-  char *U, *Un, *M, *Mr;
+  char *U, *Un, *M, *Mr;  // U, Un: the current and the other buffer
   uint32_t tb;  // bytes of one real-valued component array
   int total, si, sj;
   int G, n0, n1, n2;
@@ -110,6 +110,15 @@ struct Item {
   int hi[3];   // range upper bounds (exclusive)
   int lo[3];   // range lower bounds
 };
+
+// Programmatic dependent launch: the kernels of a step are launched while their
+// predecessor drains (launch_dependent).  A kernel first looks its first tile
+// up in the directory, which nothing writes during a step, then waits until
+// every earlier kernel has completed and its writes are visible.  CTAs without
+// work may leave before the wait, but never CTA 0: a kernel must not complete
+// before its predecessor has.
+__device__ __forceinline__ void let_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void wait_for_predecessors() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 struct NoTileEnd {
   __device__ void operator()(int) const {}
@@ -216,13 +225,19 @@ __device__ __forceinline__ void build_item(const Dir &D, int s, int b, int t, It
 template <class R, int KIND, class F, class E = NoTileEnd>
 __device__ __forceinline__ void for_items(const Dir &D, F &&f, E &&end = E{}) {
   __shared__ int sh[3];
+  let_dependents_launch();
   const int total = D.solve_tile_prefix[KIND][D.nsolves];
   const int tid = threadIdx.x;
+  if ((int)blockIdx.x >= total) {
+    if (blockIdx.x == 0) wait_for_predecessors();
+    return;
+  }
   for (int w = blockIdx.x; w < total; w += gridDim.x) {
     if (tid == 0) lookup_item<KIND>(D, w, sh[0], sh[1], sh[2]);
     __syncthreads();
     const int s = sh[0], b = sh[1], t = sh[2];
     __syncthreads();
+    if (w == (int)blockIdx.x) wait_for_predecessors();
     if (!solve_active(D, s)) continue;  // inactive solve (the whole CTA agrees)
     Item it;
     V<R> B;
@@ -372,7 +387,7 @@ __device__ __forceinline__ void build_vec_item(const Dir &D, int s, int b, int t
   const DevSolve &S = D.solves[s];
   const DevBlock &DB = S.blocks[b];
   const RangeBox r = range_of(KIND, DB.n, S.c.nghost);
-  set_view(B, DB, D.state[s].cur);
+  set_view(B, DB, 0);  // the buffers of cur = 0: use_current after the state can be read
   B.U = uniform(B.U);
   B.Un = uniform(B.Un);
   B.M = uniform(B.M);
@@ -404,25 +419,39 @@ __device__ __forceinline__ void build_vec_item(const Dir &D, int s, int b, int t
   it.o = (uint32_t)B.off(it.i, it.j, it.k) * (uint32_t)sizeof(R);
 }
 
+template <class R>
+__device__ __forceinline__ void use_current(V<R> &B, int cur) {
+  char *const a = B.U, *const b = B.Un;
+  B.U = cur ? b : a;
+  B.Un = cur ? a : b;
+}
+
 // Work-item loop over the vector ranges: f(S, B, item) for every tile of
 // range KIND of every active solve.  Thread 0 looks the next tile up while the
 // CTA works on the current one (one barrier per tile).
 template <class R, int KIND, class F>
 __device__ __forceinline__ void for_vec_items(const Dir &D, F &&f) {
   __shared__ int sh[2][3];
+  let_dependents_launch();
   const int total = D.solve_tile_prefix[KIND][D.nsolves];
   int w = blockIdx.x, p = 0;
-  if (threadIdx.x == 0 && w < total) lookup_item<KIND>(D, w, sh[0][0], sh[0][1], sh[0][2]);
+  if (w >= total) {
+    if (w == 0) wait_for_predecessors();
+    return;
+  }
+  if (threadIdx.x == 0) lookup_item<KIND>(D, w, sh[0][0], sh[0][1], sh[0][2]);
   __syncthreads();
   for (; w < total; w += gridDim.x, p ^= 1) {
     const int s = uniform(sh[p][0]), b = uniform(sh[p][1]), t = uniform(sh[p][2]);
     if (threadIdx.x == 0 && w + (int)gridDim.x < total)
       lookup_item<KIND>(D, w + gridDim.x, sh[p ^ 1][0], sh[p ^ 1][1], sh[p ^ 1][2]);
     __syncwarp();
+    VItem it;
+    VV<R> B;
+    build_vec_item<R, KIND>(D, s, b, t, it, B);
+    if (w == (int)blockIdx.x) wait_for_predecessors();
     if (uniform((int)solve_active(D, s))) {
-      VItem it;
-      VV<R> B;
-      build_vec_item<R, KIND>(D, s, b, t, it, B);
+      use_current(B, uniform(D.state[s].cur));
       f(D.solves[s], B, it);
     }
     __syncthreads();
@@ -841,15 +870,21 @@ template <class R, int VT>
 __global__ void __launch_bounds__(fluid_threads(VT), fluid_ctas(VT, sizeof(R))) k_fluid(Dir D) {
   constexpr int KIND = fluid_kind(VT), NS = fluid_species(sizeof(R)), TI = fluid_tile(VT).i;
   __shared__ int sh[3];
+  let_dependents_launch();
   const int items = D.solve_tile_prefix[KIND][D.nsolves] / NS;
   const int split = items < (int)gridDim.x ? TI : 1;
   const int li = TI / split;
+  if ((int)blockIdx.x >= items * split) {
+    if (blockIdx.x == 0) wait_for_predecessors();
+    return;
+  }
   for (int q = blockIdx.x; q < items * split; q += gridDim.x) {
     const int part = q % split;
     if (threadIdx.x == 0) lookup_item<KIND>(D, q / split * NS, sh[0], sh[1], sh[2]);
     __syncthreads();
     const int is = sh[0], ib = sh[1], t = sh[2];
     __syncthreads();
+    if (q == (int)blockIdx.x) wait_for_predecessors();
     if (!solve_active(D, is)) continue;  // inactive solve (the whole CTA agrees)
     Item it;
     V<R> B;
@@ -1495,6 +1530,8 @@ __global__ void __launch_bounds__(kTileThreads) k_res_cg_sum(Dir D, int op, cons
                                                              ResCtl *ctl, double *chunks, unsigned int *sarr,
                                                              cudaGraphConditionalHandle handle, int in_graph) {
   __shared__ double sh[2][kWarpsPerTile];
+  let_dependents_launch();
+  wait_for_predecessors();
   const int s = blockIdx.x / kCgChunks, c = blockIdx.x % kCgChunks;
   const bool act = s < D.nsolves && solve_active(D, s);  // the whole CTA agrees
   bool last_of_solve = false;
@@ -1885,22 +1922,37 @@ __global__ void __launch_bounds__(256) k_sync(Dir D, SyncOps ops) {
   const int stride = (gridDim.x * blockDim.x) >> 3;
   const int *pre0 = op_prefix(D, ops.op[0]);
   const int *pre1 = ops.n > 1 ? op_prefix(D, ops.op[1]) : nullptr;
+  let_dependents_launch();
   const int t0 = pre0[D.nsolves];
   const int total = t0 + (pre1 ? pre1[D.nsolves] : 0);
+  bool first = true;
+  if (((int)(blockIdx.x * blockDim.x) >> 3) >= total) {
+    if (blockIdx.x == 0) wait_for_predecessors();
+    return;
+  }
   for (int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; g < total; g += stride) {
     const bool second = g >= t0;
     const SyncOp &op = second ? ops.op[1] : ops.op[0];
     const int *pre = second ? pre1 : pre0;
     const int e = second ? g - t0 : g;
     const int s = find_solve(pre, D.nsolves, e);
-    if (!solve_active(D, s)) continue;
     const DevSolve &S = D.solves[s];
     const int q = e - pre[s];
+    const bool copy = op.kind == SYNC_COPY;
+    const DevAlias &A = op.arg ? S.aliasJ : S.aliasE;
+    // the tables are as static as the directory
+    int64_t dcode = 0, scode = 0, rw = 0;
+    if (copy) {
+      const int64_t *w = S.tab[op.arg][op.phase].seg + kSegWords * (int64_t)q;
+      dcode = w[0];
+      scode = w[1];
+      rw = w[2];
+    }
+    if (first) wait_for_predecessors();
+    first = false;
+    if (!solve_active(D, s)) continue;
     const int cur = D.state[s].cur;
-    if (op.kind == SYNC_COPY) {
-      const DevTable &T = S.tab[op.arg][op.phase];
-      const int64_t *w = T.seg + kSegWords * (int64_t)q;
-      const int64_t dcode = w[0], scode = w[1], rw = w[2];
+    if (copy) {
       const int len = (int)((dcode >> kSegLenShift) & 31) + 1;
       const int n = len * ((int)(rw & 0xffff) + 1);
       const int64_t stride = rw >> kSegStrideShift;  // bytes between runs
@@ -1923,7 +1975,6 @@ __global__ void __launch_bounds__(256) k_sync(Dir D, SyncOps ops) {
       for (int u = 0; u < kSegElems / 8; ++u)
         if (lane + 8 * u < n) *(R *)(dst + off[u]) = op.mark ? R(0.0) : (neg ? -v[u] : v[u]);
     } else {
-      const DevAlias &A = op.arg ? S.aliasJ : S.aliasE;
       const int c = q * 8 + lane;
       if (c < A.n) {
         R sum = R(0.0);
@@ -1954,8 +2005,10 @@ __device__ __forceinline__ V<R> block_view(const Dir &D, int s, int b) {
 // writes, so they run in any order.
 template <class R>
 __global__ void __launch_bounds__(256) k_phys(Dir D, int which) {
+  let_dependents_launch();
   const int *pre = D.phys_prefix[which];
   const int total = pre[D.nsolves];
+  wait_for_predecessors();
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   // a warp takes 32 consecutive operations, one per lane; the constant
@@ -2041,7 +2094,9 @@ __global__ void __launch_bounds__(256) k_phys(Dir D, int which) {
 // One thread per singular edge of every active solve.
 template <class F>
 __device__ __forceinline__ void for_singular(const Dir &D, F &&f) {
+  let_dependents_launch();
   const int total = D.sing_prefix[D.nsolves];
+  wait_for_predecessors();
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
     const int s = find_solve(D.sing_prefix, D.nsolves, e);
     if (!solve_active(D, s)) continue;
@@ -2230,6 +2285,8 @@ __global__ void k_sing_j(Dir D) {
 // (Z4_Mercury/src/MercurySolver_Driver.cpp:40-45), record a dt failure (the
 // reference's exit(-1), Timestep.cpp:129-140) and re-arm the dt reduction.
 __global__ void k_flip(Dir D) {
+  let_dependents_launch();
+  wait_for_predecessors();
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < D.nsolves; s += gridDim.x * blockDim.x) {
     SolveState &st = D.state[s];
     if (!st.remaining) continue;
@@ -2254,6 +2311,8 @@ __global__ void k_flip(Dir D) {
 
 // End of a step: one step fewer to go (after every pass of the step has run).
 __global__ void k_retire(Dir D) {
+  let_dependents_launch();
+  wait_for_predecessors();
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < D.nsolves; s += gridDim.x * blockDim.x) {
     SolveState &st = D.state[s];
     if (st.remaining > 0) st.remaining -= 1;
@@ -2271,6 +2330,28 @@ static int g_grid_tiles = 0;
 static int g_grid_kernel[SK_COUNT];
 static int g_grid_fluid[kNumFluidTiles];  // the fluid kernel's, per tile variant
 
+template <class T>
+struct SameAs {
+  using type = T;
+};
+template <class T>
+using Same = typename SameAs<T>::type;
+// A launch that may begin while its predecessor in the stream drains; the kernel
+// waits itself (wait_for_predecessors).
+template <class... P>
+static void launch_dependent(void (*fn)(P...), int grid, int threads, cudaStream_t st, Same<P>... args) {
+  cudaLaunchAttribute a[1];
+  a[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.stream = st;
+  cfg.attrs = a;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, fn, args...);
+}
+
 template <class R>
 static const void *fluid_fn(int v) {
   switch (v) {
@@ -2287,8 +2368,7 @@ static_assert(kNumFluidTiles == 7, "fluid_fn lists every variant");
 template <class R>
 static void launch_fluid(int v, const Dir &D, cudaStream_t st) {
   v = (v >= 0 && v < kNumFluidTiles) ? v : 0;
-  void *args[] = {(void *)&D};
-  cudaLaunchKernel(fluid_fn<R>(v), dim3(g_grid_fluid[v]), dim3(fluid_threads(v)), args, 0, st);
+  launch_dependent((void (*)(Dir))fluid_fn<R>(v), g_grid_fluid[v], fluid_threads(v), st, D);
 }
 
 template <class R>
@@ -2372,44 +2452,44 @@ static void launch_as(StepKernel k, const Dir &D, cudaStream_t st, const SyncOps
                       ResScratch rs) {
   const int G = g_grid_kernel[k];
   switch (k) {
-    case SK_FACE_EMF: k_face_emf<R><<<G, kVecThreads, 0, st>>>(D); break;
-    case SK_EDGE_EMF: k_edge_emf<R><<<G, kVecThreads, 0, st>>>(D); break;
-    case SK_HALL_EDGE: k_hall_edge<R><<<G, kVecThreads, 0, st>>>(D); break;
-    case SK_ADD_HALL: k_add_hall<R><<<G, kVecThreads, 0, st>>>(D); break;
+    case SK_FACE_EMF: launch_dependent(k_face_emf<R>, G, kVecThreads, st, D); break;
+    case SK_EDGE_EMF: launch_dependent(k_edge_emf<R>, G, kVecThreads, st, D); break;
+    case SK_HALL_EDGE: launch_dependent(k_hall_edge<R>, G, kVecThreads, st, D); break;
+    case SK_ADD_HALL: launch_dependent(k_add_hall<R>, G, kVecThreads, st, D); break;
     case SK_FLUID: launch_fluid<R>(iarg, D, st); break;  // iarg: the tile variant
-    case SK_BFACE: k_bface<R><<<G, kVecThreads, 0, st>>>(D); break;
-    case SK_BCELL_JEDGE: k_bcell_jedge<R><<<G, kVecThreads, 0, st>>>(D); break;
-    case SK_JCELL: k_jcell<R><<<G, kVecThreads, 0, st>>>(D); break;
-    case SK_PV_UPLUS: k_pv_uplus<R><<<G, kVecThreads, 0, st>>>(D); break;
-    case SK_SYNC: k_sync<R><<<G, kTileThreads, 0, st>>>(D, *ops); break;
+    case SK_BFACE: launch_dependent(k_bface<R>, G, kVecThreads, st, D); break;
+    case SK_BCELL_JEDGE: launch_dependent(k_bcell_jedge<R>, G, kVecThreads, st, D); break;
+    case SK_JCELL: launch_dependent(k_jcell<R>, G, kVecThreads, st, D); break;
+    case SK_PV_UPLUS: launch_dependent(k_pv_uplus<R>, G, kVecThreads, st, D); break;
+    case SK_SYNC: launch_dependent(k_sync<R>, G, kTileThreads, st, D, *ops); break;
     case SK_FACE_NORMALS: k_face_normals<R><<<G, kVecThreads, 0, st>>>(D); break;
     case SK_DIVB: k_div_b<R><<<G, kVecThreads, 0, st>>>(D); break;
     case SK_RES_SEED: k_res_seed<R><<<G, kVecThreads, 0, st>>>(D); break;
     case SK_RES_W: k_res_w<R><<<G, kVecThreads, 0, st>>>(D); break;
-    case SK_RES_VEC: k_res_vec<R><<<G, kTileThreads, 0, st>>>(D, iarg); break;
-    case SK_RES_DB: k_res_db<R><<<G, kTileThreads, 0, st>>>(D); break;
-    case SK_RES_DJ: k_res_dj<R><<<G, kTileThreads, 0, st>>>(D); break;
-    case SK_RES_Q: k_res_q<R><<<G, kTileThreads, 0, st>>>(D); break;
+    case SK_RES_VEC: launch_dependent(k_res_vec<R>, G, kTileThreads, st, D, iarg); break;
+    case SK_RES_DB: launch_dependent(k_res_db<R>, G, kTileThreads, st, D); break;
+    case SK_RES_DJ: launch_dependent(k_res_dj<R>, G, kTileThreads, st, D); break;
+    case SK_RES_Q: launch_dependent(k_res_q<R>, G, kTileThreads, st, D); break;
     case SK_RES_DOT: k_res_dot<R><<<g_grid_tiles, kTileThreads, 0, st>>>(D, rs.partial); break;
     case SK_RES_SUM: k_res_sum<<<1, 32, 0, st>>>(rs.partial, g_grid_tiles, rs.result); break;
-    case SK_RES_COPYB: k_res_copyb<R><<<G, kTileThreads, 0, st>>>(D, iarg); break;
-    case SK_RES_BUPDATE: k_res_bupdate<R><<<G, kTileThreads, 0, st>>>(D); break;
+    case SK_RES_COPYB: launch_dependent(k_res_copyb<R>, G, kTileThreads, st, D, iarg); break;
+    case SK_RES_BUPDATE: launch_dependent(k_res_bupdate<R>, G, kTileThreads, st, D); break;
     case SK_RES_CG:
-      k_res_cg<R><<<g_grid_tiles, kTileThreads, 0, st>>>(D, iarg, rs.tpartial, rs.cg, rs.handle, rs.in_graph);
+      launch_dependent(k_res_cg<R>, g_grid_tiles, kTileThreads, st, D, iarg, rs.tpartial, rs.cg, rs.handle, rs.in_graph);
       break;
     case SK_RES_CGSUM:
-      k_res_cg_sum<<<D.nsolves * kCgChunks, kTileThreads, 0, st>>>(D, iarg, rs.tpartial, rs.cg, rs.ctl, rs.chunks,
-                                                                   rs.sarrivals, rs.handle, rs.in_graph);
+      launch_dependent(k_res_cg_sum, D.nsolves * kCgChunks, kTileThreads, st, D, iarg, rs.tpartial, rs.cg, rs.ctl, rs.chunks,
+                       rs.sarrivals, rs.handle, rs.in_graph);
       break;
-    case SK_RES_PUPD_E: k_res_pupd_e<R><<<G, kTileThreads, 0, st>>>(D, rs.cg); break;
-    case SK_FLIP: k_flip<<<1, 128, 0, st>>>(D); break;
-    case SK_RETIRE: k_retire<<<1, 128, 0, st>>>(D); break;
-    case SK_PHYS: k_phys<R><<<G, 256, 0, st>>>(D, iarg); break;
+    case SK_RES_PUPD_E: launch_dependent(k_res_pupd_e<R>, G, kTileThreads, st, D, rs.cg); break;
+    case SK_FLIP: launch_dependent(k_flip, 1, 128, st, D); break;
+    case SK_RETIRE: launch_dependent(k_retire, 1, 128, st, D); break;
+    case SK_PHYS: launch_dependent(k_phys<R>, G, 256, st, D, iarg); break;
     // one thread per singular edge (8 radial lines of nr edges per shell)
     case SK_SING_SETUP: k_sing_setup<R><<<g_grid_tiles / 2, 64, 0, st>>>(D); break;
-    case SK_SING_EMF: k_sing_emf<R><<<g_grid_tiles / 2, 64, 0, st>>>(D); break;
-    case SK_SING_J: k_sing_j<R><<<g_grid_tiles / 2, 64, 0, st>>>(D); break;
-    case SK_RES_CLEARB: k_res_clearb<R><<<G, kTileThreads, 0, st>>>(D); break;
+    case SK_SING_EMF: launch_dependent(k_sing_emf<R>, g_grid_tiles / 2, 64, st, D); break;
+    case SK_SING_J: launch_dependent(k_sing_j<R>, g_grid_tiles / 2, 64, st, D); break;
+    case SK_RES_CLEARB: launch_dependent(k_res_clearb<R>, G, kTileThreads, st, D); break;
     default: break;
   }
 }
@@ -2463,7 +2543,7 @@ __global__ void __launch_bounds__(kTileThreads) k_res_cross(Dir D, int op) {
 void launch_res_cross(const Dir &D, int op, cudaStream_t st) {
   grids<float>();
   if (op == RES_X_STATIC) k_res_cross<kFull><<<g_grid_tiles, kTileThreads, 0, st>>>(D, op);
-  else k_res_cross<kResK><<<g_grid_tiles, kTileThreads, 0, st>>>(D, op);
+  else launch_dependent(k_res_cross<kResK>, g_grid_tiles, kTileThreads, st, D, op);
 }
 
 void launch_step_kernel_f32(StepKernel k, const Dir &D, cudaStream_t st, const SyncOps *ops, int iarg, double darg,
