@@ -1100,7 +1100,7 @@ void res_apply(mhd_batch *b, int *nk) {
 }
 
 // The CG iteration loop of every masked solve as one CUDA graph: k_res_cg
-// and k_res_cg_sum (CG_INIT) set the loop condition, then a conditional
+// (CG_INIT) sets the loop condition, then a conditional
 // WHILE node repeats the iteration (operator, q and (p.q)_W, the x / r update
 // and the stop test, the direction update) while some solve's device CG
 // state says it is still running; a solve whose loop ends leaves the mask.
@@ -1127,20 +1127,12 @@ int build_cg_graph(mhd_batch *b) {
       cudaSuccess)
     return fin(e, "capture");
   launch(b, 1, SK_RES_CG, &nk, nullptr, CG_INIT);
-  launch(b, 1, SK_RES_CGSUM, &nk, nullptr, CG_INIT);
   if ((e = cudaStreamEndCapture(b->stream, &g)) != cudaSuccess) return fin(e, "capture");
-  // the loop node follows the chain's last node
-  cudaGraphNode_t nodes[2] = {};
-  size_t n = 2;
-  if ((e = cudaGraphGetNodes(g, nodes, &n)) != cudaSuccess || n != 2)
-    return fin(e != cudaSuccess ? e : cudaErrorUnknown, "init nodes");
+  // the loop node follows the start
   cudaGraphNode_t init = nullptr;
-  for (cudaGraphNode_t c : nodes) {
-    size_t nd = 0;
-    if ((e = cudaGraphNodeGetDependentNodes(c, nullptr, &nd)) != cudaSuccess) return fin(e, "init nodes");
-    if (nd == 0) init = c;
-  }
-  if (!init) return fin(cudaErrorUnknown, "init nodes");
+  size_t n = 1;
+  if ((e = cudaGraphGetNodes(g, &init, &n)) != cudaSuccess || n != 1)
+    return fin(e != cudaSuccess ? e : cudaErrorUnknown, "init node");
   cudaGraphNodeParams p{};
   p.type = cudaGraphNodeTypeConditional;
   p.conditional.handle = h;
@@ -1154,9 +1146,7 @@ int build_cg_graph(mhd_batch *b) {
     return fin(e, "body capture");
   res_apply_core(b, &nk);
   launch(b, 1, SK_RES_CG, &nk, nullptr, CG_PQ);
-  launch(b, 1, SK_RES_CGSUM, &nk, nullptr, CG_PQ);
   launch(b, 1, SK_RES_CG, &nk, nullptr, CG_RR);
-  launch(b, 1, SK_RES_CGSUM, &nk, nullptr, CG_RR);
   launch(b, 1, SK_RES_PUPD_E, &nk);
   if ((e = cudaStreamEndCapture(b->stream, &body)) != cudaSuccess) return fin(e, "body capture");
   e = cudaGraphInstantiate(&b->graph_cg, g, 0);
@@ -1170,14 +1160,14 @@ int build_cg_graph(mhd_batch *b) {
   return MHD_OK;
 }
 
-// The per-warp tile partials of the batched CG: 2 doubles per warp of every
+// The tile partials of the batched CG: 2 doubles per
 // kResK tile of the batch's solves (grown on demand; the loop graph holds the
 // pointer, so a new buffer means a new graph).
 int ensure_tpartial(mhd_batch *b) {
   size_t tiles = 0;
   for (int s = 0; s < b->capacity; ++s)
     if (const Solve *S = b->slots[s]) tiles += (size_t)(S->dres_prefix ? S->res_tiles : S->T->tiles[kResK]);
-  const size_t need = std::max<size_t>(tiles, 1) * kWarpsPerTile * 2;
+  const size_t need = std::max<size_t>(tiles, 1) * 2;
   if (need <= b->tpart_elems) return MHD_OK;
   CUDA_TRY(cudaStreamSynchronize(b->stream));  // no loop graph in flight
   if (b->graph_cg) {
@@ -1236,7 +1226,6 @@ int res_cg_batch(mhd_batch *b, const std::vector<CgJob> &jobs) {
   } else {  // the same kernels launched from the host, the states read back after every iteration
     int nk = 0;
     launch(b, 1, SK_RES_CG, &nk, nullptr, CG_INIT);
-    launch(b, 1, SK_RES_CGSUM, &nk, nullptr, CG_INIT);
     for (;;) {
       CUDA_TRY(cudaMemcpyAsync(b->hcg, b->res.cg, sizeof(ResCG) * b->capacity, cudaMemcpyDeviceToHost, b->stream));
       CUDA_TRY(cudaStreamSynchronize(b->stream));
@@ -1245,9 +1234,7 @@ int res_cg_batch(mhd_batch *b, const std::vector<CgJob> &jobs) {
       if (!running) break;  // every solve's loop ends by its own max_it at the latest
       res_apply_core(b, &nk);
       launch(b, 1, SK_RES_CG, &nk, nullptr, CG_PQ);
-      launch(b, 1, SK_RES_CGSUM, &nk, nullptr, CG_PQ);
       launch(b, 1, SK_RES_CG, &nk, nullptr, CG_RR);
-      launch(b, 1, SK_RES_CGSUM, &nk, nullptr, CG_RR);
       launch(b, 1, SK_RES_PUPD_E, &nk);
     }
   }
@@ -1497,9 +1484,6 @@ int mhd_batch_create(int capacity, int precision, mhd_batch **out) {
   if (cudaMalloc(&b->res.partial, sizeof(double) * 2 * res_dot_grid()) != cudaSuccess ||
       cudaMalloc(&b->res.result, sizeof(double) * 2) != cudaSuccess ||
       cudaMalloc(&b->res.cg, sizeof(ResCG) * capacity) != cudaSuccess ||
-      cudaMalloc(&b->res.ctl, sizeof(ResCtl)) != cudaSuccess ||
-      cudaMemsetAsync(b->res.ctl, 0, sizeof(ResCtl), b->stream) != cudaSuccess ||
-      cudaMalloc(&b->res.chunks, sizeof(double) * 2 * kCgChunks * capacity) != cudaSuccess ||
       cudaMalloc(&b->res.sarrivals, sizeof(unsigned int) * capacity) != cudaSuccess ||
       cudaMemsetAsync(b->res.sarrivals, 0, sizeof(unsigned int) * capacity, b->stream) != cudaSuccess ||
       cudaMallocHost(&b->hres, sizeof(double) * 2) != cudaSuccess ||
@@ -1527,8 +1511,6 @@ int mhd_batch_destroy(mhd_batch *b) {
   cudaFree(b->res.partial);
   cudaFree(b->res.result);
   cudaFree(b->res.cg);
-  cudaFree(b->res.ctl);
-  cudaFree(b->res.chunks);
   cudaFree(b->res.sarrivals);
   cudaFree(b->res.tpartial);
   if (b->hres) cudaFreeHost(b->hres);

@@ -331,7 +331,7 @@ __host__ __device__ inline RangeBox range_of(int kind, const int n[3], int g) {
 // The vector ranges: their passes take 16-byte groups of consecutive k
 // positions (mhd_kernels.cu, Vec).
 __host__ __device__ constexpr bool vector_kind(int kind) {
-  return kind == kCells || kind == kBox || kind == kExt || kind == kAlloc;
+  return kind == kCells || kind == kBox || kind == kExt || kind == kAlloc || kind == kResK;
 }
 // The aligned 16-byte groups of a row that hold positions of the range.
 struct RowGroups {

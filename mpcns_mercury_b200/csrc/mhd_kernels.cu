@@ -120,10 +120,6 @@ struct Item {
 __device__ __forceinline__ void let_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void wait_for_predecessors() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-struct NoTileEnd {
-  __device__ void operator()(int) const {}
-};
-
 // The solve s, its block b and the block's tile t of work item w of range
 // KIND (two binary searches over the directory's prefix sums).
 template <int KIND>
@@ -181,7 +177,6 @@ __device__ __forceinline__ void build_item(const Dir &D, int s, int b, int t, It
   const DevSolve &S = D.solves[s];
   const DevBlock &DB = S.blocks[b];
   RangeBox r = range_of(KIND, DB.n, S.c.nghost);
-  if constexpr (KIND == kResK) r.hi[2] = DB.reskhi;
   it.s = s;
   it.blk = b;
   for (int a = 0; a < 3; ++a) {
@@ -219,11 +214,10 @@ __device__ __forceinline__ void build_item(const Dir &D, int s, int b, int t, It
 }
 
 // Work-item loop: for every tile of range `KIND` of every active solve, call
-// f(S, B, item), then end(w) with the tile's index w over all solves (every
-// thread of the CTA).  Tile lookup by thread 0, broadcast through shared
+// f(S, B, item).  Tile lookup by thread 0, broadcast through shared
 // memory.
-template <class R, int KIND, class F, class E = NoTileEnd>
-__device__ __forceinline__ void for_items(const Dir &D, F &&f, E &&end = E{}) {
+template <class R, int KIND, class F>
+__device__ __forceinline__ void for_items(const Dir &D, F &&f) {
   __shared__ int sh[3];
   let_dependents_launch();
   const int total = D.solve_tile_prefix[KIND][D.nsolves];
@@ -243,7 +237,6 @@ __device__ __forceinline__ void for_items(const Dir &D, F &&f, E &&end = E{}) {
     V<R> B;
     build_item<R, KIND>(D, s, b, t, it, B);
     f(D.solves[s], B, it);
-    end(w);
   }
 }
 
@@ -319,7 +312,7 @@ __device__ __forceinline__ Vec<R> vup(const Vec<R> &a, R next) {
 // One thread's part of a vector item: positions k .. k + N - 1 of row (i, j),
 // of which [klo, khi) are in the range.
 struct VItem {
-  int s, blk, i, j, k;
+  int s, blk, w, i, j, k;  // w: the tile's index over all solves
   bool in;
   uint32_t o;  // byte offset of position (i, j, k) in a real-valued component array
   int klo, khi;
@@ -386,7 +379,8 @@ template <class R, int KIND>
 __device__ __forceinline__ void build_vec_item(const Dir &D, int s, int b, int t, VItem &it, VV<R> &B) {
   const DevSolve &S = D.solves[s];
   const DevBlock &DB = S.blocks[b];
-  const RangeBox r = range_of(KIND, DB.n, S.c.nghost);
+  RangeBox r = range_of(KIND, DB.n, S.c.nghost);
+  if constexpr (KIND == kResK) r.hi[2] = DB.reskhi;
   set_view(B, DB, 0);  // the buffers of cur = 0: use_current after the state can be read
   B.U = uniform(B.U);
   B.Un = uniform(B.Un);
@@ -449,6 +443,7 @@ __device__ __forceinline__ void for_vec_items(const Dir &D, F &&f) {
     VItem it;
     VV<R> B;
     build_vec_item<R, KIND>(D, s, b, t, it, B);
+    it.w = w;
     if (w == (int)blockIdx.x) wait_for_predecessors();
     if (uniform((int)solve_active(D, s))) {
       use_current(B, uniform(D.state[s].cur));
@@ -1310,22 +1305,24 @@ __global__ void __launch_bounds__(kVecThreads) k_res_kmax(Dir D, int *out) {
 
 // Vector operations of the CG on the unknowns (W > 0); other entries stay 0.
 template <class R>
-__global__ void __launch_bounds__(kTileThreads) k_res_vec(Dir D, int op) {
-  for_items<R, kResK>(D, [&](const DevSolve &S, const V<R> &B, const Item &it) {
-    if (!it.in) return;
-    const int o = B.off(it.i, it.j, it.k);
+__global__ void __launch_bounds__(kVecThreads) k_res_vec(Dir D, int op) {
+  for_vec_items<R, kResK>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
+    const uint32_t o = it.o;
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
-      const bool dof = B.c(cRW + a)[o] > R(0.0);
-      R *x = B.c(cRX + a) + o, *r = B.c(cRR + a) + o, *p = B.c(cRP + a) + o;
+      const Vec<R> W = B.lv(cRW + a, o);
+      auto put = [&](int comp, const Vec<R> &v) {  // v on the unknowns, 0 elsewhere
+        B.st(comp + a, it, vmap<R>([&](int e) { return W.v[e] > R(0.0) ? v.v[e] : R(0.0); }), it.klo, it.khi);
+      };
       switch (op) {
         case RES_INIT:  // r = b = eta J (PackImplicitJedgeToVec_, :395-418); the CG's start sets x and p
-          *r = dof ? R(0.0) + B.c(cETAR + a)[o] * B.c(cJX + a)[o] : R(0.0);
+          put(cRR, R(0.0) + B.lv(cETAR + a, o) * B.lv(cJX + a, o));
           break;
-        case RES_E_FROM_P: B.c(cEX + a)[o] = dof ? *p : R(0.0); break;  // UnpackVecToImplicitEres_ (:294-312)
-        case RES_E_FROM_X: B.c(cEX + a)[o] = dof ? *x : R(0.0); break;
-        case RES_P_FROM_X: *p = dof ? *x : R(0.0); break;
+        case RES_E_FROM_P: put(cEX, B.lv(cRP + a, o)); break;  // UnpackVecToImplicitEres_ (:294-312)
+        case RES_E_FROM_X: put(cEX, B.lv(cRX + a, o)); break;
+        case RES_P_FROM_X: put(cRP, B.lv(cRX + a, o)); break;
         case RES_RESID:  // r = b - q, b kept in the B* snapshot arrays (FP64 companion of a mixed solve)
-          *r = dof ? B.c(cRBS + a)[o] - B.c(cRQ + a)[o] : R(0.0);
+          put(cRR, B.lv(cRBS + a, o) - B.lv(cRQ + a, o));
           break;
         default: break;
       }
@@ -1336,42 +1333,42 @@ __global__ void __launch_bounds__(kTileThreads) k_res_vec(Dir D, int op) {
 // dB = -dt curl E on the owned faces (CurlEdgeToFace with multiplier -dt,
 // Z4_Mercury/src/operators/CTOperators.cpp:6-56; MatMultImplicitResistive_, :420-445).
 template <class R>
-__global__ void __launch_bounds__(kTileThreads) k_res_db(Dir D) {
-  for_items<R, kResK>(D, [&](const DevSolve &S, const V<R> &B, const Item &it) {
-    if (!it.in) return;
+__global__ void __launch_bounds__(kVecThreads) k_res_db(Dir D) {
+  for_vec_items<R, kResK>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
     const R m = R(-D.state[it.s].dt);
-    const int i = it.i, j = it.j, k = it.k;
-    if (j < B.n1 && k < B.n2)
-      AT(cBX, i, j, k) = m * ((AT(cEY, i, j, k) - AT(cEY, i, j, k + 1)) + (AT(cEZ, i, j + 1, k) - AT(cEZ, i, j, k)));
-    if (i < B.n0 && k < B.n2)
-      AT(cBY, i, j, k) = m * ((AT(cEX, i, j, k + 1) - AT(cEX, i, j, k)) + (AT(cEZ, i, j, k) - AT(cEZ, i + 1, j, k)));
-    if (i < B.n0 && j < B.n1)
-      AT(cBZ, i, j, k) = m * ((AT(cEX, i, j, k) - AT(cEX, i, j + 1, k)) + (AT(cEY, i + 1, j, k) - AT(cEY, i, j, k)));
+    const uint32_t o = it.o, di = B.di, dj = B.dj;
+    const bool ic = it.i < B.n0, jc = it.j < B.n1;
+    const int hi = min(B.n2, it.khi);
+    const Vec<R> ex = B.lv(cEX, o), ey = B.lv(cEY, o), ez = B.lv(cEZ, o);
+    B.st(cBX, it, m * ((ey - B.upper(ey, cEY, o)) + (B.lv(cEZ, o + dj) - ez)), 0, hi, jc);
+    B.st(cBY, it, m * ((B.upper(ex, cEX, o) - ex) + (ez - B.lv(cEZ, o + di))), 0, hi, ic);
+    B.st(cBZ, it, m * ((ex - B.lv(cEX, o + dj)) + (B.lv(cEY, o + di) - ey)), 0, it.khi, ic && jc);
   });
+}
+
+// alpha CurlAdjFaceToEdge(beta B) on this thread's edges (CTOperators.cpp:59-110):
+// J of the field in the face arrays.
+template <class R>
+__device__ __forceinline__ void edge_current(const VV<R> &B, uint32_t o, Vec<R> J[3]) {
+  const uint32_t di = B.di, dj = B.dj;
+  constexpr uint32_t es = sizeof(R);
+  const Vec<R> fx = B.lv(cBFX, o) * B.lv(cBX, o), fy = B.lv(cBFY, o) * B.lv(cBY, o), fz = B.lv(cBFZ, o) * B.lv(cBZ, o);
+  auto below = [&](int a, uint32_t d) { return B.lv(cBFX + a, o - d) * B.lv(cBX + a, o - d); };
+  J[0] = ((vdown(fy, B.ld(cBFY, o - es) * B.ld(cBY, o - es)) - fy) + (fz - below(2, dj))) * R(1.0) * B.lv(cALX, o);
+  J[1] = ((fx - vdown(fx, B.ld(cBFX, o - es) * B.ld(cBX, o - es))) + (below(2, di) - fz)) * R(1.0) * B.lv(cALY, o);
+  J[2] = ((below(0, dj) - fx) + (fy - below(1, di))) * R(1.0) * B.lv(cALZ, o);
 }
 
 // dJ = alpha CurlAdjFaceToEdge(beta dB) on the owned edges (CalcImplicitDeltaJedgeFromDeltaB_,
 // Mercury_ImplicitResistive.cpp:314-393; CTOperators.cpp:59-110).
 template <class R>
-__global__ void __launch_bounds__(kTileThreads) k_res_dj(Dir D) {
-  for_items<R, kResK>(D, [&](const DevSolve &S, const V<R> &B, const Item &it) {
-    if (!it.in) return;
-    const int i = it.i, j = it.j, k = it.k;
-    if (i < B.n0) {
-      const R v = ((AT(cBFY, i, j, k - 1) * AT(cBY, i, j, k - 1) - AT(cBFY, i, j, k) * AT(cBY, i, j, k)) +
-                   (AT(cBFZ, i, j, k) * AT(cBZ, i, j, k) - AT(cBFZ, i, j - 1, k) * AT(cBZ, i, j - 1, k))) * R(1.0);
-      AT(cJX, i, j, k) = v * AT(cALX, i, j, k);
-    }
-    if (j < B.n1) {
-      const R v = ((AT(cBFX, i, j, k) * AT(cBX, i, j, k) - AT(cBFX, i, j, k - 1) * AT(cBX, i, j, k - 1)) +
-                   (AT(cBFZ, i - 1, j, k) * AT(cBZ, i - 1, j, k) - AT(cBFZ, i, j, k) * AT(cBZ, i, j, k))) * R(1.0);
-      AT(cJY, i, j, k) = v * AT(cALY, i, j, k);
-    }
-    if (k < B.n2) {
-      const R v = ((AT(cBFX, i, j - 1, k) * AT(cBX, i, j - 1, k) - AT(cBFX, i, j, k) * AT(cBX, i, j, k)) +
-                   (AT(cBFY, i, j, k) * AT(cBY, i, j, k) - AT(cBFY, i - 1, j, k) * AT(cBY, i - 1, j, k))) * R(1.0);
-      AT(cJZ, i, j, k) = v * AT(cALZ, i, j, k);
-    }
+__global__ void __launch_bounds__(kVecThreads) k_res_dj(Dir D) {
+  for_vec_items<R, kResK>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
+    Vec<R> J[3];
+    edge_current(B, it.o, J);
+    B.st(cJX, it, J[0], 0, it.khi, it.i < B.n0);
+    B.st(cJY, it, J[1], 0, it.khi, it.j < B.n1);
+    B.st(cJZ, it, J[2], 0, min(B.n2, it.khi));
   });
 }
 
@@ -1394,232 +1391,222 @@ __global__ void __launch_bounds__(kTileThreads) k_res_clearb(Dir D) {
 
 // q = A p = E_res - eta dJ on the unknowns (MatMultImplicitResistive_, :446-468).
 template <class R>
-__global__ void __launch_bounds__(kTileThreads) k_res_q(Dir D) {
-  for_items<R, kResK>(D, [&](const DevSolve &S, const V<R> &B, const Item &it) {
-    if (!it.in) return;
-    const int o = B.off(it.i, it.j, it.k);
+__global__ void __launch_bounds__(kVecThreads) k_res_q(Dir D) {
+  for_vec_items<R, kResK>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
+    const uint32_t o = it.o;
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
-      const bool dof = B.c(cRW + a)[o] > R(0.0);
-      B.c(cRQ + a)[o] = dof ? B.c(cEX + a)[o] - B.c(cETAR + a)[o] * B.c(cJX + a)[o] : R(0.0);
+      const Vec<R> W = B.lv(cRW + a, o), q = B.lv(cEX + a, o) - B.lv(cETAR + a, o) * B.lv(cJX + a, o);
+      B.st(cRQ + a, it, vmap<R>([&](int e) { return W.v[e] > R(0.0) ? q.v[e] : R(0.0); }), it.klo, it.khi);
     }
   });
 }
 
-// Dot products of r on the unknowns of the masked solve: (sum W r r, sum r r).  Per-CTA partial sums in a fixed order (deterministic).
-template <class R>
-__global__ void __launch_bounds__(kTileThreads) k_res_dot(Dir D, double *partial) {
-  __shared__ double sh[2][kTileThreads / 32];
-  double acc0 = 0.0, acc1 = 0.0;
-  for_items<R, kResK>(D, [&](const DevSolve &S, const V<R> &B, const Item &it) {
-    if (!it.in) return;
-    const int o = B.off(it.i, it.j, it.k);
-    for (int a = 0; a < 3; ++a) {
-      const double w = (double)B.c(cRW + a)[o];
-      if (!(w > 0.0)) continue;
-      const double r = (double)B.c(cRR + a)[o];
-      acc0 += w * r * r;
-      acc1 += r * r;
-    }
-  });
-  for (int of = 16; of > 0; of >>= 1) {
-    acc0 += __shfl_xor_sync(0xffffffffu, acc0, of);
-    acc1 += __shfl_xor_sync(0xffffffffu, acc1, of);
+// The CTA's sums of two values, in thread 0 (fixed order).
+__device__ __forceinline__ void cta_sum(double &a, double &b) {
+  __shared__ double sh[2][kVecThreads / 32];
+  for (int w = 16; w > 0; w >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, w);
+    b += __shfl_xor_sync(0xffffffffu, b, w);
   }
+  __syncthreads();  // sh of the previous sum has been read
   if ((threadIdx.x & 31) == 0) {
-    sh[0][threadIdx.x >> 5] = acc0;
-    sh[1][threadIdx.x >> 5] = acc1;
+    sh[0][threadIdx.x >> 5] = a;
+    sh[1][threadIdx.x >> 5] = b;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    double s0 = 0.0, s1 = 0.0;
-    for (int w = 0; w < kTileThreads / 32; ++w) {
-      s0 += sh[0][w];
-      s1 += sh[1][w];
+    a = b = 0.0;
+    for (int w = 0; w < kVecThreads / 32; ++w) {
+      a += sh[0][w];
+      b += sh[1][w];
     }
-    partial[2 * blockIdx.x] = s0;
-    partial[2 * blockIdx.x + 1] = s1;
+  }
+}
+
+// Dot products of r on the unknowns of the masked solve: (sum W r r, sum r r).  Per-CTA partial sums in a fixed order (deterministic).
+template <class R>
+__global__ void __launch_bounds__(kVecThreads) k_res_dot(Dir D, double *partial) {
+  double acc0 = 0.0, acc1 = 0.0;
+  for_vec_items<R, kResK>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const Vec<R> W = B.lv(cRW + a, it.o), r = B.lv(cRR + a, it.o);
+#pragma unroll
+      for (int e = 0; e < Vec<R>::N; ++e) {
+        if (!it.in || !it.has(e) || !(W.v[e] > R(0.0))) continue;
+        const double w = (double)W.v[e], x = (double)r.v[e];
+        acc0 += w * x * x;
+        acc1 += x * x;
+      }
+    }
+  });
+  cta_sum(acc0, acc1);
+  if (threadIdx.x == 0) {
+    partial[2 * blockIdx.x] = acc0;
+    partial[2 * blockIdx.x + 1] = acc1;
   }
 }
 __global__ void k_res_sum(const double *partial, int n, double *result) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double s0 = 0.0, s1 = 0.0;
-    for (int q = 0; q < n; ++q) {
-      s0 += partial[2 * q];
-      s1 += partial[2 * q + 1];
-    }
+  double s0 = 0.0, s1 = 0.0;
+  for (int q = threadIdx.x; q < n; q += 32) {
+    s0 += partial[2 * q];
+    s1 += partial[2 * q + 1];
+  }
+  for (int w = 16; w > 0; w >>= 1) {
+    s0 += __shfl_xor_sync(0xffffffffu, s0, w);
+    s1 += __shfl_xor_sync(0xffffffffu, s1, w);
+  }
+  if (threadIdx.x == 0) {
     result[0] = s0;
     result[1] = s1;
   }
 }
 
-// One step of the CG iteration of every masked solve with its dot products:
-// each warp writes its sums over each tile to its own slot of tpart (2
-// doubles per warp and tile), k_res_cg_sum then adds a solve's slots in a
-// fixed order (deterministic) and updates its scalars.  CG_PQ first clears
-// the loop condition, so a loop whose stop test did not run ends.  Both
-// kernels write the condition of the loop graph they belong to
-// (build_cg_graph) only when launched inside it (in_graph; the host-driven
-// loop of res_cg_batch reads the states instead).
-template <class R>
-__global__ void __launch_bounds__(kTileThreads) k_res_cg(Dir D, int op, double *tpart, const ResCG *cg,
-                                                         cudaGraphConditionalHandle handle, int in_graph) {
-  if (in_graph && op == CG_PQ && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(handle, 0u);
-  double acc0 = 0.0, acc1 = 0.0;
-  for_items<R, kResK>(
-      D,
-      [&](const DevSolve &S, const V<R> &B, const Item &it) {
-        if (!it.in) return;
-        const R alpha = R(cg[it.s].alpha);
-        const int o = B.off(it.i, it.j, it.k);
-        for (int a = 0; a < 3; ++a) {
-          const R wr = B.c(cRW + a)[o];
-          const bool dof = wr > R(0.0);
-          const double w = (double)wr;
-          R *x = B.c(cRX + a) + o, *r = B.c(cRR + a) + o, *p = B.c(cRP + a) + o, *q = B.c(cRQ + a) + o;
-          if (op == CG_INIT) {  // x = 0, p = r (the start), E_res = p
-            const R pv = dof ? *r : R(0.0);
-            *x = R(0.0);
-            *p = pv;
-            B.c(cEX + a)[o] = pv;
-            if (w > 0.0) {
-              const double rv = (double)*r;
-              acc0 += w * rv * rv;
-              acc1 += rv * rv;
-            }
-          } else if (op == CG_PQ) {
-            const R qv = dof ? B.c(cEX + a)[o] - B.c(cETAR + a)[o] * B.c(cJX + a)[o] : R(0.0);
-            *q = qv;
-            if (w > 0.0) acc0 += w * (double)*p * (double)qv;
-          } else {
-            if (dof) {
-              *x += alpha * *p;
-              *r -= alpha * *q;
-            }
-            if (w > 0.0) {
-              const double rv = (double)*r;
-              acc0 += w * rv * rv;
-              acc1 += rv * rv;
-            }
-          }
-        }
-      },
-      [&](int w) {  // the warp's sums over this tile
-        for (int of = 16; of > 0; of >>= 1) {
-          acc0 += __shfl_xor_sync(0xffffffffu, acc0, of);
-          acc1 += __shfl_xor_sync(0xffffffffu, acc1, of);
-        }
-        if ((threadIdx.x & 31) == 0) {
-          const int64_t slot = (int64_t)w * kWarpsPerTile + (threadIdx.x >> 5);
-          tpart[2 * slot] = acc0;
-          tpart[2 * slot + 1] = acc1;
-        }
-        acc0 = acc1 = 0.0;
-      });
+// The end of a k_res_cg step of solve s, by one thread, from its sums t0, t1:
+// the solve's scalars, and whether its loop ends (converged, max_it,
+// breakdown): it then leaves the mask, so the following kernels skip it.
+__device__ __forceinline__ void res_cg_end(ResCG &cs, int op, double t0, double t1) {
+  if (op == CG_INIT) {
+    cs.rho = t0;
+    cs.r0 = cs.rnorm = sqrt(t1);
+    cs.tol = cs.tol_factor * cs.r0;
+    cs.it = 0;
+    cs.converged = cs.rnorm <= cs.tol;
+    cs.done = cs.converged || cs.max_it <= 0;
+  } else if (op == CG_PQ) {
+    if (!(t0 > 0.0)) cs.done = 1;  // breakdown: not positive definite on these unknowns
+    else cs.alpha = cs.rho / t0;
+  } else {
+    cs.it += 1;
+    cs.rnorm = sqrt(t1);
+    if (cs.rnorm <= cs.tol) cs.converged = cs.done = 1;
+    else if (cs.it >= cs.max_it) cs.done = 1;
+    cs.beta = t0 / cs.rho;
+    cs.rho = t0;
+  }
 }
 
-// The per-solve end of a k_res_cg step: kCgChunks CTAs per slot, CTA c of
-// solve s adds chunk c of the solve's tile partials (threads stride over it,
-// then a fixed tree); the last of them (atomic ticket per solve) adds the
-// chunks in order and updates the solve's state; a solve whose loop ends
-// (converged, max_it, breakdown) leaves the mask, so the following kernels
-// skip it.  The last slot to report (atomic ticket) sets the loop condition
-// after CG_INIT and CG_RR: some solve still running.  Every sum has fixed
-// bounds and order (deterministic, and the same for a solve alone or in a
-// batch).
-__global__ void __launch_bounds__(kTileThreads) k_res_cg_sum(Dir D, int op, const double *tpart, ResCG *cg,
-                                                             ResCtl *ctl, double *chunks, unsigned int *sarr,
-                                                             cudaGraphConditionalHandle handle, int in_graph) {
-  __shared__ double sh[2][kWarpsPerTile];
-  let_dependents_launch();
-  wait_for_predecessors();
-  const int s = blockIdx.x / kCgChunks, c = blockIdx.x % kCgChunks;
-  const bool act = s < D.nsolves && solve_active(D, s);  // the whole CTA agrees
-  bool last_of_solve = false;
-  if (act) {
+// One step of the CG iteration of every masked solve with its dot products.
+// Each tile's sums go to its own slot of tpart (2 doubles); the CTA that
+// finishes a solve's last tile (a ticket per solve) adds the solve's slots in a
+// fixed order (deterministic, and the same for a solve alone or in a batch)
+// and ends the step.  Warps without an unknown skip the vectors.  CG_PQ first
+// clears the condition of the loop graph (build_cg_graph), and a solve that goes
+// on sets it, so a loop whose stop test did not run ends; the condition is only
+// written when launched inside the graph (in_graph; the host-driven loop of
+// res_cg_batch reads the states instead).
+template <class R, int OP>
+__global__ void __launch_bounds__(kVecThreads) k_res_cg(Dir D, double *tpart, ResCG *cg, unsigned int *sarr,
+                                                        cudaGraphConditionalHandle handle, int in_graph) {
+  if (in_graph && OP == CG_PQ && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(handle, 0u);
+  for_vec_items<R, kResK>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
+    constexpr int N = Vec<R>::N;
+    const uint32_t o = it.o;
+    double acc0 = 0.0, acc1 = 0.0;
+    Vec<R> W[3];
+    bool some = false;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      W[a] = B.lv(cRW + a, o);
+#pragma unroll
+      for (int e = 0; e < N; ++e) some = some || W[a].v[e] > R(0.0);
+    }
+    if (OP == CG_INIT || __any_sync(0xffffffffu, some && it.in)) {
+      const R alpha = R(cg[it.s].alpha);
+      auto mask = [&](int a, const Vec<R> &v) { return vmap<R>([&](int e) { return W[a].v[e] > R(0.0) ? v.v[e] : R(0.0); }); };
+      auto counts = [&](int a, int e) { return it.in && it.has(e) && W[a].v[e] > R(0.0); };
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        if (OP == CG_INIT) {  // x = 0, p = r (the start), E_res = p
+          const Vec<R> r = B.lv(cRR + a, o), p = mask(a, r);
+          B.st(cRX + a, it, vset(R(0.0)), it.klo, it.khi);
+          B.st(cRP + a, it, p, it.klo, it.khi);
+          B.st(cEX + a, it, p, it.klo, it.khi);
+#pragma unroll
+          for (int e = 0; e < N; ++e) {
+            if (!counts(a, e)) continue;
+            const double w = (double)W[a].v[e], rv = (double)r.v[e];
+            acc0 += w * rv * rv;
+            acc1 += rv * rv;
+          }
+        } else if (OP == CG_PQ) {
+          const Vec<R> q = mask(a, B.lv(cEX + a, o) - B.lv(cETAR + a, o) * B.lv(cJX + a, o)), p = B.lv(cRP + a, o);
+          B.st(cRQ + a, it, q, it.klo, it.khi);
+#pragma unroll
+          for (int e = 0; e < N; ++e)
+            if (counts(a, e)) acc0 += (double)W[a].v[e] * (double)p.v[e] * (double)q.v[e];
+        } else {
+          const Vec<R> x = B.own(cRX + a, o), r = B.own(cRR + a, o), p = B.lv(cRP + a, o), q = B.lv(cRQ + a, o);
+          Vec<R> xn = x, rn = r;
+#pragma unroll
+          for (int e = 0; e < N; ++e) {
+            if (!(W[a].v[e] > R(0.0))) continue;
+            xn.v[e] += alpha * p.v[e];
+            rn.v[e] -= alpha * q.v[e];
+            if (!counts(a, e)) continue;
+            const double w = (double)W[a].v[e], rv = (double)rn.v[e];
+            acc0 += w * rv * rv;
+            acc1 += rv * rv;
+          }
+          B.st(cRX + a, it, xn, it.klo, it.khi);
+          B.st(cRR + a, it, rn, it.klo, it.khi);
+        }
+      }
+    }
+    __shared__ int last;
+    cta_sum(acc0, acc1);
     const int *sp = D.solve_tile_prefix[kResK];
-    const int64_t a0 = (int64_t)sp[s] * kWarpsPerTile, n = (int64_t)(sp[s + 1] - sp[s]) * kWarpsPerTile;
-    const int64_t len = (n + kCgChunks - 1) / kCgChunks;
-    const int64_t a = a0 + min(n, (int64_t)c * len), e = a0 + min(n, (int64_t)(c + 1) * len);
-    double u0 = 0.0, u1 = 0.0;
-    for (int64_t q = a + threadIdx.x; q < e; q += kTileThreads) {
-      u0 += tpart[2 * q];
-      u1 += tpart[2 * q + 1];
-    }
-    for (int of = 16; of > 0; of >>= 1) {
-      u0 += __shfl_xor_sync(0xffffffffu, u0, of);
-      u1 += __shfl_xor_sync(0xffffffffu, u1, of);
-    }
-    if ((threadIdx.x & 31) == 0) {
-      sh[0][threadIdx.x >> 5] = u0;
-      sh[1][threadIdx.x >> 5] = u1;
+    const int t0 = sp[it.s], nt = sp[it.s + 1] - t0;
+    if (threadIdx.x == 0) {
+      tpart[2 * (int64_t)it.w] = acc0;
+      tpart[2 * (int64_t)it.w + 1] = acc1;
+      __threadfence();
+      last = atomicAdd(&sarr[it.s], 1u) == (unsigned)nt - 1;
     }
     __syncthreads();
+    if (!last) return;
+    __threadfence();  // every tile of the solve is in
+    double s0 = 0.0, s1 = 0.0;
+    for (int q = threadIdx.x; q < nt; q += kVecThreads) {
+      const double2 v = __ldcg((const double2 *)tpart + t0 + q);
+      s0 += v.x;
+      s1 += v.y;
+    }
+    cta_sum(s0, s1);
     if (threadIdx.x == 0) {
-      double t0 = 0.0, t1 = 0.0;
-      for (int w = 0; w < kWarpsPerTile; ++w) {
-        t0 += sh[0][w];
-        t1 += sh[1][w];
-      }
-      chunks[2 * (s * kCgChunks + c)] = t0;
-      chunks[2 * (s * kCgChunks + c) + 1] = t1;
-      __threadfence();
-      last_of_solve = atomicAdd(&sarr[s], 1u) == kCgChunks - 1;
+      sarr[it.s] = 0;
+      res_cg_end(cg[it.s], OP, s0, s1);
+      if (cg[it.s].done) D.state[it.s].mask = 0;
+      else if (in_graph && OP != CG_PQ) cudaGraphSetConditional(handle, 1u);
     }
-  }
-  if (threadIdx.x != 0) return;
-  if (act ? !last_of_solve : c != 0) return;  // one report per slot: its last chunk, or chunk 0 of an idle slot
-  if (act) {  // every chunk of solve s is in
-    __threadfence();
-    sarr[s] = 0;
-    double t0 = 0.0, t1 = 0.0;
-    for (int q = 0; q < kCgChunks; ++q) {
-      t0 += __ldcg(chunks + 2 * (s * kCgChunks + q));
-      t1 += __ldcg(chunks + 2 * (s * kCgChunks + q) + 1);
-    }
-    ResCG &cs = cg[s];
-    if (op == CG_INIT) {
-      cs.rho = t0;
-      cs.r0 = cs.rnorm = sqrt(t1);
-      cs.tol = cs.tol_factor * cs.r0;
-      cs.it = 0;
-      cs.converged = cs.rnorm <= cs.tol;
-      cs.done = cs.converged || cs.max_it <= 0;
-    } else if (op == CG_PQ) {
-      if (!(t0 > 0.0)) cs.done = 1;  // breakdown: not positive definite on these unknowns
-      else cs.alpha = cs.rho / t0;
-    } else {
-      cs.it += 1;
-      cs.rnorm = sqrt(t1);
-      if (cs.rnorm <= cs.tol) cs.converged = cs.done = 1;
-      else if (cs.it >= cs.max_it) cs.done = 1;
-      cs.beta = t0 / cs.rho;
-      cs.rho = t0;
-    }
-    if (cs.done) D.state[s].mask = 0;
-    else atomicAdd(&ctl->running, 1);
-  }
-  __threadfence();
-  if (atomicAdd(&ctl->arrivals, 1u) != (unsigned)(gridDim.x / kCgChunks) - 1) return;  // the last slot to report
-  __threadfence();
-  const int running = atomicAdd(&ctl->running, 0);
-  ctl->arrivals = 0;
-  ctl->running = 0;
-  if (in_graph && op != CG_PQ) cudaGraphSetConditional(handle, running > 0 ? 1u : 0u);
+  });
 }
 
 // p = r + beta p and E_res = p on the unknowns (the next iteration's
-// operator input) of every solve still iterating (in the mask).
+// operator input) of every solve still iterating (in the mask); warps without an
+// unknown have nothing to update (their E_res is 0, or an owner copy that the
+// next operator writes again).
 template <class R>
-__global__ void __launch_bounds__(kTileThreads) k_res_pupd_e(Dir D, const ResCG *cg) {
-  for_items<R, kResK>(D, [&](const DevSolve &S, const V<R> &B, const Item &it) {
-    if (!it.in) return;
-    const R beta = R(cg[it.s].beta);
-    const int o = B.off(it.i, it.j, it.k);
+__global__ void __launch_bounds__(kVecThreads) k_res_pupd_e(Dir D, const ResCG *cg) {
+  for_vec_items<R, kResK>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
+    constexpr int N = Vec<R>::N;
+    const uint32_t o = it.o;
+    Vec<R> W[3];
+    bool some = false;
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
-      const bool dof = B.c(cRW + a)[o] > R(0.0);
-      R *p = B.c(cRP + a) + o;
-      if (dof) *p = B.c(cRR + a)[o] + beta * *p;
-      B.c(cEX + a)[o] = dof ? *p : R(0.0);
+      W[a] = B.lv(cRW + a, o);
+#pragma unroll
+      for (int e = 0; e < N; ++e) some = some || W[a].v[e] > R(0.0);
+    }
+    if (!__any_sync(0xffffffffu, some && it.in)) return;
+    const R beta = R(cg[it.s].beta);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const Vec<R> p = B.own(cRP + a, o), pn = B.lv(cRR + a, o) + beta * p;
+      B.st(cRP + a, it, vmap<R>([&](int e) { return W[a].v[e] > R(0.0) ? pn.v[e] : p.v[e]; }), it.klo, it.khi);
+      B.st(cEX + a, it, vmap<R>([&](int e) { return W[a].v[e] > R(0.0) ? pn.v[e] : R(0.0); }), it.klo, it.khi);
     }
   });
 }
@@ -1641,25 +1628,19 @@ __global__ void __launch_bounds__(kTileThreads) k_res_copyb(Dir D, int op) {
 // B += dt (-curl E_res) on the owned faces (ApplyImplicitResistiveUpdate_, :557-575;
 // ApplyUpdate_Euler_BfaceOnly_, Z4_Mercury/src/physics/MercurySolver_MagExplicit_Hall.cpp:435-473).
 template <class R>
-__global__ void __launch_bounds__(kTileThreads) k_res_bupdate(Dir D) {
-  for_items<R, kResK>(D, [&](const DevSolve &S, const V<R> &B, const Item &it) {
-    if (!it.in) return;
+__global__ void __launch_bounds__(kVecThreads) k_res_bupdate(Dir D) {
+  for_vec_items<R, kResK>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
     const R dt = R(D.state[it.s].dt);
-    const int i = it.i, j = it.j, k = it.k;
+    const uint32_t o = it.o, di = B.di, dj = B.dj;
+    const bool ic = it.i < B.n0, jc = it.j < B.n1;
     // the faces whose edges E_res covers (k + 1 below the range's bound);
     // above them E_res is 0 and B does not change
-    if (j < B.n1 && k + 1 < it.hi[2]) {
-      const R rb = R(-1.0) * ((AT(cEY, i, j, k) - AT(cEY, i, j, k + 1)) + (AT(cEZ, i, j + 1, k) - AT(cEZ, i, j, k)));
-      AT(cBX, i, j, k) += dt * rb;
-    }
-    if (i < B.n0 && k + 1 < it.hi[2]) {
-      const R rb = R(-1.0) * ((AT(cEX, i, j, k + 1) - AT(cEX, i, j, k)) + (AT(cEZ, i, j, k) - AT(cEZ, i + 1, j, k)));
-      AT(cBY, i, j, k) += dt * rb;
-    }
-    if (i < B.n0 && j < B.n1) {
-      const R rb = R(-1.0) * ((AT(cEX, i, j, k) - AT(cEX, i, j + 1, k)) + (AT(cEY, i + 1, j, k) - AT(cEY, i, j, k)));
-      AT(cBZ, i, j, k) += dt * rb;
-    }
+    const int hi = it.khi - 1;
+    const Vec<R> ex = B.lv(cEX, o), ey = B.lv(cEY, o), ez = B.lv(cEZ, o);
+    B.st(cBX, it, B.own(cBX, o) + dt * (R(-1.0) * ((ey - B.upper(ey, cEY, o)) + (B.lv(cEZ, o + dj) - ez))), 0, hi, jc);
+    B.st(cBY, it, B.own(cBY, o) + dt * (R(-1.0) * ((B.upper(ex, cEX, o) - ex) + (ez - B.lv(cEZ, o + di)))), 0, hi, ic);
+    B.st(cBZ, it, B.own(cBZ, o) + dt * (R(-1.0) * ((ex - B.lv(cEX, o + dj)) + (B.lv(cEY, o + di) - ey))), 0, it.khi,
+         ic && jc);
   });
 }
 
@@ -2394,11 +2375,10 @@ static const void *kernel_fn(StepKernel k) {
     case SK_RES_Q: return (const void *)k_res_q<R>;
     case SK_RES_COPYB: return (const void *)k_res_copyb<R>;
     case SK_RES_BUPDATE: return (const void *)k_res_bupdate<R>;
-    case SK_RES_CG: return (const void *)k_res_cg<R>;
+    case SK_RES_CG: return (const void *)k_res_cg<R, CG_RR>;
     case SK_RES_PUPD_E: return (const void *)k_res_pupd_e<R>;
     case SK_PHYS: return (const void *)k_phys<R>;
     case SK_RES_CLEARB: return (const void *)k_res_clearb<R>;
-    case SK_RES_CGSUM: return (const void *)k_res_cg_sum;
     default: return nullptr;
   }
 }
@@ -2408,6 +2388,8 @@ static int kernel_threads(StepKernel k) {
   switch (k) {
     case SK_FACE_EMF: case SK_EDGE_EMF: case SK_HALL_EDGE: case SK_ADD_HALL: case SK_BFACE: case SK_BCELL_JEDGE:
     case SK_JCELL: case SK_PV_UPLUS: case SK_FACE_NORMALS: case SK_DIVB: case SK_RES_SEED: case SK_RES_W:
+    case SK_RES_VEC: case SK_RES_DB: case SK_RES_DJ: case SK_RES_Q: case SK_RES_BUPDATE: case SK_RES_CG:
+    case SK_RES_PUPD_E:
       return kVecThreads;
     default: return kTileThreads;
   }
@@ -2466,22 +2448,26 @@ static void launch_as(StepKernel k, const Dir &D, cudaStream_t st, const SyncOps
     case SK_DIVB: k_div_b<R><<<G, kVecThreads, 0, st>>>(D); break;
     case SK_RES_SEED: k_res_seed<R><<<G, kVecThreads, 0, st>>>(D); break;
     case SK_RES_W: k_res_w<R><<<G, kVecThreads, 0, st>>>(D); break;
-    case SK_RES_VEC: launch_dependent(k_res_vec<R>, G, kTileThreads, st, D, iarg); break;
-    case SK_RES_DB: launch_dependent(k_res_db<R>, G, kTileThreads, st, D); break;
-    case SK_RES_DJ: launch_dependent(k_res_dj<R>, G, kTileThreads, st, D); break;
-    case SK_RES_Q: launch_dependent(k_res_q<R>, G, kTileThreads, st, D); break;
-    case SK_RES_DOT: k_res_dot<R><<<g_grid_tiles, kTileThreads, 0, st>>>(D, rs.partial); break;
+    case SK_RES_VEC: launch_dependent(k_res_vec<R>, G, kVecThreads, st, D, iarg); break;
+    case SK_RES_DB: launch_dependent(k_res_db<R>, G, kVecThreads, st, D); break;
+    case SK_RES_DJ: launch_dependent(k_res_dj<R>, G, kVecThreads, st, D); break;
+    case SK_RES_Q: launch_dependent(k_res_q<R>, G, kVecThreads, st, D); break;
+    case SK_RES_DOT: k_res_dot<R><<<g_grid_tiles, kVecThreads, 0, st>>>(D, rs.partial); break;
     case SK_RES_SUM: k_res_sum<<<1, 32, 0, st>>>(rs.partial, g_grid_tiles, rs.result); break;
     case SK_RES_COPYB: launch_dependent(k_res_copyb<R>, G, kTileThreads, st, D, iarg); break;
-    case SK_RES_BUPDATE: launch_dependent(k_res_bupdate<R>, G, kTileThreads, st, D); break;
+    case SK_RES_BUPDATE: launch_dependent(k_res_bupdate<R>, G, kVecThreads, st, D); break;
     case SK_RES_CG:
-      launch_dependent(k_res_cg<R>, g_grid_tiles, kTileThreads, st, D, iarg, rs.tpartial, rs.cg, rs.handle, rs.in_graph);
+      if (iarg == CG_INIT)
+        launch_dependent(k_res_cg<R, CG_INIT>, G, kVecThreads, st, D, rs.tpartial, rs.cg, rs.sarrivals, rs.handle,
+                         rs.in_graph);
+      else if (iarg == CG_PQ)
+        launch_dependent(k_res_cg<R, CG_PQ>, G, kVecThreads, st, D, rs.tpartial, rs.cg, rs.sarrivals, rs.handle,
+                         rs.in_graph);
+      else
+        launch_dependent(k_res_cg<R, CG_RR>, G, kVecThreads, st, D, rs.tpartial, rs.cg, rs.sarrivals, rs.handle,
+                         rs.in_graph);
       break;
-    case SK_RES_CGSUM:
-      launch_dependent(k_res_cg_sum, D.nsolves * kCgChunks, kTileThreads, st, D, iarg, rs.tpartial, rs.cg, rs.ctl, rs.chunks,
-                       rs.sarrivals, rs.handle, rs.in_graph);
-      break;
-    case SK_RES_PUPD_E: launch_dependent(k_res_pupd_e<R>, G, kTileThreads, st, D, rs.cg); break;
+    case SK_RES_PUPD_E: launch_dependent(k_res_pupd_e<R>, G, kVecThreads, st, D, rs.cg); break;
     case SK_FLIP: launch_dependent(k_flip, 1, 128, st, D); break;
     case SK_RETIRE: launch_dependent(k_retire, 1, 128, st, D); break;
     case SK_PHYS: launch_dependent(k_phys<R>, G, 256, st, D, iarg); break;
@@ -2511,30 +2497,66 @@ static void launch_as(StepKernel k, const Dir &D, cudaStream_t st, const SyncOps
 // RES_X_DEMOTE_R: r = (float) companion r (the next correction's right-hand side).
 // RES_X_ADD_X: companion x += x (the correction).
 // RES_X_DEMOTE_X: x = (float) companion x (the solution).
-template <int KIND>
-__global__ void __launch_bounds__(kTileThreads) k_res_cross(Dir D, int op) {
-  for_items<float, KIND>(D, [&](const DevSolve &S, const V<float> &B, const Item &it) {
+__global__ void __launch_bounds__(kTileThreads) k_res_cross_static(Dir D) {
+  for_items<float, kFull>(D, [&](const DevSolve &S, const V<float> &B, const Item &it) {
     if (!it.in) return;
-    const DevBlock &CB = S.companion[it.blk];
-    if (op == RES_X_SETUP && it.blk == 0 && it.i == it.lo[0] && it.j == it.lo[1] && it.k == it.lo[2]) {
+    V<double> C;
+    set_view(C, S.companion[it.blk], 0);
+    const int o = B.off(it.i, it.j, it.k), oc = C.off(it.i, it.j, it.k);
+    for (int a = 0; a < 3; ++a)
+      for (int c : {cALX, cBFX, cETAR, cRW}) C.c(c + a)[oc] = (double)B.c(c + a)[o];
+  });
+}
+template <int OP>
+__global__ void __launch_bounds__(kVecThreads) k_res_cross(Dir D) {
+  for_vec_items<float, kResK>(D, [&](const DevSolve &S, const VV<float> &B, const VItem &it) {
+    if (OP == RES_X_SETUP && threadIdx.x == 0 && it.w == D.solve_tile_prefix[kResK][it.s]) {
       S.companion_state->dt = D.state[it.s].dt;  // the step's dt, once per solve
       S.companion_state->dt_bits = D.state[it.s].dt_bits;
     }
     V<double> C;
-    set_view(C, CB, 0);
-    const int o = B.off(it.i, it.j, it.k), oc = C.off(it.i, it.j, it.k);
+    set_view(C, S.companion[it.blk], 0);
+    // the four positions in the companion's arrays (the same box: twice the byte offset, 32-byte aligned)
+    auto at = [&](int comp) { return (double2 *)((char *)C.c(comp) + 2 * (uint64_t)it.o); };
+    auto widen = [&](int comp, const Vec<float> &v) {  // positions outside the range keep their values
+      double2 *p = at(comp);
+      if (!it.in) return;
+      if (it.k >= it.klo && it.k + 4 <= it.khi) {
+        p[0] = make_double2((double)v.v[0], (double)v.v[1]);
+        p[1] = make_double2((double)v.v[2], (double)v.v[3]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (it.has(e)) ((double *)p)[e] = (double)v.v[e];
+      }
+    };
+    auto narrow = [&](int comp) {
+      const double2 *p = at(comp);
+      const double2 a = p[0], b = p[1];
+      Vec<float> v;
+      v.v[0] = (float)a.x;
+      v.v[1] = (float)a.y;
+      v.v[2] = (float)b.x;
+      v.v[3] = (float)b.y;
+      return v;
+    };
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
-      switch (op) {
-        case RES_X_STATIC:
-          for (int c : {cALX, cBFX, cETAR, cRW}) C.c(c + a)[oc] = (double)B.c(c + a)[o];
-          break;
-        case RES_X_SETUP:
-          C.c(cRBS + a)[oc] = C.c(cRR + a)[oc] = (double)B.c(cRR + a)[o];
-          C.c(cRX + a)[oc] = 0.0;
-          break;
-        case RES_X_DEMOTE_R: B.c(cRR + a)[o] = (float)C.c(cRR + a)[oc]; break;
-        case RES_X_ADD_X: C.c(cRX + a)[oc] += (double)B.c(cRX + a)[o]; break;
-        default: B.c(cRX + a)[o] = (float)C.c(cRX + a)[oc]; break;  // RES_X_DEMOTE_X
+      if (OP == RES_X_SETUP) {
+        const Vec<float> r = B.lv(cRR + a, it.o);
+        widen(cRBS + a, r);
+        widen(cRR + a, r);
+        widen(cRX + a, vset(0.0f));
+      } else if (OP == RES_X_DEMOTE_R) {
+        B.st(cRR + a, it, narrow(cRR + a), it.klo, it.khi);
+      } else if (OP == RES_X_ADD_X) {
+        const Vec<float> x = B.lv(cRX + a, it.o);
+        double *p = (double *)at(cRX + a);
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (it.in && it.has(e)) p[e] += (double)x.v[e];
+      } else {  // RES_X_DEMOTE_X
+        B.st(cRX + a, it, narrow(cRX + a), it.klo, it.khi);
       }
     }
   });
@@ -2542,8 +2564,13 @@ __global__ void __launch_bounds__(kTileThreads) k_res_cross(Dir D, int op) {
 
 void launch_res_cross(const Dir &D, int op, cudaStream_t st) {
   grids<float>();
-  if (op == RES_X_STATIC) k_res_cross<kFull><<<g_grid_tiles, kTileThreads, 0, st>>>(D, op);
-  else launch_dependent(k_res_cross<kResK>, g_grid_tiles, kTileThreads, st, D, op);
+  switch (op) {
+    case RES_X_STATIC: k_res_cross_static<<<g_grid_tiles, kTileThreads, 0, st>>>(D); break;
+    case RES_X_SETUP: launch_dependent(k_res_cross<RES_X_SETUP>, g_grid_tiles, kVecThreads, st, D); break;
+    case RES_X_DEMOTE_R: launch_dependent(k_res_cross<RES_X_DEMOTE_R>, g_grid_tiles, kVecThreads, st, D); break;
+    case RES_X_ADD_X: launch_dependent(k_res_cross<RES_X_ADD_X>, g_grid_tiles, kVecThreads, st, D); break;
+    default: launch_dependent(k_res_cross<RES_X_DEMOTE_X>, g_grid_tiles, kVecThreads, st, D); break;
+  }
 }
 
 void launch_step_kernel_f32(StepKernel k, const Dir &D, cudaStream_t st, const SyncOps *ops, int iarg, double darg,
@@ -2602,7 +2629,7 @@ const char *step_kernel_name(StepKernel k) {
                                 "k_res_seed", "k_res_w",    "k_res_vec",     "k_res_db",   "k_res_dj",
                                 "k_res_q",    "k_res_dot",  "k_res_sum",     "k_res_copyb", "k_res_bupdate",
                                 "k_res_cg",   "k_res_pupd_e", "k_phys",      "k_sing_setup", "k_sing_emf",
-                                "k_sing_j",   "k_res_clearb", "k_res_cg_sum"};
+                                "k_sing_j",   "k_res_clearb"};
   static_assert(sizeof(names) / sizeof(names[0]) == SK_COUNT, "a name per kernel");
   return (k >= 0 && k < SK_COUNT) ? names[k] : "?";
 }

@@ -15,9 +15,7 @@ enum StepKernel {
   // grids with physical boundaries and singular edges
   SK_PHYS, SK_SING_SETUP, SK_SING_EMF, SK_SING_J,
   // implicit resistive substep on grids with physical boundaries: zero the ghost faces of dB
-  SK_RES_CLEARB,
-  // the batched CG's per-solve sums
-  SK_RES_CGSUM, SK_COUNT
+  SK_RES_CLEARB, SK_COUNT
 };
 
 // One launch of k_sync runs up to two independent sync operations: a copy
@@ -43,7 +41,7 @@ enum ResCopyOp { RES_SNAPSHOT = 0, RES_RESTORE };
 
 // CG state of one solve on the device (one per slot), for the iteration
 // loop run as a CUDA graph over every masked solve at once (k_res_cg,
-// k_res_cg_sum, k_res_pupd_e): the host sets tol_factor and max_it (and
+// k_res_pupd_e): the host sets tol_factor and max_it (and
 // zeros the rest) before the graph and reads it back after.
 struct ResCG {
   double rho, alpha, beta;  // W-weighted r.r, step length, direction update
@@ -52,32 +50,23 @@ struct ResCG {
   int it, max_it;           // iterations taken, at most max_it
   int done, converged;      // loop over (converged, max_it reached, or breakdown)
 };
-// The loop's shared counters: slots of k_res_cg_sum reported, solves still iterating.
-struct ResCtl {
-  unsigned int arrivals;
-  int running;
-};
 // Steps of k_res_cg: CG_INIT: x = 0, p = r, E = p, (r.r)_W and r.r, sets rho, r0, tol;
 // CG_PQ: q = A p (its last part, E - eta dJ) and (p.q)_W, sets alpha;
 // CG_RR: x += alpha p, r -= alpha q, (r.r)_W and r.r, the stop test and beta.
-// k_res_cg writes one partial pair per warp and tile; k_res_cg_sum
-// (kCgChunks CTAs per slot) sums a solve's pairs in fixed chunks and a fixed
-// order and updates its state; a solve whose loop is over leaves the mask.
+// Every tile writes its pair of partial sums; the CTA that finishes a solve's
+// last tile adds them in a fixed order and updates the solve's state; a solve
+// whose loop is over leaves the mask.
 enum ResCgOp { CG_INIT = 0, CG_PQ, CG_RR };
-constexpr int kWarpsPerTile = kTileThreads / 32;
-constexpr int kCgChunks = 32;
 
 // Scratch of the CG dot products: per-CTA partial sums and the two results
-// (k_res_dot, one masked solve); the per-slot CG states, the per-warp tile
-// partials of the batched loop, its counters and the graph's loop condition.
+// (k_res_dot, one masked solve); the per-slot CG states, the tile partials of
+// the batched loop, its tickets and the graph's loop condition.
 struct ResScratch {
   double *partial;  // 2 * grid
   double *result;   // 2
   ResCG *cg = nullptr;
-  double *tpartial = nullptr;  // 2 per warp of every kResK tile
-  ResCtl *ctl = nullptr;
-  double *chunks = nullptr;           // 2 per chunk of every slot (k_res_cg_sum)
-  unsigned int *sarrivals = nullptr;  // per slot: its chunks summed so far
+  double *tpartial = nullptr;         // 2 per kResK tile
+  unsigned int *sarrivals = nullptr;  // per slot: its tiles summed so far
   unsigned long long handle = 0;  // cudaGraphConditionalHandle of the loop
   int in_graph = 0;               // the CG kernels set the loop condition (launched inside the loop graph)
 };
