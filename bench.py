@@ -60,9 +60,7 @@ L2_BYTES = 126 * 1024 * 1024
 # allocated cells.
 KERNEL_COMPS = {
     "k_face_emf": (3 + 3 + 3 + 9 + 2 + 1 + 9 + 3, 0),        # B, Badd, UCON, p x2, grad coef -> Eface, node p_e, grad p_e
-    "k_edge_emf": (9 + 3 + 3 + 1 + 2 + 3, 0),                # Eface, UCON, B, node p_e, rho x2 -> E
-    "k_hall_edge": (3 + 1 + 9 + 6 + 3 + 3 + 3, 0),           # EHC, beta, dr, Hall ratios, B, taper -> Ehall
-    "k_add_hall": (3 + 3 + 3, 0),                            # E += Ehall
+    "k_edge_emf": (9 + 3 + 3 + 1 + 2 + 3 + 1 + 9 + 6 + 3 + 3 + 3, 0),  # Eface, UCON, B, node p_e, rho x2, EHC, beta, dr, Hall ratios, taper -> E, Ehall
     "k_fluid": (10 + 10 + 3 + 10 + 3 + 3 + 3 + 3 + 1 + 3 + 10, 0),  # U, PV, |JD|, JD + 1/Jac, grad p_e, U+, B_cell, J_cell, Photo, xyz -> U'
     "k_bface": (3 + 3 + 3, 0),                               # B += dt curl E
     "k_bcell_jedge": (3 + 3 + 18 + 3 + 3 + 3 + 3 + 3, 0),    # B, Badd, W_B, beta, alpha -> B_cell, Bind, J edges

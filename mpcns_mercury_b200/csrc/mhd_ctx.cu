@@ -163,6 +163,9 @@ struct Tables {
   // Every halo, staged and physical write of Sync(Eres) and Sync(Jedge) lands
   // on a ghost position (res_light_syncs)
   bool res_ghost_writes_only = false;
+  // Some write of the E alias reduction, the singular edges or Sync(Ehall) lands
+  // on an edge inside a block (hall_writes_inside)
+  bool hall_late = false;
 };
 
 struct Solve {
@@ -243,6 +246,7 @@ struct mhd_batch {
   int *dprefix_copy[kMaxGroups][kNumPhases] = {};
   int *dprefix_phys[kNumPhys] = {};
   int *dprefix_sing = nullptr;
+  unsigned int *tickets = nullptr;  // Dir::tickets
   int *dprefix_aliasE = nullptr, *dprefix_aliasJ = nullptr;
   cudaGraphExec_t graph = nullptr;
   cudaGraphExec_t graph_a = nullptr, graph_b = nullptr;  // the step split around implicit resistive solves
@@ -279,6 +283,7 @@ struct mhd_batch {
   int snap_next = 0;
   // eager profiling
   bool profiling = false;
+  bool after_flip = false;  // the last kernel launched was k_bface
   int fluid_tile = 0;  // the fluid kernel's tile variant (fluid_tile)
   std::vector<cudaEvent_t> prof_events;
   std::vector<const char *> prof_names;
@@ -297,6 +302,7 @@ struct mhd_batch {
     d.aliasJ_prefix = dprefix_aliasJ;
     for (int q = 0; q < kNumPhys; ++q) d.phys_prefix[q] = dprefix_phys[q];
     d.sing_prefix = dprefix_sing;
+    d.tickets = tickets;
     return d;
   }
 };
@@ -321,7 +327,8 @@ void mark(mhd_batch *b, const char *name) {
 
 void launch(mhd_batch *b, int mode, StepKernel k, int *nk, const SyncOps *ops = nullptr, int iarg = 0,
             double darg = 0.0) {
-  launch_step_kernel(k, b->dir(mode), b->stream, ops, b->precision, iarg, darg, b->res);
+  launch_step_kernel(k, b->dir(mode), b->stream, ops, b->precision, iarg, darg, b->res, b->after_flip);
+  b->after_flip = k == SK_BFACE;  // it flips the solves' states, which the next kernels read ahead of their wait
   ++*nk;
   mark(b, step_kernel_name(k));
 }
@@ -388,7 +395,7 @@ void enqueue_sync(mhd_batch *b, int mode, int g, int *nk, bool full = false) {
 // Sync(Jedge), in the same order per field as the reference; the singular
 // edges' current replaces their owners' after the alias reduction
 // (Calc_J_Edge, Z4_Mercury/src/physics/MercurySolver_Current.cpp:140-201).
-void enqueue_derived(mhd_batch *b, int mode, int *nk) {
+void enqueue_derived(mhd_batch *b, int mode, int *nk, bool end_of_step = false) {
   launch(b, mode, SK_BCELL_JEDGE, nk);
   sync_pre(b, mode, MHD_SYNC_B_CELL, nk);
   sync2(b, mode, copy_op(MHD_SYNC_B_CELL, kPhHalo), alias_op(1), nk);
@@ -400,7 +407,7 @@ void enqueue_derived(mhd_batch *b, int mode, int *nk) {
   sync1(b, mode, copy_op(MHD_SYNC_JEDGE, kPhOwner), nk);
   launch(b, mode, SK_JCELL, nk);
   enqueue_sync(b, mode, MHD_SYNC_J_CELL, nk);
-  launch(b, mode, SK_PV_UPLUS, nk);
+  launch(b, mode, SK_PV_UPLUS, nk, nullptr, end_of_step);
 }
 
 // StepOnce (Z4_Mercury/src/MercurySolver_Driver.cpp:21-61) for every active slot, in two
@@ -412,7 +419,6 @@ void enqueue_step_a(mhd_batch *b, int *nk) {
   // AssembleRHS_Induction_CT_ (Z4_Mercury/src/physics/MercurySolver_MagneticRHS.cpp:90-171)
   launch(b, m, SK_FACE_EMF, nk);
   launch(b, m, SK_EDGE_EMF, nk);
-  launch(b, m, SK_HALL_EDGE, nk);
   if (b->live_sing > 0 || b->live_phys[MHD_SYNC_EHALL] > 0 || b->live_tables[MHD_SYNC_EHALL][kPhStash] > 0) {
     // the E alias reduction, the singular edges' EMF and Hall EMF, Sync(Ehall)
     sync1(b, m, alias_op(0), nk);
@@ -422,14 +428,13 @@ void enqueue_step_a(mhd_batch *b, int *nk) {
     sync2(b, m, alias_op(0), copy_op(MHD_SYNC_EHALL, kPhHalo), nk);
     sync1(b, m, copy_op(MHD_SYNC_EHALL, kPhOwner), nk);
   }
-  launch(b, m, SK_ADD_HALL, nk);
+  launch(b, m, SK_ADD_HALL, nk);  // on the edges in the blocks' faces
   phys1(b, m, kMaxGroups, nk);  // the wall EMF: E_t = 0 on solid-wall edges
   enqueue_sync(b, m, MHD_SYNC_EEDGE, nk);
   // AssembleRHS_Fluid_ + ApplyUpdate_Euler_ (state into the other buffer) and
   // the constrained-transport face update (Z4_Mercury/src/physics/MercurySolver_Advance.cpp:73-147)
   launch(b, m, SK_FLUID, nk, nullptr, b->fluid_tile);
   launch(b, m, SK_BFACE, nk);
-  launch(b, m, SK_FLIP, nk);
   // the reference's Sync(Ucell) reads ghosts it does not overwrite first at
   // their values from the previous sync, which after the flip are in the
   // other buffer
@@ -443,8 +448,7 @@ void enqueue_step_a(mhd_batch *b, int *nk) {
 void enqueue_step_b(mhd_batch *b, int *nk, bool resync_b) {
   const int m = 0;
   if (resync_b) enqueue_sync(b, m, MHD_SYNC_BFACE, nk);
-  enqueue_derived(b, m, nk);
-  launch(b, m, SK_RETIRE, nk);
+  enqueue_derived(b, m, nk, true);
 }
 void enqueue_step(mhd_batch *b, int *nk) {
   enqueue_step_a(b, nk);
@@ -499,6 +503,7 @@ int publish(mhd_batch *b) {
     d.arena = S->arena;
     d.ubuf = S->ubuf;
     d.nblocks = S->nblocks;
+    d.hall_late = S->T->hall_late;
     for (int r = 0; r < kNumRanges; ++r) d.tile_prefix[r] = S->T->dtile_prefix[r];
     if (S->dres_prefix) d.tile_prefix[kResK] = S->dres_prefix;
     for (int g = 0; g < kMaxGroups; ++g)
@@ -1477,7 +1482,10 @@ int mhd_batch_create(int capacity, int precision, mhd_batch **out) {
       if (cudaMalloc(&b->dprefix_copy[g][p], sizeof(int) * C1) != cudaSuccess) return bail(fail(MHD_ERR_OOM, "prefix"));
   for (int q = 0; q < kNumPhys; ++q)
     if (cudaMalloc(&b->dprefix_phys[q], sizeof(int) * C1) != cudaSuccess) return bail(fail(MHD_ERR_OOM, "prefix"));
-  if (cudaMalloc(&b->dprefix_sing, sizeof(int) * C1) != cudaSuccess) return bail(fail(MHD_ERR_OOM, "prefix"));
+  if (cudaMalloc(&b->dprefix_sing, sizeof(int) * C1) != cudaSuccess ||
+      cudaMalloc(&b->tickets, sizeof(unsigned int) * 2) != cudaSuccess ||
+      cudaMemsetAsync(b->tickets, 0, sizeof(unsigned int) * 2, b->stream) != cudaSuccess)
+    return bail(fail(MHD_ERR_OOM, "prefix"));
   if (cudaMalloc(&b->dprefix_aliasE, sizeof(int) * C1) != cudaSuccess ||
       cudaMalloc(&b->dprefix_aliasJ, sizeof(int) * C1) != cudaSuccess)
     return bail(fail(MHD_ERR_OOM, "prefix"));
@@ -1531,6 +1539,7 @@ int mhd_batch_destroy(mhd_batch *b) {
     for (int p = 0; p < kNumPhases; ++p) cudaFree(b->dprefix_copy[g][p]);
   for (int q = 0; q < kNumPhys; ++q) cudaFree(b->dprefix_phys[q]);
   cudaFree(b->dprefix_sing);
+  cudaFree(b->tickets);
   cudaFree(b->dprefix_aliasE);
   cudaFree(b->dprefix_aliasJ);
   for (auto e : b->prof_events) cudaEventDestroy(e);
@@ -1689,6 +1698,39 @@ static bool res_ghost_writes_only(const Solve *S, const mhd_desc *desc) {
   }
   return true;
 }
+
+// Whether the E alias reduction, the singular edges' EMF or Sync(Ehall) writes
+// an owned edge that does not lie in one of its block's faces: E + Ehall may
+// then not be summed ahead of them (k_edge_emf).  False on every grid whose
+// blocks meet in their faces.
+static bool hall_writes_inside(const Solve *S, const mhd_desc *desc) {
+  auto inside = [&](int axis, const mhd_dof &d) {
+    if (d.block < 0 || d.block >= S->nblocks) return false;
+    const int *n = S->boxes[d.block].n;
+    const int q[3] = {d.i, d.j, d.k};
+    for (int a = 0; a < 3; ++a)
+      if (a == axis ? (q[a] < 0 || q[a] >= n[a]) : (q[a] <= 0 || q[a] >= n[a])) return false;
+    return true;
+  };
+  auto hall = [&](const mhd_dof &d) {
+    return d.field >= MHD_EHALL_XI && d.field <= MHD_EHALL_ZETA && inside(d.field - MHD_EHALL_XI, d);
+  };
+  const mhd_sync_group &g = desc->groups[MHD_SYNC_EHALL];
+  for (int q = 0; q < g.n_halo; ++q)
+    if (hall(g.halo[q].dst)) return true;
+  for (int q = 0; q < g.n_owner; ++q)
+    if (hall(g.owner[q].dst)) return true;
+  for (int q = 0; q < 2 * g.n_stash; ++q)
+    if (hall(g.stash[q].dst)) return true;
+  for (int q = 0; q < g.n_phys; ++q)
+    if (hall(g.phys[q].dst)) return true;
+  for (int c = 0; c < desc->edge_aliases.n_classes; ++c)
+    if (inside(desc->edge_aliases.owner[c].field, desc->edge_aliases.owner[c])) return true;
+  for (int e = 0; e < desc->singular.n_edges; ++e)
+    if (inside(desc->singular.owner[e].field, desc->singular.owner[e])) return true;
+  return false;
+}
+
 
 static int upload_phys(Solve *S, const mhd_desc *desc, cudaStream_t st) {
   for (int q = 0; q < kNumPhys; ++q) {
@@ -2013,11 +2055,13 @@ static int add_solve(mhd_batch *b, const mhd_desc *desc, bool periodic, int *slo
   try {
     if (periodic) {
       if ((rc = upload_groups_periodic(S, st)) || (rc = upload_aliases_periodic(S, st))) return bail(rc);
+      S->T->res_ghost_writes_only = true;  // a periodic block's halo copies write ghosts
     } else {
       if ((rc = upload_groups(S, desc->groups, st))) return bail(rc);
       if ((rc = upload_aliases(S, desc->edge_aliases, st))) return bail(rc);
       if ((rc = upload_phys(S, desc, st))) return bail(rc);
       if ((rc = upload_singular(S, desc->singular, st)) || (rc = alloc_singular_geo(S, st))) return bail(rc);
+      S->T->hall_late = hall_writes_inside(S, desc);
       if (S->consts.resistive) {
         S->T->res_kdown = res_kdown(desc);
         S->T->res_ghost_writes_only = res_ghost_writes_only(S, desc);

@@ -264,6 +264,7 @@ struct DevSolve {
   char *arena;                        // base of the sync codes
   int64_t ubuf;                       // bytes per U buffer
   int nblocks;
+  int hall_late;                      // E += Ehall on every edge after Sync(Ehall), not ahead of it inside the blocks
   const int *tile_prefix[kNumRanges]; // per range: nblocks + 1 prefix sums of tile counts
   DevTable tab[kMaxGroups][kNumPhases];
   DevAlias aliasE, aliasJ;
@@ -291,6 +292,7 @@ struct Dir {
   // prefix sums over the solves
   const int *phys_prefix[kNumPhys];
   const int *sing_prefix;
+  unsigned int *tickets;  // two zeros: CTAs done of the kernels that end by changing every solve's state
 };
 
 template <class R>

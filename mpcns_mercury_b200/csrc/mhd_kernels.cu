@@ -169,6 +169,18 @@ __device__ __forceinline__ T *uniform(T *p) {
   return (T *)(((unsigned long long)hi << 32) | lo);
 }
 
+// Whether solve s is active and which U buffer is current.  In a step (mode 0)
+// they only change in its passes that end by them (flip_solve in k_bface,
+// retire_solve in k_pv_uplus), whose successors are launched after them in full,
+// so they may be read ahead of the wait; the mask of a targeted pass may not.
+struct Status {
+  int active, cur;
+};
+__device__ __forceinline__ Status status_of(const Dir &D, int s) {
+  const SolveState &st = D.state[s];
+  return Status{D.mode ? st.mask != 0 : st.remaining != 0, st.cur};
+}
+
 // The work item (s, b, t) of range KIND as this thread sees it, and the
 // block's fields of the current step.
 template <class R, int KIND>
@@ -444,13 +456,33 @@ __device__ __forceinline__ void for_vec_items(const Dir &D, F &&f) {
     VV<R> B;
     build_vec_item<R, KIND>(D, s, b, t, it, B);
     it.w = w;
+    Status st{};
+    if (D.mode == 0) st = status_of(D, s);
     if (w == (int)blockIdx.x) wait_for_predecessors();
-    if (uniform((int)solve_active(D, s))) {
-      use_current(B, uniform(D.state[s].cur));
+    if (D.mode != 0) st = status_of(D, s);
+    if (uniform(st.active)) {
+      use_current(B, uniform(st.cur));
       f(D.solves[s], B, it);
     }
     __syncthreads();
   }
+}
+// Runs f(state) for every solve once all CTAs of this kernel that had tiles of
+// range KIND have done them (a ticket): the last of them does it.
+template <int KIND, class F>
+__device__ __forceinline__ void after_all_tiles(const Dir &D, unsigned int *ticket, F &&f) {
+  const int total = D.solve_tile_prefix[KIND][D.nsolves];
+  if ((int)blockIdx.x >= total) return;
+  __shared__ int last;
+  if (threadIdx.x == 0) {  // the CTA's tiles are done (for_vec_items ends in a barrier)
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == (unsigned)min(total, (int)gridDim.x) - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int s = threadIdx.x; s < D.nsolves; s += blockDim.x) f(D.state[s]);
+  if (threadIdx.x == 0) *ticket = 0;
 }
 // The same, position by position: f(S, B, pos) (passes that run once per solve).
 struct Pos {
@@ -645,13 +677,18 @@ __device__ __forceinline__ Vec<R> add_artificial(const VV<R> &B, const ConstsT<R
 }
 
 // AssembleEdgeEMF_FromFaceE_Ideal_ (Ideal.cpp:138-372) + AddAmbipolarEdgeEMF_
-// (Z4_Mercury/src/physics/MercurySolver_MagExplicit_Ambipo.cpp:3-143) on the owned edges.
+// (Z4_Mercury/src/physics/MercurySolver_MagExplicit_Ambipo.cpp:3-143), then the Hall EMF
+// (BuildHallFaceEMF_Rusanov_diff_ steps 2-4, Hall.cpp:148-400) on the owned
+// edges.  An edge inside the block has no alias: its sum E + Ehall
+// (MercurySolver_MagneticRHS.cpp:135-147) is written at once, so only the edges
+// on the block's faces wait for the alias reduction and k_add_hall.
 template <class R>
-__global__ void __launch_bounds__(kVecThreads, 4) k_edge_emf(Dir D) {
+__global__ void __launch_bounds__(kVecThreads, 3) k_edge_emf(Dir D) {
   for_vec_items<R, kBox>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
     const ConstsT<R> &c = consts_of<R>(S);
     const uint32_t o = it.o, di = B.di, dj = B.dj;
     const R Cuct = R(0.5);
+    Vec<R> E[3];
     const R pc = c.pe_coeff;
     auto lowk = [&](const Vec<R> &v, int comp, uint32_t q) { return B.lower(v, comp, q); };
     // max |u^a| over the four cells at an edge: this row, the row below along
@@ -696,7 +733,7 @@ __global__ void __launch_bounds__(kVecThreads, 4) k_edge_emf(Dir D) {
       const Vec<R> d2 = by - lowk(by, cBY, o);
       Vec<R> e = Ec + Cuct * (R(0.5) * ae * d1 - R(0.5) * az * d2);
       if (ambi) e = e - pc * (B.lv(cPEN, o + di) - pn) / ne_of(rho_k(cUH, dj), rho_k(cUN, dj));
-      B.st(cEX, it, add_artificial(B, c, 0, o, e), 0, B.n2 + 1, it.i < B.n0);
+      E[0] = add_artificial(B, c, 0, o, e);
     }
     {
       const Vec<R> fx = B.lv(cEFX + 1, o), bx = B.lv(cBX, o);
@@ -706,7 +743,7 @@ __global__ void __launch_bounds__(kVecThreads, 4) k_edge_emf(Dir D) {
       const Vec<R> d2 = B.lv(cBZ, o) - B.lv(cBZ, o - di);
       Vec<R> e = Ec + Cuct * (R(0.5) * az * d1 - R(0.5) * ax * d2);
       if (ambi) e = e - pc * (B.lv(cPEN, o + dj) - pn) / ne_of(rho_k(cUH, di), rho_k(cUN, di));
-      B.st(cEY, it, add_artificial(B, c, 1, o, e), 0, B.n2 + 1, it.j < B.n1);
+      E[1] = add_artificial(B, c, 1, o, e);
     }
     {
       const Vec<R> Ec =
@@ -716,17 +753,17 @@ __global__ void __launch_bounds__(kVecThreads, 4) k_edge_emf(Dir D) {
       const Vec<R> d2 = B.lv(cBX, o) - B.lv(cBX, o - dj);
       Vec<R> e = Ec + Cuct * (R(0.5) * ax * d1 - R(0.5) * ae * d2);
       if (ambi) e = e - pc * (B.upper(pn, cPEN, o) - pn) / ne_of(rho_ij(cUH), rho_ij(cUN));
-      B.st(cEZ, it, add_artificial(B, c, 2, o, e), 0, B.n2);
+      E[2] = add_artificial(B, c, 2, o, e);
     }
-  });
-}
-
-// ------------------------------------------------------------------ Hall EMF
-// BuildHallFaceEMF_Rusanov_diff_ steps 2-4 (Hall.cpp:148-400).
-template <class R>
-__global__ void __launch_bounds__(kVecThreads, 3) k_hall_edge(Dir D) {
-  for_vec_items<R, kBox>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
-    const uint32_t o = it.o, di = B.di, dj = B.dj;
+    // E_Hall of family ax, and E: with it inside the block, without on its faces
+    const bool late = S.hall_late != 0;
+    auto put = [&](int ax, const Vec<R> &h, int hi, bool owned, bool face, bool kfaces) {
+      B.st(cHX + ax, it, h, 0, hi, owned);
+      B.st(cEX + ax, it, vmap<R>([&](int e) {
+             const bool f = face || (kfaces && (it.k + e == 0 || it.k + e == B.n2));
+             return f ? E[ax].v[e] : E[ax].v[e] + h.v[e];
+           }), 0, hi, owned);
+    };
     const R Cwh = R(0.1);
     // over the four cells at an edge, in the reference's order: lower row and
     // lower k first
@@ -752,33 +789,51 @@ __global__ void __launch_bounds__(kVecThreads, 3) k_hall_edge(Dir D) {
       const Vec<R> Ecen = mean_k(cEHC, dj) * B.lv(cDRX, o) + mean_k(cEHC + 1, dj) * B.lv(cDRX + 1, o) +
                           mean_k(cEHC + 2, dj) * B.lv(cDRX + 2, o);
       const Vec<R> by = B.lv(cBY, o);
-      B.st(cHX, it, tail(0, Ecen, max_k(cHB, dj), B.lv(cBZ, o) - B.lv(cBZ, o - dj), by - B.lower(by, cBY, o)), 0,
-           B.n2 + 1, it.i < B.n0);
+      put(0, tail(0, Ecen, max_k(cHB, dj), B.lv(cBZ, o) - B.lv(cBZ, o - dj), by - B.lower(by, cBY, o)), B.n2 + 1, it.i < B.n0,
+          late || it.j == 0 || it.j == B.n1, true);
     }
     {
       const Vec<R> Ecen = mean_k(cEHC, di) * B.lv(cDRY, o) + mean_k(cEHC + 1, di) * B.lv(cDRY + 1, o) +
                           mean_k(cEHC + 2, di) * B.lv(cDRY + 2, o);
       const Vec<R> bx = B.lv(cBX, o);
-      B.st(cHY, it, tail(1, Ecen, max_k(cHB, di), bx - B.lower(bx, cBX, o), B.lv(cBZ, o) - B.lv(cBZ, o - di)), 0,
-           B.n2 + 1, it.j < B.n1);
+      put(1, tail(1, Ecen, max_k(cHB, di), bx - B.lower(bx, cBX, o), B.lv(cBZ, o) - B.lv(cBZ, o - di)), B.n2 + 1, it.j < B.n1,
+          late || it.i == 0 || it.i == B.n0, true);
     }
     {
       const Vec<R> Ecen =
           mean_ij(cEHC) * B.lv(cDRZ, o) + mean_ij(cEHC + 1) * B.lv(cDRZ + 1, o) + mean_ij(cEHC + 2) * B.lv(cDRZ + 2, o);
       const Vec<R> be = vmax(vmax(B.lv(cHB, o - di - dj), B.lv(cHB, o - di)), vmax(B.lv(cHB, o - dj), B.lv(cHB, o)));
-      B.st(cHZ, it, tail(2, Ecen, be, B.lv(cBY, o) - B.lv(cBY, o - di), B.lv(cBX, o) - B.lv(cBX, o - dj)), 0, B.n2);
+      put(2, tail(2, Ecen, be, B.lv(cBY, o) - B.lv(cBY, o - di), B.lv(cBX, o) - B.lv(cBX, o - dj)), B.n2, true,
+          late || it.i == 0 || it.i == B.n0 || it.j == 0 || it.j == B.n1, false);
     }
   });
 }
 
-// E += Ehall on owned edges (Z4_Mercury/src/physics/MercurySolver_MagneticRHS.cpp:135-147).
+// E += Ehall (Z4_Mercury/src/physics/MercurySolver_MagneticRHS.cpp:135-147) on the owned
+// edges that lie in the block's faces (k_edge_emf has summed the others).
 template <class R>
 __global__ void __launch_bounds__(kVecThreads) k_add_hall(Dir D) {
   for_vec_items<R, kBox>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
+    const bool late = S.hall_late != 0;  // every edge
+    const bool fi = late || it.i == 0 || it.i == B.n0, fj = late || it.j == 0 || it.j == B.n1;
+    const bool k0 = it.k <= 0, k1 = it.k <= B.n2 && it.k + Vec<R>::N > B.n2;
+    if (!it.in || !(fi || fj || k0 || k1)) return;
     // each thread reads and writes its own positions only
-    B.st(cEX, it, B.own(cEX, it.o) + B.lv(cHX, it.o), 0, B.n2 + 1, it.i < B.n0);
-    B.st(cEY, it, B.own(cEY, it.o) + B.lv(cHY, it.o), 0, B.n2 + 1, it.j < B.n1);
-    B.st(cEZ, it, B.own(cEZ, it.o) + B.lv(cHZ, it.o), 0, B.n2);
+    auto add = [&](int ax, int lo, int hi, bool cond) {
+      B.st(cEX + ax, it, B.own(cEX + ax, it.o) + B.lv(cHX + ax, it.o), lo, hi, cond);
+    };
+    // family xi: on the eta faces whole rows, else the ends of the row; eta likewise; zeta: whole rows
+    if (it.i < B.n0) {
+      add(0, 0, B.n2 + 1, fj);
+      add(0, 0, 1, !fj && k0);
+      add(0, B.n2, B.n2 + 1, !fj && k1);
+    }
+    if (it.j < B.n1) {
+      add(1, 0, B.n2 + 1, fi);
+      add(1, 0, 1, !fi && k0);
+      add(1, B.n2, B.n2 + 1, !fi && k1);
+    }
+    if (fi || fj) add(2, 0, B.n2, true);
   });
 }
 
@@ -879,16 +934,16 @@ __global__ void __launch_bounds__(fluid_threads(VT), fluid_ctas(VT, sizeof(R))) 
     __syncthreads();
     const int is = sh[0], ib = sh[1], t = sh[2];
     __syncthreads();
-    if (q == (int)blockIdx.x) wait_for_predecessors();
-    if (!solve_active(D, is)) continue;  // inactive solve (the whole CTA agrees)
     Item it;
     V<R> B;
     build_item<R, KIND>(D, is, ib, t, it, B);
+    if (q == (int)blockIdx.x) wait_for_predecessors();
+    if (!solve_active(D, is)) continue;  // inactive solve (the whole CTA agrees)
     it.i += part;
     const DevSolve &S = D.solves[is];
     const ConstsT<R> &c = consts_of<R>(S);
     const R dt = __longlong_as_double((long long)D.state[it.s].dt_bits);
-    // the reference aborts; k_flip records the status (and a solve with a
+    // the reference aborts; flip_solve records the status (and a solve with a
     // non-finite cell is not advanced)
     if (!(dt >= R(1e-7)) || !isfinite(dt) || D.state[it.s].nonfinite || !it.in || it.i >= it.hi[0]) continue;
     const int j = it.j, k = it.k;
@@ -1009,12 +1064,40 @@ __global__ void __launch_bounds__(fluid_threads(VT), fluid_ctas(VT, sizeof(R))) 
   }
 }
 
-// B_face += dt * (-curl E) on the owned faces (CTOperators.cpp:6-56 with multiplier -1).
+// After the updates: flip the state buffer, account time/step
+// (Z4_Mercury/src/MercurySolver_Driver.cpp:40-45), record a dt failure (the
+// reference's exit(-1), Timestep.cpp:129-140) and re-arm the dt reduction.
+__device__ __forceinline__ void flip_solve(SolveState &st) {
+  if (!st.remaining) return;
+  if (st.nonfinite) {  // a NaN/Inf cell: retire the solve, the others go on
+    st.status = MHD_ERR_NONFINITE;
+    st.remaining = 0;
+    return;
+  }
+  const double dt = __longlong_as_double((long long)st.dt_bits);
+  if (!(dt >= 1e-7) || !isfinite(dt)) {
+    st.status = MHD_ERR_DT;
+    st.remaining = 0;
+    return;
+  }
+  st.cur ^= 1;
+  st.dt = dt;
+  st.time += dt;
+  st.step += 1;
+  st.dt_bits = (unsigned long long)__double_as_longlong(1e100);
+}
+// End of a step: one step fewer to go (after every pass of the step has run).
+__device__ __forceinline__ void retire_solve(SolveState &st) {
+  if (st.remaining > 0) st.remaining -= 1;
+}
+
+// B_face += dt * (-curl E) on the owned faces (CTOperators.cpp:6-56 with multiplier -1),
+// and, the fluid update before it being complete, the flip of every solve's state.
 template <class R>
 __global__ void __launch_bounds__(kVecThreads) k_bface(Dir D) {
   for_vec_items<R, kBox>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
     const R dt = __longlong_as_double((long long)D.state[it.s].dt_bits);
-    if (uniform((int)(!(dt >= R(1e-7)) || !isfinite(dt) || D.state[it.s].nonfinite))) return;  // k_flip records the status
+    if (uniform((int)(!(dt >= R(1e-7)) || !isfinite(dt) || D.state[it.s].nonfinite))) return;  // flip_solve records the status
     const uint32_t o = it.o, di = B.di, dj = B.dj;
     const bool ic = it.i < B.n0, jc = it.j < B.n1;
     const Vec<R> ex = B.lv(cEX, o), ey = B.lv(cEY, o), ez = B.lv(cEZ, o);
@@ -1031,6 +1114,7 @@ __global__ void __launch_bounds__(kVecThreads) k_bface(Dir D) {
       B.st(cBZ, it, B.own(cBZ, o) + dt * rb, 0, B.n2 + 1, ic && jc);
     }
   });
+  after_all_tiles<kBox>(D, D.tickets, [](SolveState &st) { flip_solve(st); });
 }
 
 // ------------------------------------------------------------------ derived fields
@@ -1759,9 +1843,9 @@ __global__ void __launch_bounds__(kVecThreads) k_face_normals(Dir D) {
 // cell range the step keeps, the fluid fluxes' cell terms, the contravariant
 // velocities UCON and the next step's Hall cell field there, and the next
 // step's CFL dt on owned cells (warp min, one atomicMin per warp on the bit
-// pattern of the positive double).
+// pattern of the positive double).  The step's last pass ends it (retire_solve).
 template <class R>
-__global__ void __launch_bounds__(kVecThreads, 4) k_pv_uplus(Dir D) {
+__global__ void __launch_bounds__(kVecThreads, 4) k_pv_uplus(Dir D, int end_of_step) {
   for_vec_items<R, kAlloc>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
     constexpr int N = Vec<R>::N;
     const ConstsT<R> &c = consts_of<R>(S);
@@ -1866,6 +1950,7 @@ __global__ void __launch_bounds__(kVecThreads, 4) k_pv_uplus(Dir D) {
       atomicMin(&D.state[it.s].dt_bits, (unsigned long long)__double_as_longlong(dtl));
     if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicExch(&D.state[it.s].nonfinite, 1);
   });
+  if (end_of_step) after_all_tiles<kAlloc>(D, D.tickets + 1, [](SolveState &st) { retire_solve(st); });
 }
 
 #undef AT
@@ -1929,10 +2014,32 @@ __global__ void __launch_bounds__(256) k_sync(Dir D, SyncOps ops) {
       scode = w[1];
       rw = w[2];
     }
+    // a class's first members (most have two or four)
+    constexpr int kAhead = 4;
+    int m0 = 0, m1 = 0;
+    int64_t mcode[kAhead], ocode = 0;
+    double msign[kAhead], osign = 0.0;
+    const int cls = q * 8 + lane;
+    const bool alias = !copy && cls < A.n;
+    if (alias) {
+      m0 = A.offset[cls];
+      m1 = A.offset[cls + 1];
+      ocode = A.owner[cls];
+      osign = A.osign[cls];
+#pragma unroll
+      for (int m = 0; m < kAhead; ++m) {
+        const bool has = m0 + m < m1;
+        mcode[m] = has ? A.member[m0 + m] : ocode;
+        msign[m] = has ? A.msign[m0 + m] : 0.0;
+      }
+    }
+    Status st{};
+    if (D.mode == 0) st = status_of(D, s);
     if (first) wait_for_predecessors();
     first = false;
-    if (!solve_active(D, s)) continue;
-    const int cur = D.state[s].cur;
+    if (D.mode != 0) st = status_of(D, s);
+    if (!st.active) continue;
+    const int cur = st.cur;
     if (copy) {
       const int len = (int)((dcode >> kSegLenShift) & 31) + 1;
       const int n = len * ((int)(rw & 0xffff) + 1);
@@ -1955,13 +2062,16 @@ __global__ void __launch_bounds__(256) k_sync(Dir D, SyncOps ops) {
 #pragma unroll
       for (int u = 0; u < kSegElems / 8; ++u)
         if (lane + 8 * u < n) *(R *)(dst + off[u]) = op.mark ? R(0.0) : (neg ? -v[u] : v[u]);
-    } else {
-      const int c = q * 8 + lane;
-      if (c < A.n) {
-        R sum = R(0.0);
-        for (int m = A.offset[c]; m < A.offset[c + 1]; ++m) sum += R(A.msign[m]) * *at_code<R>(S, cur, A.member[m]);
-        *at_code<R>(S, cur, A.owner[c]) = R(A.osign[c]) * sum / (R)(A.offset[c + 1] - A.offset[c]);
-      }
+    } else if (alias) {
+      R v[kAhead];
+#pragma unroll
+      for (int m = 0; m < kAhead; ++m) v[m] = *at_code<R>(S, cur, mcode[m]);
+      R sum = R(0.0);
+#pragma unroll
+      for (int m = 0; m < kAhead; ++m)
+        if (m0 + m < m1) sum += R(msign[m]) * v[m];
+      for (int m = m0 + kAhead; m < m1; ++m) sum += R(A.msign[m]) * *at_code<R>(S, cur, A.member[m]);
+      *at_code<R>(S, cur, ocode) = R(osign) * sum / (R)(m1 - m0);
     }
   }
 }
@@ -2262,44 +2372,6 @@ __global__ void k_sing_j(Dir D) {
 #undef AT
 #undef ATM
 
-// After the updates: flip the state buffer, account time/step
-// (Z4_Mercury/src/MercurySolver_Driver.cpp:40-45), record a dt failure (the
-// reference's exit(-1), Timestep.cpp:129-140) and re-arm the dt reduction.
-__global__ void k_flip(Dir D) {
-  let_dependents_launch();
-  wait_for_predecessors();
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < D.nsolves; s += gridDim.x * blockDim.x) {
-    SolveState &st = D.state[s];
-    if (!st.remaining) continue;
-    if (st.nonfinite) {  // a NaN/Inf cell: retire the solve, the others go on
-      st.status = MHD_ERR_NONFINITE;
-      st.remaining = 0;
-      continue;
-    }
-    const double dt = __longlong_as_double((long long)st.dt_bits);
-    if (!(dt >= 1e-7) || !isfinite(dt)) {
-      st.status = MHD_ERR_DT;
-      st.remaining = 0;
-      continue;
-    }
-    st.cur ^= 1;
-    st.dt = dt;
-    st.time += dt;
-    st.step += 1;
-    st.dt_bits = (unsigned long long)__double_as_longlong(1e100);
-  }
-}
-
-// End of a step: one step fewer to go (after every pass of the step has run).
-__global__ void k_retire(Dir D) {
-  let_dependents_launch();
-  wait_for_predecessors();
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < D.nsolves; s += gridDim.x * blockDim.x) {
-    SolveState &st = D.state[s];
-    if (st.remaining > 0) st.remaining -= 1;
-  }
-}
-
 }  // namespace
 
 // ------------------------------------------------------------------ launchers
@@ -2318,12 +2390,13 @@ struct SameAs {
 template <class T>
 using Same = typename SameAs<T>::type;
 // A launch that may begin while its predecessor in the stream drains; the kernel
-// waits itself (wait_for_predecessors).
+// waits itself (wait_for_predecessors).  t_full: after it instead, in full.
+static thread_local bool t_full = false;
 template <class... P>
 static void launch_dependent(void (*fn)(P...), int grid, int threads, cudaStream_t st, Same<P>... args) {
   cudaLaunchAttribute a[1];
   a[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  a[0].val.programmaticStreamSerializationAllowed = 1;
+  a[0].val.programmaticStreamSerializationAllowed = t_full ? 0 : 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(threads);
@@ -2357,7 +2430,6 @@ static const void *kernel_fn(StepKernel k) {
   switch (k) {
     case SK_FACE_EMF: return (const void *)k_face_emf<R>;
     case SK_EDGE_EMF: return (const void *)k_edge_emf<R>;
-    case SK_HALL_EDGE: return (const void *)k_hall_edge<R>;
     case SK_ADD_HALL: return (const void *)k_add_hall<R>;
     case SK_FLUID: return fluid_fn<R>(0);
     case SK_BFACE: return (const void *)k_bface<R>;
@@ -2386,7 +2458,7 @@ static const void *kernel_fn(StepKernel k) {
 // Threads of a kernel's CTAs.
 static int kernel_threads(StepKernel k) {
   switch (k) {
-    case SK_FACE_EMF: case SK_EDGE_EMF: case SK_HALL_EDGE: case SK_ADD_HALL: case SK_BFACE: case SK_BCELL_JEDGE:
+    case SK_FACE_EMF: case SK_EDGE_EMF: case SK_ADD_HALL: case SK_BFACE: case SK_BCELL_JEDGE:
     case SK_JCELL: case SK_PV_UPLUS: case SK_FACE_NORMALS: case SK_DIVB: case SK_RES_SEED: case SK_RES_W:
     case SK_RES_VEC: case SK_RES_DB: case SK_RES_DJ: case SK_RES_Q: case SK_RES_BUPDATE: case SK_RES_CG:
     case SK_RES_PUPD_E:
@@ -2436,13 +2508,12 @@ static void launch_as(StepKernel k, const Dir &D, cudaStream_t st, const SyncOps
   switch (k) {
     case SK_FACE_EMF: launch_dependent(k_face_emf<R>, G, kVecThreads, st, D); break;
     case SK_EDGE_EMF: launch_dependent(k_edge_emf<R>, G, kVecThreads, st, D); break;
-    case SK_HALL_EDGE: launch_dependent(k_hall_edge<R>, G, kVecThreads, st, D); break;
     case SK_ADD_HALL: launch_dependent(k_add_hall<R>, G, kVecThreads, st, D); break;
     case SK_FLUID: launch_fluid<R>(iarg, D, st); break;  // iarg: the tile variant
     case SK_BFACE: launch_dependent(k_bface<R>, G, kVecThreads, st, D); break;
     case SK_BCELL_JEDGE: launch_dependent(k_bcell_jedge<R>, G, kVecThreads, st, D); break;
     case SK_JCELL: launch_dependent(k_jcell<R>, G, kVecThreads, st, D); break;
-    case SK_PV_UPLUS: launch_dependent(k_pv_uplus<R>, G, kVecThreads, st, D); break;
+    case SK_PV_UPLUS: launch_dependent(k_pv_uplus<R>, G, kVecThreads, st, D, iarg); break;
     case SK_SYNC: launch_dependent(k_sync<R>, G, kTileThreads, st, D, *ops); break;
     case SK_FACE_NORMALS: k_face_normals<R><<<G, kVecThreads, 0, st>>>(D); break;
     case SK_DIVB: k_div_b<R><<<G, kVecThreads, 0, st>>>(D); break;
@@ -2468,8 +2539,6 @@ static void launch_as(StepKernel k, const Dir &D, cudaStream_t st, const SyncOps
                          rs.in_graph);
       break;
     case SK_RES_PUPD_E: launch_dependent(k_res_pupd_e<R>, G, kVecThreads, st, D, rs.cg); break;
-    case SK_FLIP: launch_dependent(k_flip, 1, 128, st, D); break;
-    case SK_RETIRE: launch_dependent(k_retire, 1, 128, st, D); break;
     case SK_PHYS: launch_dependent(k_phys<R>, G, 256, st, D, iarg); break;
     // one thread per singular edge (8 radial lines of nr edges per shell)
     case SK_SING_SETUP: k_sing_setup<R><<<g_grid_tiles / 2, 64, 0, st>>>(D); break;
@@ -2564,6 +2633,7 @@ __global__ void __launch_bounds__(kVecThreads) k_res_cross(Dir D) {
 
 void launch_res_cross(const Dir &D, int op, cudaStream_t st) {
   grids<float>();
+  t_full = false;
   switch (op) {
     case RES_X_STATIC: k_res_cross_static<<<g_grid_tiles, kTileThreads, 0, st>>>(D); break;
     case RES_X_SETUP: launch_dependent(k_res_cross<RES_X_SETUP>, g_grid_tiles, kVecThreads, st, D); break;
@@ -2574,8 +2644,9 @@ void launch_res_cross(const Dir &D, int op, cudaStream_t st) {
 }
 
 void launch_step_kernel_f32(StepKernel k, const Dir &D, cudaStream_t st, const SyncOps *ops, int iarg, double darg,
-                            ResScratch rs) {
+                            ResScratch rs, bool full) {
   grids<float>();
+  t_full = full;
   launch_as<float>(k, D, st, ops, iarg, darg, rs);
 }
 
@@ -2598,14 +2669,15 @@ void launch_res_kmax(const Dir &D, int precision, int *out, cudaStream_t st) {
 }
 
 void launch_step_kernel_f32(StepKernel k, const Dir &D, cudaStream_t st, const SyncOps *ops, int iarg, double darg,
-                            ResScratch rs);
+                            ResScratch rs, bool full);
 
 void launch_step_kernel(StepKernel k, const Dir &D, cudaStream_t st, const SyncOps *ops, int precision, int iarg,
-                        double darg, ResScratch rs) {
+                        double darg, ResScratch rs, bool full) {
   if (precision == kMixed) {
-    launch_step_kernel_f32(k, D, st, ops, iarg, darg, rs);
+    launch_step_kernel_f32(k, D, st, ops, iarg, darg, rs, full);
   } else {
     grids<double>();
+    t_full = full;
     launch_as<double>(k, D, st, ops, iarg, darg, rs);
   }
 }
@@ -2623,9 +2695,9 @@ int res_dot_grid() {
 }
 
 const char *step_kernel_name(StepKernel k) {
-  static const char *names[] = {"k_face_emf", "k_edge_emf", "k_hall_edge", "k_add_hall",
+  static const char *names[] = {"k_face_emf", "k_edge_emf", "k_add_hall",
                                 "k_fluid",    "k_bface",    "k_bcell_jedge", "k_jcell",   "k_pv_uplus",
-                                "k_sync",     "k_flip",     "k_retire",      "k_face_normals", "k_div_b",
+                                "k_sync",     "k_face_normals", "k_div_b",
                                 "k_res_seed", "k_res_w",    "k_res_vec",     "k_res_db",   "k_res_dj",
                                 "k_res_q",    "k_res_dot",  "k_res_sum",     "k_res_copyb", "k_res_bupdate",
                                 "k_res_cg",   "k_res_pupd_e", "k_phys",      "k_sing_setup", "k_sing_emf",

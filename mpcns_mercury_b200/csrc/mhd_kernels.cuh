@@ -7,8 +7,8 @@
 namespace mhd {
 
 enum StepKernel {
-  SK_FACE_EMF = 0, SK_EDGE_EMF, SK_HALL_EDGE, SK_ADD_HALL, SK_FLUID, SK_BFACE, SK_BCELL_JEDGE,
-  SK_JCELL, SK_PV_UPLUS, SK_SYNC, SK_FLIP, SK_RETIRE, SK_FACE_NORMALS, SK_DIVB,
+  SK_FACE_EMF = 0, SK_EDGE_EMF, SK_ADD_HALL, SK_FLUID, SK_BFACE, SK_BCELL_JEDGE,
+  SK_JCELL, SK_PV_UPLUS, SK_SYNC, SK_FACE_NORMALS, SK_DIVB,
   // implicit resistive substep
   SK_RES_SEED, SK_RES_W, SK_RES_VEC, SK_RES_DB, SK_RES_DJ, SK_RES_Q, SK_RES_DOT, SK_RES_SUM, SK_RES_COPYB,
   SK_RES_BUPDATE, SK_RES_CG, SK_RES_PUPD_E,
@@ -73,9 +73,10 @@ struct ResScratch {
 
 // Launch one engine kernel over the directory D (ops: SK_SYNC only) in the
 // batch's precision (Precision); iarg / darg: the operation and scalar of the
-// implicit resistive kernels.
+// implicit resistive kernels (SK_PV_UPLUS: iarg = 1 ends the step).  full: the launch
+// waits for its predecessor to complete instead of overlapping its end.
 void launch_step_kernel(StepKernel k, const Dir &D, cudaStream_t st, const SyncOps *ops, int precision, int iarg = 0,
-                        double darg = 0.0, ResScratch rs = ResScratch{nullptr, nullptr});
+                        double darg = 0.0, ResScratch rs = ResScratch{nullptr, nullptr}, bool full = false);
 int res_dot_grid();
 // Mixed-precision implicit substep: moves its coefficients (RES_X_STATIC, at
 // prepare) and vectors between every masked solve of the FP32 directory D and
