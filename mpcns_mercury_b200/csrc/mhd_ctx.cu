@@ -283,7 +283,7 @@ struct mhd_batch {
   int snap_next = 0;
   // eager profiling
   bool profiling = false;
-  bool after_flip = false;  // the last kernel launched was k_bface
+  bool after_flip = false;  // the last kernel launched was k_bface or k_face_normals
   int fluid_tile = 0;  // the fluid kernel's tile variant (fluid_tile)
   std::vector<cudaEvent_t> prof_events;
   std::vector<const char *> prof_names;
@@ -328,7 +328,8 @@ void mark(mhd_batch *b, const char *name) {
 void launch(mhd_batch *b, int mode, StepKernel k, int *nk, const SyncOps *ops = nullptr, int iarg = 0,
             double darg = 0.0) {
   launch_step_kernel(k, b->dir(mode), b->stream, ops, b->precision, iarg, darg, b->res, b->after_flip);
-  b->after_flip = k == SK_BFACE;  // it flips the solves' states, which the next kernels read ahead of their wait
+  // it flips the solves' states, or writes static fields: the next kernels read those ahead of their wait
+  b->after_flip = k == SK_BFACE || k == SK_FACE_NORMALS;
   ++*nk;
   mark(b, step_kernel_name(k));
 }

@@ -335,12 +335,16 @@ __host__ __device__ inline RangeBox range_of(int kind, const int n[3], int g) {
 __host__ __device__ constexpr bool vector_kind(int kind) {
   return kind == kCells || kind == kBox || kind == kExt || kind == kAlloc || kind == kResK;
 }
-// The aligned 16-byte groups of a row that hold positions of the range.
+// Positions of a thread's group (es: bytes per real): 16 bytes of an array
+// (8 bytes in the primitive pass, whose long chains of divisions and square
+// roots want threads).
+__host__ __device__ constexpr int group_size(int kind, int es) { return (kind == kAlloc ? 8 : 16) / es; }
+// The aligned groups (of n positions) of a row that hold positions of the range.
 struct RowGroups {
   int first, count;
 };
-__host__ __device__ inline RowGroups row_groups(const RangeBox &r, int G, int es) {
-  const int n = 16 / es, first = (r.lo[2] + G) / n;
+__host__ __device__ inline RowGroups row_groups(const RangeBox &r, int G, int n) {
+  const int first = (r.lo[2] + G) / n;
   return RowGroups{first, (r.hi[2] - 1 + G) / n - first + 1};
 }
 // Work items of a block: the fluid kinds use 3-D tiles of their variant's
@@ -359,7 +363,7 @@ __host__ __device__ inline int tiles_of(const RangeBox &r, int kind, int G, int 
     return tk * tj * ti * 2;
   }
   if (vector_kind(kind)) {
-    const int64_t groups = (int64_t)(r.hi[0] - r.lo[0]) * (r.hi[1] - r.lo[1]) * row_groups(r, G, es).count;
+    const int64_t groups = (int64_t)(r.hi[0] - r.lo[0]) * (r.hi[1] - r.lo[1]) * row_groups(r, G, group_size(kind, es)).count;
     return (int)((groups + kVecThreads - 1) / kVecThreads);
   }
   const int64_t vol = (int64_t)(r.hi[0] - r.lo[0]) * (r.hi[1] - r.lo[1]) * (r.hi[2] - r.lo[2]);

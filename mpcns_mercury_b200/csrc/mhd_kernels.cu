@@ -27,6 +27,9 @@ namespace mhd {
 
 namespace {
 
+// Slots of k_pv_uplus's stage, and its resident CTAs per SM.
+constexpr int kPvSlots = 30;
+constexpr int kPvCtas = 5;
 constexpr int cUH = 0, cUN = 5;
 constexpr int cBX = kComp.first[MHD_B_XI], cBY = kComp.first[MHD_B_ETA], cBZ = kComp.first[MHD_B_ZETA];
 constexpr int cPVH = kComp.first[MHD_PV_H], cPVN = kComp.first[MHD_PV_NA], cUP = kComp.first[MHD_U_PLUS];
@@ -256,69 +259,64 @@ __device__ __forceinline__ void for_items(const Dir &D, F &&f) {
 // The step's stencil passes take 16 bytes of consecutive k positions (4 FP32 or
 // 2 FP64 values, aligned: block rows start on 64-byte boundaries) per thread and
 // array, element by element with the operations of the scalar form.
-template <class R>
-struct alignas(16) Vec {
-  static constexpr int N = 16 / (int)sizeof(R);
-  R v[N];
+template <class R, int M = 16 / (int)sizeof(R)>
+struct alignas(M * sizeof(R)) Vec {
+  static constexpr int N = M;
+  R v[M];
 };
-template <class R, class F>
-__device__ __forceinline__ Vec<R> vmap(F &&f) {
-  Vec<R> r;
+template <class R, int M = 16 / (int)sizeof(R), class F>
+__device__ __forceinline__ Vec<R, M> vmap(F &&f) {
+  Vec<R, M> r;
 #pragma unroll
-  for (int e = 0; e < Vec<R>::N; ++e) r.v[e] = f(e);
+  for (int e = 0; e < M; ++e) r.v[e] = f(e);
   return r;
 }
-#define MHD_VEC_OP(op)                                                                                                \
-  template <class R>                                                                                                  \
-  __device__ __forceinline__ Vec<R> operator op(const Vec<R> &a, const Vec<R> &b) {                                  \
-    return vmap<R>([&](int e) { return a.v[e] op b.v[e]; });                                                          \
-  }                                                                                                                   \
-  template <class R>                                                                                                  \
-  __device__ __forceinline__ Vec<R> operator op(R a, const Vec<R> &b) {                                              \
-    return vmap<R>([&](int e) { return a op b.v[e]; });                                                               \
-  }                                                                                                                   \
-  template <class R>                                                                                                  \
-  __device__ __forceinline__ Vec<R> operator op(const Vec<R> &a, R b) {                                              \
-    return vmap<R>([&](int e) { return a.v[e] op b; });                                                               \
+#define MHD_VEC_OP(op)                                                                  \
+  template <class R, int M>                                                             \
+  __device__ __forceinline__ Vec<R, M> operator op(const Vec<R, M> &a, const Vec<R, M> &b) { \
+    return vmap<R, M>([&](int e) { return a.v[e] op b.v[e]; });                         \
+  }                                                                                     \
+  template <class R, int M>                                                             \
+  __device__ __forceinline__ Vec<R, M> operator op(R a, const Vec<R, M> &b) {           \
+    return vmap<R, M>([&](int e) { return a op b.v[e]; });                              \
+  }                                                                                     \
+  template <class R, int M>                                                             \
+  __device__ __forceinline__ Vec<R, M> operator op(const Vec<R, M> &a, R b) {           \
+    return vmap<R, M>([&](int e) { return a.v[e] op b; });                              \
   }
 MHD_VEC_OP(+)
 MHD_VEC_OP(-)
 MHD_VEC_OP(*)
 MHD_VEC_OP(/)
 #undef MHD_VEC_OP
-template <class R>
-__device__ __forceinline__ Vec<R> operator-(const Vec<R> &a) {
-  return vmap<R>([&](int e) { return -a.v[e]; });
+template <class R, int M>
+__device__ __forceinline__ Vec<R, M> operator-(const Vec<R, M> &a) {
+  return vmap<R, M>([&](int e) { return -a.v[e]; });
 }
-template <class R>
-__device__ __forceinline__ Vec<R> vset(R x) {
-  return vmap<R>([&](int) { return x; });
+template <class R, int M = 16 / (int)sizeof(R)>
+__device__ __forceinline__ Vec<R, M> vset(R x) {
+  return vmap<R, M>([&](int) { return x; });
 }
-template <class R>
-__device__ __forceinline__ Vec<R> vabs(const Vec<R> &a) {
-  return vmap<R>([&](int e) { return fabs(a.v[e]); });
+template <class R, int M>
+__device__ __forceinline__ Vec<R, M> vabs(const Vec<R, M> &a) {
+  return vmap<R, M>([&](int e) { return fabs(a.v[e]); });
 }
-template <class R>
-__device__ __forceinline__ Vec<R> vsqrt(const Vec<R> &a) {
-  return vmap<R>([&](int e) { return sqrt(a.v[e]); });
+template <class R, int M>
+__device__ __forceinline__ Vec<R, M> vsqrt(const Vec<R, M> &a) {
+  return vmap<R, M>([&](int e) { return sqrt(a.v[e]); });
 }
-template <class R>
-__device__ __forceinline__ Vec<R> vmax(const Vec<R> &a, const Vec<R> &b) {
-  return vmap<R>([&](int e) { return dmax(a.v[e], b.v[e]); });
-}
-template <class R>
-__device__ __forceinline__ Vec<R> vmax(const Vec<R> &a, R b) {
-  return vmap<R>([&](int e) { return dmax(a.v[e], b); });
+template <class R, int M>
+__device__ __forceinline__ Vec<R, M> vmax(const Vec<R, M> &a, const Vec<R, M> &b) {
+  return vmap<R, M>([&](int e) { return dmax(a.v[e], b.v[e]); });
 }
 // The values one k lower (the lowest from `prev`), one k higher (the highest from `next`).
-template <class R>
-__device__ __forceinline__ Vec<R> vdown(const Vec<R> &a, R prev) {
-  return vmap<R>([&](int e) { return e == 0 ? prev : a.v[e > 0 ? e - 1 : 0]; });
+template <class R, int M>
+__device__ __forceinline__ Vec<R, M> vdown(const Vec<R, M> &a, R prev) {
+  return vmap<R, M>([&](int e) { return e == 0 ? prev : a.v[e > 0 ? e - 1 : 0]; });
 }
-template <class R>
-__device__ __forceinline__ Vec<R> vup(const Vec<R> &a, R next) {
-  constexpr int N = Vec<R>::N;
-  return vmap<R>([&](int e) { return e == N - 1 ? next : a.v[e < N - 1 ? e + 1 : e]; });
+template <class R, int M>
+__device__ __forceinline__ Vec<R, M> vup(const Vec<R, M> &a, R next) {
+  return vmap<R, M>([&](int e) { return e == M - 1 ? next : a.v[e < M - 1 ? e + 1 : e]; });
 }
 
 // One thread's part of a vector item: positions k .. k + N - 1 of row (i, j),
@@ -330,65 +328,95 @@ struct VItem {
   int klo, khi;
   __device__ __forceinline__ bool has(int e) const { return k + e >= klo && k + e < khi; }
 };
-template <class R>
+// The static operands of a pass (weights, metric terms: set by mhd_prepare) stream
+// through shared memory: every thread copies its own 16 bytes of each array
+// with cp.async and reads them back itself, so no barrier is needed, all of
+// them are in flight at once, and the first tile's are issued ahead of the wait
+// for the predecessors, which do not write them.
+// This thread's address in slot 0 of a stage of `size`-byte groups.
+__device__ __forceinline__ uint32_t stage_base(int size) {
+  extern __shared__ __align__(16) unsigned char stage_smem[];
+  return (uint32_t)__cvta_generic_to_shared(stage_smem) + threadIdx.x * (uint32_t)size;
+}
+constexpr int stage_bytes(int slots, int size) { return slots * kVecThreads * size; }
+__device__ __forceinline__ void staged_arrived() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+template <class R, int M = 16 / (int)sizeof(R)>
 struct VV : V<R> {
-  static constexpr int N = Vec<R>::N;
+  static constexpr int N = M;
+  using Vc = Vec<R, M>;
   using V<R>::c;
   using V<R>::m;
   uint32_t di, dj;  // bytes to the neighbour along i and j (k: sizeof(R))
-  __device__ __forceinline__ Vec<R> lv(int comp, uint32_t o) const {
-    Vec<R> r;
+  // 4, 8 or 16 aligned bytes as one load
+  template <class T>
+  __device__ __forceinline__ static void load(T *to, const void *p) {
+    if constexpr (sizeof(R) * M == 16) *(float4 *)to = __ldg((const float4 *)p);
+    else if constexpr (sizeof(R) * M == 8) *(float2 *)to = __ldg((const float2 *)p);
+    else *(float *)to = __ldg((const float *)p);
+  }
+  __device__ __forceinline__ Vc lv(int comp, uint32_t o) const {
+    Vc r;
     const char *p = (const char *)c(comp) + o;
-    if constexpr (sizeof(R) == 4) *(float4 *)r.v = __ldg((const float4 *)p);
-    else *(double2 *)r.v = __ldg((const double2 *)p);
+    if constexpr (M == 1) r.v[0] = __ldg((const R *)p);
+    else if constexpr (sizeof(R) == 8) *(double2 *)r.v = __ldg((const double2 *)p);
+    else load(r.v, p);
     return r;
   }
   // the values one k lower / higher than lv(comp, o), of which v holds the shared ones
-  __device__ __forceinline__ Vec<R> lower(const Vec<R> &v, int comp, uint32_t o) const {
+  __device__ __forceinline__ Vc lower(const Vc &v, int comp, uint32_t o) const {
     return vdown(v, this->ld(comp, o - (uint32_t)sizeof(R)));
   }
-  __device__ __forceinline__ Vec<R> upper(const Vec<R> &v, int comp, uint32_t o) const {
-    return vup(v, this->ld(comp, o + 16u));
+  __device__ __forceinline__ Vc upper(const Vc &v, int comp, uint32_t o) const {
+    return vup(v, this->ld(comp, o + (uint32_t)sizeof(Vc)));
+  }
+  // lv(comp, o) copied to this thread's bytes of slot q of the CTA's stage
+  // (cp.async: in flight without holding a register) and, after staged_arrived, read back
+  __device__ __forceinline__ void stage(uint32_t base, int q, int comp, uint32_t o) const {
+    const uint32_t to = base + (uint32_t)q * (uint32_t)(kVecThreads * sizeof(Vc));
+    const char *from = (const char *)c(comp) + o;
+    if constexpr (sizeof(Vc) == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(from) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(to), "l"(from), "n"(sizeof(Vc)) : "memory");
+  }
+  __device__ __forceinline__ Vc staged(int q) const {
+    extern __shared__ __align__(16) unsigned char stage_smem[];
+    return reinterpret_cast<const Vc *>(stage_smem)[q * kVecThreads + (int)threadIdx.x];
   }
   // values that the kernel itself updates (this thread's positions only)
-  __device__ __forceinline__ Vec<R> own(int comp, uint32_t o) const {
-    Vec<R> r;
-    const char *p = (const char *)c(comp) + o;
-    if constexpr (sizeof(R) == 4) *(float4 *)r.v = *(const float4 *)p;
-    else *(double2 *)r.v = *(const double2 *)p;
-    return r;
-  }
+  __device__ __forceinline__ Vc own(int comp, uint32_t o) const { return *(const Vc *)((const char *)c(comp) + o); }
   // metric values (double) at the item's positions
-  __device__ __forceinline__ Vec<R> lm(int comp, uint32_t o) const {
-    const char *p = (const char *)m(comp) + (uint64_t)o * (8 / sizeof(R));
-    Vec<R> r;
-    if constexpr (sizeof(R) == 4) {
-      const double2 a = __ldg((const double2 *)p), b = __ldg((const double2 *)p + 1);
-      r.v[0] = (R)a.x;
-      r.v[1] = (R)a.y;
-      r.v[2] = (R)b.x;
-      r.v[3] = (R)b.y;
+  __device__ __forceinline__ Vc lm(int comp, uint32_t o) const {
+    const double *p = (const double *)((const char *)m(comp) + (uint64_t)o * (8 / sizeof(R)));
+    Vc r;
+    if constexpr (M == 1) {
+      r.v[0] = (R)__ldg(p);
     } else {
-      *(double2 *)r.v = __ldg((const double2 *)p);
+#pragma unroll
+      for (int e = 0; e < M; e += 2) {
+        const double2 a = __ldg((const double2 *)p + e / 2);
+        r.v[e] = (R)a.x;
+        r.v[e + 1] = (R)a.y;
+      }
     }
     return r;
   }
   // writes the positions k + e in [lo, hi) where the item is in the range and `cond`
-  __device__ __forceinline__ void st(int comp, const VItem &it, const Vec<R> &v, int lo, int hi, bool cond = true) const {
+  __device__ __forceinline__ void st(int comp, const VItem &it, const Vc &v, int lo, int hi, bool cond = true) const {
     char *p = (char *)c(comp) + it.o;
     const bool w = it.in && cond, all = w && it.k >= lo && it.k + N <= hi;
-    if (all) {
-      if constexpr (sizeof(R) == 4) *(float4 *)p = *(const float4 *)v.v;
-      else *(double2 *)p = *(const double2 *)v.v;
-    }
+    if (all) *(Vc *)p = v;
+    if constexpr (M > 1) {
 #pragma unroll
-    for (int e = 0; e < N; ++e)
-      if (w && !all && it.k + e >= lo && it.k + e < hi) ((R *)p)[e] = v.v[e];
+      for (int e = 0; e < N; ++e)
+        if (w && !all && it.k + e >= lo && it.k + e < hi) ((R *)p)[e] = v.v[e];
+    }
   }
 };
 
 template <class R, int KIND>
-__device__ __forceinline__ void build_vec_item(const Dir &D, int s, int b, int t, VItem &it, VV<R> &B) {
+__device__ __forceinline__ void build_vec_item(const Dir &D, int s, int b, int t, VItem &it,
+                                               VV<R, group_size(KIND, sizeof(R))> &B) {
+  constexpr int N = group_size(KIND, sizeof(R));
   const DevSolve &S = D.solves[s];
   const DevBlock &DB = S.blocks[b];
   RangeBox r = range_of(KIND, DB.n, S.c.nghost);
@@ -405,20 +433,20 @@ __device__ __forceinline__ void build_vec_item(const Dir &D, int s, int b, int t
   B.n0 = uniform(B.n0);
   B.n1 = uniform(B.n1);
   B.n2 = uniform(B.n2);
-  const RowGroups g = row_groups(r, B.G, sizeof(R));
+  const RowGroups g = row_groups(r, B.G, N);
   const int ej = r.hi[1] - r.lo[1];
   const int L = t * kVecThreads + (int)threadIdx.x;
   const int row = L / g.count, ri = row / ej;
   it.s = s;
   it.blk = b;
-  it.k = (g.first + (L - row * g.count)) * Vec<R>::N - B.G;
+  it.k = (g.first + (L - row * g.count)) * N - B.G;
   it.j = r.lo[1] + (row - ri * ej);
   it.i = r.lo[0] + ri;
   it.in = it.i < r.hi[0];
   if (!it.in) {  // past the last row: work on the first one and write nothing (no divergence)
     it.i = r.lo[0];
     it.j = r.lo[1];
-    it.k = g.first * Vec<R>::N - B.G;
+    it.k = g.first * N - B.G;
   }
   it.klo = r.lo[2];
   it.khi = r.hi[2];
@@ -433,10 +461,15 @@ __device__ __forceinline__ void use_current(V<R> &B, int cur) {
 }
 
 // Work-item loop over the vector ranges: f(S, B, item) for every tile of
-// range KIND of every active solve.  Thread 0 looks the next tile up while the
+// range KIND of every active solve, pre(B, item) before it (staged static
+// operands).  Thread 0 looks the next tile up while the
 // CTA works on the current one (one barrier per tile).
-template <class R, int KIND, class F>
-__device__ __forceinline__ void for_vec_items(const Dir &D, F &&f) {
+struct NoStage {
+  template <class B>
+  __device__ void operator()(const B &, const VItem &) const {}
+};
+template <class R, int KIND, class F, class P = NoStage>
+__device__ __forceinline__ void for_vec_items(const Dir &D, F &&f, P &&pre = P{}) {
   __shared__ int sh[2][3];
   let_dependents_launch();
   const int total = D.solve_tile_prefix[KIND][D.nsolves];
@@ -453,9 +486,10 @@ __device__ __forceinline__ void for_vec_items(const Dir &D, F &&f) {
       lookup_item<KIND>(D, w + gridDim.x, sh[p ^ 1][0], sh[p ^ 1][1], sh[p ^ 1][2]);
     __syncwarp();
     VItem it;
-    VV<R> B;
+    VV<R, group_size(KIND, sizeof(R))> B;
     build_vec_item<R, KIND>(D, s, b, t, it, B);
     it.w = w;
+    pre(B, it);  // loads of what no pass of the step writes
     Status st{};
     if (D.mode == 0) st = status_of(D, s);
     if (w == (int)blockIdx.x) wait_for_predecessors();
@@ -463,6 +497,8 @@ __device__ __forceinline__ void for_vec_items(const Dir &D, F &&f) {
     if (uniform(st.active)) {
       use_current(B, uniform(st.cur));
       f(D.solves[s], B, it);
+    } else if constexpr (!std::is_same_v<P, NoStage>) {
+      staged_arrived();  // the next tile takes the same slots
     }
     __syncthreads();
   }
@@ -490,9 +526,9 @@ struct Pos {
 };
 template <class R, int KIND, class F>
 __device__ __forceinline__ void for_positions(const Dir &D, F &&f) {
-  for_vec_items<R, KIND>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
+  for_vec_items<R, KIND>(D, [&](const DevSolve &S, const auto &B, const VItem &it) {
 #pragma unroll 1
-    for (int e = 0; e < Vec<R>::N; ++e)
+    for (int e = 0; e < group_size(KIND, sizeof(R)); ++e)
       if (it.in && it.has(e)) f(S, B, Pos{it.s, it.blk, it.i, it.j, it.k + e});
   });
 }
@@ -1180,24 +1216,22 @@ __global__ void __launch_bounds__(kVecThreads, 3) k_jcell(Dir D) {
 #pragma unroll
       for (int x = 0; x < 3; ++x) j[x] = j[x] + B.lv(cWJ + 12 * x + q, o) * s;
     };
-    {
-      const Vec<R> a = B.lv(cJX, o), b = B.lv(cJX, o + dj);
-      add(0, a);
-      add(1, b);
-      add(2, B.upper(a, cJX, o));
-      add(3, B.upper(b, cJX, o + dj));
-    }
-    {
-      const Vec<R> a = B.lv(cJY, o), b = B.lv(cJY, o + di);
-      add(4, a);
-      add(5, b);
-      add(6, B.upper(a, cJY, o));
-      add(7, B.upper(b, cJY, o + di));
-    }
-    add(8, B.lv(cJZ, o));
-    add(9, B.lv(cJZ, o + di));
-    add(10, B.lv(cJZ, o + dj));
-    add(11, B.lv(cJZ, o + di + dj));
+    const Vec<R> ax = B.lv(cJX, o), bx = B.lv(cJX, o + dj), ay = B.lv(cJY, o), by = B.lv(cJY, o + di);
+    const Vec<R> ux = B.upper(ax, cJX, o), vx = B.upper(bx, cJX, o + dj);
+    const Vec<R> uy = B.upper(ay, cJY, o), vy = B.upper(by, cJY, o + di);
+    const Vec<R> z0 = B.lv(cJZ, o), z1 = B.lv(cJZ, o + di), z2 = B.lv(cJZ, o + dj), z3 = B.lv(cJZ, o + di + dj);
+    add(0, ax);
+    add(1, bx);
+    add(2, ux);
+    add(3, vx);
+    add(4, ay);
+    add(5, by);
+    add(6, uy);
+    add(7, vy);
+    add(8, z0);
+    add(9, z1);
+    add(10, z2);
+    add(11, z3);
 #pragma unroll
     for (int x = 0; x < 3; ++x) B.st(cJC + x, it, j[x], 0, B.n2);
   });
@@ -1239,19 +1273,19 @@ __device__ __forceinline__ R fast_cf(R cs2, R vA2, R vAn2) {
   if (disc < R(0.0)) disc = R(0.0);
   return sqrt(R(0.5) * (term + sqrt(disc)));
 }
-template <class R>
-__device__ __forceinline__ R cells_dt(const VV<R> &B, const ConstsT<R> &c, const VItem &it, bool own, const Vec<R> &Bx,
-                                      const Vec<R> &By, const Vec<R> &Bz, bool &bad) {
-  constexpr int N = Vec<R>::N;
+template <class R, int N>
+__device__ __forceinline__ R cells_dt(const VV<R, N> &B, const ConstsT<R> &c, const VItem &it, bool own,
+                                      const Vec<R, N> &Bx, const Vec<R, N> &By, const Vec<R, N> &Bz, bool &bad) {
+  using Vc = Vec<R, N>;
   const uint32_t o = it.o;
-  const Vec<R> Vol = vabs(B.lm(cJAC, o));
-  const Vec<R> B2 = Bx * Bx + By * By + Bz * Bz;
-  Vec<R> d = vset(R(1e100));
+  const Vc Vol = vabs(B.lm(cJAC, o));
+  const Vc B2 = Bx * Bx + By * By + Bz * Bz;
+  Vc d = vset<R, N>(R(1e100));
 #pragma unroll 1
   for (int s = 0; s < 2; ++s) {
     const int u0 = s ? cUN : cUH;
-    const Vec<R> rho0 = B.lv(u0, o), m1 = B.lv(u0 + 1, o), m2 = B.lv(u0 + 2, o), m3 = B.lv(u0 + 3, o), E = B.lv(u0 + 4, o);
-    Vec<R> ux, uy, uz, cs2, vA2, den = vset(R(0.0)), rho, y;
+    const Vc rho0 = B.lv(u0, o), m1 = B.lv(u0 + 1, o), m2 = B.lv(u0 + 2, o), m3 = B.lv(u0 + 3, o), E = B.lv(u0 + 4, o);
+    Vc ux, uy, uz, cs2, vA2, den = vset<R, N>(R(0.0)), rho, y;
 #pragma unroll
     for (int e = 0; e < N; ++e) {
       rho.v[e] = dmax(rho0.v[e], R(1e-2));
@@ -1267,10 +1301,11 @@ __device__ __forceinline__ R cells_dt(const VV<R> &B, const ConstsT<R> &c, const
       uz.v[e] = w;
     }
     // faces xi-, xi+, eta-, eta+, zeta-, zeta+ (the reference's summation order)
-    auto face = [&](const Vec<R> &px, const Vec<R> &py, const Vec<R> &pz, const Vec<R> &An, bool up) {
+    // (the outward normal's sign changes neither |u . n| nor (B . n)^2)
+    auto face = [&](const Vc &px, const Vc &py, const Vc &pz, const Vc &An) {
 #pragma unroll
       for (int e = 0; e < N; ++e) {
-        const R nx = up ? px.v[e] : -px.v[e], ny = up ? py.v[e] : -py.v[e], nz = up ? pz.v[e] : -pz.v[e];
+        const R nx = px.v[e], ny = py.v[e], nz = pz.v[e];
         const R un = ux.v[e] * nx + uy.v[e] * ny + uz.v[e] * nz;
         const R Bn = Bx.v[e] * nx + By.v[e] * ny + Bz.v[e] * nz;
         const Divisor<R> by(rho.v[e], y.v[e]);
@@ -1279,15 +1314,13 @@ __device__ __forceinline__ R cells_dt(const VV<R> &B, const ConstsT<R> &c, const
       }
     };
 #pragma unroll 1
-    for (int a = 0; a < 2; ++a) {  // rolled: two axes' face loads in flight at once spill
-      const int cn = cFNX + 4 * a;
-      const uint32_t q = o + (a == 0 ? B.di : B.dj);
-      face(B.lv(cn, o), B.lv(cn + 1, o), B.lv(cn + 2, o), B.lv(cn + 3, o), false);
-      face(B.lv(cn, q), B.lv(cn + 1, q), B.lv(cn + 2, q), B.lv(cn + 3, q), true);
+    for (int a = 0; a < 2; ++a) {
+      face(B.staged(8 * a), B.staged(8 * a + 1), B.staged(8 * a + 2), B.staged(8 * a + 3));
+      face(B.staged(8 * a + 4), B.staged(8 * a + 5), B.staged(8 * a + 6), B.staged(8 * a + 7));
     }
-    const Vec<R> zx = B.lv(cFNZ, o), zy = B.lv(cFNZ + 1, o), zz = B.lv(cFNZ + 2, o), zA = B.lv(cFNZ + 3, o);
-    face(zx, zy, zz, zA, false);
-    face(B.upper(zx, cFNZ, o), B.upper(zy, cFNZ + 1, o), B.upper(zz, cFNZ + 2, o), B.upper(zA, cFNZ + 3, o), true);
+    const Vc zx = B.staged(16), zy = B.staged(17), zz = B.staged(18), zA = B.staged(19);
+    face(zx, zy, zz, zA);
+    face(B.upper(zx, cFNZ, o), B.upper(zy, cFNZ + 1, o), B.upper(zz, cFNZ + 2, o), B.upper(zA, cFNZ + 3, o));
 #pragma unroll
     for (int e = 0; e < N; ++e)
       if (Vol.v[e] > R(0.0) && den.v[e] > R(0.0)) d.v[e] = dmin(d.v[e], c.CFL * Vol.v[e] / den.v[e]);
@@ -1346,7 +1379,7 @@ __device__ __forceinline__ bool edge_owned(int a, int i, int j, int k, int n0, i
 // an edge still at 1 is its own unknown.
 template <class R>
 __global__ void __launch_bounds__(kVecThreads) k_res_seed(Dir D) {
-  for_positions<R, kBox>(D, [&](const DevSolve &S, const VV<R> &B, const Pos &it) {
+  for_positions<R, kBox>(D, [&](const DevSolve &S, const auto &B, const Pos &it) {
     const int o = B.off(it.i, it.j, it.k);
     for (int a = 0; a < 3; ++a) B.c(cEX + a)[o] = R(1.0);
   });
@@ -1356,7 +1389,7 @@ __global__ void __launch_bounds__(kVecThreads) k_res_seed(Dir D) {
 // alpha > 0: BuildImplicitResistiveEdgeDofMap_, Mercury_ImplicitResistive.cpp:168-226), 0 elsewhere.
 template <class R>
 __global__ void __launch_bounds__(kVecThreads) k_res_w(Dir D) {
-  for_positions<R, kBox>(D, [&](const DevSolve &S, const VV<R> &B, const Pos &it) {
+  for_positions<R, kBox>(D, [&](const DevSolve &S, const auto &B, const Pos &it) {
     const int o = B.off(it.i, it.j, it.k);
     for (int a = 0; a < 3; ++a) {
       R w = R(0.0);
@@ -1740,7 +1773,7 @@ __global__ void __launch_bounds__(kVecThreads) k_res_bupdate(Dir D) {
 // the fluid fluxes' face JD and 1 / Jac in the real type.
 template <class R>
 __global__ void __launch_bounds__(kVecThreads) k_face_normals(Dir D) {
-  for_positions<R, kAlloc>(D, [&](const DevSolve &S, const VV<R> &B, const Pos &it) {
+  for_positions<R, kAlloc>(D, [&](const DevSolve &S, const auto &B, const Pos &it) {
     {
       // Coefficients of the contravariant velocities (calc_Uplus,
       // Tools.cpp:159-301) on the cells k_pv_uplus refreshes them on: the
@@ -1844,26 +1877,32 @@ __global__ void __launch_bounds__(kVecThreads) k_face_normals(Dir D) {
 // velocities UCON and the next step's Hall cell field there, and the next
 // step's CFL dt on owned cells (warp min, one atomicMin per warp on the bit
 // pattern of the positive double).  The step's last pass ends it (retire_solve).
+// Bound by latency: a cell is a chain of divisions and square roots behind some
+// 50 operands.  So 8-byte groups (twice the threads of 16-byte ones), and the 30
+// static operands on their way before the wait (kPvCtas x the stage fits an SM):
+// a step takes 55 us for a box of 8^3 FP64 cells (62 with 16-byte groups and
+// plain loads), 85 (93) for 32^3, 153 (163) for 64^3 mixed.
 template <class R>
-__global__ void __launch_bounds__(kVecThreads, 4) k_pv_uplus(Dir D, int end_of_step) {
-  for_vec_items<R, kAlloc>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
-    constexpr int N = Vec<R>::N;
+__global__ void __launch_bounds__(kVecThreads, kPvCtas) k_pv_uplus(Dir D, int end_of_step) {
+  for_vec_items<R, kAlloc>(D, [&](const DevSolve &S, const auto &B, const VItem &it) {
+    constexpr int N = group_size(kAlloc, sizeof(R));
+    using Vc = Vec<R, N>;
     const ConstsT<R> &c = consts_of<R>(S);
     R dtl = R(1e100);
     bool bad = false;
     {
       const uint32_t o = it.o;
-      auto put = [&](int comp, const Vec<R> &v) { B.st(comp, it, v, it.klo, it.khi); };
-      Vec<R> rho[2], vel[2][3];
-      Vec<R> chk = vset(R(0.0));  // sum of the conserved components: non-finite if any of them is
+      auto put = [&](int comp, const Vc &v) { B.st(comp, it, v, it.klo, it.khi); };
+      Vc rho[2], vel[2][3];
+      Vc chk = vset<R, N>(R(0.0));  // sum of the conserved components: non-finite if any of them is
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
         const int pv0 = s ? cPVN : cPVH, u0 = s ? cUN : cUH;
         const R coeff = s ? c.state_coeff_Na : c.state_coeff_H;
-        const Vec<R> r0 = B.lv(u0, o), m1 = B.lv(u0 + 1, o), m2 = B.lv(u0 + 2, o), m3 = B.lv(u0 + 3, o), E = B.lv(u0 + 4, o);
+        const Vc r0 = B.lv(u0, o), m1 = B.lv(u0 + 1, o), m2 = B.lv(u0 + 2, o), m3 = B.lv(u0 + 3, o), E = B.lv(u0 + 4, o);
         rho[s] = r0;
         chk = chk + (((r0 + m1) + (m2 + m3)) + E);
-        Vec<R> pr, T, re, cs;
+        Vc pr, T, re, cs;
 #pragma unroll
         for (int e = 0; e < N; ++e) {
           const R rh = dmax(r0.v[e], R(1e-12));
@@ -1896,8 +1935,8 @@ __global__ void __launch_bounds__(kVecThreads, 4) k_pv_uplus(Dir D, int end_of_s
         put(cFT + 2 * s, re);
         put(cFT + 2 * s + 1, cs);
       }
-      const Vec<R> Bx = B.lv(cBC, o), By = B.lv(cBC + 1, o), Bz = B.lv(cBC + 2, o);
-      Vec<R> alpha, up[3];
+      const Vc Bx = B.lv(cBC, o), By = B.lv(cBC + 1, o), Bz = B.lv(cBC + 2, o);
+      Vc alpha, up[3];
 #pragma unroll
       for (int e = 0; e < N; ++e) {
         const R rH = dmax(rho[0].v[e], R(0.0)), rN = dmax(rho[1].v[e], R(0.0));
@@ -1915,7 +1954,7 @@ __global__ void __launch_bounds__(kVecThreads, 4) k_pv_uplus(Dir D, int end_of_s
         // (Z4_Mercury/src/physics/MercurySolver_MagExplicit_Hall.cpp:110-146): its inputs (J_cell,
         // B_cell, the densities) are final here (num_limiter clamps the
         // densities at zero itself, so it is the limiter of the raw densities)
-        const Vec<R> Jx = B.lv(cJC, o), Jy = B.lv(cJC + 1, o), Jz = B.lv(cJC + 2, o);
+        const Vc Jx = B.lv(cJC, o), Jy = B.lv(cJC + 1, o), Jz = B.lv(cJC + 2, o);
         put(cEHC, alpha * (Jy * Bz - Jz * By));
         put(cEHC + 1, alpha * (Jz * Bx - Jx * Bz));
         put(cEHC + 2, alpha * (Jx * By - Jy * Bx));
@@ -1927,18 +1966,19 @@ __global__ void __launch_bounds__(kVecThreads, 4) k_pv_uplus(Dir D, int end_of_s
       const bool near = it.i >= -gm && it.i < B.n0 + gm && it.j >= -gm && it.j < B.n1 + gm;
       {
         // coefficients (cell-averaged JD, 1 / (|Jac| + 1e-30)) from k_face_normals
-        const Vec<R> inv_jac = B.lv(cUCK + 9, o);
+        staged_arrived();
+        const Vc inv_jac = B.staged(29);
 #pragma unroll
         for (int axis = 0; axis < 3; ++axis)
           B.st(cUC + axis, it,
-               (B.lv(cUCK + 3 * axis, o) * up[0] + B.lv(cUCK + 3 * axis + 1, o) * up[1] +
-                B.lv(cUCK + 3 * axis + 2, o) * up[2]) *
+               (B.staged(20 + 3 * axis) * up[0] + B.staged(21 + 3 * axis) * up[1] +
+                B.staged(22 + 3 * axis) * up[2]) *
                    inv_jac,
                max(it.klo, -gm), min(it.khi, B.n2 + gm), near);
       }
       const bool own = it.in && it.i >= 0 && it.i < B.n0 && it.j >= 0 && it.j < B.n1;
       if (__any_sync(0xffffffffu, own)) {
-        dtl = cells_dt(B, c, it, own, Bx, By, Bz, bad);
+        dtl = cells_dt<R, N>(B, c, it, own, Bx, By, Bz, bad);
         // the pressure floors can hide a non-finite energy from the dt
 #pragma unroll
         for (int e = 0; e < N; ++e) bad = bad || (own && it.k + e >= 0 && it.k + e < B.n2 && !isfinite(chk.v[e]));
@@ -1949,6 +1989,18 @@ __global__ void __launch_bounds__(kVecThreads, 4) k_pv_uplus(Dir D, int end_of_s
     if ((threadIdx.x & 31) == 0 && dtl < R(1e100))
       atomicMin(&D.state[it.s].dt_bits, (unsigned long long)__double_as_longlong(dtl));
     if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicExch(&D.state[it.s].nonfinite, 1);
+  }, [&](const auto &B, const VItem &it) {
+    const uint32_t w = stage_base(group_size(kAlloc, sizeof(R)) * (int)sizeof(R)), o = it.o;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {  // the faces' normals and |a|: xi-, xi+, eta-, eta+, zeta-
+      B.stage(w, q, cFNX + q, o);
+      B.stage(w, 4 + q, cFNX + q, o + B.di);
+      B.stage(w, 8 + q, cFNY + q, o);
+      B.stage(w, 12 + q, cFNY + q, o + B.dj);
+      B.stage(w, 16 + q, cFNZ + q, o);
+    }
+#pragma unroll
+    for (int q = 0; q < 10; ++q) B.stage(w, 20 + q, cUCK + q, o);
   });
   if (end_of_step) after_all_tiles<kAlloc>(D, D.tickets + 1, [](SolveState &st) { retire_solve(st); });
 }
@@ -2392,6 +2444,7 @@ using Same = typename SameAs<T>::type;
 // A launch that may begin while its predecessor in the stream drains; the kernel
 // waits itself (wait_for_predecessors).  t_full: after it instead, in full.
 static thread_local bool t_full = false;
+static thread_local int t_smem = 0;  // dynamic shared memory of the next launch
 template <class... P>
 static void launch_dependent(void (*fn)(P...), int grid, int threads, cudaStream_t st, Same<P>... args) {
   cudaLaunchAttribute a[1];
@@ -2401,9 +2454,11 @@ static void launch_dependent(void (*fn)(P...), int grid, int threads, cudaStream
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(threads);
   cfg.stream = st;
+  cfg.dynamicSmemBytes = (size_t)t_smem;
   cfg.attrs = a;
   cfg.numAttrs = 1;
   cudaLaunchKernelEx(&cfg, fn, args...);
+  t_smem = 0;
 }
 
 template <class R>
@@ -2467,6 +2522,15 @@ static int kernel_threads(StepKernel k) {
   }
 }
 
+// Dynamic shared memory of a kernel (its stage).
+template <class R>
+static int kernel_smem(StepKernel k) {
+  switch (k) {
+    case SK_PV_UPLUS: return stage_bytes(kPvSlots, group_size(kAlloc, sizeof(R)) * (int)sizeof(R));
+    default: return 0;
+  }
+}
+
 static std::once_flag g_grids_once;
 
 template <class R>
@@ -2477,7 +2541,9 @@ static void grids_init() {
   for (int k = 0; k < SK_COUNT; ++k) {
     int per_sm = 8;
     const void *fn = kernel_fn<R>((StepKernel)k);
-    if (fn && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kernel_threads((StepKernel)k), 0) != cudaSuccess ||
+    const int smem = kernel_smem<R>((StepKernel)k);
+    if (smem > 0) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (fn && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kernel_threads((StepKernel)k), smem) != cudaSuccess ||
                per_sm < 1)) {
       cudaGetLastError();
       per_sm = 1;
@@ -2505,6 +2571,7 @@ template <class R>
 static void launch_as(StepKernel k, const Dir &D, cudaStream_t st, const SyncOps *ops, int iarg, double darg,
                       ResScratch rs) {
   const int G = g_grid_kernel[k];
+  t_smem = kernel_smem<R>(k);
   switch (k) {
     case SK_FACE_EMF: launch_dependent(k_face_emf<R>, G, kVecThreads, st, D); break;
     case SK_EDGE_EMF: launch_dependent(k_edge_emf<R>, G, kVecThreads, st, D); break;
