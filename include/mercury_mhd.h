@@ -79,7 +79,7 @@ enum mhd_field {
   MHD_LOCAL_ETA_XI, MHD_LOCAL_ETA_ETA, MHD_LOCAL_ETA_ZETA,         /* local artificial resistivity per edge */
   MHD_ETA_RES_XI, MHD_ETA_RES_ETA, MHD_ETA_RES_ZETA,               /* implicit resistivity per owned edge */
   /* work of the implicit resistive solve (3 components: xi, eta, zeta edges;
-   * BSTAR: xi, eta, zeta faces) */
+   * BSTAR: xi, eta, zeta faces, the operator's dB) */
   MHD_RES_W, MHD_RES_X, MHD_RES_R, MHD_RES_P, MHD_RES_Q, MHD_RES_BSTAR,
   MHD_NUM_FIELDS
 };
@@ -90,8 +90,9 @@ enum mhd_location { MHD_CELL = 0, MHD_FACE_XI, MHD_FACE_ETA, MHD_FACE_ZETA, MHD_
 /* Sync groups: MercuryBoundary::Sync names (Z4_Mercury/src/boundary/Boundary_Build.cpp:564-703).
  * MHD_SYNC_ERES and MHD_SYNC_DB are the implicit resistive substep's Sync("Eres")
  * and Sync("dB") (Z4_Mercury/src/implicit/Mercury_ImplicitResistive.cpp:321,440): the
- * engine keeps E_res in the E edge arrays and dB in the B face arrays, so their
- * tables address those fields; they differ from MHD_SYNC_EEDGE and MHD_SYNC_BFACE
+ * engine keeps E_res in the E edge arrays and dB in arrays of its own
+ * (MHD_RES_BSTAR), B's twins: the tables address the E edges and the B faces, and
+ * mhd_sync of either group acts on these; they differ from MHD_SYNC_EEDGE and MHD_SYNC_BFACE
  * only in the physical handlers (Farfield: copy, Coupled-Solid: nothing).  dJ
  * (in the J edge arrays) shares MHD_SYNC_JEDGE's handlers and tables.  Only
  * solves with the implicit resistive substep read them.  MHD_SYNC_BADD is

@@ -519,6 +519,7 @@ int publish(mhd_batch *b) {
     if (S->shadow_slot >= 0 && b->shadow && b->shadow->slots[S->shadow_slot]) {
       d.companion = b->shadow->slots[S->shadow_slot]->dblocks;
       d.companion_state = b->shadow->dstate + S->shadow_slot;
+      d.companion_slot = S->shadow_slot;
     }
   }
   CUDA_TRY(cudaMemcpyAsync(b->dsolves, ds.data(), sizeof(DevSolve) * C, cudaMemcpyHostToDevice, b->stream));
@@ -558,15 +559,26 @@ struct Encoded {
 
 constexpr int kEncodeChunk = 1 << 13;
 
-// Encodes entries [t0, t1) of a table; records the first invalid entry of
+// The DOF that a table of `group` addresses: Sync(dB)'s tables name the face
+// fluxes, whose dB lies in arrays of its own.
+mhd_dof table_dof(int group, mhd_dof d) {
+  if (group == MHD_SYNC_DB && d.field >= MHD_B_XI && d.field <= MHD_B_ZETA) {
+    d.comp = d.field - MHD_B_XI;
+    d.field = MHD_RES_BSTAR;
+  }
+  return d;
+}
+
+// Encodes entries [t0, t1) of a table of `group`; records the first invalid entry of
 // the chunk and whether its destinations ascend.
-void encode_chunk(const Solve *S, const mhd_copy *tab, int t0, int t1, Encoded *e, int *bad, int *kind, char *asc) {
+void encode_chunk(const Solve *S, int group, const mhd_copy *tab, int t0, int t1, Encoded *e, int *bad, int *kind,
+                  char *asc) {
   *bad = -1;
   *asc = 1;
   for (int t = t0; t < t1; ++t) {
     bool o1, o2;
-    const int64_t dc = S->code(tab[t].dst, &o1);
-    const int64_t sc = S->code(tab[t].src, &o2);
+    const int64_t dc = S->code(table_dof(group, tab[t].dst), &o1);
+    const int64_t sc = S->code(table_dof(group, tab[t].src), &o2);
     if (!o1 || !o2 || (tab[t].sign != 1.0 && tab[t].sign != -1.0)) {
       *bad = t;
       *kind = (!o1 || !o2) ? 1 : 2;
@@ -812,11 +824,15 @@ int upload_groups_periodic(Solve *S, cudaStream_t st) {
   }
   // Sync(Eres) and Sync(dB) of a periodic block: the E edge and B face
   // copies (no physical boundary tells them apart)
-  if (S->consts.resistive)
+  if (S->consts.resistive) {
+    const int64_t to_db = S->comp_base(0, kComp.first[MHD_RES_BSTAR], 0) - S->comp_base(0, kComp.first[MHD_B_XI], 0);
     for (int p = 0; p < 2; ++p) {
       enc[2 * MHD_SYNC_ERES + p] = enc[2 * MHD_SYNC_EEDGE + p];
-      enc[2 * MHD_SYNC_DB + p] = enc[2 * MHD_SYNC_BFACE + p];
+      Encoded &db = enc[2 * MHD_SYNC_DB + p] = enc[2 * MHD_SYNC_BFACE + p];
+      for (int64_t &c : db.dst) c += to_db;  // table_dof
+      for (int64_t &c : db.src) c += to_db;
     }
+  }
   return upload_encoded(S, enc, st);
 }
 
@@ -874,7 +890,7 @@ int upload_groups(Solve *S, const mhd_sync_group *groups, cudaStream_t st) {
   mhd::parallel_for(nch, [&](int c) {
     const int q = chunk_table[c];
     const int t0 = (c - first_chunk[q]) * kEncodeChunk, t1 = std::min(ntab[q], t0 + kEncodeChunk);
-    encode_chunk(S, tabs[q], t0, t1, &enc[q], &bad[c], &kind[c], &asc[c]);
+    encode_chunk(S, q / 4, tabs[q], t0, t1, &enc[q], &bad[c], &kind[c], &asc[c]);
   });
   for (int q = 0; q < NT; ++q) {
     const int g = q / 4, p = q % 4;
@@ -927,6 +943,17 @@ int upload_aliases(Solve *S, const mhd_alias_classes &a, cudaStream_t st) {
       (rc = dev_upload(S->pool, oJ, &S->T->al_ownJ, st)) || (rc = dev_upload(S->pool, ms, &S->T->al_msign, st)) ||
       (rc = dev_upload(S->pool, os, &S->T->al_osign, st)))
     return rc;
+  return MHD_OK;
+}
+
+// The blocks of the FP64 companion C read the static fields of the implicit
+// substep from the FP32 blocks of S (DevBlock::narrow).
+int link_companion(const Solve *S, const Solve *C, cudaStream_t st) {
+  std::vector<char *> narrow(S->nblocks);
+  for (int bi = 0; bi < S->nblocks; ++bi)
+    narrow[bi] = S->arena + S->main_off + S->mbase[bi] + (int64_t)kNumMetric * S->boxes[bi].total * 8;
+  CUDA_TRY(cudaMemcpy2DAsync((char *)C->dblocks + offsetof(DevBlock, narrow), sizeof(DevBlock), narrow.data(),
+                             sizeof(char *), sizeof(char *), (size_t)S->nblocks, cudaMemcpyHostToDevice, st));
   return MHD_OK;
 }
 
@@ -1094,9 +1121,9 @@ void res_apply_core(mhd_batch *b, int *nk) {  // from E_res (set) to dJ (synced)
   res_sync_eres(b, nk);
   launch(b, 1, SK_RES_DB, nk);  // the ghost faces were cleared at the substep's start (res_step)
   enqueue_sync(b, 1, MHD_SYNC_DB, nk);
-  launch(b, 1, SK_RES_DJ, nk);
+  launch(b, 1, SK_RES_DJ, nk, nullptr, RES_OF_DB);
   sync1(b, 1, alias_op(1), nk);
-  if (b->live_sing > 0) launch(b, 1, SK_SING_J, nk);  // AssembleSingularEdgeCurrent_(dB, dJ)
+  if (b->live_sing > 0) launch(b, 1, SK_SING_J, nk, nullptr, RES_OF_DB);  // AssembleSingularEdgeCurrent_(dB, dJ)
   res_sync_dj(b, nk);
 }
 void res_apply(mhd_batch *b, int *nk) {
@@ -1206,12 +1233,13 @@ struct CgJob {
 };
 
 // CG on every job's solve at once, each from x = 0 and p = r = its
-// right-hand side (r already set), until ||r|| <= tol_factor ||r_0|| or max_it
+// right-hand side (r already set; the solution is final_x of x and the states), until ||r|| <= tol_factor ||r_0|| or max_it
 // iterations, the loop on the device (build_cg_graph); the jobs' masks are
 // set here and are all clear on return; one host round trip at the end.
 // Each job's final state is in b->hcg[slot].
 int res_cg_batch(mhd_batch *b, const std::vector<CgJob> &jobs) {
   int rc;
+  b->res.use_p = !res_light_syncs(b);
   if ((rc = ensure_tpartial(b)) || (!b->cg_host_loop && (rc = build_cg_graph(b)))) return rc;
   std::vector<int> on((size_t)b->capacity, 0);
   for (int s = 0; s < b->capacity; ++s) {
@@ -1251,7 +1279,7 @@ int res_cg_batch(mhd_batch *b, const std::vector<CgJob> &jobs) {
 }
 
 // The mixed-precision solve of (I + dt eta alpha C^T beta C) E = b on the
-// solve's FP64 companion (widened alpha, beta, eta, W; its own copies of the
+// solve's FP64 companion (the solve's own alpha, beta, eta, W; its copies of the
 // E / B / J syncs); b = eta J(B*) is the FP32 step's current (the state is
 // FP32).  While the previous substep took at most res_direct iterations
 // the companion runs the CG itself in FP64 (one host round trip); after a
@@ -1302,7 +1330,7 @@ int res_refine(mhd_batch *b, int slot, Solve *S, bool *converged) {
     launch_res_cross(Dm, RES_X_DEMOTE_R, st);
     if ((rc = res_cg_batch(b, {CgJob{slot, kInnerRtol, S->res_max_it}}))) return rc;
     if ((rc = apply_masks(b, mb))) return rc;  // the loop cleared it
-    launch_res_cross(Dm, RES_X_ADD_X, st);
+    launch_res_cross(Dm, RES_X_ADD_X, st, b->res.cg, b->res.use_p);
     S->res_iters += b->hcg[slot].it;
     ++S->res_refinements;
   }
@@ -1315,7 +1343,7 @@ int res_refine(mhd_batch *b, int slot, Solve *S, bool *converged) {
 
 // The implicit resistive substep (SolveImplicitResistiveDiffusion_,
 // Mercury_ImplicitResistive.cpp:475-555) of every listed solve at once,
-// after the explicit update and its Sync(B faces): B* snapshot, J(B*),
+// after the explicit update and its Sync(B faces): J(B*),
 // b = eta J(B*), the solves (FP64: CG in the inner product weighted by
 // 1 / (eta alpha), in which A is self-adjoint, all solves in one device
 // loop; mixed precision: the short ones as FP64 CG on their companions in
@@ -1330,16 +1358,14 @@ int res_step(mhd_batch *b, const std::vector<int> &slots) {
   int rc = apply_masks(b, on);
   if (rc) return rc;
   int nk = 0;
-  launch(b, 1, SK_RES_COPYB, &nk, nullptr, RES_SNAPSHOT);
   // Calc_J_Edge on B* over the substep's range (the formula of k_bcell_jedge's
   // J part; B_cell is refreshed after the substep)
-  launch(b, 1, SK_RES_DJ, &nk);
+  launch(b, 1, SK_RES_DJ, &nk, nullptr, RES_OF_B);
   sync1(b, 1, alias_op(1), &nk);
   if (b->live_sing > 0) launch(b, 1, SK_SING_J, &nk);  // reads B* around the singular edges
   res_sync_dj(b, &nk);
   launch(b, 1, SK_RES_VEC, &nk, nullptr, RES_INIT);
-  // the B arrays turn into the operator's dB: its ghost faces start at zero
-  // (restored with B* at the end)
+  // the operator's dB: its ghost faces start at zero
   if (open_grids(b)) launch(b, 1, SK_RES_CLEARB, &nk);
   std::vector<char> conv((size_t)b->capacity, 0);
   auto take = [&](Solve *S, const ResCG &h, int s) {
@@ -1374,10 +1400,10 @@ int res_step(mhd_batch *b, const std::vector<int> &slots) {
         jobs.push_back(CgJob{S->shadow_slot, S->res_rtol > 0.0 ? S->res_rtol : 1e-10, S->res_max_it});
       }
       if ((rc = apply_masks(b, mb)) || (rc = apply_masks(sh, ms))) return rc;
-      launch_res_cross(b->dir(1), RES_X_SETUP, st);
+      launch_res_cross(b->dir(1), RES_X_SETUP, st, sh->res.cg);
       if (open_grids(sh)) launch(sh, 1, SK_RES_CLEARB, &nk);  // the companions' dB ghost faces
       if ((rc = res_cg_batch(sh, jobs))) return rc;
-      launch_res_cross(b->dir(1), RES_X_DEMOTE_X, st);
+      launch_res_cross(b->dir(1), RES_X_DEMOTE_X, st, sh->res.cg, sh->res.use_p);
       CUDA_TRY(cudaGetLastError());
       for (int s : direct) take(b->slots[s], sh->hcg[b->slots[s]->shadow_slot], s);
     }
@@ -1394,9 +1420,8 @@ int res_step(mhd_batch *b, const std::vector<int> &slots) {
       if ((rc = set_state_field(b, s, offsetof(SolveState, status), &e, sizeof e))) return rc;
     }
   // E_res = x, its owner copies; B = B* + dt (-curl E_res) on the owned faces
-  launch(b, 1, SK_RES_VEC, &nk, nullptr, RES_E_FROM_X);
+  launch(b, 1, SK_RES_VEC, &nk, nullptr, b->precision == kMixed ? RES_E_FROM_X : RES_E_FROM_CG);
   res_sync_eres(b, &nk);
-  launch(b, 1, SK_RES_COPYB, &nk, nullptr, RES_RESTORE);
   launch(b, 1, SK_RES_BUPDATE, &nk);
   CUDA_TRY(cudaGetLastError());
   std::fill(on.begin(), on.end(), 0);
@@ -1744,7 +1769,7 @@ static int upload_phys(Solve *S, const mhd_desc *desc, cudaStream_t st) {
     for (int t = 0; t < n; ++t) {
       const mhd_phys_op &o = ops[t];
       bool ok1 = false, ok2 = true;
-      const int64_t dc = S->code(o.dst, &ok1);
+      const int64_t dc = S->code(table_dof(q, o.dst), &ok1);
       if (!ok1) return fail(MHD_ERR_ARG, "physical operation %d of table %d: destination out of range", t, q);
       if (o.kind == MHD_PHYS_SET) {
         if (o.arg < 0 || o.arg >= MHD_NUM_BC) return fail(MHD_ERR_ARG, "physical operation %d: value index %d", t, o.arg);
@@ -1793,7 +1818,7 @@ static int upload_phys(Solve *S, const mhd_desc *desc, cudaStream_t st) {
       std::unordered_set<int64_t> written;
       for (int t = 0; t < n; ++t) {
         bool ok = false;
-        written.insert(S->code(ops[t].dst, &ok));
+        written.insert(S->code(table_dof(q, ops[t].dst), &ok));
       }
       const mhd_sync_group &G = desc->groups[q];
       auto ghost = [&](const mhd_dof &d) {
@@ -1809,7 +1834,7 @@ static int upload_phys(Solve *S, const mhd_desc *desc, cudaStream_t st) {
         for (int t = 0; t < m; ++t) {
           if (!ghost(tab[t].src)) continue;
           bool ok = false;
-          const int64_t c = S->code(tab[t].src, &ok);
+          const int64_t c = S->code(table_dof(q, tab[t].src), &ok);
           if (ok && written.insert(c).second) set.push_back(c | ((int64_t)MHD_BC_ZERO << kPhysArgShift));
         }
       };
@@ -2097,6 +2122,7 @@ static int add_solve(mhd_batch *b, const mhd_desc *desc, bool periodic, int *slo
       return rc;
     }
     S->shadow_slot = cs;
+    if ((rc = link_companion(S, b->shadow->slots[cs], st))) return rc;
     if ((rc = publish(b))) return rc;  // the directory entry's companion
   }
   *slot_out = slot;
@@ -2200,6 +2226,7 @@ int mhd_batch_add_like(mhd_batch *b, int src_slot, const mhd_constants *constant
       return rc;
     }
     S->shadow_slot = cs;
+    if ((rc = link_companion(S, b->shadow->slots[cs], st))) return rc;
     if ((rc = publish(b))) return rc;  // the directory entry's companion
   }
   *slot_out = slot;  // asynchronous: stream-ordered with the batch's other work
@@ -2382,7 +2409,13 @@ int mhd_batch_sync(mhd_batch *b, int slot, int group) {
   int rc = slot_check(b, slot);
   if (rc) return rc;
   if (group < 0 || group >= MHD_NUM_GROUPS) return fail(MHD_ERR_ARG, "mhd_sync: bad group %d", group);
-  return targeted(b, slot, [&](int *nk) { enqueue_sync(b, 1, group, nk, true); });  // asynchronous
+  // asynchronous; Sync(dB) on the face fluxes, through dB's arrays
+  const bool db = group == MHD_SYNC_DB && b->slots[slot]->consts.resistive;
+  return targeted(b, slot, [&](int *nk) {
+    if (db) launch(b, 1, SK_RES_COPYB, nk, nullptr, RES_DB_FROM_B);
+    enqueue_sync(b, 1, group, nk, true);
+    if (db) launch(b, 1, SK_RES_COPYB, nk, nullptr, RES_B_FROM_DB);
+  });
 }
 
 // The implicit substep's work range of one solve (kResK), after its
@@ -2471,8 +2504,6 @@ int mhd_batch_prepare(mhd_batch *b, int slot, double time, int64_t step) {
     if (S->T->sg_n > 0)  // the singular edges' geometry, FP64 in both
       CUDA_TRY(cudaMemcpyAsync(b->shadow->slots[S->shadow_slot]->sg_geo, S->sg_geo, sizeof(double) * 4 * S->T->sg_n,
                                cudaMemcpyDeviceToDevice, b->stream));
-    // the operator's coefficients (alpha, beta, eta, W), widened into the companion once
-    if ((rc = targeted(b, slot, [&](int *) { launch_res_cross(b->dir(1), RES_X_STATIC, b->stream); }))) return rc;
   }
   b->slots[slot]->prepared = true;  // asynchronous: stream-ordered with the batch's other work
   return MHD_OK;

@@ -101,6 +101,8 @@ __host__ __device__ constexpr int rslot(int comp) {
 struct DevBlock {
   void *U[2];         // U_H, U_Na components (10) of buffer 0 / 1
   char *M;
+  // of an FP64 companion's block: the real-valued components of the FP32 block it companions (else null)
+  char *narrow;
   int64_t total, si, sj;
   int G, n[3];
   int solve;          // index of the owning solve in the directory
@@ -274,6 +276,7 @@ struct DevSolve {
   // and its state in the companion batch (null without one)
   const DevBlock *companion;
   SolveState *companion_state;
+  int companion_slot;
 };
 
 // The directory handed to every kernel (by value).

@@ -79,6 +79,7 @@ __device__ __forceinline__ R dmin(R a, R b) { return (b < a) ? b : a; }
 template <class R>
 struct V {
   char *U, *Un, *M, *Mr;  // U, Un: the current and the other buffer
+  char *narrow;           // DevBlock::narrow
   uint32_t tb;  // bytes of one real-valued component array
   int total, si, sj;
   int G, n0, n1, n2;
@@ -154,6 +155,7 @@ __device__ __forceinline__ void set_view(V<R> &B, const DevBlock &DB, int cur) {
   B.total = (int)DB.total;
   B.tb = (uint32_t)B.total * (uint32_t)sizeof(R);
   B.Mr = DB.M + (int64_t)kNumMetric * DB.total * 8;
+  B.narrow = DB.narrow;
   B.si = (int)DB.si;
   B.sj = (int)DB.sj;
   B.G = DB.G;
@@ -363,6 +365,26 @@ struct VV : V<R> {
     else load(r.v, p);
     return r;
   }
+  // lv of a static field of the implicit substep: an FP64 companion reads the
+  // FP32 values it was widened from (half the bytes, the same numbers)
+  __device__ __forceinline__ Vc stat(int comp, uint32_t o) const {
+    if constexpr (sizeof(R) == 8 && M == 2) {
+      if (this->narrow) {
+        const float2 f = __ldg((const float2 *)(this->narrow + (uint64_t)rslot(comp) * (this->tb / 2) + o / 2));
+        Vc r;
+        r.v[0] = (R)f.x;
+        r.v[1] = (R)f.y;
+        return r;
+      }
+    }
+    return lv(comp, o);
+  }
+  __device__ __forceinline__ R stat1(int comp, uint32_t o) const {  // one value of stat
+    if constexpr (sizeof(R) == 8 && M == 2)
+      if (this->narrow)
+        return (R)__ldg((const float *)(this->narrow + (uint64_t)rslot(comp) * (this->tb / 2) + o / 2));
+    return this->ld(comp, o);
+  }
   // the values one k lower / higher than lv(comp, o), of which v holds the shared ones
   __device__ __forceinline__ Vc lower(const Vc &v, int comp, uint32_t o) const {
     return vdown(v, this->ld(comp, o - (uint32_t)sizeof(R)));
@@ -426,6 +448,7 @@ __device__ __forceinline__ void build_vec_item(const Dir &D, int s, int b, int t
   B.Un = uniform(B.Un);
   B.M = uniform(B.M);
   B.Mr = uniform(B.Mr);
+  B.narrow = uniform(B.narrow);
   B.tb = uniform((int)B.tb);
   B.di = uniform((int)((uint32_t)B.si * (uint32_t)sizeof(R)));
   B.dj = uniform((int)((uint32_t)B.sj * (uint32_t)sizeof(R)));
@@ -1420,26 +1443,46 @@ __global__ void __launch_bounds__(kVecThreads) k_res_kmax(Dir D, int *out) {
   });
 }
 
+// The solution of a CG loop: x with the last direction's step where the loop
+// ended ahead of it (k_res_pupd_e updates x for a loop that goes on).
+template <class R>
+__device__ __forceinline__ R final_x(const ResCG &cg, R x, R p) {
+  if (cg.it == 0) return R(0.0);
+  if (!cg.pending) return x;
+  const R step = R(cg.alpha) * p;
+  return cg.it == 1 ? step : x + step;
+}
+// The direction p of the CG: E_res holds it on the unknowns; a solve whose
+// Sync(Eres) may write those keeps it in RES_P as well (use_p).
+__device__ __forceinline__ int dir_comp(int use_p) { return use_p ? cRP : cEX; }
+
 // Vector operations of the CG on the unknowns (W > 0); other entries stay 0.
 template <class R>
-__global__ void __launch_bounds__(kVecThreads) k_res_vec(Dir D, int op) {
+__global__ void __launch_bounds__(kVecThreads) k_res_vec(Dir D, int op, const ResCG *cg, int use_p) {
   for_vec_items<R, kResK>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
     const uint32_t o = it.o;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      const Vec<R> W = B.lv(cRW + a, o);
+      const Vec<R> W = B.stat(cRW + a, o);
       auto put = [&](int comp, const Vec<R> &v) {  // v on the unknowns, 0 elsewhere
         B.st(comp + a, it, vmap<R>([&](int e) { return W.v[e] > R(0.0) ? v.v[e] : R(0.0); }), it.klo, it.khi);
       };
       switch (op) {
-        case RES_INIT:  // r = b = eta J (PackImplicitJedgeToVec_, :395-418); the CG's start sets x and p
-          put(cRR, R(0.0) + B.lv(cETAR + a, o) * B.lv(cJX + a, o));
+        case RES_INIT:  // r = b = eta J (PackImplicitJedgeToVec_, :395-418); the CG's start sets p
+          put(cRR, R(0.0) + B.stat(cETAR + a, o) * B.lv(cJX + a, o));
           break;
         case RES_E_FROM_P: put(cEX, B.lv(cRP + a, o)); break;  // UnpackVecToImplicitEres_ (:294-312)
         case RES_E_FROM_X: put(cEX, B.lv(cRX + a, o)); break;
+        case RES_E_FROM_CG: {  // the solution of the finished CG
+          const Vec<R> p = B.own(dir_comp(use_p) + a, o), x0 = B.own(cRX + a, o);
+          const Vec<R> x = vmap<R>([&](int e) { return final_x(cg[it.s], x0.v[e], p.v[e]); });
+          put(cRX, x);
+          put(cEX, x);
+          break;
+        }
         case RES_P_FROM_X: put(cRP, B.lv(cRX + a, o)); break;
-        case RES_RESID:  // r = b - q, b kept in the B* snapshot arrays (FP64 companion of a mixed solve)
-          put(cRR, B.lv(cRBS + a, o) - B.lv(cRQ + a, o));
+        case RES_RESID:  // r = b - q, b kept in the face arrays (FP64 companion of a mixed solve)
+          put(cRR, B.lv(cBX + a, o) - B.lv(cRQ + a, o));
           break;
         default: break;
       }
@@ -1449,6 +1492,7 @@ __global__ void __launch_bounds__(kVecThreads) k_res_vec(Dir D, int op) {
 
 // dB = -dt curl E on the owned faces (CurlEdgeToFace with multiplier -dt,
 // Z4_Mercury/src/operators/CTOperators.cpp:6-56; MatMultImplicitResistive_, :420-445).
+// dB has arrays of its own (RES_BSTAR), so B keeps B* and nothing is saved or restored.
 template <class R>
 __global__ void __launch_bounds__(kVecThreads) k_res_db(Dir D) {
   for_vec_items<R, kResK>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
@@ -1457,32 +1501,33 @@ __global__ void __launch_bounds__(kVecThreads) k_res_db(Dir D) {
     const bool ic = it.i < B.n0, jc = it.j < B.n1;
     const int hi = min(B.n2, it.khi);
     const Vec<R> ex = B.lv(cEX, o), ey = B.lv(cEY, o), ez = B.lv(cEZ, o);
-    B.st(cBX, it, m * ((ey - B.upper(ey, cEY, o)) + (B.lv(cEZ, o + dj) - ez)), 0, hi, jc);
-    B.st(cBY, it, m * ((B.upper(ex, cEX, o) - ex) + (ez - B.lv(cEZ, o + di))), 0, hi, ic);
-    B.st(cBZ, it, m * ((ex - B.lv(cEX, o + dj)) + (B.lv(cEY, o + di) - ey)), 0, it.khi, ic && jc);
+    B.st(cRBS, it, m * ((ey - B.upper(ey, cEY, o)) + (B.lv(cEZ, o + dj) - ez)), 0, hi, jc);
+    B.st(cRBS + 1, it, m * ((B.upper(ex, cEX, o) - ex) + (ez - B.lv(cEZ, o + di))), 0, hi, ic);
+    B.st(cRBS + 2, it, m * ((ex - B.lv(cEX, o + dj)) + (B.lv(cEY, o + di) - ey)), 0, it.khi, ic && jc);
   });
 }
 
 // alpha CurlAdjFaceToEdge(beta B) on this thread's edges (CTOperators.cpp:59-110):
-// J of the field in the face arrays.
+// J of the field in the face arrays from component cb.
 template <class R>
-__device__ __forceinline__ void edge_current(const VV<R> &B, uint32_t o, Vec<R> J[3]) {
+__device__ __forceinline__ void edge_current(const VV<R> &B, int cb, uint32_t o, Vec<R> J[3]) {
   const uint32_t di = B.di, dj = B.dj;
   constexpr uint32_t es = sizeof(R);
-  const Vec<R> fx = B.lv(cBFX, o) * B.lv(cBX, o), fy = B.lv(cBFY, o) * B.lv(cBY, o), fz = B.lv(cBFZ, o) * B.lv(cBZ, o);
-  auto below = [&](int a, uint32_t d) { return B.lv(cBFX + a, o - d) * B.lv(cBX + a, o - d); };
-  J[0] = ((vdown(fy, B.ld(cBFY, o - es) * B.ld(cBY, o - es)) - fy) + (fz - below(2, dj))) * R(1.0) * B.lv(cALX, o);
-  J[1] = ((fx - vdown(fx, B.ld(cBFX, o - es) * B.ld(cBX, o - es))) + (below(2, di) - fz)) * R(1.0) * B.lv(cALY, o);
-  J[2] = ((below(0, dj) - fx) + (fy - below(1, di))) * R(1.0) * B.lv(cALZ, o);
+  auto on = [&](int a, uint32_t q) { return B.stat(cBFX + a, q) * B.lv(cb + a, q); };
+  auto before = [&](int a) { return R(B.stat1(cBFX + a, o - es)) * B.ld(cb + a, o - es); };
+  const Vec<R> fx = on(0, o), fy = on(1, o), fz = on(2, o);
+  J[0] = ((vdown(fy, before(1)) - fy) + (fz - on(2, o - dj))) * R(1.0) * B.stat(cALX, o);
+  J[1] = ((fx - vdown(fx, before(0))) + (on(2, o - di) - fz)) * R(1.0) * B.stat(cALY, o);
+  J[2] = ((on(0, o - dj) - fx) + (fy - on(1, o - di))) * R(1.0) * B.stat(cALZ, o);
 }
 
 // dJ = alpha CurlAdjFaceToEdge(beta dB) on the owned edges (CalcImplicitDeltaJedgeFromDeltaB_,
-// Mercury_ImplicitResistive.cpp:314-393; CTOperators.cpp:59-110).
+// Mercury_ImplicitResistive.cpp:314-393; CTOperators.cpp:59-110), or J of B (ResField).
 template <class R>
-__global__ void __launch_bounds__(kVecThreads) k_res_dj(Dir D) {
+__global__ void __launch_bounds__(kVecThreads) k_res_dj(Dir D, int field) {
   for_vec_items<R, kResK>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
     Vec<R> J[3];
-    edge_current(B, it.o, J);
+    edge_current(B, field == RES_OF_B ? cBX : cRBS, it.o, J);
     B.st(cJX, it, J[0], 0, it.khi, it.i < B.n0);
     B.st(cJY, it, J[1], 0, it.khi, it.j < B.n1);
     B.st(cJZ, it, J[2], 0, min(B.n2, it.khi));
@@ -1500,9 +1545,9 @@ __global__ void __launch_bounds__(kTileThreads) k_res_clearb(Dir D) {
     const int i = it.i, j = it.j, k = it.k;
     const bool ci = i >= 0 && i < B.n0, cj = j >= 0 && j < B.n1, ck = k >= 0 && k < B.n2;
     const int o = B.off(i, j, k);
-    if (!(i >= 0 && i <= B.n0 && cj && ck)) B.c(cBX)[o] = R(0.0);
-    if (!(ci && j >= 0 && j <= B.n1 && ck)) B.c(cBY)[o] = R(0.0);
-    if (!(ci && cj && k >= 0 && k <= B.n2)) B.c(cBZ)[o] = R(0.0);
+    if (!(i >= 0 && i <= B.n0 && cj && ck)) B.c(cRBS)[o] = R(0.0);
+    if (!(ci && j >= 0 && j <= B.n1 && ck)) B.c(cRBS + 1)[o] = R(0.0);
+    if (!(ci && cj && k >= 0 && k <= B.n2)) B.c(cRBS + 2)[o] = R(0.0);
   });
 }
 
@@ -1513,7 +1558,7 @@ __global__ void __launch_bounds__(kVecThreads) k_res_q(Dir D) {
     const uint32_t o = it.o;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      const Vec<R> W = B.lv(cRW + a, o), q = B.lv(cEX + a, o) - B.lv(cETAR + a, o) * B.lv(cJX + a, o);
+      const Vec<R> W = B.stat(cRW + a, o), q = B.lv(cEX + a, o) - B.stat(cETAR + a, o) * B.lv(cJX + a, o);
       B.st(cRQ + a, it, vmap<R>([&](int e) { return W.v[e] > R(0.0) ? q.v[e] : R(0.0); }), it.klo, it.khi);
     }
   });
@@ -1548,7 +1593,7 @@ __global__ void __launch_bounds__(kVecThreads) k_res_dot(Dir D, double *partial)
   for_vec_items<R, kResK>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      const Vec<R> W = B.lv(cRW + a, it.o), r = B.lv(cRR + a, it.o);
+      const Vec<R> W = B.stat(cRW + a, it.o), r = B.lv(cRR + a, it.o);
 #pragma unroll
       for (int e = 0; e < Vec<R>::N; ++e) {
         if (!it.in || !it.has(e) || !(W.v[e] > R(0.0))) continue;
@@ -1589,6 +1634,7 @@ __device__ __forceinline__ void res_cg_end(ResCG &cs, int op, double t0, double 
     cs.r0 = cs.rnorm = sqrt(t1);
     cs.tol = cs.tol_factor * cs.r0;
     cs.it = 0;
+    cs.pending = 0;
     cs.converged = cs.rnorm <= cs.tol;
     cs.done = cs.converged || cs.max_it <= 0;
   } else if (op == CG_PQ) {
@@ -1599,6 +1645,7 @@ __device__ __forceinline__ void res_cg_end(ResCG &cs, int op, double t0, double 
     cs.rnorm = sqrt(t1);
     if (cs.rnorm <= cs.tol) cs.converged = cs.done = 1;
     else if (cs.it >= cs.max_it) cs.done = 1;
+    cs.pending = cs.done;  // x lacks alpha p: k_res_pupd_e adds it while the loop goes on
     cs.beta = t0 / cs.rho;
     cs.rho = t0;
   }
@@ -1615,7 +1662,7 @@ __device__ __forceinline__ void res_cg_end(ResCG &cs, int op, double t0, double 
 // res_cg_batch reads the states instead).
 template <class R, int OP>
 __global__ void __launch_bounds__(kVecThreads) k_res_cg(Dir D, double *tpart, ResCG *cg, unsigned int *sarr,
-                                                        cudaGraphConditionalHandle handle, int in_graph) {
+                                                        cudaGraphConditionalHandle handle, int in_graph, int use_p) {
   if (in_graph && OP == CG_PQ && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(handle, 0u);
   for_vec_items<R, kResK>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
     constexpr int N = Vec<R>::N;
@@ -1625,7 +1672,7 @@ __global__ void __launch_bounds__(kVecThreads) k_res_cg(Dir D, double *tpart, Re
     bool some = false;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      W[a] = B.lv(cRW + a, o);
+      W[a] = B.stat(cRW + a, o);
 #pragma unroll
       for (int e = 0; e < N; ++e) some = some || W[a].v[e] > R(0.0);
     }
@@ -1635,10 +1682,9 @@ __global__ void __launch_bounds__(kVecThreads) k_res_cg(Dir D, double *tpart, Re
       auto counts = [&](int a, int e) { return it.in && it.has(e) && W[a].v[e] > R(0.0); };
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
-        if (OP == CG_INIT) {  // x = 0, p = r (the start), E_res = p
+        if (OP == CG_INIT) {  // x = 0 (final_x), p = r (the start), E_res = p
           const Vec<R> r = B.lv(cRR + a, o), p = mask(a, r);
-          B.st(cRX + a, it, vset(R(0.0)), it.klo, it.khi);
-          B.st(cRP + a, it, p, it.klo, it.khi);
+          if (use_p) B.st(cRP + a, it, p, it.klo, it.khi);
           B.st(cEX + a, it, p, it.klo, it.khi);
 #pragma unroll
           for (int e = 0; e < N; ++e) {
@@ -1648,25 +1694,24 @@ __global__ void __launch_bounds__(kVecThreads) k_res_cg(Dir D, double *tpart, Re
             acc1 += rv * rv;
           }
         } else if (OP == CG_PQ) {
-          const Vec<R> q = mask(a, B.lv(cEX + a, o) - B.lv(cETAR + a, o) * B.lv(cJX + a, o)), p = B.lv(cRP + a, o);
+          const Vec<R> E = B.lv(cEX + a, o), q = mask(a, E - B.stat(cETAR + a, o) * B.lv(cJX + a, o));
+          const Vec<R> p = use_p ? B.lv(cRP + a, o) : E;
           B.st(cRQ + a, it, q, it.klo, it.khi);
 #pragma unroll
           for (int e = 0; e < N; ++e)
             if (counts(a, e)) acc0 += (double)W[a].v[e] * (double)p.v[e] * (double)q.v[e];
         } else {
-          const Vec<R> x = B.own(cRX + a, o), r = B.own(cRR + a, o), p = B.lv(cRP + a, o), q = B.lv(cRQ + a, o);
-          Vec<R> xn = x, rn = r;
+          const Vec<R> r = B.own(cRR + a, o), q = B.lv(cRQ + a, o);
+          Vec<R> rn = r;
 #pragma unroll
           for (int e = 0; e < N; ++e) {
             if (!(W[a].v[e] > R(0.0))) continue;
-            xn.v[e] += alpha * p.v[e];
             rn.v[e] -= alpha * q.v[e];
             if (!counts(a, e)) continue;
             const double w = (double)W[a].v[e], rv = (double)rn.v[e];
             acc0 += w * rv * rv;
             acc1 += rv * rv;
           }
-          B.st(cRX + a, it, xn, it.klo, it.khi);
           B.st(cRR + a, it, rn, it.klo, it.khi);
         }
       }
@@ -1700,12 +1745,12 @@ __global__ void __launch_bounds__(kVecThreads) k_res_cg(Dir D, double *tpart, Re
   });
 }
 
-// p = r + beta p and E_res = p on the unknowns (the next iteration's
-// operator input) of every solve still iterating (in the mask); warps without an
-// unknown have nothing to update (their E_res is 0, or an owner copy that the
-// next operator writes again).
+// x += alpha p, then p = r + beta p and E_res = p (the next iteration's operator
+// input) on the unknowns of every solve still iterating (in the mask): p is read
+// once for both.  Warps without an unknown have nothing to update (their E_res
+// is 0, or an owner copy that the next operator writes again).
 template <class R>
-__global__ void __launch_bounds__(kVecThreads) k_res_pupd_e(Dir D, const ResCG *cg) {
+__global__ void __launch_bounds__(kVecThreads) k_res_pupd_e(Dir D, const ResCG *cg, int use_p) {
   for_vec_items<R, kResK>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
     constexpr int N = Vec<R>::N;
     const uint32_t o = it.o;
@@ -1713,30 +1758,35 @@ __global__ void __launch_bounds__(kVecThreads) k_res_pupd_e(Dir D, const ResCG *
     bool some = false;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      W[a] = B.lv(cRW + a, o);
+      W[a] = B.stat(cRW + a, o);
 #pragma unroll
       for (int e = 0; e < N; ++e) some = some || W[a].v[e] > R(0.0);
     }
     if (!__any_sync(0xffffffffu, some && it.in)) return;
-    const R beta = R(cg[it.s].beta);
+    const R alpha = R(cg[it.s].alpha), beta = R(cg[it.s].beta);
+    const bool first = cg[it.s].it == 1;  // x = 0 until now
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      const Vec<R> p = B.own(cRP + a, o), pn = B.lv(cRR + a, o) + beta * p;
-      B.st(cRP + a, it, vmap<R>([&](int e) { return W[a].v[e] > R(0.0) ? pn.v[e] : p.v[e]; }), it.klo, it.khi);
-      B.st(cEX + a, it, vmap<R>([&](int e) { return W[a].v[e] > R(0.0) ? pn.v[e] : R(0.0); }), it.klo, it.khi);
+      const Vec<R> p = B.own(dir_comp(use_p) + a, o), pn = B.lv(cRR + a, o) + beta * p, step = alpha * p;
+      Vec<R> x = step;
+      if (!first) x = B.own(cRX + a, o) + step;
+      B.st(cRX + a, it, vmap<R>([&](int e) { return W[a].v[e] > R(0.0) ? x.v[e] : R(0.0); }), it.klo, it.khi);
+      const Vec<R> e1 = vmap<R>([&](int e) { return W[a].v[e] > R(0.0) ? pn.v[e] : R(0.0); });
+      if (use_p) B.st(cRP + a, it, e1, it.klo, it.khi);
+      B.st(cEX + a, it, e1, it.klo, it.khi);
     }
   });
 }
 
-// B* snapshot / restore over the whole box (SnapshotImplicitResistiveBstar_,
-// RestoreImplicitResistiveBstar_, :260-292).
+// B into dB's arrays and back over the whole box (an explicit Sync(dB), which is
+// asked of the face fluxes).
 template <class R>
 __global__ void __launch_bounds__(kTileThreads) k_res_copyb(Dir D, int op) {
   for_items<R, kFull>(D, [&](const DevSolve &S, const V<R> &B, const Item &it) {
     if (!it.in) return;
     const int o = B.off(it.i, it.j, it.k);
     for (int a = 0; a < 3; ++a) {
-      if (op == RES_SNAPSHOT) B.c(cRBS + a)[o] = B.c(cBX + a)[o];
+      if (op == RES_DB_FROM_B) B.c(cRBS + a)[o] = B.c(cBX + a)[o];
       else B.c(cBX + a)[o] = B.c(cRBS + a)[o];
     }
   });
@@ -2406,7 +2456,7 @@ __global__ void k_sing_emf(Dir D) {
 // over the incident owner faces of the signed beta B, times the owner's
 // orientation.
 template <class R>
-__global__ void k_sing_j(Dir D) {
+__global__ void k_sing_j(Dir D, int field) {
   for_singular(D, [&](int s, const DevSingular &G, int e) {
     const R ih = (R)G.geo[4 * e + 3];
     R sum = R(0.0);
@@ -2415,7 +2465,11 @@ __global__ void k_sing_j(Dir D) {
       if (r[5] == 0) continue;
       const V<R> B = block_view<R>(D, s, r[0]);
       const int ax = r[1];
-      sum += ih * R(r[5]) * AT(cBFX + ax, r[2], r[3], r[4]) * AT((ax == 0 ? cBX : ax == 1 ? cBY : cBZ), r[2], r[3], r[4]);
+      R beta = R(0.0);
+      if constexpr (sizeof(R) == 8)
+        if (B.narrow) beta = (R)((const float *)(B.narrow + (uint64_t)rslot(cBFX + ax) * (B.tb / 2)))[B.off(r[2], r[3], r[4])];
+      if (sizeof(R) == 4 || !B.narrow) beta = AT(cBFX + ax, r[2], r[3], r[4]);
+      sum += ih * R(r[5]) * beta * AT((field == RES_OF_DB ? cRBS : cBX) + ax, r[2], r[3], r[4]);
     }
     *at_code<R>(D.solves[s], D.state[s].cur, G.owner[3 * e + 2]) = R(G.osign[e]) * sum;
   });
@@ -2586,9 +2640,9 @@ static void launch_as(StepKernel k, const Dir &D, cudaStream_t st, const SyncOps
     case SK_DIVB: k_div_b<R><<<G, kVecThreads, 0, st>>>(D); break;
     case SK_RES_SEED: k_res_seed<R><<<G, kVecThreads, 0, st>>>(D); break;
     case SK_RES_W: k_res_w<R><<<G, kVecThreads, 0, st>>>(D); break;
-    case SK_RES_VEC: launch_dependent(k_res_vec<R>, G, kVecThreads, st, D, iarg); break;
+    case SK_RES_VEC: launch_dependent(k_res_vec<R>, G, kVecThreads, st, D, iarg, rs.cg, rs.use_p); break;
     case SK_RES_DB: launch_dependent(k_res_db<R>, G, kVecThreads, st, D); break;
-    case SK_RES_DJ: launch_dependent(k_res_dj<R>, G, kVecThreads, st, D); break;
+    case SK_RES_DJ: launch_dependent(k_res_dj<R>, G, kVecThreads, st, D, iarg); break;
     case SK_RES_Q: launch_dependent(k_res_q<R>, G, kVecThreads, st, D); break;
     case SK_RES_DOT: k_res_dot<R><<<g_grid_tiles, kVecThreads, 0, st>>>(D, rs.partial); break;
     case SK_RES_SUM: k_res_sum<<<1, 32, 0, st>>>(rs.partial, g_grid_tiles, rs.result); break;
@@ -2597,20 +2651,20 @@ static void launch_as(StepKernel k, const Dir &D, cudaStream_t st, const SyncOps
     case SK_RES_CG:
       if (iarg == CG_INIT)
         launch_dependent(k_res_cg<R, CG_INIT>, G, kVecThreads, st, D, rs.tpartial, rs.cg, rs.sarrivals, rs.handle,
-                         rs.in_graph);
+                         rs.in_graph, rs.use_p);
       else if (iarg == CG_PQ)
         launch_dependent(k_res_cg<R, CG_PQ>, G, kVecThreads, st, D, rs.tpartial, rs.cg, rs.sarrivals, rs.handle,
-                         rs.in_graph);
+                         rs.in_graph, rs.use_p);
       else
         launch_dependent(k_res_cg<R, CG_RR>, G, kVecThreads, st, D, rs.tpartial, rs.cg, rs.sarrivals, rs.handle,
-                         rs.in_graph);
+                         rs.in_graph, rs.use_p);
       break;
-    case SK_RES_PUPD_E: launch_dependent(k_res_pupd_e<R>, G, kVecThreads, st, D, rs.cg); break;
+    case SK_RES_PUPD_E: launch_dependent(k_res_pupd_e<R>, G, kVecThreads, st, D, rs.cg, rs.use_p); break;
     case SK_PHYS: launch_dependent(k_phys<R>, G, 256, st, D, iarg); break;
     // one thread per singular edge (8 radial lines of nr edges per shell)
     case SK_SING_SETUP: k_sing_setup<R><<<g_grid_tiles / 2, 64, 0, st>>>(D); break;
     case SK_SING_EMF: launch_dependent(k_sing_emf<R>, g_grid_tiles / 2, 64, st, D); break;
-    case SK_SING_J: launch_dependent(k_sing_j<R>, g_grid_tiles / 2, 64, st, D); break;
+    case SK_SING_J: launch_dependent(k_sing_j<R>, g_grid_tiles / 2, 64, st, D, iarg); break;
     case SK_RES_CLEARB: launch_dependent(k_res_clearb<R>, G, kTileThreads, st, D); break;
     default: break;
   }
@@ -2623,28 +2677,17 @@ static void launch_as(StepKernel k, const Dir &D, cudaStream_t st, const SyncOps
 #if MHD_KERNELS_F32
 // Vectors of the mixed-precision implicit substep between a solve's FP32
 // arena (every masked solve of D) and its FP64 companion (DevSolve::companion:
-// the companion's blocks, the same boxes):
-// RES_X_STATIC (the whole box, once at prepare): companion alpha, beta, eta,
-//   W = the solve's (widened).
-// The others over the substep's range (kResK), where its unknowns are:
-// RES_X_SETUP: the companion's b (B* snapshot arrays) and r = the solve's r
-//   (the FP32 right-hand side eta J(B*)); companion x = 0; the companion's
-//   dt = the step's.
+// the companion's blocks, the same boxes)
+// over the substep's range (kResK), where its unknowns are:
+// RES_X_SETUP: the companion's r = the solve's r (the FP32 right-hand side
+//   eta J(B*)) and its dt = the step's; without cg (refinement) also its b (in
+//   its face arrays) = r and x = 0.
 // RES_X_DEMOTE_R: r = (float) companion r (the next correction's right-hand side).
-// RES_X_ADD_X: companion x += x (the correction).
-// RES_X_DEMOTE_X: x = (float) companion x (the solution).
-__global__ void __launch_bounds__(kTileThreads) k_res_cross_static(Dir D) {
-  for_items<float, kFull>(D, [&](const DevSolve &S, const V<float> &B, const Item &it) {
-    if (!it.in) return;
-    V<double> C;
-    set_view(C, S.companion[it.blk], 0);
-    const int o = B.off(it.i, it.j, it.k), oc = C.off(it.i, it.j, it.k);
-    for (int a = 0; a < 3; ++a)
-      for (int c : {cALX, cBFX, cETAR, cRW}) C.c(c + a)[oc] = (double)B.c(c + a)[o];
-  });
-}
+// RES_X_ADD_X: companion x += the correction (the solve's CG cg).
+// RES_X_DEMOTE_X: x = (float) companion x: the solution of the companion's CG cg,
+//   or without it the refined x.
 template <int OP>
-__global__ void __launch_bounds__(kVecThreads) k_res_cross(Dir D) {
+__global__ void __launch_bounds__(kVecThreads) k_res_cross(Dir D, const ResCG *cg, int use_p) {
   for_vec_items<float, kResK>(D, [&](const DevSolve &S, const VV<float> &B, const VItem &it) {
     if (OP == RES_X_SETUP && threadIdx.x == 0 && it.w == D.solve_tile_prefix[kResK][it.s]) {
       S.companion_state->dt = D.state[it.s].dt;  // the step's dt, once per solve
@@ -2680,33 +2723,42 @@ __global__ void __launch_bounds__(kVecThreads) k_res_cross(Dir D) {
     for (int a = 0; a < 3; ++a) {
       if (OP == RES_X_SETUP) {
         const Vec<float> r = B.lv(cRR + a, it.o);
-        widen(cRBS + a, r);
         widen(cRR + a, r);
-        widen(cRX + a, vset(0.0f));
+        if (!cg) {  // refinement: b and x
+          widen(cBX + a, r);
+          widen(cRX + a, vset(0.0f));
+        }
       } else if (OP == RES_X_DEMOTE_R) {
         B.st(cRR + a, it, narrow(cRR + a), it.klo, it.khi);
       } else if (OP == RES_X_ADD_X) {
-        const Vec<float> x = B.lv(cRX + a, it.o);
+        const Vec<float> x = B.lv(cRX + a, it.o), d = B.lv(dir_comp(use_p) + a, it.o), W = B.lv(cRW + a, it.o);
         double *p = (double *)at(cRX + a);
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          if (it.in && it.has(e)) p[e] += (double)x.v[e];
-      } else {  // RES_X_DEMOTE_X
+          if (it.in && it.has(e) && W.v[e] > 0.0f) p[e] += (double)final_x(cg[it.s], x.v[e], d.v[e]);
+      } else if (cg) {  // RES_X_DEMOTE_X of a finished CG on the companion (its own slot's state)
+        const ResCG &c = cg[S.companion_slot];
+        const double *x = (const double *)at(cRX + a), *p = (const double *)at(dir_comp(use_p) + a);
+        const Vec<float> W = B.lv(cRW + a, it.o);
+        Vec<float> v;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v.v[e] = W.v[e] > 0.0f ? (float)final_x(c, x[e], p[e]) : 0.0f;
+        B.st(cRX + a, it, v, it.klo, it.khi);
+      } else {  // RES_X_DEMOTE_X of a refined solution
         B.st(cRX + a, it, narrow(cRX + a), it.klo, it.khi);
       }
     }
   });
 }
 
-void launch_res_cross(const Dir &D, int op, cudaStream_t st) {
+void launch_res_cross(const Dir &D, int op, cudaStream_t st, const ResCG *cg, int use_p) {
   grids<float>();
   t_full = false;
   switch (op) {
-    case RES_X_STATIC: k_res_cross_static<<<g_grid_tiles, kTileThreads, 0, st>>>(D); break;
-    case RES_X_SETUP: launch_dependent(k_res_cross<RES_X_SETUP>, g_grid_tiles, kVecThreads, st, D); break;
-    case RES_X_DEMOTE_R: launch_dependent(k_res_cross<RES_X_DEMOTE_R>, g_grid_tiles, kVecThreads, st, D); break;
-    case RES_X_ADD_X: launch_dependent(k_res_cross<RES_X_ADD_X>, g_grid_tiles, kVecThreads, st, D); break;
-    default: launch_dependent(k_res_cross<RES_X_DEMOTE_X>, g_grid_tiles, kVecThreads, st, D); break;
+    case RES_X_SETUP: launch_dependent(k_res_cross<RES_X_SETUP>, g_grid_tiles, kVecThreads, st, D, cg, use_p); break;
+    case RES_X_DEMOTE_R: launch_dependent(k_res_cross<RES_X_DEMOTE_R>, g_grid_tiles, kVecThreads, st, D, cg, use_p); break;
+    case RES_X_ADD_X: launch_dependent(k_res_cross<RES_X_ADD_X>, g_grid_tiles, kVecThreads, st, D, cg, use_p); break;
+    default: launch_dependent(k_res_cross<RES_X_DEMOTE_X>, g_grid_tiles, kVecThreads, st, D, cg, use_p); break;
   }
 }
 

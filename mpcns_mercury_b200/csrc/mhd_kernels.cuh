@@ -35,9 +35,10 @@ struct SyncOps {
   int n;
 };
 
-// Operations of SK_RES_VEC / SK_RES_DOT / SK_RES_COPYB (the arg of the launch).
-enum ResVecOp { RES_INIT = 0, RES_E_FROM_P, RES_E_FROM_X, RES_P_FROM_X, RES_RESID };
-enum ResCopyOp { RES_SNAPSHOT = 0, RES_RESTORE };
+// Operations of SK_RES_VEC / SK_RES_COPYB / SK_RES_DJ (the arg of the launch).
+enum ResVecOp { RES_INIT = 0, RES_E_FROM_P, RES_E_FROM_X, RES_E_FROM_CG, RES_P_FROM_X, RES_RESID };
+enum ResCopyOp { RES_DB_FROM_B = 0, RES_B_FROM_DB };
+enum ResField { RES_OF_B = 0, RES_OF_DB };  // SK_RES_DJ, SK_SING_J: the current of B, or of the operator's dB
 
 // CG state of one solve on the device (one per slot), for the iteration
 // loop run as a CUDA graph over every masked solve at once (k_res_cg,
@@ -49,10 +50,12 @@ struct ResCG {
   double tol_factor;
   int it, max_it;           // iterations taken, at most max_it
   int done, converged;      // loop over (converged, max_it reached, or breakdown)
+  int pending, pad_;        // x lacks the last step alpha p (final_x)
 };
-// Steps of k_res_cg: CG_INIT: x = 0, p = r, E = p, (r.r)_W and r.r, sets rho, r0, tol;
+// Steps of k_res_cg: CG_INIT: p = r, E = p, (r.r)_W and r.r, sets rho, r0, tol;
 // CG_PQ: q = A p (its last part, E - eta dJ) and (p.q)_W, sets alpha;
-// CG_RR: x += alpha p, r -= alpha q, (r.r)_W and r.r, the stop test and beta.
+// CG_RR: r -= alpha q, (r.r)_W and r.r, the stop test and beta (k_res_pupd_e then
+// updates x and p).
 // Every tile writes its pair of partial sums; the CTA that finishes a solve's
 // last tile adds them in a fixed order and updates the solve's state; a solve
 // whose loop is over leaves the mask.
@@ -69,6 +72,7 @@ struct ResScratch {
   unsigned int *sarrivals = nullptr;  // per slot: its tiles summed so far
   unsigned long long handle = 0;  // cudaGraphConditionalHandle of the loop
   int in_graph = 0;               // the CG kernels set the loop condition (launched inside the loop graph)
+  int use_p = 0;                  // the direction is kept in RES_P beside E_res
 };
 
 // Launch one engine kernel over the directory D (ops: SK_SYNC only) in the
@@ -78,12 +82,12 @@ struct ResScratch {
 void launch_step_kernel(StepKernel k, const Dir &D, cudaStream_t st, const SyncOps *ops, int precision, int iarg = 0,
                         double darg = 0.0, ResScratch rs = ResScratch{nullptr, nullptr}, bool full = false);
 int res_dot_grid();
-// Mixed-precision implicit substep: moves its coefficients (RES_X_STATIC, at
-// prepare) and vectors between every masked solve of the FP32 directory D and
-// its FP64 companion (DevSolve::companion; RES_X_SETUP also hands over the
-// step's dt) (k_res_cross, FP32 translation unit).
-enum ResCrossOp { RES_X_SETUP = 0, RES_X_DEMOTE_R, RES_X_ADD_X, RES_X_DEMOTE_X, RES_X_STATIC };
-void launch_res_cross(const Dir &D, int op, cudaStream_t st);
+// Mixed-precision implicit substep: moves its vectors between every masked
+// solve of the FP32 directory D and its FP64 companion (DevSolve::companion;
+// RES_X_SETUP also hands over the step's dt) (k_res_cross, FP32 translation
+// unit).  cg, use_p: the states and the direction of the CG whose solution is taken.
+enum ResCrossOp { RES_X_SETUP = 0, RES_X_DEMOTE_R, RES_X_ADD_X, RES_X_DEMOTE_X };
+void launch_res_cross(const Dir &D, int op, cudaStream_t st, const ResCG *cg = nullptr, int use_p = 0);
 // Per block of the masked solve of D: the largest k of an unknown of the
 // implicit substep into out[block] (atomic max; out starts at -1).
 void launch_res_kmax(const Dir &D, int precision, int *out, cudaStream_t st);
