@@ -268,9 +268,15 @@ struct mhd_batch {
   ResCG *hcg = nullptr;                                 // pinned copy of res.cg (one per slot)
   size_t tpart_elems = 0;                               // doubles allocated at res.tpartial
   bool cg_host_loop = false;                            // CG iterations launched one by one from the host
-  // device time of the implicit substep: events around the last one, the sum and count so far
-  cudaEvent_t res_ev[2] = {nullptr, nullptr};
-  bool res_ev_pending = false;
+  // device time of the implicit substep: events around the last two, the sum and count so far
+  cudaEvent_t res_ev[2][2] = {};
+  bool res_ev_pending[2] = {};
+  int res_ev_next = 0;
+  // the last substep's CG states on their way to the host (cg_done: they are in
+  // hcg, the companion batch's for mixed precision); its solves, null once removed
+  cudaEvent_t cg_done = nullptr;
+  bool cg_pending = false;
+  std::vector<Solve *> cg_solves;
   double res_ms = 0.0;
   int64_t res_steps = 0;
   int kernels_per_step = 0;
@@ -467,6 +473,11 @@ int ensure_staging(mhd_batch *b, size_t elems) {  // elems doubles
   return MHD_OK;
 }
 
+// The CG's stop factor where the constants give none, and its iteration cap (the
+// loop runs on the device: a hard bound).
+double default_rtol(const mhd_batch *b) { return b->precision == kMixed ? 1e-10 : 1e-13; }
+int cg_cap(int max_it) { return std::max(0, std::min(max_it, 100000)); }
+
 // Rewrites the directory: per-range and per-table prefix sums over the slots
 // and every slot's DevSolve (empty slots contribute no items).
 int publish(mhd_batch *b) {
@@ -521,6 +532,8 @@ int publish(mhd_batch *b) {
       d.companion_state = b->shadow->dstate + S->shadow_slot;
       d.companion_slot = S->shadow_slot;
     }
+    d.res_tol = S->res_rtol > 0.0 ? S->res_rtol : default_rtol(b);
+    d.res_max_it = cg_cap(S->res_max_it);
   }
   CUDA_TRY(cudaMemcpyAsync(b->dsolves, ds.data(), sizeof(DevSolve) * C, cudaMemcpyHostToDevice, b->stream));
   return MHD_OK;
@@ -1250,7 +1263,7 @@ int res_cg_batch(mhd_batch *b, const std::vector<CgJob> &jobs) {
     ResCG &h = b->hcg[j.slot];
     h.done = 0;
     h.tol_factor = j.tol_factor;
-    h.max_it = std::max(0, std::min(j.max_it, 100000));  // the loop runs on the device: a hard bound
+    h.max_it = cg_cap(j.max_it);
     on[j.slot] = 1;
   }
   if ((rc = apply_masks(b, on))) return rc;
@@ -1307,7 +1320,7 @@ int res_refine(mhd_batch *b, int slot, Solve *S, bool *converged) {
   launch_res_cross(Dm, RES_X_SETUP, st);
   if (open_grids(sh)) launch(sh, 1, SK_RES_CLEARB, &nk);
   CUDA_TRY(cudaGetLastError());
-  const double rtol = S->res_rtol > 0.0 ? S->res_rtol : 1e-10;
+  const double rtol = S->res_rtol > 0.0 ? S->res_rtol : default_rtol(b);
   if ((rc = res_dot(sh))) return rc;
   const double bnorm = std::sqrt(sh->hres[1]);
   double rn = bnorm;
@@ -1341,6 +1354,85 @@ int res_refine(mhd_batch *b, int slot, Solve *S, bool *converged) {
   return apply_masks(sh, ms);
 }
 
+// The right-hand side r = b = eta J(B*) of every masked solve: Calc_J_Edge on B*
+// over the substep's range (the formula of k_bcell_jedge's J part; B_cell is
+// refreshed after the substep).
+void res_rhs(mhd_batch *b, int *nk) {
+  launch(b, 1, SK_RES_DJ, nk, nullptr, RES_OF_B);
+  sync1(b, 1, alias_op(1), nk);
+  if (b->live_sing > 0) launch(b, 1, SK_SING_J, nk, nullptr, RES_OF_B);  // reads B* around the singular edges
+  res_sync_dj(b, nk);
+  launch(b, 1, SK_RES_VEC, nk, nullptr, RES_INIT);
+}
+// E_res = x, its owner copies; B = B* + dt (-curl E_res) on the owned faces.
+void res_finish(mhd_batch *b, int *nk) {
+  launch(b, 1, SK_RES_VEC, nk, nullptr, b->precision == kMixed ? RES_E_FROM_X : RES_E_FROM_CG);
+  res_sync_eres(b, nk);
+  launch(b, 1, SK_RES_BUPDATE, nk);
+}
+
+void take_cg(Solve *S, const ResCG &h) {
+  S->res_iters = h.it;
+  S->res_refinements = 0;
+  S->res_relres = h.r0 > 0.0 ? h.rnorm / h.r0 : 0.0;
+}
+
+// The figures of the last substep that res_step_device queued, once its CG is
+// over (waits for it).
+int fold_cg(mhd_batch *b) {
+  if (!b->cg_pending) return MHD_OK;
+  CUDA_TRY(cudaEventSynchronize(b->cg_done));
+  b->cg_pending = false;
+  bool any = false;
+  for (int s = 0; s < b->capacity; ++s) {
+    Solve *S = b->cg_solves[s];
+    if (!S) continue;
+    const ResCG &h = b->precision == kMixed ? b->shadow->hcg[S->shadow_slot] : b->hcg[s];
+    if (!h.ran) continue;
+    any = true;
+    take_cg(S, h);
+  }
+  b->res_ev_pending[b->res_ev_next ^ 1] = any;
+  return MHD_OK;
+}
+
+// Mixed precision: a solve whose last substep took few iterations runs the CG in
+// FP64 on its companion, another one by refinement (res_refine).
+bool runs_direct(const Solve *S) { return S->res_direct >= 0 && S->res_iters <= S->res_direct; }
+
+// The substep of every resistive solve with steps left, queued without a
+// look at the device (FP64, or mixed precision with every solve direct): which
+// solves take part, their masks, CG states and status are set there
+// (launch_res_begin, launch_res_end), and the figures follow in fold_cg.  The
+// host waits for the CG of a step only before it queues the next step's
+// substep, by when the rest of the step and the next explicit part are queued: with
+// a round trip ahead of the substep and one behind its CG, and the masks and
+// states sent from the host, a step of the resistive shell of 24 x 24 x 40
+// cells took 519 us.
+int res_step_device(mhd_batch *b) {
+  const bool mixed = b->precision == kMixed;
+  mhd_batch *c = mixed ? b->shadow : b;  // runs the CG
+  int rc, nk = 0;
+  if ((rc = ensure_tpartial(c)) || (rc = build_cg_graph(c))) return rc;
+  c->res.use_p = !res_light_syncs(c);
+  launch_res_begin(b->dir(1), c->res.cg, mixed, b->stream);
+  res_rhs(b, &nk);
+  if (mixed) launch_res_cross(b->dir(1), RES_X_SETUP, b->stream, c->res.cg);
+  if (open_grids(c)) launch(c, 1, SK_RES_CLEARB, &nk);
+  CUDA_TRY(cudaGraphLaunch(c->graph_cg, b->stream));
+  launch_res_end(b->dir(1), c->res.cg, c->hcg, c->capacity, mixed, false, b->stream);
+  b->cg_solves.assign((size_t)b->capacity, nullptr);
+  for (int s = 0; s < b->capacity; ++s)
+    if (b->slots[s] && b->slots[s]->consts.resistive) b->cg_solves[s] = b->slots[s];
+  CUDA_TRY(cudaEventRecord(b->cg_done, b->stream));
+  b->cg_pending = true;
+  if (mixed) launch_res_cross(b->dir(1), RES_X_DEMOTE_X, b->stream, c->res.cg, c->res.use_p);
+  res_finish(b, &nk);
+  launch_res_end(b->dir(1), c->res.cg, c->hcg, c->capacity, mixed, true, b->stream);
+  CUDA_TRY(cudaGetLastError());
+  return MHD_OK;
+}
+
 // The implicit resistive substep (SolveImplicitResistiveDiffusion_,
 // Mercury_ImplicitResistive.cpp:475-555) of every listed solve at once,
 // after the explicit update and its Sync(B faces): J(B*),
@@ -1358,27 +1450,19 @@ int res_step(mhd_batch *b, const std::vector<int> &slots) {
   int rc = apply_masks(b, on);
   if (rc) return rc;
   int nk = 0;
-  // Calc_J_Edge on B* over the substep's range (the formula of k_bcell_jedge's
-  // J part; B_cell is refreshed after the substep)
-  launch(b, 1, SK_RES_DJ, &nk, nullptr, RES_OF_B);
-  sync1(b, 1, alias_op(1), &nk);
-  if (b->live_sing > 0) launch(b, 1, SK_SING_J, &nk);  // reads B* around the singular edges
-  res_sync_dj(b, &nk);
-  launch(b, 1, SK_RES_VEC, &nk, nullptr, RES_INIT);
+  res_rhs(b, &nk);
   // the operator's dB: its ghost faces start at zero
   if (open_grids(b)) launch(b, 1, SK_RES_CLEARB, &nk);
   std::vector<char> conv((size_t)b->capacity, 0);
   auto take = [&](Solve *S, const ResCG &h, int s) {
-    S->res_iters = h.it;
-    S->res_refinements = 0;
-    S->res_relres = h.r0 > 0.0 ? h.rnorm / h.r0 : 0.0;
+    take_cg(S, h);
     conv[s] = h.converged != 0;
   };
   if (b->precision != kMixed) {
     std::vector<CgJob> jobs;
     for (int s : slots) {
       const Solve *S = b->slots[s];
-      jobs.push_back(CgJob{s, S->res_rtol > 0.0 ? S->res_rtol : 1e-13, S->res_max_it});
+      jobs.push_back(CgJob{s, S->res_rtol > 0.0 ? S->res_rtol : default_rtol(b), S->res_max_it});
     }
     if ((rc = res_cg_batch(b, jobs))) return rc;
     for (int s : slots) take(b->slots[s], b->hcg[s], s);
@@ -1387,7 +1471,7 @@ int res_step(mhd_batch *b, const std::vector<int> &slots) {
     std::vector<int> direct, refine;
     for (int s : slots) {
       const Solve *S = b->slots[s];
-      (S->res_direct >= 0 && S->res_iters <= S->res_direct ? direct : refine).push_back(s);
+      (runs_direct(S) ? direct : refine).push_back(s);
     }
     if (!direct.empty()) {
       // FP64 CG on the companions of the short solves, from x = 0, p = r = b
@@ -1397,7 +1481,7 @@ int res_step(mhd_batch *b, const std::vector<int> &slots) {
         const Solve *S = b->slots[s];
         mb[s] = 1;
         ms[S->shadow_slot] = 1;
-        jobs.push_back(CgJob{S->shadow_slot, S->res_rtol > 0.0 ? S->res_rtol : 1e-10, S->res_max_it});
+        jobs.push_back(CgJob{S->shadow_slot, S->res_rtol > 0.0 ? S->res_rtol : default_rtol(b), S->res_max_it});
       }
       if ((rc = apply_masks(b, mb)) || (rc = apply_masks(sh, ms))) return rc;
       launch_res_cross(b->dir(1), RES_X_SETUP, st, sh->res.cg);
@@ -1419,10 +1503,7 @@ int res_step(mhd_batch *b, const std::vector<int> &slots) {
       const int e = MHD_ERR_SOLVE;
       if ((rc = set_state_field(b, s, offsetof(SolveState, status), &e, sizeof e))) return rc;
     }
-  // E_res = x, its owner copies; B = B* + dt (-curl E_res) on the owned faces
-  launch(b, 1, SK_RES_VEC, &nk, nullptr, b->precision == kMixed ? RES_E_FROM_X : RES_E_FROM_CG);
-  res_sync_eres(b, &nk);
-  launch(b, 1, SK_RES_BUPDATE, &nk);
+  res_finish(b, &nk);
   CUDA_TRY(cudaGetLastError());
   std::fill(on.begin(), on.end(), 0);
   return apply_masks(b, on);
@@ -1540,8 +1621,10 @@ int mhd_batch_destroy(mhd_batch *b) {
   if (b->graph_a) cudaGraphExecDestroy(b->graph_a);
   if (b->graph_b) cudaGraphExecDestroy(b->graph_b);
   if (b->graph_cg) cudaGraphExecDestroy(b->graph_cg);
-  for (cudaEvent_t e : b->res_ev)
-    if (e) cudaEventDestroy(e);
+  for (auto &pair : b->res_ev)
+    for (cudaEvent_t e : pair)
+      if (e) cudaEventDestroy(e);
+  if (b->cg_done) cudaEventDestroy(b->cg_done);
   cudaFree(b->res.partial);
   cudaFree(b->res.result);
   cudaFree(b->res.cg);
@@ -2309,6 +2392,7 @@ int mhd_batch_remove(mhd_batch *b, int slot) {
   Solve *S = b->slots[slot];
   if (S->shadow_slot >= 0 && (rc = mhd_batch_remove(b->shadow, S->shadow_slot))) return rc;
   b->slots[slot] = nullptr;
+  if (slot < (int)b->cg_solves.size()) b->cg_solves[slot] = nullptr;
   if (S->consts.resistive) --b->n_res;
   count_tables(b, S, -1);
   SolveState s0{};
@@ -2748,18 +2832,21 @@ int mhd_batch_request(mhd_batch *b, int slot, int64_t nsteps) {
   return set_state_field(b, slot, offsetof(SolveState, remaining), &n, sizeof n);
 }
 
-// Adds the last substep's event time to the batch's sum (its events have
-// completed: the caller synchronised the stream after them).
-static void fold_substep_time(mhd_batch *b) {
-  if (!b->res_ev_pending) return;
-  float ms = 0.0f;
-  if (cudaEventElapsedTime(&ms, b->res_ev[0], b->res_ev[1]) == cudaSuccess) {
-    b->res_ms += ms;
-    ++b->res_steps;
-  } else {
-    cudaGetLastError();
+// Adds the event time of the substeps before the last one (all: of the last one
+// too) to the batch's sum; their events have completed (the caller waited for
+// work behind them).
+static void fold_substep_time(mhd_batch *b, bool all) {
+  for (int p = 0; p < 2; ++p) {
+    if (!b->res_ev_pending[p] || (!all && p == (b->res_ev_next ^ 1))) continue;
+    float ms = 0.0f;
+    if (cudaEventElapsedTime(&ms, b->res_ev[p][0], b->res_ev[p][1]) == cudaSuccess) {
+      b->res_ms += ms;
+      ++b->res_steps;
+    } else {
+      cudaGetLastError();
+    }
+    b->res_ev_pending[p] = false;
   }
-  b->res_ev_pending = false;
 }
 
 int mhd_batch_cg_host_loop(mhd_batch *b, int on) {
@@ -2772,7 +2859,8 @@ int mhd_batch_cg_host_loop(mhd_batch *b, int on) {
 int mhd_batch_substep_ms(mhd_batch *b, double *ms_per_step) {
   if (!b || !ms_per_step) return fail(MHD_ERR_ARG, "mhd_batch_substep_ms: bad arguments");
   CUDA_TRY(cudaStreamSynchronize(b->stream));
-  fold_substep_time(b);
+  if (const int rc = fold_cg(b)) return rc;
+  fold_substep_time(b, true);
   *ms_per_step = b->res_steps > 0 ? b->res_ms / (double)b->res_steps : 0.0;
   b->res_ms = 0.0;
   b->res_steps = 0;
@@ -2787,28 +2875,43 @@ int mhd_batch_run(mhd_batch *b, int nsteps) {
     for (int s = 0; s < nsteps; ++s) CUDA_TRY(cudaGraphLaunch(b->graph, b->stream));
     return MHD_OK;
   }
-  // with implicit resistive solves: part A, their substep (all at once, host-driven), part B
+  // with implicit resistive solves: part A, their substep (all at once), part B
   if ((rc = capture(b, &b->graph_a, nullptr, [&](int *nk) { enqueue_step_a(b, nk); }))) return rc;
   if ((rc = capture(b, &b->graph_b, nullptr, [&](int *nk) { enqueue_step_b(b, nk, true); }))) return rc;
-  if (!b->res_ev[0]) {
-    CUDA_TRY(cudaEventCreate(&b->res_ev[0]));
-    CUDA_TRY(cudaEventCreate(&b->res_ev[1]));
+  if (!b->cg_done) {
+    for (auto &pair : b->res_ev)
+      for (cudaEvent_t &e : pair) CUDA_TRY(cudaEventCreate(&e));
+    CUDA_TRY(cudaEventCreateWithFlags(&b->cg_done, cudaEventDisableTiming));
   }
   std::vector<int> slots;
   for (int s = 0; s < nsteps; ++s) {
     CUDA_TRY(cudaGraphLaunch(b->graph_a, b->stream));
-    if ((rc = read_state(b))) return rc;
-    fold_substep_time(b);  // the previous step's substep is complete
-    slots.clear();
-    for (int q = 0; q < b->capacity; ++q) {
-      const Solve *S = b->slots[q];
-      if (S && S->consts.resistive && b->hstate[q].remaining > 0 && b->hstate[q].status == 0) slots.push_back(q);
-    }
-    if (!slots.empty()) CUDA_TRY(cudaEventRecord(b->res_ev[0], b->stream));
-    if ((rc = res_step(b, slots))) return rc;
-    if (!slots.empty()) {
-      CUDA_TRY(cudaEventRecord(b->res_ev[1], b->stream));
-      b->res_ev_pending = true;
+    if ((rc = fold_cg(b))) return rc;  // the previous step's
+    fold_substep_time(b, false);
+    bool device = !b->cg_host_loop;
+    if (b->precision == kMixed)
+      for (const Solve *S : b->slots) device = device && !(S && S->consts.resistive && !runs_direct(S));
+    const int p = b->res_ev_next;
+    if (device) {
+      CUDA_TRY(cudaEventRecord(b->res_ev[p][0], b->stream));
+      if ((rc = res_step_device(b))) return rc;
+      CUDA_TRY(cudaEventRecord(b->res_ev[p][1], b->stream));
+      b->res_ev_next ^= 1;
+    } else {
+      if ((rc = read_state(b))) return rc;
+      fold_substep_time(b, true);
+      slots.clear();
+      for (int q = 0; q < b->capacity; ++q) {
+        const Solve *S = b->slots[q];
+        if (S && S->consts.resistive && b->hstate[q].remaining > 0 && b->hstate[q].status == 0) slots.push_back(q);
+      }
+      if (!slots.empty()) CUDA_TRY(cudaEventRecord(b->res_ev[p][0], b->stream));
+      if ((rc = res_step(b, slots))) return rc;
+      if (!slots.empty()) {
+        CUDA_TRY(cudaEventRecord(b->res_ev[p][1], b->stream));
+        b->res_ev_pending[p] = true;
+        b->res_ev_next ^= 1;
+      }
     }
     CUDA_TRY(cudaGraphLaunch(b->graph_b, b->stream));
   }
@@ -2833,7 +2936,7 @@ static void fill_solve_info(const mhd_batch *b, int s, mhd_info *info) {
 int mhd_batch_poll(mhd_batch *b, mhd_info *infos) {
   if (!b || !infos) return fail(MHD_ERR_ARG, "mhd_batch_poll: bad arguments");
   int rc = read_state(b);
-  if (rc) return rc;
+  if (rc || (rc = fold_cg(b))) return rc;
   for (int s = 0; s < b->capacity; ++s) {
     const SolveState &st = b->hstate[s];
     std::memset(&infos[s], 0, sizeof(mhd_info));
@@ -2874,6 +2977,14 @@ int mhd_batch_poll_async(mhd_batch *b, int *ticket) {
 int mhd_batch_poll_wait(mhd_batch *b, int ticket, mhd_info *infos) {
   if (!b || !infos || ticket < 0 || ticket > 1) return fail(MHD_ERR_ARG, "mhd_batch_poll_wait: bad arguments");
   CUDA_TRY(cudaEventSynchronize(b->snap_ev[ticket]));
+  // the substeps ahead of the snapshot are over; a later one's figures are not waited for
+  if (b->cg_pending) {
+    if (cudaEventQuery(b->cg_done) == cudaSuccess) {
+      if (const int rc = fold_cg(b)) return rc;
+    } else {
+      cudaGetLastError();  // not ready
+    }
+  }
   fill_infos(b, b->hsnap[ticket], infos);
   return MHD_OK;
 }

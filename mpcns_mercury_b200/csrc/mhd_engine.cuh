@@ -277,6 +277,9 @@ struct DevSolve {
   const DevBlock *companion;
   SolveState *companion_state;
   int companion_slot;
+  // the CG's stop factor and iteration cap in a substep on the device (launch_res_begin)
+  double res_tol;
+  int res_max_it;
 };
 
 // The directory handed to every kernel (by value).

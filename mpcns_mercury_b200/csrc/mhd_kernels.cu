@@ -2787,6 +2787,42 @@ void launch_res_kmax(const Dir &D, int precision, int *out, cudaStream_t st) {
   }
 }
 
+__global__ void k_res_begin(Dir D, ResCG *cg, int mixed) {
+  for (int s = threadIdx.x; s < D.nsolves; s += blockDim.x) {
+    const DevSolve &S = D.solves[s];
+    SolveState &st = D.state[s];
+    const bool on = S.nblocks > 0 && S.c.resistive && st.remaining > 0 && st.status == 0;
+    st.mask = on;
+    if (mixed && !(S.nblocks > 0 && S.c.resistive)) continue;
+    ResCG h{};
+    h.done = !on;
+    h.ran = on;
+    h.tol_factor = S.res_tol;
+    h.max_it = S.res_max_it;
+    cg[mixed ? S.companion_slot : s] = h;
+    if (mixed) S.companion_state->mask = on;
+  }
+}
+__global__ void k_res_end(Dir D, const ResCG *cg, ResCG *host, int n, int mixed, int last) {
+  for (int s = threadIdx.x; s < D.nsolves; s += blockDim.x) {
+    const DevSolve &S = D.solves[s];
+    SolveState &st = D.state[s];
+    if (!(S.nblocks > 0 && S.c.resistive)) continue;
+    const ResCG &h = cg[mixed ? S.companion_slot : s];
+    st.mask = !last && h.ran;
+    if (!last && h.ran && !h.converged) st.status = MHD_ERR_SOLVE;
+  }
+  if (!last)
+    for (int q = threadIdx.x; q < n; q += blockDim.x) host[q] = cg[q];
+}
+
+void launch_res_begin(const Dir &D, ResCG *cg, bool mixed, cudaStream_t st) {
+  k_res_begin<<<1, 256, 0, st>>>(D, cg, mixed);
+}
+void launch_res_end(const Dir &D, const ResCG *cg, ResCG *host, int n, bool mixed, bool last, cudaStream_t st) {
+  k_res_end<<<1, 256, 0, st>>>(D, cg, host, n, mixed, last);
+}
+
 void launch_step_kernel_f32(StepKernel k, const Dir &D, cudaStream_t st, const SyncOps *ops, int iarg, double darg,
                             ResScratch rs, bool full);
 

@@ -50,7 +50,8 @@ struct ResCG {
   double tol_factor;
   int it, max_it;           // iterations taken, at most max_it
   int done, converged;      // loop over (converged, max_it reached, or breakdown)
-  int pending, pad_;        // x lacks the last step alpha p (final_x)
+  int pending;              // x lacks the last step alpha p (final_x)
+  int ran;                  // the solve took part in the last substep (launch_res_begin)
 };
 // Steps of k_res_cg: CG_INIT: p = r, E = p, (r.r)_W and r.r, sets rho, r0, tol;
 // CG_PQ: q = A p (its last part, E - eta dJ) and (p.q)_W, sets alpha;
@@ -88,6 +89,13 @@ int res_dot_grid();
 // unit).  cg, use_p: the states and the direction of the CG whose solution is taken.
 enum ResCrossOp { RES_X_SETUP = 0, RES_X_DEMOTE_R, RES_X_ADD_X, RES_X_DEMOTE_X };
 void launch_res_cross(const Dir &D, int op, cudaStream_t st, const ResCG *cg = nullptr, int use_p = 0);
+// The ends of a substep whose decisions stay on the device.  launch_res_begin
+// masks the resistive solves that take this step (and their companions; mixed:
+// the CG runs on these) and sets up their CG states.  launch_res_end after the
+// CG: masks them again, gives a solve that did not converge MHD_ERR_SOLVE and
+// writes the n states to host (pinned); with last, clears the masks.
+void launch_res_begin(const Dir &D, ResCG *cg, bool mixed, cudaStream_t st);
+void launch_res_end(const Dir &D, const ResCG *cg, ResCG *host, int n, bool mixed, bool last, cudaStream_t st);
 // Per block of the masked solve of D: the largest k of an unknown of the
 // implicit substep into out[block] (atomic max; out starts at -1).
 void launch_res_kmax(const Dir &D, int precision, int *out, cudaStream_t st);
