@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cmath>
 #include <cstdarg>
@@ -166,6 +167,13 @@ struct Tables {
   // Some write of the E alias reduction, the singular edges or Sync(Ehall) lands
   // on an edge inside a block (hall_writes_inside)
   bool hall_late = false;
+  // The step's syncs may run in fewer launches (joined_syncs); Sync(dB) of the
+  // substep needs its halo and owner copies only (plain_db); one block periodic
+  // in every direction (upload_groups_periodic)
+  bool sync_joined = false, db_plain = false, periodic = false;
+  bool one_pass[kMaxGroups] = {};  // halo, staged and owner copies of the step touch one another's data nowhere
+  bool two_pass[kMaxGroups] = {};  // the halo and the staged copies do not
+  bool db_apart = false;           // no copy of Sync(dB) reads what its halo or staged copies write
 };
 
 struct Solve {
@@ -258,6 +266,8 @@ struct mhd_batch {
   int live_phys[kNumPhys] = {};
   int live_sing = 0;
   int n_res = 0;                                        // slots whose solve has the implicit resistive substep
+  // solves whose syncs need the general order, whose Sync(dB) does, and that are not periodic blocks
+  int n_sync_general = 0, n_db_general = 0, n_open = 0;
   int n_res_full = 0;                                   // of them, solves whose substep runs the full E / J syncs
   // FP64 batch of the companions of mixed-precision resistive solves, which
   // runs on this batch's stream and pool (borrowed = true in the companion)
@@ -341,7 +351,8 @@ void launch(mhd_batch *b, int mode, StepKernel k, int *nk, const SyncOps *ops = 
 }
 
 SyncOp copy_op(int g, int phase, int prev = 0, int mark = 0) { return SyncOp{SYNC_COPY, g, phase, prev, mark}; }
-SyncOp alias_op(int which) { return SyncOp{SYNC_ALIAS, which, 0, 0, 0}; }
+// all: the value goes to every member of a class, not only to its owner
+SyncOp alias_op(int which, int all = 0) { return SyncOp{SYNC_ALIAS, which, 0, 0, all}; }
 
 // A sync operation some solve of the batch has work for (a copy phase whose
 // table is empty in every solve is left out: the depth-0 halos of E, E_Hall
@@ -351,18 +362,15 @@ bool op_live(const mhd_batch *b, const SyncOp &o) {
   return o.kind != SYNC_COPY || o.phase == kPhHaloFull || b->live_tables[o.arg][o.phase] > 0;
 }
 
-// One k_sync launch running one or two independent sync operations.
-void sync1(mhd_batch *b, int mode, SyncOp a, int *nk) {
-  if (!op_live(b, a)) return;
-  SyncOps ops{{a, a}, 1};
-  launch(b, mode, SK_SYNC, nk, &ops);
+// One k_sync launch running up to kMaxSyncOps independent sync operations.
+void sync_ops(mhd_batch *b, int mode, std::initializer_list<SyncOp> list, int *nk) {
+  SyncOps ops{};
+  for (const SyncOp &o : list)
+    if (op_live(b, o)) ops.op[ops.n++] = o;
+  if (ops.n > 0) launch(b, mode, SK_SYNC, nk, &ops);
 }
-void sync2(mhd_batch *b, int mode, SyncOp a, SyncOp c, int *nk) {
-  if (!op_live(b, a)) return sync1(b, mode, c, nk);
-  if (!op_live(b, c)) return sync1(b, mode, a, nk);
-  SyncOps ops{{a, c}, 2};
-  launch(b, mode, SK_SYNC, nk, &ops);
-}
+void sync1(mhd_batch *b, int mode, SyncOp a, int *nk) { sync_ops(b, mode, {a}, nk); }
+void sync2(mhd_batch *b, int mode, SyncOp a, SyncOp c, int *nk) { sync_ops(b, mode, {a, c}, nk); }
 
 // The physical boundary operations of table `which` (a group, or the wall
 // EMF), when some solve has them.
@@ -396,6 +404,47 @@ void enqueue_sync(mhd_batch *b, int mode, int g, int *nk, bool full = false) {
   sync1(b, mode, copy_op(g, kPhOwner), nk);
 }
 
+// The step's syncs in fewer launches, for batches whose solves' tables all allow
+// it (joined_syncs; the edge and cell groups then need two launches at most,
+// where MercuryBoundary::Sync's phases take four).  Results are the same bits:
+// - the staging of a group's ghosts, which only that group's sync writes, runs
+//   beside the alias reduction ahead of it (U's ahead of the buffer flip, from
+//   the buffer that is the other one after it);
+// - a group's halo, staged and owner copies run in one launch (of Sync(B faces),
+//   whose halo copies read owner copies, the owner copies follow);
+// - on periodic blocks the alias reduction writes every member of a class, and
+//   E + Ehall, the same sum at each of them, needs no owner copies.
+// A k_sync launch costs 3 to 4 us whatever it copies.
+SyncOp stash_op(int g) { return copy_op(g, kPhStash); }
+bool has_pre(const mhd_batch *b, int g) { return b->live_phys[g] > 0 || b->live_tables[g][kPhStash] > 0; }
+
+// enqueue_derived
+void enqueue_derived_joined(mhd_batch *b, int mode, int *nk, bool end_of_step) {
+  const int B = MHD_SYNC_B_CELL, J = MHD_SYNC_JEDGE, C = MHD_SYNC_J_CELL;
+  const bool all = b->n_open == 0, early = b->live_tables[B][kPhStash] == 0;
+  const SyncOp bhalo = copy_op(B, kPhHalo);
+  launch(b, mode, SK_BCELL_JEDGE, nk);
+  phys1(b, mode, B, nk);
+  sync_ops(b, mode, {alias_op(1, all), early ? bhalo : stash_op(B), stash_op(J), stash_op(C)}, nk);
+  if (b->live_sing > 0) launch(b, mode, SK_SING_J, nk);
+  phys1(b, mode, J, nk);
+  SyncOps ops{};
+  auto add = [&](const SyncOp &o) {
+    if (op_live(b, o)) ops.op[ops.n++] = o;
+  };
+  if (!early) add(bhalo);
+  add(copy_op(B, kPhUnstash));
+  add(copy_op(B, kPhOwner));
+  add(copy_op(J, kPhHalo));
+  add(copy_op(J, kPhUnstash));
+  if (!all) add(copy_op(J, kPhOwner));
+  if (ops.n > 0) launch(b, mode, SK_SYNC, nk, &ops);
+  launch(b, mode, SK_JCELL, nk);
+  phys1(b, mode, C, nk);
+  sync_ops(b, mode, {copy_op(C, kPhHalo), copy_op(C, kPhUnstash), copy_op(C, kPhOwner)}, nk);
+  launch(b, mode, SK_PV_UPLUS, nk, nullptr, end_of_step);
+}
+
 // UpdateDerivedFields_ (Z4_Mercury/src/physics/MercurySolver_Tools.cpp:309-321) plus the
 // contravariant velocities and the next step's CFL dt.  Independent sync
 // stages share a launch: Sync(B_cell) runs beside the J alias reduction and
@@ -403,6 +452,7 @@ void enqueue_sync(mhd_batch *b, int mode, int g, int *nk, bool full = false) {
 // edges' current replaces their owners' after the alias reduction
 // (Calc_J_Edge, Z4_Mercury/src/physics/MercurySolver_Current.cpp:140-201).
 void enqueue_derived(mhd_batch *b, int mode, int *nk, bool end_of_step = false) {
+  if (b->n_sync_general == 0) return enqueue_derived_joined(b, mode, nk, end_of_step);
   launch(b, mode, SK_BCELL_JEDGE, nk);
   sync_pre(b, mode, MHD_SYNC_B_CELL, nk);
   sync2(b, mode, copy_op(MHD_SYNC_B_CELL, kPhHalo), alias_op(1), nk);
@@ -417,6 +467,31 @@ void enqueue_derived(mhd_batch *b, int mode, int *nk, bool end_of_step = false) 
   launch(b, mode, SK_PV_UPLUS, nk, nullptr, end_of_step);
 }
 
+// enqueue_step_a after the edge EMF
+void enqueue_step_a_joined(mhd_batch *b, int *nk) {
+  const int m = 0, H = MHD_SYNC_EHALL, E = MHD_SYNC_EEDGE, U = MHD_SYNC_UCELL, F = MHD_SYNC_BFACE;
+  const bool all = b->n_open == 0;
+  if (b->live_sing > 0 || has_pre(b, H)) {
+    sync_ops(b, m, {alias_op(0, all), stash_op(H), stash_op(E), stash_op(U), stash_op(F)}, nk);
+    if (b->live_sing > 0) launch(b, m, SK_SING_EMF, nk);
+    phys1(b, m, H, nk);
+    sync_ops(b, m, {copy_op(H, kPhHalo), copy_op(H, kPhUnstash), copy_op(H, kPhOwner)}, nk);
+  } else {
+    sync_ops(b, m, {alias_op(0, all), stash_op(E), stash_op(U), stash_op(F), copy_op(H, kPhHalo), copy_op(H, kPhOwner)},
+             nk);
+  }
+  launch(b, m, SK_ADD_HALL, nk);  // on the edges in the blocks' faces
+  phys1(b, m, kMaxGroups, nk);    // the wall EMF: E_t = 0 on solid-wall edges
+  phys1(b, m, E, nk);
+  if (!all) sync_ops(b, m, {copy_op(E, kPhHalo), copy_op(E, kPhUnstash), copy_op(E, kPhOwner)}, nk);
+  launch(b, m, SK_FLUID, nk, nullptr, b->fluid_tile);
+  launch(b, m, SK_BFACE, nk);
+  phys1(b, m, U, nk);
+  phys1(b, m, F, nk);
+  sync_ops(b, m, {copy_op(U, kPhHalo), copy_op(F, kPhHalo), copy_op(U, kPhUnstash), copy_op(F, kPhUnstash)}, nk);
+  sync_ops(b, m, {copy_op(U, kPhOwner), copy_op(F, kPhOwner)}, nk);
+}
+
 // StepOnce (Z4_Mercury/src/MercurySolver_Driver.cpp:21-61) for every active slot, in two
 // parts: A up to the Euler update and Sync(U), Sync(B faces); B the derived
 // refresh.  With implicit resistive solves, their substep
@@ -426,6 +501,7 @@ void enqueue_step_a(mhd_batch *b, int *nk) {
   // AssembleRHS_Induction_CT_ (Z4_Mercury/src/physics/MercurySolver_MagneticRHS.cpp:90-171)
   launch(b, m, SK_FACE_EMF, nk);
   launch(b, m, SK_EDGE_EMF, nk);
+  if (b->n_sync_general == 0) return enqueue_step_a_joined(b, nk);
   if (b->live_sing > 0 || b->live_phys[MHD_SYNC_EHALL] > 0 || b->live_tables[MHD_SYNC_EHALL][kPhStash] > 0) {
     // the E alias reduction, the singular edges' EMF and Hall EMF, Sync(Ehall)
     sync1(b, m, alias_op(0), nk);
@@ -454,7 +530,13 @@ void enqueue_step_a(mhd_batch *b, int *nk) {
 }
 void enqueue_step_b(mhd_batch *b, int *nk, bool resync_b) {
   const int m = 0;
-  if (resync_b) enqueue_sync(b, m, MHD_SYNC_BFACE, nk);
+  if (resync_b && b->n_sync_general == 0) {
+    sync_pre(b, m, MHD_SYNC_BFACE, nk);
+    sync2(b, m, copy_op(MHD_SYNC_BFACE, kPhHalo), copy_op(MHD_SYNC_BFACE, kPhUnstash), nk);
+    sync1(b, m, copy_op(MHD_SYNC_BFACE, kPhOwner), nk);
+  } else if (resync_b) {
+    enqueue_sync(b, m, MHD_SYNC_BFACE, nk);
+  }
   enqueue_derived(b, m, nk, true);
 }
 void enqueue_step(mhd_batch *b, int *nk) {
@@ -698,6 +780,38 @@ std::vector<int64_t> build_segments(const Encoded &e, int es, int max_depth, con
   return seg;
 }
 
+// A set of arena codes, each with a number (open addressing, at most a quarter
+// full: a code that is not in it is mostly answered by the first slot).
+struct CodeSet {
+  struct Slot {
+    int64_t code = -1, value = 0;
+  };
+  std::vector<Slot> slot;
+  size_t mask;
+  explicit CodeSet(size_t n) {
+    size_t size = 4;
+    while (size < 4 * n) size *= 2;
+    slot.resize(size);
+    mask = size - 1;
+  }
+  size_t at(int64_t c) const {
+    size_t q = (size_t)(((uint64_t)c * 0x9e3779b97f4a7c15ull) >> 20) & mask;
+    while (slot[q].code != -1 && slot[q].code != c) q = (q + 1) & mask;
+    return q;
+  }
+  void add(int64_t c, int64_t value = 0) {
+    Slot &s = slot[at(c)];
+    s.code = c;
+    s.value = value;
+  }
+  bool has(int64_t c) const { return slot[at(c)].code == c; }
+};
+CodeSet code_set(const std::vector<int64_t> &v) {
+  CodeSet s(v.size());
+  for (int64_t c : v) s.add(c);
+  return s;
+}
+
 // The three phases of every group (pruned halo, owner, full halo) segmented
 // on the host threads from the encoded halo (2 g) and owner (2 g + 1)
 // tables, and uploaded.
@@ -709,26 +823,66 @@ std::vector<int64_t> build_segments(const Encoded &e, int es, int max_depth, con
 std::vector<char> step_halo_mask(const Encoded &h, const Encoded *owner, const Encoded *stash, int max_depth) {
   const size_t n = h.dst.size();
   std::vector<char> keep(n, 0);
-  std::unordered_map<int64_t, size_t> by_dst;
-  by_dst.reserve(n * 2);
-  for (size_t t = 0; t < n; ++t) by_dst[h.dst[t]] = t;  // the later entry wins a destination written twice
   std::vector<int64_t> todo;
+  size_t deep = 0;
+  for (size_t t = 0; t < n; ++t) {
+    keep[t] = h.depth[t] <= max_depth;
+    if (keep[t]) todo.push_back(h.src[t]);
+    else ++deep;
+  }
+  if (deep == 0) return keep;
+  CodeSet by_dst(deep);
   for (size_t t = 0; t < n; ++t)
-    if (h.depth[t] <= max_depth) {
-      keep[t] = 1;
-      todo.push_back(h.src[t]);
-    }
+    if (!keep[t]) by_dst.add(h.dst[t], (int64_t)t);  // the later entry wins a destination written twice
   for (const Encoded *o : {owner, stash})
     if (o) todo.insert(todo.end(), o->src.begin(), o->src.end());
   while (!todo.empty()) {
     const int64_t c = todo.back();
     todo.pop_back();
-    auto it = by_dst.find(c);
-    if (it == by_dst.end() || keep[it->second]) continue;
-    keep[it->second] = 1;
-    todo.push_back(h.src[it->second]);
+    const CodeSet::Slot &e = by_dst.slot[by_dst.at(c)];
+    if (e.code != c || keep[e.value]) continue;
+    keep[e.value] = 1;
+    todo.push_back(h.src[e.value]);
   }
   return keep;
+}
+
+// Whether a group's copies of the step may run at once: the kept halo copies h,
+// the owner copies o and the copies from the staging slots u write different
+// positions and none reads what another phase writes (*one); the same of the
+// halo copies and the staged ones alone (*two).
+void pass_flags(const Encoded &h, const std::vector<char> &keep, const Encoded &o, const Encoded *u, bool *one,
+                bool *two) {
+  static const std::vector<int64_t> kNone;
+  const std::vector<int64_t> &udst = u ? u->dst : kNone;
+  const CodeSet od = code_set(o.dst), os = code_set(o.src), ud = code_set(udst);
+  bool halo_u = true, halo_o = true, o_u = true;
+  if (!udst.empty() || !o.dst.empty())
+    for (size_t t = 0; t < h.dst.size() && (halo_u || halo_o); ++t) {
+      if (!keep[t]) continue;
+      halo_u = halo_u && !ud.has(h.dst[t]) && !ud.has(h.src[t]);
+      halo_o = halo_o && !od.has(h.dst[t]) && !os.has(h.dst[t]) && !od.has(h.src[t]);
+    }
+  for (int64_t c : udst) o_u = o_u && !od.has(c) && !os.has(c);
+  *two = halo_u;
+  *one = halo_u && halo_o && o_u;
+}
+
+// No kept halo copy and no owner copy reads a position that a kept halo copy or a
+// staged one writes.
+bool reads_no_ghost_write(const Encoded &h, const std::vector<char> &keep, const Encoded &o, const Encoded *u) {
+  size_t n = u ? u->dst.size() : 0;
+  for (char k : keep) n += k != 0;
+  CodeSet w(n);
+  if (u)
+    for (int64_t c : u->dst) w.add(c);
+  for (size_t t = 0; t < h.dst.size(); ++t)
+    if (keep[t]) w.add(h.dst[t]);
+  for (size_t t = 0; t < h.src.size(); ++t)
+    if (keep[t] && w.has(h.src[t])) return false;
+  for (int64_t c : o.src)
+    if (w.has(c)) return false;
+  return true;
 }
 
 // Every group's phases (CopyPhase) segmented on the host threads from its
@@ -745,6 +899,8 @@ int upload_encoded(Solve *S, const std::vector<Encoded> &enc, cudaStream_t st, i
       case kPhHalo: {
         const std::vector<char> keep = step_halo_mask(h, &o, stash, kHaloDepth[g]);
         seg[q] = build_segments(h, S->es, -1, &keep);
+        pass_flags(h, keep, o, unstash, &S->T->one_pass[g], &S->T->two_pass[g]);
+        if (g == MHD_SYNC_DB) S->T->db_apart = S->T->two_pass[g] && reads_no_ghost_write(h, keep, o, unstash);
         break;
       }
       case kPhOwner: seg[q] = build_segments(o, S->es, -1); break;
@@ -1065,6 +1221,14 @@ bool count_tables(mhd_batch *b, const Solve *S, int d) {
     grew = grew || (d > 0 && b->live_sing == 0);
     b->live_sing += d;
   }
+  auto count = [&](bool has, int *n) {
+    if (!has) return;
+    grew = grew || (d > 0 && *n == 0);
+    *n += d;
+  };
+  count(!S->T->sync_joined, &b->n_sync_general);
+  count(S->consts.resistive && !S->T->db_plain, &b->n_db_general);
+  count(!S->T->periodic, &b->n_open);
   if (S->consts.resistive && !S->T->res_ghost_writes_only) {
     grew = grew || (d > 0 && b->n_res_full == 0);
     b->n_res_full += d;
@@ -1133,7 +1297,12 @@ void res_sync_dj(mhd_batch *b, int *nk) {  // after the current's alias reductio
 void res_apply_core(mhd_batch *b, int *nk) {  // from E_res (set) to dJ (synced)
   res_sync_eres(b, nk);
   launch(b, 1, SK_RES_DB, nk);  // the ghost faces were cleared at the substep's start (res_step)
-  enqueue_sync(b, 1, MHD_SYNC_DB, nk);
+  if (b->n_db_general > 0) {
+    enqueue_sync(b, 1, MHD_SYNC_DB, nk);
+  } else {  // plain_db; on periodic blocks dB comes out the same on a face and its image
+    sync1(b, 1, copy_op(MHD_SYNC_DB, kPhHalo), nk);
+    if (b->n_open > 0) sync1(b, 1, copy_op(MHD_SYNC_DB, kPhOwner), nk);
+  }
   launch(b, 1, SK_RES_DJ, nk, nullptr, RES_OF_DB);
   sync1(b, 1, alias_op(1), nk);
   if (b->live_sing > 0) launch(b, 1, SK_SING_J, nk, nullptr, RES_OF_DB);  // AssembleSingularEdgeCurrent_(dB, dJ)
@@ -1841,6 +2010,67 @@ static bool hall_writes_inside(const Solve *S, const mhd_desc *desc) {
 }
 
 
+// Whether the step's syncs may run joined (enqueue_step_a_joined): the groups'
+// copies allow it (pass_flags); every staged source is a ghost that no physical
+// operation of its group (or the wall EMF) writes, so it holds the last sync's
+// value until its group's next copies; and groups staged in one launch have
+// slots of their own.  Tables without these properties take the phases in order.
+static bool joined_syncs(const Solve *S, const mhd_desc *desc) {
+  for (int g : {(int)MHD_SYNC_EHALL, (int)MHD_SYNC_EEDGE, (int)MHD_SYNC_JEDGE, (int)MHD_SYNC_B_CELL, (int)MHD_SYNC_J_CELL})
+    if (!S->T->one_pass[g]) return false;
+  for (int g : {(int)MHD_SYNC_UCELL, (int)MHD_SYNC_BFACE})
+    if (!S->T->two_pass[g]) return false;
+  const int sets[2][4] = {{MHD_SYNC_EHALL, MHD_SYNC_EEDGE, MHD_SYNC_UCELL, MHD_SYNC_BFACE},
+                          {MHD_SYNC_B_CELL, MHD_SYNC_JEDGE, MHD_SYNC_J_CELL, -1}};
+  for (const auto &set : sets) {
+    std::vector<char> used((size_t)std::max(S->n_staging, 0), 0);
+    for (int g : set) {
+      if (g < 0) continue;
+      const mhd_sync_group &G = desc->groups[g];
+      for (int t = 0; t < G.n_stash; ++t) {
+        const int slot = G.stash[t].dst.i;
+        if (G.stash[t].dst.field != MHD_STAGING || slot < 0 || slot >= S->n_staging || used[slot]++) return false;
+      }
+    }
+  }
+  std::atomic<bool> good{true};
+  mhd::parallel_for(8, [&](int q) {
+    const int g = sets[q / 4][q % 4];
+    // U is staged from the buffer that the step's writes leave alone
+    if (g < 0 || g == MHD_SYNC_UCELL || desc->groups[g].n_stash <= 0) return;
+    const mhd_sync_group &G = desc->groups[g];
+    bool ok = false;
+    CodeSet src((size_t)G.n_stash);
+    for (int t = 0; t < G.n_stash; ++t) {
+      if (dof_depth(S, G.stash[t].src) == 0) good = false;
+      src.add(S->code(G.stash[t].src, &ok));
+    }
+    auto writes = [&](const mhd_phys_op *ops, int n) {
+      for (int t = 0; t < n; ++t)
+        if (src.has(S->code(ops[t].dst, &ok))) good = false;
+    };
+    writes(G.phys, G.n_phys);
+    if (g == MHD_SYNC_EEDGE) writes(desc->wall, desc->n_wall);
+  });
+  return good;
+}
+
+// Whether Sync(dB) of the substep needs its halo and owner copies only: no
+// physical operation; every staged source a ghost face, zero when it is staged
+// (clear_triplet), so the staged copies write the zeros that the substep's
+// start left there (k_res_clearb); and no other copy reads a ghost face that a
+// copy writes, so none has to be zeroed again.
+static bool plain_db(const Solve *S, const mhd_desc *desc) {
+  const mhd_sync_group &G = desc->groups[MHD_SYNC_DB];
+  if (G.n_phys > 0) return false;
+  if (!S->T->db_apart) return false;
+  for (int t = 0; t < G.n_stash; ++t)
+    if (G.stash[t].src.field == MHD_STAGING || dof_depth(S, G.stash[t].src) == 0 ||
+        dof_depth(S, G.stash[G.n_stash + t].dst) == 0)
+      return false;
+  return true;
+}
+
 static int upload_phys(Solve *S, const mhd_desc *desc, cudaStream_t st) {
   for (int q = 0; q < kNumPhys; ++q) {
     const mhd_phys_op *ops = q < kMaxGroups ? desc->groups[q].phys : desc->wall;
@@ -2165,14 +2395,17 @@ static int add_solve(mhd_batch *b, const mhd_desc *desc, bool periodic, int *slo
     if (periodic) {
       if ((rc = upload_groups_periodic(S, st)) || (rc = upload_aliases_periodic(S, st))) return bail(rc);
       S->T->res_ghost_writes_only = true;  // a periodic block's halo copies write ghosts
+      S->T->sync_joined = S->T->db_plain = S->T->periodic = true;
     } else {
       if ((rc = upload_groups(S, desc->groups, st))) return bail(rc);
       if ((rc = upload_aliases(S, desc->edge_aliases, st))) return bail(rc);
       if ((rc = upload_phys(S, desc, st))) return bail(rc);
       if ((rc = upload_singular(S, desc->singular, st)) || (rc = alloc_singular_geo(S, st))) return bail(rc);
       S->T->hall_late = hall_writes_inside(S, desc);
+      S->T->sync_joined = joined_syncs(S, desc);
       if (S->consts.resistive) {
         S->T->res_kdown = res_kdown(desc);
+        S->T->db_plain = plain_db(S, desc);
         S->T->res_ghost_writes_only = res_ghost_writes_only(S, desc);
       }
     }

@@ -2078,31 +2078,39 @@ __device__ __forceinline__ const int *op_prefix(const Dir &D, const SyncOp &op) 
 
 // MercuryBoundary::Sync_ stages (Z4_Mercury/src/boundary/Boundary_Sync_.cpp:4-110) and
 // ReduceEdgeAliasCandidatesToOwners_ (Z4_Mercury/src/physics/MercurySolver_Current.cpp:3-57)
-// for every active solve, up to two independent operations per launch.
+// for every active solve, up to kMaxSyncOps independent operations per launch.
 // Work unit: a group of 8 lanes.  A copy phase gives each group one segment
 // (dst <- sign * src on up to kSegElems elements: reps strided runs of len
 // consecutive elements); an alias reduction gives each lane one class, whose
 // members are summed in stored order from 0.0 and written to the owner as
 // owner_sign * sum / count.
-template <class R>
+template <class R, int N>  // N: the most operations of the launch
 __global__ void __launch_bounds__(256) k_sync(Dir D, SyncOps ops) {
   const int lane = threadIdx.x & 7;
   const int stride = (gridDim.x * blockDim.x) >> 3;
-  const int *pre0 = op_prefix(D, ops.op[0]);
-  const int *pre1 = ops.n > 1 ? op_prefix(D, ops.op[1]) : nullptr;
   let_dependents_launch();
-  const int t0 = pre0[D.nsolves];
-  const int total = t0 + (pre1 ? pre1[D.nsolves] : 0);
+  // the operations' work units follow one another
+  int end[N], total = 0;
+#pragma unroll
+  for (int p = 0; p < N; ++p) {
+    if (N <= 2 || p < ops.n) total += op_prefix(D, ops.op[p])[D.nsolves];
+    end[p] = total;
+  }
   bool first = true;
   if (((int)(blockIdx.x * blockDim.x) >> 3) >= total) {
     if (blockIdx.x == 0) wait_for_predecessors();
     return;
   }
   for (int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; g < total; g += stride) {
-    const bool second = g >= t0;
-    const SyncOp &op = second ? ops.op[1] : ops.op[0];
-    const int *pre = second ? pre1 : pre0;
-    const int e = second ? g - t0 : g;
+    SyncOp op = ops.op[0];
+    int e = g;
+#pragma unroll
+    for (int p = 1; p < N; ++p)
+      if (g >= end[p - 1]) {
+        op = ops.op[p];
+        e = g - end[p - 1];
+      }
+    const int *pre = op_prefix(D, op);
     const int s = find_solve(pre, D.nsolves, e);
     const DevSolve &S = D.solves[s];
     const int q = e - pre[s];
@@ -2173,7 +2181,15 @@ __global__ void __launch_bounds__(256) k_sync(Dir D, SyncOps ops) {
       for (int m = 0; m < kAhead; ++m)
         if (m0 + m < m1) sum += R(msign[m]) * v[m];
       for (int m = m0 + kAhead; m < m1; ++m) sum += R(A.msign[m]) * *at_code<R>(S, cur, A.member[m]);
-      *at_code<R>(S, cur, ocode) = R(osign) * sum / (R)(m1 - m0);
+      const R mean = R(osign) * sum / (R)(m1 - m0);
+      *at_code<R>(S, cur, ocode) = mean;
+      if (op.mark) {
+#pragma unroll
+        for (int m = 0; m < kAhead; ++m)
+          if (m0 + m < m1) *at_code<R>(S, cur, mcode[m]) = msign[m] == osign ? mean : -mean;
+        for (int m = m0 + kAhead; m < m1; ++m)
+          *at_code<R>(S, cur, A.member[m]) = A.msign[m] == osign ? mean : -mean;
+      }
     }
   }
 }
@@ -2545,7 +2561,7 @@ static const void *kernel_fn(StepKernel k) {
     case SK_BCELL_JEDGE: return (const void *)k_bcell_jedge<R>;
     case SK_JCELL: return (const void *)k_jcell<R>;
     case SK_PV_UPLUS: return (const void *)k_pv_uplus<R>;
-    case SK_SYNC: return (const void *)k_sync<R>;
+    case SK_SYNC: return (const void *)k_sync<R, kMaxSyncOps>;
     case SK_FACE_NORMALS: return (const void *)k_face_normals<R>;
     case SK_DIVB: return (const void *)k_div_b<R>;
     case SK_RES_SEED: return (const void *)k_res_seed<R>;
@@ -2635,7 +2651,11 @@ static void launch_as(StepKernel k, const Dir &D, cudaStream_t st, const SyncOps
     case SK_BCELL_JEDGE: launch_dependent(k_bcell_jedge<R>, G, kVecThreads, st, D); break;
     case SK_JCELL: launch_dependent(k_jcell<R>, G, kVecThreads, st, D); break;
     case SK_PV_UPLUS: launch_dependent(k_pv_uplus<R>, G, kVecThreads, st, D, iarg); break;
-    case SK_SYNC: launch_dependent(k_sync<R>, G, kTileThreads, st, D, *ops); break;
+    case SK_SYNC:
+      if (ops->n == 1) launch_dependent(k_sync<R, 1>, G, kTileThreads, st, D, *ops);
+      else if (ops->n == 2) launch_dependent(k_sync<R, 2>, G, kTileThreads, st, D, *ops);
+      else launch_dependent(k_sync<R, kMaxSyncOps>, G, kTileThreads, st, D, *ops);
+      break;
     case SK_FACE_NORMALS: k_face_normals<R><<<G, kVecThreads, 0, st>>>(D); break;
     case SK_DIVB: k_div_b<R><<<G, kVecThreads, 0, st>>>(D); break;
     case SK_RES_SEED: k_res_seed<R><<<G, kVecThreads, 0, st>>>(D); break;

@@ -18,7 +18,7 @@ enum StepKernel {
   SK_RES_CLEARB, SK_COUNT
 };
 
-// One launch of k_sync runs up to two independent sync operations: a copy
+// One launch of k_sync runs up to kMaxSyncOps independent sync operations: a copy
 // phase of a group (halo or owner copies) or an edge alias reduction.
 enum SyncKind { SYNC_COPY = 0, SYNC_ALIAS = 1 };
 struct SyncOp {
@@ -28,10 +28,12 @@ struct SyncOp {
   int prev;   // SYNC_COPY: read U components from the other buffer (1) -- the staged
               // ghosts of Sync(U) inside the step, whose last synced values are there
   int mark;   // SYNC_COPY: write 0 to every destination instead of the copy (marks
-              // the phase's destinations, e.g. the non-owner aliases of an owner phase)
+              // the phase's destinations, e.g. the non-owner aliases of an owner phase);
+              // SYNC_ALIAS: write every member of a class, not only its owner
 };
+constexpr int kMaxSyncOps = 6;
 struct SyncOps {
-  SyncOp op[2];
+  SyncOp op[kMaxSyncOps];
   int n;
 };
 
