@@ -168,9 +168,10 @@ struct Tables {
   // on an edge inside a block (hall_writes_inside)
   bool hall_late = false;
   // The step's syncs may run in fewer launches (joined_syncs); Sync(dB) of the
-  // substep needs its halo and owner copies only (plain_db); one block periodic
-  // in every direction (upload_groups_periodic)
-  bool sync_joined = false, db_plain = false, periodic = false;
+  // substep needs its halo and owner copies only (plain_db), and not the owner
+  // copies either (same_db); the alias reductions replace the owner copies of E,
+  // E_Hall and J (alias_owners)
+  bool sync_joined = false, db_plain = false, db_same = false, alias_all = false;
   bool one_pass[kMaxGroups] = {};  // halo, staged and owner copies of the step touch one another's data nowhere
   bool two_pass[kMaxGroups] = {};  // the halo and the staged copies do not
   bool db_apart = false;           // no copy of Sync(dB) reads what its halo or staged copies write
@@ -266,8 +267,9 @@ struct mhd_batch {
   int live_phys[kNumPhys] = {};
   int live_sing = 0;
   int n_res = 0;                                        // slots whose solve has the implicit resistive substep
-  // solves whose syncs need the general order, whose Sync(dB) does, and that are not periodic blocks
-  int n_sync_general = 0, n_db_general = 0, n_open = 0;
+  // solves whose syncs need the general order, whose Sync(dB) does, whose Sync(dB)
+  // needs owner copies, and whose alias reductions do not replace the owner copies
+  int n_sync_general = 0, n_db_general = 0, n_db_owner = 0, n_alias_owner = 0;
   int n_res_full = 0;                                   // of them, solves whose substep runs the full E / J syncs
   // FP64 batch of the companions of mixed-precision resistive solves, which
   // runs on this batch's stream and pool (borrowed = true in the companion)
@@ -377,6 +379,11 @@ void sync2(mhd_batch *b, int mode, SyncOp a, SyncOp c, int *nk) { sync_ops(b, mo
 void phys1(mhd_batch *b, int mode, int which, int *nk) {
   if (b->live_phys[which] > 0) launch(b, mode, SK_PHYS, nk, nullptr, which);
 }
+// Two tables that write different positions and read none the other writes.
+void phys2(mhd_batch *b, int mode, int t0, int t1, int *nk) {
+  if (b->live_phys[t0] == 0 || b->live_phys[t1] == 0) return phys1(b, mode, b->live_phys[t0] > 0 ? t0 : t1, nk);
+  launch(b, mode, SK_PHYS, nk, nullptr, t0 | (t1 + 1) << 8);
+}
 // Before a group's halo copies: its physical operations, then the staging of
 // the sources its halo copies overwrite; after them: the staged copies.
 // prev: the group's U ghosts hold their last synced values in the other
@@ -412,8 +419,9 @@ void enqueue_sync(mhd_batch *b, int mode, int g, int *nk, bool full = false) {
 //   the buffer that is the other one after it);
 // - a group's halo, staged and owner copies run in one launch (of Sync(B faces),
 //   whose halo copies read owner copies, the owner copies follow);
-// - on periodic blocks the alias reduction writes every member of a class, and
-//   E + Ehall, the same sum at each of them, needs no owner copies.
+// - where every owner copy of E, E_Hall and J is one of an alias class
+//   (alias_owners), the reduction writes every member, and E + Ehall, the same sum
+//   at each of them, needs no owner copies.
 // A k_sync launch costs 3 to 4 us whatever it copies.
 SyncOp stash_op(int g) { return copy_op(g, kPhStash); }
 bool has_pre(const mhd_batch *b, int g) { return b->live_phys[g] > 0 || b->live_tables[g][kPhStash] > 0; }
@@ -421,10 +429,10 @@ bool has_pre(const mhd_batch *b, int g) { return b->live_phys[g] > 0 || b->live_
 // enqueue_derived
 void enqueue_derived_joined(mhd_batch *b, int mode, int *nk, bool end_of_step) {
   const int B = MHD_SYNC_B_CELL, J = MHD_SYNC_JEDGE, C = MHD_SYNC_J_CELL;
-  const bool all = b->n_open == 0, early = b->live_tables[B][kPhStash] == 0;
+  const bool all = b->n_alias_owner == 0, early = b->live_tables[B][kPhStash] == 0;
   const SyncOp bhalo = copy_op(B, kPhHalo);
   launch(b, mode, SK_BCELL_JEDGE, nk);
-  phys1(b, mode, B, nk);
+  if (!end_of_step) phys1(b, mode, B, nk);  // a step wrote them already
   sync_ops(b, mode, {alias_op(1, all), early ? bhalo : stash_op(B), stash_op(J), stash_op(C)}, nk);
   if (b->live_sing > 0) launch(b, mode, SK_SING_J, nk);
   phys1(b, mode, J, nk);
@@ -470,7 +478,7 @@ void enqueue_derived(mhd_batch *b, int mode, int *nk, bool end_of_step = false) 
 // enqueue_step_a after the edge EMF
 void enqueue_step_a_joined(mhd_batch *b, int *nk) {
   const int m = 0, H = MHD_SYNC_EHALL, E = MHD_SYNC_EEDGE, U = MHD_SYNC_UCELL, F = MHD_SYNC_BFACE;
-  const bool all = b->n_open == 0;
+  const bool all = b->n_alias_owner == 0;
   if (b->live_sing > 0 || has_pre(b, H)) {
     sync_ops(b, m, {alias_op(0, all), stash_op(H), stash_op(E), stash_op(U), stash_op(F)}, nk);
     if (b->live_sing > 0) launch(b, m, SK_SING_EMF, nk);
@@ -481,12 +489,11 @@ void enqueue_step_a_joined(mhd_batch *b, int *nk) {
              nk);
   }
   launch(b, m, SK_ADD_HALL, nk);  // on the edges in the blocks' faces
-  phys1(b, m, kMaxGroups, nk);    // the wall EMF: E_t = 0 on solid-wall edges
-  phys1(b, m, E, nk);
+  phys2(b, m, kMaxGroups, E, nk);  // the wall EMF (E_t = 0 on solid-wall edges), Sync(E)'s operations
   if (!all) sync_ops(b, m, {copy_op(E, kPhHalo), copy_op(E, kPhUnstash), copy_op(E, kPhOwner)}, nk);
   launch(b, m, SK_FLUID, nk, nullptr, b->fluid_tile);
   launch(b, m, SK_BFACE, nk);
-  phys1(b, m, U, nk);
+  phys2(b, m, U, MHD_SYNC_B_CELL, nk);  // the latter's are constants: ahead of enqueue_derived_joined
   phys1(b, m, F, nk);
   sync_ops(b, m, {copy_op(U, kPhHalo), copy_op(F, kPhHalo), copy_op(U, kPhUnstash), copy_op(F, kPhUnstash)}, nk);
   sync_ops(b, m, {copy_op(U, kPhOwner), copy_op(F, kPhOwner)}, nk);
@@ -1228,7 +1235,8 @@ bool count_tables(mhd_batch *b, const Solve *S, int d) {
   };
   count(!S->T->sync_joined, &b->n_sync_general);
   count(S->consts.resistive && !S->T->db_plain, &b->n_db_general);
-  count(!S->T->periodic, &b->n_open);
+  count(S->consts.resistive && !S->T->db_same, &b->n_db_owner);
+  count(!S->T->alias_all, &b->n_alias_owner);
   if (S->consts.resistive && !S->T->res_ghost_writes_only) {
     grew = grew || (d > 0 && b->n_res_full == 0);
     b->n_res_full += d;
@@ -1299,9 +1307,9 @@ void res_apply_core(mhd_batch *b, int *nk) {  // from E_res (set) to dJ (synced)
   launch(b, 1, SK_RES_DB, nk);  // the ghost faces were cleared at the substep's start (res_step)
   if (b->n_db_general > 0) {
     enqueue_sync(b, 1, MHD_SYNC_DB, nk);
-  } else {  // plain_db; on periodic blocks dB comes out the same on a face and its image
+  } else {
     sync1(b, 1, copy_op(MHD_SYNC_DB, kPhHalo), nk);
-    if (b->n_open > 0) sync1(b, 1, copy_op(MHD_SYNC_DB, kPhOwner), nk);
+    if (b->n_db_owner > 0 || !res_light_syncs(b)) sync1(b, 1, copy_op(MHD_SYNC_DB, kPhOwner), nk);
   }
   launch(b, 1, SK_RES_DJ, nk, nullptr, RES_OF_DB);
   sync1(b, 1, alias_op(1), nk);
@@ -2013,13 +2021,27 @@ static bool hall_writes_inside(const Solve *S, const mhd_desc *desc) {
 // Whether the step's syncs may run joined (enqueue_step_a_joined): the groups'
 // copies allow it (pass_flags); every staged source is a ghost that no physical
 // operation of its group (or the wall EMF) writes, so it holds the last sync's
-// value until its group's next copies; and groups staged in one launch have
-// slots of their own.  Tables without these properties take the phases in order.
+// value until its group's next copies; groups staged in one launch have slots of
+// their own; and the wall EMF and the operations of E are apart, those of B_cell
+// constants, to share launches.  Tables without these properties take the phases in order.
 static bool joined_syncs(const Solve *S, const mhd_desc *desc) {
   for (int g : {(int)MHD_SYNC_EHALL, (int)MHD_SYNC_EEDGE, (int)MHD_SYNC_JEDGE, (int)MHD_SYNC_B_CELL, (int)MHD_SYNC_J_CELL})
     if (!S->T->one_pass[g]) return false;
   for (int g : {(int)MHD_SYNC_UCELL, (int)MHD_SYNC_BFACE})
     if (!S->T->two_pass[g]) return false;
+  const mhd_sync_group &GE = desc->groups[MHD_SYNC_EEDGE], &GB = desc->groups[MHD_SYNC_B_CELL];
+  for (int t = 0; t < GB.n_phys; ++t)
+    if (GB.phys[t].kind != MHD_PHYS_SET || GB.phys[t].dst.field == MHD_U_H || GB.phys[t].dst.field == MHD_U_NA)
+      return false;
+  if (desc->n_wall > 0 && GE.n_phys > 0) {
+    bool ok = false;
+    CodeSet wall((size_t)desc->n_wall);
+    for (int t = 0; t < desc->n_wall; ++t) wall.add(S->code(desc->wall[t].dst, &ok));
+    for (int t = 0; t < GE.n_phys; ++t)
+      if (GE.phys[t].kind == MHD_PHYS_WALL || wall.has(S->code(GE.phys[t].dst, &ok))) return false;
+    for (int t = 0; t < desc->n_wall; ++t)
+      if (desc->wall[t].kind == MHD_PHYS_WALL) return false;
+  }
   const int sets[2][4] = {{MHD_SYNC_EHALL, MHD_SYNC_EEDGE, MHD_SYNC_UCELL, MHD_SYNC_BFACE},
                           {MHD_SYNC_B_CELL, MHD_SYNC_JEDGE, MHD_SYNC_J_CELL, -1}};
   for (const auto &set : sets) {
@@ -2068,6 +2090,83 @@ static bool plain_db(const Solve *S, const mhd_desc *desc) {
     if (G.stash[t].src.field == MHD_STAGING || dof_depth(S, G.stash[t].src) == 0 ||
         dof_depth(S, G.stash[G.n_stash + t].dst) == 0)
       return false;
+  return true;
+}
+
+// Whether the alias reductions of E and J may write every member of a class in
+// place of the owner copies that follow: the owner copies of E, E_Hall and J are
+// exactly the non-owner members of the classes, each from its class's owner with
+// its sign; and nothing (a singular edge, a physical operation, the wall EMF, a
+// halo copy that the step keeps) changes E or J between the two.
+static bool alias_owners(const Solve *S, const mhd_desc *desc) {
+  const mhd_alias_classes &a = desc->edge_aliases;
+  if (desc->singular.n_edges > 0 || desc->n_wall > 0 || a.n_classes < 0) return false;
+  for (int g : {(int)MHD_SYNC_EEDGE, (int)MHD_SYNC_JEDGE})
+    if (desc->groups[g].n_phys > 0 || desc->groups[g].n_stash > 0 || S->T->tab_n[g][kPhHalo] > 0) return false;
+  bool ok = false;
+  auto code = [&](mhd_dof d, int base) {  // of the E edge that stands for d
+    d.field = MHD_E_XI + (d.field - base);
+    return d.field < MHD_E_XI || d.field > MHD_E_ZETA ? -2 : S->code(d, &ok);
+  };
+  const int nm = a.n_classes > 0 ? a.offset[a.n_classes] : 0;
+  CodeSet members((size_t)nm);
+  std::vector<int> cls(nm);
+  std::vector<int64_t> owner(a.n_classes > 0 ? a.n_classes : 0);
+  for (int c = 0; c < a.n_classes; ++c) {
+    owner[c] = code(a.owner[c], 0);
+    for (int m = a.offset[c]; m < a.offset[c + 1]; ++m) {
+      cls[m] = c;
+      members.add(code(a.member[m], 0), m);
+    }
+  }
+  const int groups[3][2] = {{MHD_SYNC_EHALL, MHD_EHALL_XI}, {MHD_SYNC_EEDGE, MHD_E_XI}, {MHD_SYNC_JEDGE, MHD_J_XI}};
+  for (const auto &gr : groups) {
+    const mhd_sync_group &G = desc->groups[gr[0]];
+    std::vector<char> seen(nm, 0);
+    for (int t = 0; t < G.n_owner; ++t) {
+      const int64_t d = code(G.owner[t].dst, gr[1]);
+      const CodeSet::Slot &e = members.slot[members.at(d)];
+      if (d < 0 || e.code != d || seen[e.value]++) return false;
+      const int m = (int)e.value;
+      if (d == owner[cls[m]] || code(G.owner[t].src, gr[1]) != owner[cls[m]] ||
+          G.owner[t].sign != a.member_sign[m] * a.owner_sign[cls[m]])
+        return false;
+    }
+    for (int m = 0; m < nm; ++m)
+      if (!seen[m] && code(a.member[m], 0) != owner[cls[m]]) return false;
+  }
+  return true;
+}
+
+// Whether Sync(dB)'s owner copies copy what is there already: each is of a face
+// whose four edges are, in order and sign, those of its owner after the owner
+// copies of E_res, so k_res_db computes the same bits on both.
+static bool same_db(const Solve *S, const mhd_desc *desc) {
+  const mhd_sync_group &E = desc->groups[MHD_SYNC_ERES], &G = desc->groups[MHD_SYNC_DB];
+  bool ok = false;
+  CodeSet copies((size_t)E.n_owner);
+  for (int t = 0; t < E.n_owner; ++t) copies.add(S->code(E.owner[t].dst, &ok), t);
+  auto value = [&](const mhd_dof &d) {  // where an edge's value comes from, and its sign
+    const int64_t c = S->code(d, &ok);
+    const CodeSet::Slot &e = copies.slot[copies.at(c)];
+    if (e.code != c) return std::make_pair(c, 1.0);
+    return std::make_pair(S->code(E.owner[e.value].src, &ok), E.owner[e.value].sign);
+  };
+  for (int t = 0; t < G.n_owner; ++t) {
+    const mhd_copy &cp = G.owner[t];
+    const int ax = cp.dst.field - MHD_B_XI;
+    if (cp.sign != 1.0 || ax < 0 || ax > 2 || cp.src.field != cp.dst.field) return false;
+    for (int q = 0; q < 4; ++q) {  // the face's edges along the other axes
+      const int along = (ax + 1 + q / 2) % 3, across = (ax + 2 - q / 2) % 3;
+      mhd_dof d = cp.dst, s = cp.src;
+      for (mhd_dof *e : {&d, &s}) {
+        e->field = MHD_E_XI + along;
+        int *x[3] = {&e->i, &e->j, &e->k};
+        *x[across] += q % 2;
+      }
+      if (value(d) != value(s)) return false;
+    }
+  }
   return true;
 }
 
@@ -2395,7 +2494,7 @@ static int add_solve(mhd_batch *b, const mhd_desc *desc, bool periodic, int *slo
     if (periodic) {
       if ((rc = upload_groups_periodic(S, st)) || (rc = upload_aliases_periodic(S, st))) return bail(rc);
       S->T->res_ghost_writes_only = true;  // a periodic block's halo copies write ghosts
-      S->T->sync_joined = S->T->db_plain = S->T->periodic = true;
+      S->T->sync_joined = S->T->db_plain = S->T->db_same = S->T->alias_all = true;
     } else {
       if ((rc = upload_groups(S, desc->groups, st))) return bail(rc);
       if ((rc = upload_aliases(S, desc->edge_aliases, st))) return bail(rc);
@@ -2403,9 +2502,11 @@ static int add_solve(mhd_batch *b, const mhd_desc *desc, bool periodic, int *slo
       if ((rc = upload_singular(S, desc->singular, st)) || (rc = alloc_singular_geo(S, st))) return bail(rc);
       S->T->hall_late = hall_writes_inside(S, desc);
       S->T->sync_joined = joined_syncs(S, desc);
+      S->T->alias_all = alias_owners(S, desc);
       if (S->consts.resistive) {
         S->T->res_kdown = res_kdown(desc);
         S->T->db_plain = plain_db(S, desc);
+        S->T->db_same = same_db(S, desc);
         S->T->res_ghost_writes_only = res_ghost_writes_only(S, desc);
       }
     }

@@ -2212,58 +2212,56 @@ __device__ __forceinline__ V<R> block_view(const Dir &D, int s, int b) {
 // MercuryBoundary's handlers, Z4_Mercury/src/boundary/Boundary_Build.cpp:5-300).
 // The operations of one table write distinct DOFs and read none another
 // writes, so they run in any order.
+// Up to two tables per launch (t1 < 0: one).  A group of 8 lanes takes a
+// constant segment (up to 32 elements) or one other operation.
 template <class R>
-__global__ void __launch_bounds__(256) k_phys(Dir D, int which) {
+__global__ void __launch_bounds__(256) k_phys(Dir D, int t0, int t1) {
   let_dependents_launch();
-  const int *pre = D.phys_prefix[which];
-  const int total = pre[D.nsolves];
-  wait_for_predecessors();
-  const int lane = threadIdx.x & 31;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  // a warp takes 32 consecutive operations, one per lane; the constant
-  // segments among them are then written by the whole warp, one element per
-  // lane (consecutive destinations to consecutive lanes)
-  for (int base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; base < total; base += nwarps * 32) {
-    const int e = base + lane;
-    unsigned long long seg_p = 0;  // the segment's first destination (0: not a segment)
-    int64_t seg_w = 0;
-    R seg_v = R(0.0);
-    const DevPhysOp *opp = nullptr;
-    const DevSolve *Sp = nullptr;
-    int cur = 0;
-    if (e < total) {
-      const int s = find_solve(pre, D.nsolves, e);
-      if (solve_active(D, s)) {
-        Sp = &D.solves[s];
-        const DevPhys &P = Sp->phys[which];
-        cur = D.state[s].cur;
-        const int q = e - pre[s];
-        if (q < P.nset) {  // destinations <- bc[arg]: nr runs of len elements, stride bytes apart
-          const int64_t w0 = P.set[2 * q];
-          seg_w = P.set[2 * q + 1];
-          seg_v = consts_of<R>(*Sp).bc[(int)((w0 >> kPhysArgShift) & 31)];
-          seg_p = (unsigned long long)at_code<R>(*Sp, cur, w0 & ~(int64_t(31) << kPhysArgShift));
-        } else {
-          opp = &P.op[q - P.nset];
-        }
-      }
-    }
-    for (unsigned m = __ballot_sync(0xffffffffu, seg_p != 0); m; m &= m - 1) {
-      const int src = __ffs(m) - 1;
-      char *p0 = (char *)__shfl_sync(0xffffffffu, seg_p, src);
-      const int64_t w1 = __shfl_sync(0xffffffffu, seg_w, src);
-      const R v = __shfl_sync(0xffffffffu, seg_v, src);
-      const int len = (int)(w1 & 255) + 1, nr = (int)((w1 >> 8) & 255) + 1;
-      const int64_t stride = w1 >> 16;
-      if (lane < len * nr) {
-        const int r = lane / len;
-        *(R *)(p0 + r * stride + (int64_t)(lane - r * len) * (int64_t)sizeof(R)) = v;
-      }
-    }
-    if (!opp) continue;
-    const DevSolve &S = *Sp;
+  const int *pre0 = D.phys_prefix[t0], *pre1 = t1 >= 0 ? D.phys_prefix[t1] : nullptr;
+  const int n0 = pre0[D.nsolves], total = n0 + (pre1 ? pre1[D.nsolves] : 0);
+  if (((int)(blockIdx.x * blockDim.x) >> 3) >= total) {
+    if (blockIdx.x == 0) wait_for_predecessors();
+    return;
+  }
+  const int lane = threadIdx.x & 7;
+  const int stride = (gridDim.x * blockDim.x) >> 3;
+  bool first = true;
+  for (int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; g < total; g += stride) {
+    const bool second = g >= n0;
+    const int *pre = second ? pre1 : pre0;
+    const int e = second ? g - n0 : g;
+    const int s = find_solve(pre, D.nsolves, e);
+    const DevSolve &S = D.solves[s];
     const ConstsT<R> &c = consts_of<R>(S);
-    const DevPhysOp &op = *opp;
+    const DevPhys &P = S.phys[second ? t1 : t0];
+    const int q = e - pre[s];
+    const bool set = q < P.nset;  // destinations <- bc[arg]: nr runs of len elements, step bytes apart
+    int64_t w0 = 0, w1 = 0;
+    R v = R(0.0);
+    if (set) {
+      w0 = P.set[2 * q];
+      w1 = P.set[2 * q + 1];
+      v = c.bc[(int)((w0 >> kPhysArgShift) & 31)];
+    }
+    Status st{};
+    if (D.mode == 0) st = status_of(D, s);
+    if (first) wait_for_predecessors();
+    first = false;
+    if (D.mode != 0) st = status_of(D, s);
+    if (!st.active) continue;
+    const int cur = st.cur;
+    if (set) {
+      char *p0 = (char *)at_code<R>(S, cur, w0 & ~(int64_t(31) << kPhysArgShift));
+      const int len = (int)(w1 & 255) + 1, nr = (int)((w1 >> 8) & 255) + 1;
+      const int64_t step = w1 >> 16;
+      for (int u = lane; u < len * nr; u += 8) {
+        const int r = u / len;
+        *(R *)(p0 + r * step + (int64_t)(u - r * len) * (int64_t)sizeof(R)) = v;
+      }
+      continue;
+    }
+    if (lane != 0) continue;
+    const DevPhysOp &op = P.op[q - P.nset];
     if (op.kind == MHD_PHYS_WALL) {
       // BC_Solid_Surface_ (Z4_Mercury/src/boundary/Boundary_Condition_Fluid.cpp:37-259), H+:
       // the boundary cell from the cell one deeper (density floor 2.5e-3,
@@ -2680,7 +2678,7 @@ static void launch_as(StepKernel k, const Dir &D, cudaStream_t st, const SyncOps
                          rs.in_graph, rs.use_p);
       break;
     case SK_RES_PUPD_E: launch_dependent(k_res_pupd_e<R>, G, kVecThreads, st, D, rs.cg, rs.use_p); break;
-    case SK_PHYS: launch_dependent(k_phys<R>, G, 256, st, D, iarg); break;
+    case SK_PHYS: launch_dependent(k_phys<R>, G, 256, st, D, iarg & 255, (iarg >> 8) - 1); break;
     // one thread per singular edge (8 radial lines of nr edges per shell)
     case SK_SING_SETUP: k_sing_setup<R><<<g_grid_tiles / 2, 64, 0, st>>>(D); break;
     case SK_SING_EMF: launch_dependent(k_sing_emf<R>, g_grid_tiles / 2, 64, st, D); break;
