@@ -301,6 +301,10 @@ struct mhd_batch {
   int snap_next = 0;
   // eager profiling
   bool profiling = false;
+  // A step graph's second branch: the fluid pass beside the EMF passes (fluid_branch)
+  cudaStream_t side = nullptr;
+  cudaEvent_t branch_ev[2] = {};
+  bool capturing = false;
   bool after_flip = false;  // the last kernel launched was k_bface or k_face_normals
   int fluid_tile = 0;  // the fluid kernel's tile variant (fluid_tile)
   std::vector<cudaEvent_t> prof_events;
@@ -350,6 +354,28 @@ void launch(mhd_batch *b, int mode, StepKernel k, int *nk, const SyncOps *ops = 
   b->after_flip = k == SK_BFACE || k == SK_FACE_NORMALS;
   ++*nk;
   mark(b, step_kernel_name(k));
+}
+
+// The fluid pass, which reads nothing that the EMF passes behind k_face_emf write
+// and writes the next state buffer only, as a branch of a captured step: from
+// behind k_face_emf to ahead of k_bface, which flips the buffers (fluid_join).
+// Outside a capture (profiling) it is launched where it joins.  The EMF passes wait
+// on loads and leave issue slots, and on small grids whole SMs, to it: a step of
+// the box of 8^3 FP64 cells takes 48 us (52 in one row), 32^3 72 (77), 64^3 mixed
+// 135 (147), 96^3 mixed 341 (346).  The branch's stream has the high priority:
+// its blocks are the long ones (0 to 1 % over the low one).
+void fluid_branch(mhd_batch *b, int mode, int *nk) {
+  if (!b->capturing) return;
+  cudaEventRecord(b->branch_ev[0], b->stream);
+  cudaStreamWaitEvent(b->side, b->branch_ev[0], 0);
+  launch_step_kernel(SK_FLUID, b->dir(mode), b->side, nullptr, b->precision, b->fluid_tile, 0.0, b->res, true);
+  cudaEventRecord(b->branch_ev[1], b->side);
+  ++*nk;
+}
+void fluid_join(mhd_batch *b, int mode, int *nk) {
+  if (!b->capturing) return launch(b, mode, SK_FLUID, nk, nullptr, b->fluid_tile);
+  cudaStreamWaitEvent(b->stream, b->branch_ev[1], 0);
+  b->after_flip = true;  // k_bface waits for both branches in full
 }
 
 SyncOp copy_op(int g, int phase, int prev = 0, int mark = 0) { return SyncOp{SYNC_COPY, g, phase, prev, mark}; }
@@ -491,7 +517,7 @@ void enqueue_step_a_joined(mhd_batch *b, int *nk) {
   launch(b, m, SK_ADD_HALL, nk);  // on the edges in the blocks' faces
   phys2(b, m, kMaxGroups, E, nk);  // the wall EMF (E_t = 0 on solid-wall edges), Sync(E)'s operations
   if (!all) sync_ops(b, m, {copy_op(E, kPhHalo), copy_op(E, kPhUnstash), copy_op(E, kPhOwner)}, nk);
-  launch(b, m, SK_FLUID, nk, nullptr, b->fluid_tile);
+  fluid_join(b, m, nk);
   launch(b, m, SK_BFACE, nk);
   phys2(b, m, U, MHD_SYNC_B_CELL, nk);  // the latter's are constants: ahead of enqueue_derived_joined
   phys1(b, m, F, nk);
@@ -507,6 +533,7 @@ void enqueue_step_a(mhd_batch *b, int *nk) {
   const int m = 0;
   // AssembleRHS_Induction_CT_ (Z4_Mercury/src/physics/MercurySolver_MagneticRHS.cpp:90-171)
   launch(b, m, SK_FACE_EMF, nk);
+  fluid_branch(b, m, nk);
   launch(b, m, SK_EDGE_EMF, nk);
   if (b->n_sync_general == 0) return enqueue_step_a_joined(b, nk);
   if (b->live_sing > 0 || b->live_phys[MHD_SYNC_EHALL] > 0 || b->live_tables[MHD_SYNC_EHALL][kPhStash] > 0) {
@@ -523,7 +550,7 @@ void enqueue_step_a(mhd_batch *b, int *nk) {
   enqueue_sync(b, m, MHD_SYNC_EEDGE, nk);
   // AssembleRHS_Fluid_ + ApplyUpdate_Euler_ (state into the other buffer) and
   // the constrained-transport face update (Z4_Mercury/src/physics/MercurySolver_Advance.cpp:73-147)
-  launch(b, m, SK_FLUID, nk, nullptr, b->fluid_tile);
+  fluid_join(b, m, nk);
   launch(b, m, SK_BFACE, nk);
   // the reference's Sync(Ucell) reads ghosts it does not overwrite first at
   // their values from the previous sync, which after the flip are in the
@@ -1195,9 +1222,17 @@ template <class F>
 int capture(mhd_batch *b, cudaGraphExec_t *out, int *nk_out, F &&enqueue) {
   if (*out) return MHD_OK;
   cudaGraph_t g = nullptr;
+  if (!b->side) {
+    int least = 0, greatest = 0;
+    CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    for (cudaEvent_t &ev : b->branch_ev) CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    CUDA_TRY(cudaStreamCreateWithPriority(&b->side, cudaStreamNonBlocking, greatest));
+  }
   CUDA_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
   int nk = 0;
+  b->capturing = true;
   enqueue(&nk);
+  b->capturing = false;
   cudaError_t e = cudaStreamEndCapture(b->stream, &g);
   if (e != cudaSuccess) return fail(MHD_ERR_CUDA, "graph capture: %s", cudaGetErrorString(e));
   e = cudaGraphInstantiate(out, g, 0);
@@ -1802,6 +1837,9 @@ int mhd_batch_destroy(mhd_batch *b) {
     for (cudaEvent_t e : pair)
       if (e) cudaEventDestroy(e);
   if (b->cg_done) cudaEventDestroy(b->cg_done);
+  for (cudaEvent_t e : b->branch_ev)
+    if (e) cudaEventDestroy(e);
+  if (b->side) cudaStreamDestroy(b->side);
   cudaFree(b->res.partial);
   cudaFree(b->res.result);
   cudaFree(b->res.cg);
