@@ -305,7 +305,7 @@ struct mhd_batch {
   cudaStream_t side = nullptr;
   cudaEvent_t branch_ev[2] = {};
   bool capturing = false;
-  bool after_flip = false;  // the last kernel launched was k_bface or k_face_normals
+  bool after_flip = false;  // the next kernel launched waits for its predecessor in full (launch)
   int fluid_tile = 0;  // the fluid kernel's tile variant (fluid_tile)
   std::vector<cudaEvent_t> prof_events;
   std::vector<const char *> prof_names;
@@ -350,8 +350,9 @@ void mark(mhd_batch *b, const char *name) {
 void launch(mhd_batch *b, int mode, StepKernel k, int *nk, const SyncOps *ops = nullptr, int iarg = 0,
             double darg = 0.0) {
   launch_step_kernel(k, b->dir(mode), b->stream, ops, b->precision, iarg, darg, b->res, b->after_flip);
-  // it flips the solves' states, or writes static fields: the next kernels read those ahead of their wait
-  b->after_flip = k == SK_BFACE || k == SK_FACE_NORMALS;
+  // it flips the solves' states, writes static fields, or ends a step: the next kernels read
+  // those, and k_sing_emf the last step's fields, ahead of their wait
+  b->after_flip = k == SK_BFACE || k == SK_FACE_NORMALS || k == SK_PV_UPLUS;
   ++*nk;
   mark(b, step_kernel_name(k));
 }
@@ -1569,16 +1570,18 @@ int res_refine(mhd_batch *b, int slot, Solve *S, bool *converged) {
 // The right-hand side r = b = eta J(B*) of every masked solve: Calc_J_Edge on B*
 // over the substep's range (the formula of k_bcell_jedge's J part; B_cell is
 // refreshed after the substep).
-void res_rhs(mhd_batch *b, int *nk) {
+void res_current(mhd_batch *b, int *nk) {  // J(B*)
   launch(b, 1, SK_RES_DJ, nk, nullptr, RES_OF_B);
   sync1(b, 1, alias_op(1), nk);
   if (b->live_sing > 0) launch(b, 1, SK_SING_J, nk, nullptr, RES_OF_B);  // reads B* around the singular edges
   res_sync_dj(b, nk);
+}
+void res_rhs(mhd_batch *b, int *nk) {
+  res_current(b, nk);
   launch(b, 1, SK_RES_VEC, nk, nullptr, RES_INIT);
 }
-// E_res = x, its owner copies; B = B* + dt (-curl E_res) on the owned faces.
+// The owner copies of E_res = x; B = B* + dt (-curl E_res) on the owned faces.
 void res_finish(mhd_batch *b, int *nk) {
-  launch(b, 1, SK_RES_VEC, nk, nullptr, b->precision == kMixed ? RES_E_FROM_X : RES_E_FROM_CG);
   res_sync_eres(b, nk);
   launch(b, 1, SK_RES_BUPDATE, nk);
 }
@@ -1628,8 +1631,12 @@ int res_step_device(mhd_batch *b) {
   if ((rc = ensure_tpartial(c)) || (rc = build_cg_graph(c))) return rc;
   c->res.use_p = !res_light_syncs(c);
   launch_res_begin(b->dir(1), c->res.cg, mixed, b->stream);
-  res_rhs(b, &nk);
-  if (mixed) launch_res_cross(b->dir(1), RES_X_SETUP, b->stream, c->res.cg);
+  if (mixed) {
+    res_current(b, &nk);
+    launch_res_cross(b->dir(1), RES_X_SETUP, b->stream, c->res.cg);
+  } else {
+    res_rhs(b, &nk);
+  }
   if (open_grids(c)) launch(c, 1, SK_RES_CLEARB, &nk);
   CUDA_TRY(cudaGraphLaunch(c->graph_cg, b->stream));
   launch_res_end(b->dir(1), c->res.cg, c->hcg, c->capacity, mixed, false, b->stream);
@@ -1639,6 +1646,7 @@ int res_step_device(mhd_batch *b) {
   CUDA_TRY(cudaEventRecord(b->cg_done, b->stream));
   b->cg_pending = true;
   if (mixed) launch_res_cross(b->dir(1), RES_X_DEMOTE_X, b->stream, c->res.cg, c->res.use_p);
+  else launch(b, 1, SK_RES_VEC, &nk, nullptr, RES_E_FROM_CG);
   res_finish(b, &nk);
   launch_res_end(b->dir(1), c->res.cg, c->hcg, c->capacity, mixed, true, b->stream);
   CUDA_TRY(cudaGetLastError());
@@ -1715,6 +1723,7 @@ int res_step(mhd_batch *b, const std::vector<int> &slots) {
       const int e = MHD_ERR_SOLVE;
       if ((rc = set_state_field(b, s, offsetof(SolveState, status), &e, sizeof e))) return rc;
     }
+  launch(b, 1, SK_RES_VEC, &nk, nullptr, b->precision == kMixed ? RES_E_FROM_X : RES_E_FROM_CG);
   res_finish(b, &nk);
   CUDA_TRY(cudaGetLastError());
   std::fill(on.begin(), on.end(), 0);
