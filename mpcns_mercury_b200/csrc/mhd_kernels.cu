@@ -9,7 +9,7 @@
 //   * the contravariant velocity u^a = (K^a . U_plus) / (|J| + 1e-30) of every
 //     cell (cell_u_contra, Z4_Mercury/src/physics/MercurySolver_MagExplicit_Ideal.cpp:180-199)
 //     is computed once per step into UCON instead of up to 16 times per edge;
-//   * the fluid update runs one work item per (cell, species);
+//   * the fluid update runs one work item per (cell, species) in FP64, per cell in FP32;
 //   * B_cell/Bind_cell and J_edge share one pass over the face fluxes;
 //   * the next step's CFL dt is reduced in the same pass that refreshes the
 //     primitive variables (both read U and B_cell after their syncs).
@@ -2213,7 +2213,9 @@ __device__ __forceinline__ V<R> block_view(const Dir &D, int s, int b) {
 // The operations of one table write distinct DOFs and read none another
 // writes, so they run in any order.
 // Up to two tables per launch (t1 < 0: one).  A group of 8 lanes takes a
-// constant segment (up to 32 elements) or one other operation.
+// constant segment (up to 32 elements) or one other operation (one per lane, eight
+// chains of scattered stores in a warp's way: a step of the shell of 8 x 8 x 12
+// cells 75 us instead of 68).
 template <class R>
 __global__ void __launch_bounds__(256) k_phys(Dir D, int t0, int t1) {
   let_dependents_launch();
