@@ -815,8 +815,7 @@ std::vector<int64_t> build_segments(const Encoded &e, int es, int max_depth, con
   return seg;
 }
 
-// A set of arena codes, each with a number (open addressing, at most a quarter
-// full: a code that is not in it is mostly answered by the first slot).
+// A set of arena codes, each with a number (open addressing, at most half full).
 struct CodeSet {
   struct Slot {
     int64_t code = -1, value = 0;
@@ -825,7 +824,7 @@ struct CodeSet {
   size_t mask;
   explicit CodeSet(size_t n) {
     size_t size = 4;
-    while (size < 4 * n) size *= 2;
+    while (size < 2 * n) size *= 2;
     slot.resize(size);
     mask = size - 1;
   }
