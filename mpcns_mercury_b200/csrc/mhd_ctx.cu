@@ -349,10 +349,12 @@ void mark(mhd_batch *b, const char *name) {
 
 void launch(mhd_batch *b, int mode, StepKernel k, int *nk, const SyncOps *ops = nullptr, int iarg = 0,
             double darg = 0.0) {
-  launch_step_kernel(k, b->dir(mode), b->stream, ops, b->precision, iarg, darg, b->res, b->after_flip);
+  // (k_fluid reads earlier passes' fields through the read-only path: always in full)
+  launch_step_kernel(k, b->dir(mode), b->stream, ops, b->precision, iarg, darg, b->res,
+                     b->after_flip || k == SK_FLUID);
   // it flips the solves' states, writes static fields, or ends a step: the next kernels read
   // those, and k_sing_emf the last step's fields, ahead of their wait
-  b->after_flip = k == SK_BFACE || k == SK_FACE_NORMALS || k == SK_PV_UPLUS;
+  b->after_flip = k == SK_BFACE || k == SK_FACE_NORMALS || k == SK_RES_W || k == SK_SING_SETUP || k == SK_PV_UPLUS;
   ++*nk;
   mark(b, step_kernel_name(k));
 }

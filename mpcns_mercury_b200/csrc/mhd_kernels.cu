@@ -93,10 +93,14 @@ struct V {
     return (double *)(M + (uint64_t)(comp - kMetricFirst) * (tb * (8 / (uint32_t)sizeof(R))));
   }
   // Component `comp` at byte offset bo of its array (bo = off() times the
-  // element size), through the read-only path.  The array's address is
+  // element size), through the read-only path: only for what no kernel writes
+  // while this one runs, the static fields, and, in kernels that are launched
+  // after their predecessor in full (k_fluid), the fields of earlier passes.  The array's address is
   // warp-uniform (build_item) and bo is 32 bits, so no thread holds 64-bit
   // addresses: without that k_fluid spilled 700 bytes at 80 registers.
-  __device__ __forceinline__ R ld(int comp, uint32_t bo) const { return __ldg((const R *)((const char *)c(comp) + bo)); }
+  __device__ __forceinline__ R fixed1(int comp, uint32_t bo) const {
+    return __ldg((const R *)((const char *)c(comp) + bo));
+  }
   __device__ __forceinline__ double ldm(int comp, uint32_t bo) const {
     return __ldg((const double *)((const char *)m(comp) + bo));
   }
@@ -357,7 +361,8 @@ struct VV : V<R> {
     else if constexpr (sizeof(R) * M == 8) *(float2 *)to = __ldg((const float2 *)p);
     else *(float *)to = __ldg((const float *)p);
   }
-  __device__ __forceinline__ Vc lv(int comp, uint32_t o) const {
+  // A static field (fixed1's conditions).
+  __device__ __forceinline__ Vc fixed(int comp, uint32_t o) const {
     Vc r;
     const char *p = (const char *)c(comp) + o;
     if constexpr (M == 1) r.v[0] = __ldg((const R *)p);
@@ -365,6 +370,18 @@ struct VV : V<R> {
     else load(r.v, p);
     return r;
   }
+  // A field that a pass of the step or of the substep writes.  These passes start
+  // while their predecessor may still write it, and the wait
+  // (wait_for_predecessors) orders ordinary loads only.  An ordinary load does not
+  // pass a store that could be to its address, so k_bcell_jedge, k_pv_uplus,
+  // k_res_db, k_res_pupd_e and k_res_bupdate load all they need ahead of their
+  // first store (on the 96^3 mixed box 0.038 ms instead of 0.041 and 0.076
+  // instead of 0.081, a step of the 8^3 FP64 box 48 us instead of 50); the EMF
+  // passes, k_bface and k_res_cg are no faster that way.  With every launch in
+  // full and read-only loads instead, a step takes 63 us on the 8^3 FP64 box,
+  // 95 (73) on 32^3, 164 (138) on 64^3 mixed.
+  __device__ __forceinline__ Vc lv(int comp, uint32_t o) const { return *(const Vc *)((const char *)c(comp) + o); }
+  __device__ __forceinline__ R ld(int comp, uint32_t bo) const { return *(const R *)((const char *)c(comp) + bo); }
   // lv of a static field of the implicit substep: an FP64 companion reads the
   // FP32 values it was widened from (half the bytes, the same numbers)
   __device__ __forceinline__ Vc stat(int comp, uint32_t o) const {
@@ -377,20 +394,23 @@ struct VV : V<R> {
         return r;
       }
     }
-    return lv(comp, o);
+    return fixed(comp, o);
   }
   __device__ __forceinline__ R stat1(int comp, uint32_t o) const {  // one value of stat
     if constexpr (sizeof(R) == 8 && M == 2)
       if (this->narrow)
         return (R)__ldg((const float *)(this->narrow + (uint64_t)rslot(comp) * (this->tb / 2) + o / 2));
-    return this->ld(comp, o);
+    return this->fixed1(comp, o);
   }
   // the values one k lower / higher than lv(comp, o), of which v holds the shared ones
   __device__ __forceinline__ Vc lower(const Vc &v, int comp, uint32_t o) const {
-    return vdown(v, this->ld(comp, o - (uint32_t)sizeof(R)));
+    return vdown(v, ld(comp, o - (uint32_t)sizeof(R)));
   }
   __device__ __forceinline__ Vc upper(const Vc &v, int comp, uint32_t o) const {
-    return vup(v, this->ld(comp, o + (uint32_t)sizeof(Vc)));
+    return vup(v, ld(comp, o + (uint32_t)sizeof(Vc)));
+  }
+  __device__ __forceinline__ Vc fixed_upper(const Vc &v, int comp, uint32_t o) const {
+    return vup(v, this->fixed1(comp, o + (uint32_t)sizeof(Vc)));
   }
   // lv(comp, o) copied to this thread's bytes of slot q of the CTA's stage
   // (cp.async: in flight without holding a register) and, after staged_arrived, read back
@@ -404,8 +424,6 @@ struct VV : V<R> {
     extern __shared__ __align__(16) unsigned char stage_smem[];
     return reinterpret_cast<const Vc *>(stage_smem)[q * kVecThreads + (int)threadIdx.x];
   }
-  // values that the kernel itself updates (this thread's positions only)
-  __device__ __forceinline__ Vc own(int comp, uint32_t o) const { return *(const Vc *)((const char *)c(comp) + o); }
   // metric values (double) at the item's positions
   __device__ __forceinline__ Vc lm(int comp, uint32_t o) const {
     const double *p = (const double *)((const char *)m(comp) + (uint64_t)o * (8 / sizeof(R)));
@@ -639,22 +657,22 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(R) == 8 ? 2 : 3) k_face_em
         const Vec<R> gi = pe(o + di) - pim, gj = pe(o + dj) - pjm, gk = vup(p0, pe1(o + 16u)) - pkm;
 #pragma unroll
         for (int q = 0; q < 3; ++q)
-          B.st(cDPE + q, it, R(0.5) * (B.lv(cAMB + q, o) * gi + B.lv(cAMB + 3 + q, o) * gj + B.lv(cAMB + 6 + q, o) * gk), 0,
+          B.st(cDPE + q, it, R(0.5) * (B.fixed(cAMB + q, o) * gi + B.fixed(cAMB + 3 + q, o) * gj + B.fixed(cAMB + 6 + q, o) * gk), 0,
                B.n2, i >= 0 && j >= 0 && i < B.n0 && j < B.n1);
       }
     }
     // induced and total B averaged to the cells (cell_beta_ind, cell_beta_tot)
     auto ind = [&](int a, uint32_t q, uint32_t d) { return R(0.5) * (B.lv(cBX + a, q) + B.lv(cBX + a, q + d)); };
     auto tot = [&](int a, uint32_t q, uint32_t d) {
-      return R(0.5) * ((B.lv(cBX + a, q) + B.lv(cBAX + a, q)) + (B.lv(cBX + a, q + d) + B.lv(cBAX + a, q + d)));
+      return R(0.5) * ((B.lv(cBX + a, q) + B.fixed(cBAX + a, q)) + (B.lv(cBX + a, q + d) + B.fixed(cBAX + a, q + d)));
     };
     auto ind_k = [&](uint32_t q) {  // along k: the cell's upper face is the next position
       const Vec<R> b = B.lv(cBZ, q);
       return R(0.5) * (b + B.upper(b, cBZ, q));
     };
     auto tot_k = [&](uint32_t q) {
-      const Vec<R> b = B.lv(cBZ, q) + B.lv(cBAZ, q);
-      return R(0.5) * (b + vup(b, B.ld(cBZ, q + 16u) + B.ld(cBAZ, q + 16u)));
+      const Vec<R> b = B.lv(cBZ, q) + B.fixed(cBAZ, q);
+      return R(0.5) * (b + vup(b, B.ld(cBZ, q + 16u) + B.fixed1(cBAZ, q + 16u)));
     };
     const Vec<R> bt[3] = {tot(0, o, di), tot(1, o, dj), tot_k(o)};
     const Vec<R> bi[3] = {ind(0, o, di), ind(1, o, dj), ind_k(o)};
@@ -670,7 +688,7 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(R) == 8 ? 2 : 3) k_face_em
     const bool ri = i < B.n0 + 1, rj = j < B.n1 + 1;  // in the range of the other families
     const int k1 = B.n2 + 1;
     {
-      const Vec<R> bff = B.lv(cBX, o) + B.lv(cBAX, o);
+      const Vec<R> bff = B.lv(cBX, o) + B.fixed(cBAX, o);
       const uint32_t q = o - di;
       const Vec<R> ufL = B.lv(cUC, q);
       const Vec<R> Ge = flux(1, 0, tot(1, q, dj), ind(1, q, dj), ufL, B.lv(cUC + 1, q), bff);
@@ -680,7 +698,7 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(R) == 8 ? 2 : 3) k_face_em
       B.st(cEFX + 2, it, -Ge, -1, k1, rj);
     }
     {
-      const Vec<R> bff = B.lv(cBY, o) + B.lv(cBAY, o);
+      const Vec<R> bff = B.lv(cBY, o) + B.fixed(cBAY, o);
       const uint32_t q = o - dj;
       const Vec<R> ufL = B.lv(cUC + 1, q);
       const Vec<R> Gx = flux(0, 1, tot(0, q, di), ind(0, q, di), ufL, B.lv(cUC, q), bff);
@@ -690,10 +708,10 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(R) == 8 ? 2 : 3) k_face_em
       B.st(cEFY + 2, it, Gx, -1, k1, ri);
     }
     {
-      const Vec<R> bff = B.lv(cBZ, o) + B.lv(cBAZ, o);
+      const Vec<R> bff = B.lv(cBZ, o) + B.fixed(cBAZ, o);
       const uint32_t q = o - (uint32_t)sizeof(R);  // the cell one k lower: its values from this thread's, and one more
       auto totL = [&](int a, uint32_t d) {
-        return vdown(bt[a], R(0.5) * ((B.ld(cBX + a, q) + B.ld(cBAX + a, q)) + (B.ld(cBX + a, q + d) + B.ld(cBAX + a, q + d))));
+        return vdown(bt[a], R(0.5) * ((B.ld(cBX + a, q) + B.fixed1(cBAX + a, q)) + (B.ld(cBX + a, q + d) + B.fixed1(cBAX + a, q + d))));
       };
       auto indL = [&](int a, uint32_t d) { return vdown(bi[a], R(0.5) * (B.ld(cBX + a, q) + B.ld(cBX + a, q + d))); };
       const Vec<R> ufL = vdown(u[2], B.ld(cUC + 2, q));
@@ -714,7 +732,7 @@ __device__ __forceinline__ Vec<R> add_artificial(const VV<R> &B, const ConstsT<R
   const int cj = cJX + axis;
   if (uniform((int)(c.arti_eta_max > R(0.0)))) {
     const int cd = axis == 0 ? cDRX : axis == 1 ? cDRY : cDRZ;
-    const Vec<R> J = B.lv(cj, o), dx = B.lv(cd, o), dy = B.lv(cd + 1, o), dz = B.lv(cd + 2, o);
+    const Vec<R> J = B.lv(cj, o), dx = B.fixed(cd, o), dy = B.fixed(cd + 1, o), dz = B.fixed(cd + 2, o);
 #pragma unroll
     for (int q = 0; q < Vec<R>::N; ++q) {
       const R dr_len = sqrt(dx.v[q] * dx.v[q] + dy.v[q] * dy.v[q] + dz.v[q] * dz.v[q]);
@@ -731,7 +749,7 @@ __device__ __forceinline__ Vec<R> add_artificial(const VV<R> &B, const ConstsT<R
       e.v[q] += eta * J.v[q];
     }
   }
-  if (uniform(c.local_arti)) e = e + B.lv(cLEX + axis, o) * B.lv(cj, o);
+  if (uniform(c.local_arti)) e = e + B.fixed(cLEX + axis, o) * B.lv(cj, o);
   return e;
 }
 
@@ -839,28 +857,28 @@ __global__ void __launch_bounds__(kVecThreads, 3) k_edge_emf(Dir D) {
     };
     auto tail = [&](int ax, const Vec<R> &Ecen, const Vec<R> &be, const Vec<R> &d1, const Vec<R> &d2) {
       const int ci = ax == 0 ? cIHX : ax == 1 ? cIHY : cIHZ;
-      const Vec<R> ih1 = B.lv(ci, o), ih2 = B.lv(ci + 1, o);
+      const Vec<R> ih1 = B.fixed(ci, o), ih2 = B.fixed(ci + 1, o);
       const Vec<R> mu1 = Cwh * be * ih1 * ih1;
       const Vec<R> mu2 = Cwh * be * ih2 * ih2;
-      return B.lv(cTPX + ax, o) * (Ecen + R(0.5) * mu1 * d1 - R(0.5) * mu2 * d2);
+      return B.fixed(cTPX + ax, o) * (Ecen + R(0.5) * mu1 * d1 - R(0.5) * mu2 * d2);
     };
     {
-      const Vec<R> Ecen = mean_k(cEHC, dj) * B.lv(cDRX, o) + mean_k(cEHC + 1, dj) * B.lv(cDRX + 1, o) +
-                          mean_k(cEHC + 2, dj) * B.lv(cDRX + 2, o);
+      const Vec<R> Ecen = mean_k(cEHC, dj) * B.fixed(cDRX, o) + mean_k(cEHC + 1, dj) * B.fixed(cDRX + 1, o) +
+                          mean_k(cEHC + 2, dj) * B.fixed(cDRX + 2, o);
       const Vec<R> by = B.lv(cBY, o);
       put(0, tail(0, Ecen, max_k(cHB, dj), B.lv(cBZ, o) - B.lv(cBZ, o - dj), by - B.lower(by, cBY, o)), B.n2 + 1, it.i < B.n0,
           late || it.j == 0 || it.j == B.n1, true);
     }
     {
-      const Vec<R> Ecen = mean_k(cEHC, di) * B.lv(cDRY, o) + mean_k(cEHC + 1, di) * B.lv(cDRY + 1, o) +
-                          mean_k(cEHC + 2, di) * B.lv(cDRY + 2, o);
+      const Vec<R> Ecen = mean_k(cEHC, di) * B.fixed(cDRY, o) + mean_k(cEHC + 1, di) * B.fixed(cDRY + 1, o) +
+                          mean_k(cEHC + 2, di) * B.fixed(cDRY + 2, o);
       const Vec<R> bx = B.lv(cBX, o);
       put(1, tail(1, Ecen, max_k(cHB, di), bx - B.lower(bx, cBX, o), B.lv(cBZ, o) - B.lv(cBZ, o - di)), B.n2 + 1, it.j < B.n1,
           late || it.i == 0 || it.i == B.n0, true);
     }
     {
       const Vec<R> Ecen =
-          mean_ij(cEHC) * B.lv(cDRZ, o) + mean_ij(cEHC + 1) * B.lv(cDRZ + 1, o) + mean_ij(cEHC + 2) * B.lv(cDRZ + 2, o);
+          mean_ij(cEHC) * B.fixed(cDRZ, o) + mean_ij(cEHC + 1) * B.fixed(cDRZ + 1, o) + mean_ij(cEHC + 2) * B.fixed(cDRZ + 2, o);
       const Vec<R> be = vmax(vmax(B.lv(cHB, o - di - dj), B.lv(cHB, o - di)), vmax(B.lv(cHB, o - dj), B.lv(cHB, o)));
       put(2, tail(2, Ecen, be, B.lv(cBY, o) - B.lv(cBY, o - di), B.lv(cBX, o) - B.lv(cBX, o - dj)), B.n2, true,
           late || it.i == 0 || it.i == B.n0 || it.j == 0 || it.j == B.n1, false);
@@ -879,7 +897,7 @@ __global__ void __launch_bounds__(kVecThreads) k_add_hall(Dir D) {
     if (!it.in || !(fi || fj || k0 || k1)) return;
     // each thread reads and writes its own positions only
     auto add = [&](int ax, int lo, int hi, bool cond) {
-      B.st(cEX + ax, it, B.own(cEX + ax, it.o) + B.lv(cHX + ax, it.o), lo, hi, cond);
+      B.st(cEX + ax, it, B.lv(cEX + ax, it.o) + B.lv(cHX + ax, it.o), lo, hi, cond);
     };
     // family xi: on the eta faces whole rows, else the ends of the row; eta likewise; zeta: whole rows
     if (it.i < B.n0) {
@@ -910,13 +928,13 @@ template <class R>
 __device__ __forceinline__ FluidCell<R> fluid_cell(const V<R> &B, int s, uint32_t o) {
   const int pv0 = s ? cPVN : cPVH, t0 = cFT + 2 * s;
   FluidCell<R> q;
-  q.rho = B.ld(s ? cUN : cUH, o);
-  q.u = B.ld(pv0, o);
-  q.v = B.ld(pv0 + 1, o);
-  q.w = B.ld(pv0 + 2, o);
-  q.p = B.ld(pv0 + 3, o);
-  q.re = B.ld(t0, o);
-  q.c = B.ld(t0 + 1, o);
+  q.rho = B.fixed1(s ? cUN : cUH, o);
+  q.u = B.fixed1(pv0, o);
+  q.v = B.fixed1(pv0 + 1, o);
+  q.w = B.fixed1(pv0 + 2, o);
+  q.p = B.fixed1(pv0 + 3, o);
+  q.re = B.fixed1(t0, o);
+  q.c = B.fixed1(t0 + 1, o);
   return q;
 }
 // A face's JD and |JD|: FP32 reads the real-typed copy (k_face_normals), FP64
@@ -931,15 +949,15 @@ __device__ __forceinline__ FluidFace<R> fluid_face(const V<R> &B, uint32_t o) {
   constexpr int cn = DIR == 0 ? cFNX : DIR == 1 ? cFNY : cFNZ;
   FluidFace<R> f;
   if constexpr (sizeof(R) == 4) {
-    f.k1 = B.ld(cm, o);
-    f.k2 = B.ld(cm + 1, o);
-    f.k3 = B.ld(cm + 2, o);
+    f.k1 = B.fixed1(cm, o);
+    f.k2 = B.fixed1(cm + 1, o);
+    f.k3 = B.fixed1(cm + 2, o);
   } else {
     f.k1 = B.ldm(cm, o);
     f.k2 = B.ldm(cm + 1, o);
     f.k3 = B.ldm(cm + 2, o);
   }
-  f.sk = B.ld(cn + 3, o);
+  f.sk = B.fixed1(cn + 3, o);
   return f;
 }
 template <class R>
@@ -1024,7 +1042,7 @@ __global__ void __launch_bounds__(fluid_threads(VT), fluid_ctas(VT, sizeof(R))) 
       }
 #pragma unroll 1
       for (int i = it.i; i < min(it.i + li, it.hi[0]); ++i, o += di) {
-        const R invJ = B.ld(cFM + 9, o);  // R(1) / R(Jac), from k_face_normals
+        const R invJ = B.fixed1(cFM + 9, o);  // R(1) / R(Jac), from k_face_normals
         R r[NS][5];
         {
           const FluidFace<R> f = fluid_face<R, 0>(B, o + di);
@@ -1057,7 +1075,7 @@ __global__ void __launch_bounds__(fluid_threads(VT), fluid_ctas(VT, sizeof(R))) 
         across(std::integral_constant<int, 1>{}, dj);
         across(std::integral_constant<int, 2>{}, dk);
         // sources (FluidRHS.cpp:206-527)
-        auto at = [&](int comp) -> R { return B.ld(comp, o); };
+        auto at = [&](int comp) -> R { return B.fixed1(comp, o); };
         const R Tn0 = R(1000.0), sk1 = R(5.0e-5), sk2 = R(1.0e-5);
         const R a4 = c.src_a4, a5 = c.src_a5;
         const R upx = at(cUP), upy = at(cUP + 1), upz = at(cUP + 2);
@@ -1162,15 +1180,15 @@ __global__ void __launch_bounds__(kVecThreads) k_bface(Dir D) {
     const Vec<R> ex = B.lv(cEX, o), ey = B.lv(cEY, o), ez = B.lv(cEZ, o);
     {
       const Vec<R> rb = -R(1.0) * ((ey - B.upper(ey, cEY, o)) + (B.lv(cEZ, o + dj) - ez));
-      B.st(cBX, it, B.own(cBX, o) + dt * rb, 0, B.n2, jc);
+      B.st(cBX, it, B.lv(cBX, o) + dt * rb, 0, B.n2, jc);
     }
     {
       const Vec<R> rb = -R(1.0) * ((B.upper(ex, cEX, o) - ex) + (ez - B.lv(cEZ, o + di)));
-      B.st(cBY, it, B.own(cBY, o) + dt * rb, 0, B.n2, ic);
+      B.st(cBY, it, B.lv(cBY, o) + dt * rb, 0, B.n2, ic);
     }
     {
       const Vec<R> rb = -R(1.0) * ((ex - B.lv(cEX, o + dj)) + (B.lv(cEY, o + di) - ey));
-      B.st(cBZ, it, B.own(cBZ, o) + dt * rb, 0, B.n2 + 1, ic && jc);
+      B.st(cBZ, it, B.lv(cBZ, o) + dt * rb, 0, B.n2 + 1, ic && jc);
     }
   });
   after_all_tiles<kBox>(D, D.tickets, [](SolveState &st) { flip_solve(st); });
@@ -1186,46 +1204,49 @@ __global__ void __launch_bounds__(kVecThreads, 3) k_bcell_jedge(Dir D) {
     const uint32_t o = it.o, di = B.di, dj = B.dj;
     const bool ic = it.i < B.n0, jc = it.j < B.n1;
     const Vec<R> bx = B.lv(cBX, o), by = B.lv(cBY, o), bz = B.lv(cBZ, o);
-    {
-      const Vec<R> ax = B.lv(cBAX, o), ay = B.lv(cBAY, o), az = B.lv(cBAZ, o);
-      const Vec<R> bxp = B.lv(cBX, o + di), byp = B.lv(cBY, o + dj), bzp = B.upper(bz, cBZ, o);
-      Vec<R> t[3] = {vset(R(0.0)), vset(R(0.0)), vset(R(0.0))}, in[3] = {t[0], t[0], t[0]};
-      auto add = [&](int q, const Vec<R> &total, const Vec<R> &induced) {  // face q of the cell
-#pragma unroll
-        for (int x = 0; x < 3; ++x) {
-          const Vec<R> w = B.lv(cWB + 6 * x + q, o);
-          t[x] = t[x] + w * total;
-          in[x] = in[x] + w * induced;
-        }
-      };
-      add(0, -bx - ax, -bx);
-      add(1, bxp + B.lv(cBAX, o + di), bxp);
-      add(2, -by - ay, -by);
-      add(3, byp + B.lv(cBAY, o + dj), byp);
-      add(4, -bz - az, -bz);
-      add(5, bzp + B.upper(az, cBAZ, o), bzp);
-#pragma unroll
-      for (int x = 0; x < 3; ++x) {
-        B.st(cBC + x, it, t[x], 0, B.n2, ic && jc);
-        B.st(cBIC + x, it, in[x], 0, B.n2, ic && jc);
-      }
-    }
     // beta B on this position's faces and the lower neighbours'
-    const Vec<R> fx = B.lv(cBFX, o) * bx, fy = B.lv(cBFY, o) * by, fz = B.lv(cBFZ, o) * bz;
-    auto below = [&](int a, uint32_t d) { return B.lv(cBFX + a, o - d) * B.lv(cBX + a, o - d); };
+    const Vec<R> fx = B.fixed(cBFX, o) * bx, fy = B.fixed(cBFY, o) * by, fz = B.fixed(cBFZ, o) * bz;
+    auto below = [&](int a, uint32_t d) { return B.fixed(cBFX + a, o - d) * B.lv(cBX + a, o - d); };
     constexpr uint32_t es = sizeof(R);
+    Vec<R> J[3];
     {
-      const Vec<R> v = ((vdown(fy, B.ld(cBFY, o - es) * B.ld(cBY, o - es)) - fy) + (fz - below(2, dj))) * R(1.0);
-      B.st(cJX, it, v * B.lv(cALX, o), 0, B.n2 + 1, ic);
+      const Vec<R> v = ((vdown(fy, B.fixed1(cBFY, o - es) * B.ld(cBY, o - es)) - fy) + (fz - below(2, dj))) * R(1.0);
+      J[0] = v * B.fixed(cALX, o);
     }
     {
-      const Vec<R> v = ((fx - vdown(fx, B.ld(cBFX, o - es) * B.ld(cBX, o - es))) + (below(2, di) - fz)) * R(1.0);
-      B.st(cJY, it, v * B.lv(cALY, o), 0, B.n2 + 1, jc);
+      const Vec<R> v = ((fx - vdown(fx, B.fixed1(cBFX, o - es) * B.ld(cBX, o - es))) + (below(2, di) - fz)) * R(1.0);
+      J[1] = v * B.fixed(cALY, o);
     }
     {
       const Vec<R> v = ((below(0, dj) - fx) + (fy - below(1, di))) * R(1.0);
-      B.st(cJZ, it, v * B.lv(cALZ, o), 0, B.n2);
+      J[2] = v * B.fixed(cALZ, o);
     }
+    const Vec<R> ax = B.fixed(cBAX, o), ay = B.fixed(cBAY, o), az = B.fixed(cBAZ, o);
+    const Vec<R> bxp = B.lv(cBX, o + di), byp = B.lv(cBY, o + dj), bzp = B.upper(bz, cBZ, o);
+    Vec<R> t[3] = {vset(R(0.0)), vset(R(0.0)), vset(R(0.0))}, in[3] = {t[0], t[0], t[0]};
+    auto add = [&](int q, const Vec<R> &total, const Vec<R> &induced) {  // face q of the cell
+#pragma unroll
+      for (int x = 0; x < 3; ++x) {
+        const Vec<R> w = B.fixed(cWB + 6 * x + q, o);
+        t[x] = t[x] + w * total;
+        in[x] = in[x] + w * induced;
+      }
+    };
+    add(0, -bx - ax, -bx);
+    add(1, bxp + B.fixed(cBAX, o + di), bxp);
+    add(2, -by - ay, -by);
+    add(3, byp + B.fixed(cBAY, o + dj), byp);
+    add(4, -bz - az, -bz);
+    add(5, bzp + B.fixed_upper(az, cBAZ, o), bzp);
+    // the stores behind every load
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+      B.st(cBC + x, it, t[x], 0, B.n2, ic && jc);
+      B.st(cBIC + x, it, in[x], 0, B.n2, ic && jc);
+    }
+    B.st(cJX, it, J[0], 0, B.n2 + 1, ic);
+    B.st(cJY, it, J[1], 0, B.n2 + 1, jc);
+    B.st(cJZ, it, J[2], 0, B.n2);
   });
 }
 
@@ -1237,7 +1258,7 @@ __global__ void __launch_bounds__(kVecThreads, 3) k_jcell(Dir D) {
     Vec<R> j[3] = {vset(R(0.0)), vset(R(0.0)), vset(R(0.0))};
     auto add = [&](int q, const Vec<R> &s) {  // edge q of the cell, the summation order of calc_Jcell
 #pragma unroll
-      for (int x = 0; x < 3; ++x) j[x] = j[x] + B.lv(cWJ + 12 * x + q, o) * s;
+      for (int x = 0; x < 3; ++x) j[x] = j[x] + B.fixed(cWJ + 12 * x + q, o) * s;
     };
     const Vec<R> ax = B.lv(cJX, o), bx = B.lv(cJX, o + dj), ay = B.lv(cJY, o), by = B.lv(cJY, o + di);
     const Vec<R> ux = B.upper(ax, cJX, o), vx = B.upper(bx, cJX, o + dj);
@@ -1343,7 +1364,7 @@ __device__ __forceinline__ R cells_dt(const VV<R, N> &B, const ConstsT<R> &c, co
     }
     const Vc zx = B.staged(16), zy = B.staged(17), zz = B.staged(18), zA = B.staged(19);
     face(zx, zy, zz, zA);
-    face(B.upper(zx, cFNZ, o), B.upper(zy, cFNZ + 1, o), B.upper(zz, cFNZ + 2, o), B.upper(zA, cFNZ + 3, o));
+    face(B.fixed_upper(zx, cFNZ, o), B.fixed_upper(zy, cFNZ + 1, o), B.fixed_upper(zz, cFNZ + 2, o), B.fixed_upper(zA, cFNZ + 3, o));
 #pragma unroll
     for (int e = 0; e < N; ++e)
       if (Vol.v[e] > R(0.0) && den.v[e] > R(0.0)) d.v[e] = dmin(d.v[e], c.CFL * Vol.v[e] / den.v[e]);
@@ -1474,7 +1495,7 @@ __global__ void __launch_bounds__(kVecThreads) k_res_vec(Dir D, int op, const Re
         case RES_E_FROM_P: put(cEX, B.lv(cRP + a, o)); break;  // UnpackVecToImplicitEres_ (:294-312)
         case RES_E_FROM_X: put(cEX, B.lv(cRX + a, o)); break;
         case RES_E_FROM_CG: {  // the solution of the finished CG
-          const Vec<R> p = B.own(dir_comp(use_p) + a, o), x0 = B.own(cRX + a, o);
+          const Vec<R> p = B.lv(dir_comp(use_p) + a, o), x0 = B.lv(cRX + a, o);
           const Vec<R> x = vmap<R>([&](int e) { return final_x(cg[it.s], x0.v[e], p.v[e]); });
           put(cRX, x);
           put(cEX, x);
@@ -1501,9 +1522,12 @@ __global__ void __launch_bounds__(kVecThreads) k_res_db(Dir D) {
     const bool ic = it.i < B.n0, jc = it.j < B.n1;
     const int hi = min(B.n2, it.khi);
     const Vec<R> ex = B.lv(cEX, o), ey = B.lv(cEY, o), ez = B.lv(cEZ, o);
-    B.st(cRBS, it, m * ((ey - B.upper(ey, cEY, o)) + (B.lv(cEZ, o + dj) - ez)), 0, hi, jc);
-    B.st(cRBS + 1, it, m * ((B.upper(ex, cEX, o) - ex) + (ez - B.lv(cEZ, o + di))), 0, hi, ic);
-    B.st(cRBS + 2, it, m * ((ex - B.lv(cEX, o + dj)) + (B.lv(cEY, o + di) - ey)), 0, it.khi, ic && jc);
+    const Vec<R> bx = m * ((ey - B.upper(ey, cEY, o)) + (B.lv(cEZ, o + dj) - ez));
+    const Vec<R> by = m * ((B.upper(ex, cEX, o) - ex) + (ez - B.lv(cEZ, o + di)));
+    const Vec<R> bz = m * ((ex - B.lv(cEX, o + dj)) + (B.lv(cEY, o + di) - ey));
+    B.st(cRBS, it, bx, 0, hi, jc);
+    B.st(cRBS + 1, it, by, 0, hi, ic);
+    B.st(cRBS + 2, it, bz, 0, it.khi, ic && jc);
   });
 }
 
@@ -1701,7 +1725,7 @@ __global__ void __launch_bounds__(kVecThreads) k_res_cg(Dir D, double *tpart, Re
           for (int e = 0; e < N; ++e)
             if (counts(a, e)) acc0 += (double)W[a].v[e] * (double)p.v[e] * (double)q.v[e];
         } else {
-          const Vec<R> r = B.own(cRR + a, o), q = B.lv(cRQ + a, o);
+          const Vec<R> r = B.lv(cRR + a, o), q = B.lv(cRQ + a, o);
           Vec<R> rn = r;
 #pragma unroll
           for (int e = 0; e < N; ++e) {
@@ -1765,15 +1789,20 @@ __global__ void __launch_bounds__(kVecThreads) k_res_pupd_e(Dir D, const ResCG *
     if (!__any_sync(0xffffffffu, some && it.in)) return;
     const R alpha = R(cg[it.s].alpha), beta = R(cg[it.s].beta);
     const bool first = cg[it.s].it == 1;  // x = 0 until now
+    Vec<R> x1[3], e1[3];  // stored behind every load
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      const Vec<R> p = B.own(dir_comp(use_p) + a, o), pn = B.lv(cRR + a, o) + beta * p, step = alpha * p;
+      const Vec<R> p = B.lv(dir_comp(use_p) + a, o), pn = B.lv(cRR + a, o) + beta * p, step = alpha * p;
       Vec<R> x = step;
-      if (!first) x = B.own(cRX + a, o) + step;
-      B.st(cRX + a, it, vmap<R>([&](int e) { return W[a].v[e] > R(0.0) ? x.v[e] : R(0.0); }), it.klo, it.khi);
-      const Vec<R> e1 = vmap<R>([&](int e) { return W[a].v[e] > R(0.0) ? pn.v[e] : R(0.0); });
-      if (use_p) B.st(cRP + a, it, e1, it.klo, it.khi);
-      B.st(cEX + a, it, e1, it.klo, it.khi);
+      if (!first) x = B.lv(cRX + a, o) + step;
+      x1[a] = vmap<R>([&](int e) { return W[a].v[e] > R(0.0) ? x.v[e] : R(0.0); });
+      e1[a] = vmap<R>([&](int e) { return W[a].v[e] > R(0.0) ? pn.v[e] : R(0.0); });
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      B.st(cRX + a, it, x1[a], it.klo, it.khi);
+      if (use_p) B.st(cRP + a, it, e1[a], it.klo, it.khi);
+      B.st(cEX + a, it, e1[a], it.klo, it.khi);
     }
   });
 }
@@ -1804,10 +1833,12 @@ __global__ void __launch_bounds__(kVecThreads) k_res_bupdate(Dir D) {
     // above them E_res is 0 and B does not change
     const int hi = it.khi - 1;
     const Vec<R> ex = B.lv(cEX, o), ey = B.lv(cEY, o), ez = B.lv(cEZ, o);
-    B.st(cBX, it, B.own(cBX, o) + dt * (R(-1.0) * ((ey - B.upper(ey, cEY, o)) + (B.lv(cEZ, o + dj) - ez))), 0, hi, jc);
-    B.st(cBY, it, B.own(cBY, o) + dt * (R(-1.0) * ((B.upper(ex, cEX, o) - ex) + (ez - B.lv(cEZ, o + di)))), 0, hi, ic);
-    B.st(cBZ, it, B.own(cBZ, o) + dt * (R(-1.0) * ((ex - B.lv(cEX, o + dj)) + (B.lv(cEY, o + di) - ey))), 0, it.khi,
-         ic && jc);
+    const Vec<R> bx = B.lv(cBX, o) + dt * (R(-1.0) * ((ey - B.upper(ey, cEY, o)) + (B.lv(cEZ, o + dj) - ez)));
+    const Vec<R> by = B.lv(cBY, o) + dt * (R(-1.0) * ((B.upper(ex, cEX, o) - ex) + (ez - B.lv(cEZ, o + di))));
+    const Vec<R> bz = B.lv(cBZ, o) + dt * (R(-1.0) * ((ex - B.lv(cEX, o + dj)) + (B.lv(cEY, o + di) - ey)));
+    B.st(cBX, it, bx, 0, hi, jc);
+    B.st(cBY, it, by, 0, hi, ic);
+    B.st(cBZ, it, bz, 0, it.khi, ic && jc);
   });
 }
 
@@ -1943,13 +1974,21 @@ __global__ void __launch_bounds__(kVecThreads, kPvCtas) k_pv_uplus(Dir D, int en
     {
       const uint32_t o = it.o;
       auto put = [&](int comp, const Vc &v) { B.st(comp, it, v, it.klo, it.khi); };
+      // every field ahead of the first store
+      Vc U[2][5];
+#pragma unroll
+      for (int s = 0; s < 2; ++s)
+#pragma unroll
+        for (int m = 0; m < 5; ++m) U[s][m] = B.lv((s ? cUN : cUH) + m, o);
+      const Vc Bx = B.lv(cBC, o), By = B.lv(cBC + 1, o), Bz = B.lv(cBC + 2, o);
+      const Vc Jx = B.lv(cJC, o), Jy = B.lv(cJC + 1, o), Jz = B.lv(cJC + 2, o);
       Vc rho[2], vel[2][3];
       Vc chk = vset<R, N>(R(0.0));  // sum of the conserved components: non-finite if any of them is
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
-        const int pv0 = s ? cPVN : cPVH, u0 = s ? cUN : cUH;
+        const int pv0 = s ? cPVN : cPVH;
         const R coeff = s ? c.state_coeff_Na : c.state_coeff_H;
-        const Vc r0 = B.lv(u0, o), m1 = B.lv(u0 + 1, o), m2 = B.lv(u0 + 2, o), m3 = B.lv(u0 + 3, o), E = B.lv(u0 + 4, o);
+        const Vc r0 = U[s][0], m1 = U[s][1], m2 = U[s][2], m3 = U[s][3], E = U[s][4];
         rho[s] = r0;
         chk = chk + (((r0 + m1) + (m2 + m3)) + E);
         Vc pr, T, re, cs;
@@ -1985,7 +2024,6 @@ __global__ void __launch_bounds__(kVecThreads, kPvCtas) k_pv_uplus(Dir D, int en
         put(cFT + 2 * s, re);
         put(cFT + 2 * s + 1, cs);
       }
-      const Vc Bx = B.lv(cBC, o), By = B.lv(cBC + 1, o), Bz = B.lv(cBC + 2, o);
       Vc alpha, up[3];
 #pragma unroll
       for (int e = 0; e < N; ++e) {
@@ -2004,7 +2042,6 @@ __global__ void __launch_bounds__(kVecThreads, kPvCtas) k_pv_uplus(Dir D, int en
         // (Z4_Mercury/src/physics/MercurySolver_MagExplicit_Hall.cpp:110-146): its inputs (J_cell,
         // B_cell, the densities) are final here (num_limiter clamps the
         // densities at zero itself, so it is the limiter of the raw densities)
-        const Vc Jx = B.lv(cJC, o), Jy = B.lv(cJC + 1, o), Jz = B.lv(cJC + 2, o);
         put(cEHC, alpha * (Jy * Bz - Jz * By));
         put(cEHC + 1, alpha * (Jz * Bx - Jx * Bz));
         put(cEHC + 2, alpha * (Jx * By - Jy * Bx));
@@ -2763,7 +2800,7 @@ __global__ void __launch_bounds__(kVecThreads) k_res_cross(Dir D, const ResCG *c
       if (OP == RES_X_SETUP) {
         Vec<float> r;
         if (cg) {  // RES_INIT
-          const Vec<float> W = B.lv(cRW + a, it.o), b = 0.0f + B.lv(cETAR + a, it.o) * B.lv(cJX + a, it.o);
+          const Vec<float> W = B.fixed(cRW + a, it.o), b = 0.0f + B.fixed(cETAR + a, it.o) * B.lv(cJX + a, it.o);
           r = vmap<float>([&](int e) { return W.v[e] > 0.0f ? b.v[e] : 0.0f; });
           B.st(cRR + a, it, r, it.klo, it.khi);
         } else {
@@ -2777,7 +2814,7 @@ __global__ void __launch_bounds__(kVecThreads) k_res_cross(Dir D, const ResCG *c
       } else if (OP == RES_X_DEMOTE_R) {
         B.st(cRR + a, it, narrow(cRR + a), it.klo, it.khi);
       } else if (OP == RES_X_ADD_X) {
-        const Vec<float> x = B.lv(cRX + a, it.o), d = B.lv(dir_comp(use_p) + a, it.o), W = B.lv(cRW + a, it.o);
+        const Vec<float> x = B.lv(cRX + a, it.o), d = B.lv(dir_comp(use_p) + a, it.o), W = B.fixed(cRW + a, it.o);
         double *p = (double *)at(cRX + a);
 #pragma unroll
         for (int e = 0; e < 4; ++e)
@@ -2785,7 +2822,7 @@ __global__ void __launch_bounds__(kVecThreads) k_res_cross(Dir D, const ResCG *c
       } else if (cg) {  // RES_X_DEMOTE_X of a finished CG on the companion (its own slot's state)
         const ResCG &c = cg[S.companion_slot];
         const double *x = (const double *)at(cRX + a), *p = (const double *)at(dir_comp(use_p) + a);
-        const Vec<float> W = B.lv(cRW + a, it.o);
+        const Vec<float> W = B.fixed(cRW + a, it.o);
         Vec<float> v;
 #pragma unroll
         for (int e = 0; e < 4; ++e) v.v[e] = W.v[e] > 0.0f ? (float)final_x(c, x[e], p[e]) : 0.0f;
