@@ -1365,7 +1365,22 @@ void res_apply(mhd_batch *b, int *nk) {
 // and the stop test, the direction update) while some solve's device CG
 // state says it is still running; a solve whose loop ends leaves the mask.
 // Captured once per batch (again after the tables or the partials change).
+// The CG's kernels take where the direction is kept (ResScratch::use_p) by value,
+// so it is set here, ahead of the capture, and a graph captured with the other
+// value is dropped.
+int set_direction(mhd_batch *b) {
+  const int use_p = !res_light_syncs(b);
+  if (b->res.use_p == use_p) return MHD_OK;
+  if (b->graph_cg) {
+    CUDA_TRY(cudaStreamSynchronize(b->stream));  // no loop graph in flight
+    cudaGraphExecDestroy(b->graph_cg);
+    b->graph_cg = nullptr;
+  }
+  b->res.use_p = use_p;
+  return MHD_OK;
+}
 int build_cg_graph(mhd_batch *b) {
+  if (const int rc = set_direction(b)) return rc;
   if (b->graph_cg) return MHD_OK;
   cudaGraph_t g = nullptr;
   CUDA_TRY(cudaGraphCreate(&g, 0));
@@ -1466,8 +1481,7 @@ struct CgJob {
 // Each job's final state is in b->hcg[slot].
 int res_cg_batch(mhd_batch *b, const std::vector<CgJob> &jobs) {
   int rc;
-  b->res.use_p = !res_light_syncs(b);
-  if ((rc = ensure_tpartial(b)) || (!b->cg_host_loop && (rc = build_cg_graph(b)))) return rc;
+  if ((rc = ensure_tpartial(b)) || (rc = b->cg_host_loop ? set_direction(b) : build_cg_graph(b))) return rc;
   std::vector<int> on((size_t)b->capacity, 0);
   for (int s = 0; s < b->capacity; ++s) {
     b->hcg[s] = ResCG{};
@@ -1630,7 +1644,6 @@ int res_step_device(mhd_batch *b) {
   mhd_batch *c = mixed ? b->shadow : b;  // runs the CG
   int rc, nk = 0;
   if ((rc = ensure_tpartial(c)) || (rc = build_cg_graph(c))) return rc;
-  c->res.use_p = !res_light_syncs(c);
   launch_res_begin(b->dir(1), c->res.cg, mixed, b->stream);
   if (mixed) {
     res_current(b, &nk);
