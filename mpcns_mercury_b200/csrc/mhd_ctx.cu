@@ -165,7 +165,7 @@ struct Tables {
   // on a ghost position (res_light_syncs)
   bool res_ghost_writes_only = false;
   // Some write of the E alias reduction, the singular edges or Sync(Ehall) lands
-  // on an edge inside a block (hall_writes_inside)
+  // on an edge inside a block, or the reduction reads one (hall_inside)
   bool hall_late = false;
   // The step's syncs may run in fewer launches (joined_syncs); Sync(dB) of the
   // substep needs its halo and owner copies only (plain_db), and not the owner
@@ -2046,11 +2046,11 @@ static bool res_ghost_writes_only(const Solve *S, const mhd_desc *desc) {
   return true;
 }
 
-// Whether the E alias reduction, the singular edges' EMF or Sync(Ehall) writes
-// an owned edge that does not lie in one of its block's faces: E + Ehall may
-// then not be summed ahead of them (k_edge_emf).  False on every grid whose
-// blocks meet in their faces.
-static bool hall_writes_inside(const Solve *S, const mhd_desc *desc) {
+// Whether the E alias reduction, the singular edges' EMF or Sync(Ehall) writes,
+// or the reduction reads, an owned edge that does not lie in one of its block's
+// faces: E + Ehall may then not be summed ahead of them (k_edge_emf).  False on
+// every grid whose blocks meet in their faces.
+static bool hall_inside(const Solve *S, const mhd_desc *desc) {
   auto inside = [&](int axis, const mhd_dof &d) {
     if (d.block < 0 || d.block >= S->nblocks) return false;
     const int *n = S->boxes[d.block].n;
@@ -2071,8 +2071,11 @@ static bool hall_writes_inside(const Solve *S, const mhd_desc *desc) {
     if (hall(g.stash[q].dst)) return true;
   for (int q = 0; q < g.n_phys; ++q)
     if (hall(g.phys[q].dst)) return true;
-  for (int c = 0; c < desc->edge_aliases.n_classes; ++c)
-    if (inside(desc->edge_aliases.owner[c].field, desc->edge_aliases.owner[c])) return true;
+  const mhd_alias_classes &a = desc->edge_aliases;
+  for (int c = 0; c < a.n_classes; ++c)
+    if (inside(a.owner[c].field, a.owner[c])) return true;
+  for (int m = 0; a.n_classes > 0 && m < a.offset[a.n_classes]; ++m)
+    if (inside(a.member[m].field, a.member[m])) return true;
   for (int e = 0; e < desc->singular.n_edges; ++e)
     if (inside(desc->singular.owner[e].field, desc->singular.owner[e])) return true;
   return false;
@@ -2561,7 +2564,7 @@ static int add_solve(mhd_batch *b, const mhd_desc *desc, bool periodic, int *slo
       if ((rc = upload_aliases(S, desc->edge_aliases, st))) return bail(rc);
       if ((rc = upload_phys(S, desc, st))) return bail(rc);
       if ((rc = upload_singular(S, desc->singular, st)) || (rc = alloc_singular_geo(S, st))) return bail(rc);
-      S->T->hall_late = hall_writes_inside(S, desc);
+      S->T->hall_late = hall_inside(S, desc);
       S->T->sync_joined = joined_syncs(S, desc);
       S->T->alias_all = alias_owners(S, desc);
       if (S->consts.resistive) {

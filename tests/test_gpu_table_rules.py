@@ -1,0 +1,181 @@
+"""Tables that break one of the rules by which the engine takes a shorter order of
+a step's passes (E + Ehall summed ahead of the alias reduction, syncs joined into
+fewer launches, a substep without the full Sync(dB)).  Every rule is checked
+against the same tables in the order without it, which a harmless further copy
+selects; all fields are the same to the bit, ghosts included."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from conftest import has_gpu
+
+pytestmark = pytest.mark.gpu
+
+G, N = 4, (6, 5, 7)
+FIELDS = ["U_H", "U_NA", "B_XI", "B_ETA", "B_ZETA", "B_CELL", "J_CELL", "J_XI", "J_ETA", "J_ZETA", "E_XI", "E_ETA", "E_ZETA"]
+
+
+class Tables:
+    """The periodic block's copy tables, with entries added or changed."""
+
+    def __init__(self, precision=0, resistive=False):
+        from mpcns_mercury_b200 import reference_constants
+        from mpcns_mercury_b200.capi import SolveDesc
+
+        self.precision, self.resistive, self.keep = precision, resistive, []
+        self.k = reference_constants(cfl=0.4)
+        for q in range(19):
+            self.k.bc[q] = 0.5 + 0.01 * q
+        if resistive:
+            self.k.resistive, self.k.res_max_it, self.k.res_rtol = 1, 50, 1e-9
+        self.desc = SolveDesc([N], G, self.k, precision=precision)
+        self.d = self.desc.desc
+
+    def group(self, name):
+        from mpcns_mercury_b200 import capi
+
+        return self.d.groups[capi.GROUPS.index(name)]
+
+    def _array(self, kind, rows):
+        a = (kind * max(len(rows), 1))(*rows)
+        self.keep.append(a)
+        return ctypes.cast(a, ctypes.POINTER(kind))
+
+    def set_copies(self, group, which, rows):
+        from mpcns_mercury_b200.capi import MhdCopy
+
+        g = self.group(group)
+        setattr(g, which, self._array(MhdCopy, rows))
+        setattr(g, "n_" + which, len(rows))
+
+    def copies(self, group, which):
+        g = self.group(group)
+        t = getattr(g, which)
+        return [t[q] for q in range(getattr(g, "n_" + which))]
+
+    def add_copy(self, group, which, dst, src, sign=1.0):
+        from mpcns_mercury_b200.capi import MhdCopy
+
+        self.set_copies(group, which, self.copies(group, which) + [MhdCopy(dst, src, sign)])
+
+    def add_set(self, group, dst, arg):
+        from mpcns_mercury_b200.capi import MhdPhysOp
+
+        g = self.group(group)
+        op = MhdPhysOp()
+        op.kind, op.arg, op.dst, op.src = 0, arg, dst, dst
+        g.phys, g.n_phys = self._array(MhdPhysOp, [g.phys[q] for q in range(g.n_phys)] + [op]), g.n_phys + 1
+
+    def classes(self):
+        """[(owner, owner_sign, [(member, sign), ...]), ...]"""
+        a = self.d.edge_aliases
+        return [(a.owner[c], a.owner_sign[c], [(a.member[m], a.member_sign[m]) for m in range(a.offset[c], a.offset[c + 1])])
+                for c in range(a.n_classes)]
+
+    def set_classes(self, classes):
+        from mpcns_mercury_b200.capi import MhdDof
+
+        a = self.d.edge_aliases
+        off = [0]
+        for c in classes:
+            off.append(off[-1] + len(c[2]))
+        a.n_classes = len(classes)
+        a.offset = self._array(ctypes.c_int32, off)
+        a.owner = self._array(MhdDof, [c[0] for c in classes])
+        a.owner_sign = self._array(ctypes.c_double, [c[1] for c in classes])
+        a.member = self._array(MhdDof, [m for c in classes for m, _ in c[2]])
+        a.member_sign = self._array(ctypes.c_double, [s for c in classes for _, s in c[2]])
+
+    def hall_late(self):
+        """E + Ehall summed behind the syncs: Sync(Ehall) copies an edge inside the block onto itself."""
+        e = dof("EHALL_XI", 2, 2, 3)
+        self.add_copy("EHALL", "owner", e, e)
+
+    def ordered(self, group="EHALL"):
+        """The syncs in their full order: an owner copy to a ghost that nothing
+        reads from one that the group's halo copies write."""
+        halo = self.copies(group, "halo")
+        far = max(range(len(halo)), key=lambda q: max(-halo[q].dst.i, -halo[q].dst.j, -halo[q].dst.k))
+        self.add_copy(group, "owner", halo[far].dst, halo[0 if far else 1].dst)
+
+    def start(self):
+        from mpcns_mercury_b200 import setup as S
+        from mpcns_mercury_b200.capi import Batch
+
+        batch = Batch(1, self.precision)
+        slot = batch.add(self.desc)
+        nodes, state = S.cube_state(N, solve_id=3)
+        batch.setup_geometry(slot, nodes)
+        if self.resistive:
+            for a, f in enumerate(("ETA_RES_XI", "ETA_RES_ETA", "ETA_RES_ZETA")):
+                hi = tuple(N[q] + (q != a) for q in range(3))
+                batch.upload(slot, f, np.full(hi + (1,), 1e-3), (0, 0, 0), hi)
+        for name, f in (("U_H", "U_H"), ("U_Na", "U_NA"), ("B_xi", "B_XI"), ("B_eta", "B_ETA"), ("B_zeta", "B_ZETA")):
+            a = state[name]
+            batch.upload(slot, f, a.data, a.lo, a.hi)
+        batch.sync(slot, "UCELL")
+        batch.sync(slot, "BFACE")
+        batch.prepare(slot)
+        return batch, slot
+
+    def run(self, steps=3):
+        batch, slot = self.start()
+        batch.request(slot, steps)
+        batch.run(steps)
+        info = batch.poll()[slot]
+        assert info.status == 0 and info.step == steps
+        out = fields(batch, slot)
+        batch.close()
+        return out
+
+
+def dof(field, i, j, k, comp=0):
+    from mpcns_mercury_b200 import capi
+    from mpcns_mercury_b200.capi import MhdDof
+
+    return MhdDof(capi.FIELD_ID[field], 0, i, j, k, comp)
+
+
+def fields(batch, slot):
+    return {f: batch.download(slot, f, (-G,) * 3, tuple(v + 1 + G for v in N)) for f in FIELDS}
+
+
+def same(a, b):
+    for f in FIELDS:
+        assert np.isfinite(b[f]).all() and np.array_equal(a[f], b[f]), (f, np.abs(a[f] - b[f]).max())
+
+
+@pytest.fixture(autouse=True)
+def gpu():
+    if not has_gpu():
+        pytest.skip("no GPU")
+
+
+PRECISIONS = pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "mixed"])
+
+
+@PRECISIONS
+def test_hall_late_changes_nothing(precision):
+    """E + Ehall ahead of the syncs and behind them, on tables where both are right."""
+    a, b = Tables(precision), Tables(precision)
+    b.hall_late()
+    same(a.run(), b.run())
+
+
+@PRECISIONS
+def test_alias_member_inside_the_block(precision):
+    """The E alias reduction reads an edge that is not in a face of its block:
+    without its Hall EMF."""
+    got = []
+    for late in (False, True):
+        t = Tables(precision)
+        c = t.classes()
+        owner, sign, members = c[0]
+        c[0] = (owner, sign, members + [(dof("JAC", 2, 2, 2), 1.0)])
+        c[0][2][-1][0].field = owner.field
+        t.set_classes(c)
+        if late:
+            t.hall_late()
+        got.append(t.run())
+    same(*got)
