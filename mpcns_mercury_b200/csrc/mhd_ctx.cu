@@ -2087,7 +2087,7 @@ static bool hall_inside(const Solve *S, const mhd_desc *desc) {
 // operation of its group (or the wall EMF) writes, so it holds the last sync's
 // value until its group's next copies; groups staged in one launch have slots of
 // their own; and the wall EMF and the operations of E are apart, those of B_cell
-// constants, to share launches.  Tables without these properties take the phases in order.
+// constants in ghosts (they run ahead of k_bcell_jedge), to share launches.  Tables without these properties take the phases in order.
 static bool joined_syncs(const Solve *S, const mhd_desc *desc) {
   for (int g : {(int)MHD_SYNC_EHALL, (int)MHD_SYNC_EEDGE, (int)MHD_SYNC_JEDGE, (int)MHD_SYNC_B_CELL, (int)MHD_SYNC_J_CELL})
     if (!S->T->one_pass[g]) return false;
@@ -2095,7 +2095,8 @@ static bool joined_syncs(const Solve *S, const mhd_desc *desc) {
     if (!S->T->two_pass[g]) return false;
   const mhd_sync_group &GE = desc->groups[MHD_SYNC_EEDGE], &GB = desc->groups[MHD_SYNC_B_CELL];
   for (int t = 0; t < GB.n_phys; ++t)
-    if (GB.phys[t].kind != MHD_PHYS_SET || GB.phys[t].dst.field == MHD_U_H || GB.phys[t].dst.field == MHD_U_NA)
+    if (GB.phys[t].kind != MHD_PHYS_SET || GB.phys[t].dst.field == MHD_U_H || GB.phys[t].dst.field == MHD_U_NA ||
+        dof_depth(S, GB.phys[t].dst) == 0)
       return false;
   if (desc->n_wall > 0 && GE.n_phys > 0) {
     bool ok = false;

@@ -179,3 +179,18 @@ def test_alias_member_inside_the_block(precision):
             t.hall_late()
         got.append(t.run())
     same(*got)
+
+
+@PRECISIONS
+def test_constant_in_an_owned_cell_of_b(precision):
+    """A physical operation of Sync(B_cell) that sets an owned cell: behind the pass that computes it."""
+    got = []
+    for ordered in (False, True):
+        t = Tables(precision)
+        t.add_set("B_CELL", dof("B_CELL", 2, 0, 3, 1), 11)
+        if ordered:
+            t.ordered()
+        got.append(t.run())
+    same(*got)
+    value = t.k.bc[11]
+    assert got[0]["B_CELL"][2 + G, 0 + G, 3 + G, 1] == (np.float32(value) if precision else value)
