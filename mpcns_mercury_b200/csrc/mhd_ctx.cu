@@ -2161,7 +2161,8 @@ static bool plain_db(const Solve *S, const mhd_desc *desc) {
 // Whether the alias reductions of E and J may write every member of a class in
 // place of the owner copies that follow: the owner copies of E, E_Hall and J are
 // exactly the non-owner members of the classes, each from its class's owner with
-// its sign; and nothing (a singular edge, a physical operation, the wall EMF, a
+// its sign; every member is an owned edge of its block (a ghost gets no E + Ehall
+// of its own: only the owner copies of E bring it there); and nothing (a singular edge, a physical operation, the wall EMF, a
 // halo copy that the step keeps) changes E or J between the two.
 static bool alias_owners(const Solve *S, const mhd_desc *desc) {
   const mhd_alias_classes &a = desc->edge_aliases;
@@ -2180,6 +2181,9 @@ static bool alias_owners(const Solve *S, const mhd_desc *desc) {
   for (int c = 0; c < a.n_classes; ++c) {
     owner[c] = code(a.owner[c], 0);
     for (int m = a.offset[c]; m < a.offset[c + 1]; ++m) {
+      mhd_dof e = a.member[m];
+      e.field += MHD_E_XI;
+      if (dof_depth(S, e) > 0) return false;
       cls[m] = c;
       members.add(code(a.member[m], 0), m);
     }

@@ -194,3 +194,29 @@ def test_constant_in_an_owned_cell_of_b(precision):
     same(*got)
     value = t.k.bc[11]
     assert got[0]["B_CELL"][2 + G, 0 + G, 3 + G, 1] == (np.float32(value) if precision else value)
+
+
+def _with_member(t, member, sign=1.0):
+    """`member` (an edge index) as a further member of the first class, with its owner copies."""
+    c = t.classes()
+    owner, osign, members = c[0]
+    axis = "XI ETA ZETA".split()[owner.field]
+    e = dof("JAC", *member)
+    e.field = owner.field
+    c[0] = (owner, osign, members + [(e, sign)])
+    t.set_classes(c)
+    for group, field in (("EHALL", "EHALL_"), ("EEDGE", "E_"), ("JEDGE", "J_")):
+        t.add_copy(group, "owner", dof(field + axis, *member), dof(field + axis, owner.i, owner.j, owner.k), sign * osign)
+
+
+@PRECISIONS
+def test_ghost_alias_member(precision):
+    """A class with a ghost edge: its E + Ehall comes with the owner copies of E."""
+    got = []
+    for ordered in (False, True):
+        t = Tables(precision)
+        _with_member(t, (N[0] + 2, N[1] + 2, 2))
+        if ordered:
+            t.ordered()
+        got.append(t.run())
+    same(*got)
