@@ -2201,8 +2201,9 @@ static bool alias_owners(const Solve *S, const mhd_desc *desc) {
           G.owner[t].sign != a.member_sign[m] * a.owner_sign[cls[m]])
         return false;
     }
+    // a member without a copy is its class's owner, with the owner's sign: it keeps the mean
     for (int m = 0; m < nm; ++m)
-      if (!seen[m] && code(a.member[m], 0) != owner[cls[m]]) return false;
+      if (!seen[m] && (code(a.member[m], 0) != owner[cls[m]] || a.member_sign[m] != a.owner_sign[cls[m]])) return false;
   }
   return true;
 }

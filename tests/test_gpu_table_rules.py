@@ -220,3 +220,22 @@ def test_ghost_alias_member(precision):
             t.ordered()
         got.append(t.run())
     same(*got)
+
+
+@PRECISIONS
+def test_owner_with_another_sign_as_a_member(precision):
+    """The owner of a class is one of its members with a sign that is not the owner's."""
+    got = []
+    for ordered in (False, True):
+        t = Tables(precision)
+        c = t.classes()
+        owner, sign, members = c[0]
+        index = lambda d: (d.field, d.block, d.i, d.j, d.k)
+        flipped = [(m, -s if index(m) == index(owner) else s) for m, s in members]
+        assert flipped != members
+        c[0] = (owner, sign, flipped)
+        t.set_classes(c)
+        if ordered:
+            t.ordered()
+        got.append(t.run())
+    same(*got)
