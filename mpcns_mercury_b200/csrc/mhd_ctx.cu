@@ -2145,8 +2145,9 @@ static bool joined_syncs(const Solve *S, const mhd_desc *desc) {
 // Whether Sync(dB) of the substep needs its halo and owner copies only: no
 // physical operation; every staged source a ghost face, zero when it is staged
 // (clear_triplet), so the staged copies write the zeros that the substep's
-// start left there (k_res_clearb); and no other copy reads a ghost face that a
-// copy writes, so none has to be zeroed again.
+// start left there (k_res_clearb); no other copy reads a ghost face that a
+// halo or staged copy writes, and the owner copies write owned faces, so none
+// has to be zeroed again.
 static bool plain_db(const Solve *S, const mhd_desc *desc) {
   const mhd_sync_group &G = desc->groups[MHD_SYNC_DB];
   if (G.n_phys > 0) return false;
@@ -2155,6 +2156,8 @@ static bool plain_db(const Solve *S, const mhd_desc *desc) {
     if (G.stash[t].src.field == MHD_STAGING || dof_depth(S, G.stash[t].src) == 0 ||
         dof_depth(S, G.stash[G.n_stash + t].dst) == 0)
       return false;
+  for (int t = 0; t < G.n_owner; ++t)
+    if (G.owner[t].dst.field == MHD_STAGING || dof_depth(S, G.owner[t].dst) > 0) return false;
   return true;
 }
 
@@ -2208,9 +2211,9 @@ static bool alias_owners(const Solve *S, const mhd_desc *desc) {
   return true;
 }
 
-// Whether Sync(dB)'s owner copies copy what is there already: each is of a face
-// whose four edges are, in order and sign, those of its owner after the owner
-// copies of E_res, so k_res_db computes the same bits on both.
+// Whether Sync(dB)'s owner copies copy what is there already: each is of an owned
+// face whose four edges are, in order and sign, those of its owner (an owned face
+// too) after the owner copies of E_res, so k_res_db computes the same bits on both.
 static bool same_db(const Solve *S, const mhd_desc *desc) {
   const mhd_sync_group &E = desc->groups[MHD_SYNC_ERES], &G = desc->groups[MHD_SYNC_DB];
   bool ok = false;
@@ -2226,6 +2229,7 @@ static bool same_db(const Solve *S, const mhd_desc *desc) {
     const mhd_copy &cp = G.owner[t];
     const int ax = cp.dst.field - MHD_B_XI;
     if (cp.sign != 1.0 || ax < 0 || ax > 2 || cp.src.field != cp.dst.field) return false;
+    if (dof_depth(S, cp.dst) > 0 || dof_depth(S, cp.src) > 0) return false;
     for (int q = 0; q < 4; ++q) {  // the face's edges along the other axes
       const int along = (ax + 1 + q / 2) % 3, across = (ax + 2 - q / 2) % 3;
       mhd_dof d = cp.dst, s = cp.src;

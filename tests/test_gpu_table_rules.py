@@ -239,3 +239,31 @@ def test_owner_with_another_sign_as_a_member(precision):
             t.ordered()
         got.append(t.run())
     same(*got)
+
+
+@PRECISIONS
+def test_owner_copy_of_a_ghost_face_in_the_substep(precision):
+    """Sync(dB) fills a ghost face by an owner copy in place of the halo copy."""
+    got = []
+    for owner in (False, True):
+        t = Tables(precision, resistive=True)
+        if owner:
+            face = (-1, 2, 3)
+            halo = t.copies("DB", "halo")
+            row = next(h for h in halo if h.dst.field == dof("B_ETA", 0, 0, 0).field and (h.dst.i, h.dst.j, h.dst.k) == face)
+            src = (row.src.i, row.src.j, row.src.k)
+            t.set_copies("DB", "halo", [h for h in halo if h is not row])
+            t.add_copy("DB", "owner", row.dst, row.src)
+            # its four edges are those of the face it stands for
+            for field, across in (("E_ZETA", 0), ("E_XI", 2)):
+                for up in (0, 1):
+                    e, s = [list(face), list(src)]
+                    e[across] += up
+                    s[across] += up
+                    if all(0 <= e[a] < N[a] + 1 for a in range(3)) or field == "E_ZETA" and e[0] == 0:
+                        continue
+                    t.add_copy("ERES", "owner", dof(field, *e), dof(field, *s))
+        got.append(t.run())
+        for f in ("E_XI", "E_ETA", "E_ZETA"):  # E_res's array: its further copies go to ghosts
+            got[-1][f] = got[-1][f][G:-G, G:-G, G:-G]
+    same(*got)
