@@ -167,6 +167,8 @@ struct Tables {
   // Some write of the E alias reduction, the singular edges or Sync(Ehall) lands
   // on an edge inside a block, or the reduction reads one (hall_inside)
   bool hall_late = false;
+  // Every copy and physical operation stays within its group's fields (group_field)
+  bool own_fields = true;
   // The step's syncs may run in fewer launches (joined_syncs); Sync(dB) of the
   // substep needs its halo and owner copies only (plain_db), and not the owner
   // copies either (same_db); the alias reductions replace the owner copies of E,
@@ -270,6 +272,7 @@ struct mhd_batch {
   // solves whose syncs need the general order, whose Sync(dB) does, whose Sync(dB)
   // needs owner copies, and whose alias reductions do not replace the owner copies
   int n_sync_general = 0, n_db_general = 0, n_db_owner = 0, n_alias_owner = 0;
+  int n_foreign = 0;  // solves with tables that name other groups' fields: every launch in full, in one row
   int n_res_full = 0;                                   // of them, solves whose substep runs the full E / J syncs
   // FP64 batch of the companions of mixed-precision resistive solves, which
   // runs on this batch's stream and pool (borrowed = true in the companion)
@@ -351,7 +354,7 @@ void launch(mhd_batch *b, int mode, StepKernel k, int *nk, const SyncOps *ops = 
             double darg = 0.0) {
   // (k_fluid reads earlier passes' fields through the read-only path: always in full)
   launch_step_kernel(k, b->dir(mode), b->stream, ops, b->precision, iarg, darg, b->res,
-                     b->after_flip || k == SK_FLUID);
+                     b->after_flip || k == SK_FLUID || b->n_foreign > 0);
   // it flips the solves' states, writes static fields, or ends a step: the next kernels read
   // those, and k_sing_emf the last step's fields, ahead of their wait
   b->after_flip = k == SK_BFACE || k == SK_FACE_NORMALS || k == SK_RES_W || k == SK_SING_SETUP || k == SK_PV_UPLUS;
@@ -362,13 +365,14 @@ void launch(mhd_batch *b, int mode, StepKernel k, int *nk, const SyncOps *ops = 
 // The fluid pass, which reads nothing that the EMF passes behind k_face_emf write
 // and writes the next state buffer only, as a branch of a captured step: from
 // behind k_face_emf to ahead of k_bface, which flips the buffers (fluid_join).
-// Outside a capture (profiling) it is launched where it joins.  The EMF passes wait
+// Outside a capture (profiling), and beside tables that could write what it reads
+// (n_foreign), it is launched where it joins.  The EMF passes wait
 // on loads and leave issue slots, and on small grids whole SMs, to it: a step of
 // the box of 8^3 FP64 cells takes 48 us (52 in one row), 32^3 72 (77), 64^3 mixed
 // 135 (147), 96^3 mixed 341 (346).  The branch's stream has the high priority:
 // its blocks are the long ones (0 to 1 % over the low one).
 void fluid_branch(mhd_batch *b, int mode, int *nk) {
-  if (!b->capturing) return;
+  if (!b->capturing || b->n_foreign > 0) return;
   cudaEventRecord(b->branch_ev[0], b->stream);
   cudaStreamWaitEvent(b->side, b->branch_ev[0], 0);
   launch_step_kernel(SK_FLUID, b->dir(mode), b->side, nullptr, b->precision, b->fluid_tile, 0.0, b->res, true);
@@ -376,7 +380,7 @@ void fluid_branch(mhd_batch *b, int mode, int *nk) {
   ++*nk;
 }
 void fluid_join(mhd_batch *b, int mode, int *nk) {
-  if (!b->capturing) return launch(b, mode, SK_FLUID, nk, nullptr, b->fluid_tile);
+  if (!b->capturing || b->n_foreign > 0) return launch(b, mode, SK_FLUID, nk, nullptr, b->fluid_tile);
   cudaStreamWaitEvent(b->stream, b->branch_ev[1], 0);
   b->after_flip = true;  // k_bface waits for both branches in full
 }
@@ -691,6 +695,23 @@ struct Encoded {
 
 constexpr int kEncodeChunk = 1 << 13;
 
+// The fields of a sync group.  A table may name any field; what the step
+// reorders or overlaps (the joined syncs, the fluid pass beside the EMF passes,
+// launches that begin while their predecessor drains) rests on each group's sync
+// writing its own.
+bool group_field(int group, int field) {
+  switch (group) {
+    case MHD_SYNC_UCELL: return field == MHD_U_H || field == MHD_U_NA;
+    case MHD_SYNC_BFACE: case MHD_SYNC_DB: return field >= MHD_B_XI && field <= MHD_B_ZETA;
+    case MHD_SYNC_EHALL: return field >= MHD_EHALL_XI && field <= MHD_EHALL_ZETA;
+    case MHD_SYNC_EEDGE: case MHD_SYNC_ERES: return field >= MHD_E_XI && field <= MHD_E_ZETA;
+    case MHD_SYNC_B_CELL: return field == MHD_B_CELL || field == MHD_BIND_CELL;
+    case MHD_SYNC_JEDGE: return field >= MHD_J_XI && field <= MHD_J_ZETA;
+    case MHD_SYNC_J_CELL: return field == MHD_J_CELL;
+    case MHD_SYNC_BADD: return field >= MHD_BADD_XI && field <= MHD_BADD_ZETA;
+    default: return false;
+  }
+}
 // The DOF that a table of `group` addresses: Sync(dB)'s tables name the face
 // fluxes, whose dB lies in arrays of its own.
 mhd_dof table_dof(int group, mhd_dof d) {
@@ -701,12 +722,14 @@ mhd_dof table_dof(int group, mhd_dof d) {
   return d;
 }
 
-// Encodes entries [t0, t1) of a table of `group`; records the first invalid entry of
-// the chunk and whether its destinations ascend.
-void encode_chunk(const Solve *S, int group, const mhd_copy *tab, int t0, int t1, Encoded *e, int *bad, int *kind,
-                  char *asc) {
+// Encodes entries [t0, t1) of table `phase` (upload_groups) of `group`; records the
+// first invalid entry of the chunk, whether its destinations ascend, and whether
+// its entries name the group's fields only (and the staging slots where it stages).
+void encode_chunk(const Solve *S, int group, int phase, const mhd_copy *tab, int t0, int t1, Encoded *e, int *bad,
+                  int *kind, char *asc, char *own) {
   *bad = -1;
   *asc = 1;
+  *own = 1;
   for (int t = t0; t < t1; ++t) {
     bool o1, o2;
     const int64_t dc = S->code(table_dof(group, tab[t].dst), &o1);
@@ -719,6 +742,9 @@ void encode_chunk(const Solve *S, int group, const mhd_copy *tab, int t0, int t1
     e->dst[t] = dc;
     e->src[t] = sc;
     e->neg[t] = tab[t].sign < 0.0;
+    if (!(phase == 2 ? tab[t].dst.field == MHD_STAGING : group_field(group, tab[t].dst.field)) ||
+        !(phase == 3 ? tab[t].src.field == MHD_STAGING : group_field(group, tab[t].src.field)))
+      *own = 0;
     const int d = tab[t].dst.field == MHD_STAGING ? 0 : dof_depth(S, tab[t].dst);
     e->depth[t] = (uint8_t)(d > 255 ? 255 : d);
     if (t > t0 && dc <= e->dst[t - 1]) *asc = 0;
@@ -1088,14 +1114,14 @@ int upload_groups(Solve *S, const mhd_sync_group *groups, cudaStream_t st) {
   }
   const int nch = first_chunk[NT];
   std::vector<int> bad(nch), kind(nch, 0);
-  std::vector<char> asc(nch);
+  std::vector<char> asc(nch), own(nch);
   std::vector<int> chunk_table(nch);
   for (int q = 0; q < NT; ++q)
     for (int c = first_chunk[q]; c < first_chunk[q + 1]; ++c) chunk_table[c] = q;
   mhd::parallel_for(nch, [&](int c) {
     const int q = chunk_table[c];
     const int t0 = (c - first_chunk[q]) * kEncodeChunk, t1 = std::min(ntab[q], t0 + kEncodeChunk);
-    encode_chunk(S, q / 4, tabs[q], t0, t1, &enc[q], &bad[c], &kind[c], &asc[c]);
+    encode_chunk(S, q / 4, q % 4, tabs[q], t0, t1, &enc[q], &bad[c], &kind[c], &asc[c], &own[c]);
   });
   for (int q = 0; q < NT; ++q) {
     const int g = q / 4, p = q % 4;
@@ -1109,6 +1135,7 @@ int upload_groups(Solve *S, const mhd_sync_group *groups, cudaStream_t st) {
       }
       const int t0 = (c - first_chunk[q]) * kEncodeChunk;
       if (!asc[c] || (t0 && e.dst[t0] <= e.dst[t0 - 1])) e.ascending = false;
+      if (!own[c]) S->T->own_fields = false;
     }
   }
   return upload_encoded(S, enc, st, 4);
@@ -1270,6 +1297,7 @@ bool count_tables(mhd_batch *b, const Solve *S, int d) {
     grew = grew || (d > 0 && *n == 0);
     *n += d;
   };
+  count(!S->T->own_fields, &b->n_foreign);
   count(!S->T->sync_joined, &b->n_sync_general);
   count(S->consts.resistive && !S->T->db_plain, &b->n_db_general);
   count(S->consts.resistive && !S->T->db_same, &b->n_db_owner);
@@ -1545,7 +1573,7 @@ int res_refine(mhd_batch *b, int slot, Solve *S, bool *converged) {
   ms[cs] = 1;
   if ((rc = apply_masks(b, mb)) || (rc = apply_masks(sh, ms))) return rc;
   // the companion's dt, b and x = 0; its dB ghost faces
-  launch_res_cross(Dm, RES_X_SETUP, st);
+  launch_res_cross(Dm, RES_X_SETUP, st, nullptr, 0, b->n_foreign > 0);
   if (open_grids(sh)) launch(sh, 1, SK_RES_CLEARB, &nk);
   CUDA_TRY(cudaGetLastError());
   const double rtol = S->res_rtol > 0.0 ? S->res_rtol : default_rtol(b);
@@ -1568,15 +1596,15 @@ int res_refine(mhd_batch *b, int slot, Solve *S, bool *converged) {
     }
     if (S->res_refinements == kMaxRefinements || !(rn == rn)) break;
     // the correction: FP32 CG on r rounded to FP32, x += d in FP64
-    launch_res_cross(Dm, RES_X_DEMOTE_R, st);
+    launch_res_cross(Dm, RES_X_DEMOTE_R, st, nullptr, 0, b->n_foreign > 0);
     if ((rc = res_cg_batch(b, {CgJob{slot, kInnerRtol, S->res_max_it}}))) return rc;
     if ((rc = apply_masks(b, mb))) return rc;  // the loop cleared it
-    launch_res_cross(Dm, RES_X_ADD_X, st, b->res.cg, b->res.use_p);
+    launch_res_cross(Dm, RES_X_ADD_X, st, b->res.cg, b->res.use_p, b->n_foreign > 0);
     S->res_iters += b->hcg[slot].it;
     ++S->res_refinements;
   }
   S->res_relres = bnorm > 0.0 ? rn / bnorm : 0.0;
-  launch_res_cross(Dm, RES_X_DEMOTE_X, st);
+  launch_res_cross(Dm, RES_X_DEMOTE_X, st, nullptr, 0, b->n_foreign > 0);
   CUDA_TRY(cudaGetLastError());
   std::fill(ms.begin(), ms.end(), 0);
   return apply_masks(sh, ms);
@@ -1647,7 +1675,7 @@ int res_step_device(mhd_batch *b) {
   launch_res_begin(b->dir(1), c->res.cg, mixed, b->stream);
   if (mixed) {
     res_current(b, &nk);
-    launch_res_cross(b->dir(1), RES_X_SETUP, b->stream, c->res.cg);
+    launch_res_cross(b->dir(1), RES_X_SETUP, b->stream, c->res.cg, 0, b->n_foreign > 0);
   } else {
     res_rhs(b, &nk);
   }
@@ -1659,7 +1687,7 @@ int res_step_device(mhd_batch *b) {
     if (b->slots[s] && b->slots[s]->consts.resistive) b->cg_solves[s] = b->slots[s];
   CUDA_TRY(cudaEventRecord(b->cg_done, b->stream));
   b->cg_pending = true;
-  if (mixed) launch_res_cross(b->dir(1), RES_X_DEMOTE_X, b->stream, c->res.cg, c->res.use_p);
+  if (mixed) launch_res_cross(b->dir(1), RES_X_DEMOTE_X, b->stream, c->res.cg, c->res.use_p, b->n_foreign > 0);
   else launch(b, 1, SK_RES_VEC, &nk, nullptr, RES_E_FROM_CG);
   res_finish(b, &nk);
   launch_res_end(b->dir(1), c->res.cg, c->hcg, c->capacity, mixed, true, b->stream);
@@ -1718,10 +1746,10 @@ int res_step(mhd_batch *b, const std::vector<int> &slots) {
         jobs.push_back(CgJob{S->shadow_slot, S->res_rtol > 0.0 ? S->res_rtol : default_rtol(b), S->res_max_it});
       }
       if ((rc = apply_masks(b, mb)) || (rc = apply_masks(sh, ms))) return rc;
-      launch_res_cross(b->dir(1), RES_X_SETUP, st, sh->res.cg);
+      launch_res_cross(b->dir(1), RES_X_SETUP, st, sh->res.cg, 0, b->n_foreign > 0);
       if (open_grids(sh)) launch(sh, 1, SK_RES_CLEARB, &nk);  // the companions' dB ghost faces
       if ((rc = res_cg_batch(sh, jobs))) return rc;
-      launch_res_cross(b->dir(1), RES_X_DEMOTE_X, st, sh->res.cg, sh->res.use_p);
+      launch_res_cross(b->dir(1), RES_X_DEMOTE_X, st, sh->res.cg, sh->res.use_p, b->n_foreign > 0);
       CUDA_TRY(cudaGetLastError());
       for (int s : direct) take(b->slots[s], sh->hcg[b->slots[s]->shadow_slot], s);
     }
@@ -2089,15 +2117,14 @@ static bool hall_inside(const Solve *S, const mhd_desc *desc) {
 // their own; and the wall EMF and the operations of E are apart, those of B_cell
 // constants in ghosts (they run ahead of k_bcell_jedge), to share launches.  Tables without these properties take the phases in order.
 static bool joined_syncs(const Solve *S, const mhd_desc *desc) {
+  if (!S->T->own_fields) return false;
   for (int g : {(int)MHD_SYNC_EHALL, (int)MHD_SYNC_EEDGE, (int)MHD_SYNC_JEDGE, (int)MHD_SYNC_B_CELL, (int)MHD_SYNC_J_CELL})
     if (!S->T->one_pass[g]) return false;
   for (int g : {(int)MHD_SYNC_UCELL, (int)MHD_SYNC_BFACE})
     if (!S->T->two_pass[g]) return false;
   const mhd_sync_group &GE = desc->groups[MHD_SYNC_EEDGE], &GB = desc->groups[MHD_SYNC_B_CELL];
   for (int t = 0; t < GB.n_phys; ++t)
-    if (GB.phys[t].kind != MHD_PHYS_SET || GB.phys[t].dst.field == MHD_U_H || GB.phys[t].dst.field == MHD_U_NA ||
-        dof_depth(S, GB.phys[t].dst) == 0)
-      return false;
+    if (GB.phys[t].kind != MHD_PHYS_SET || dof_depth(S, GB.phys[t].dst) == 0) return false;
   if (desc->n_wall > 0 && GE.n_phys > 0) {
     bool ok = false;
     CodeSet wall((size_t)desc->n_wall);
@@ -2149,6 +2176,7 @@ static bool joined_syncs(const Solve *S, const mhd_desc *desc) {
 // halo or staged copy writes, and the owner copies write owned faces, so none
 // has to be zeroed again.
 static bool plain_db(const Solve *S, const mhd_desc *desc) {
+  if (!S->T->own_fields) return false;
   const mhd_sync_group &G = desc->groups[MHD_SYNC_DB];
   if (G.n_phys > 0) return false;
   if (!S->T->db_apart) return false;
@@ -2168,6 +2196,7 @@ static bool plain_db(const Solve *S, const mhd_desc *desc) {
 // of its own: only the owner copies of E bring it there); and nothing (a singular edge, a physical operation, the wall EMF, a
 // halo copy that the step keeps) changes E or J between the two.
 static bool alias_owners(const Solve *S, const mhd_desc *desc) {
+  if (!S->T->own_fields) return false;
   const mhd_alias_classes &a = desc->edge_aliases;
   if (desc->singular.n_edges > 0 || desc->n_wall > 0 || a.n_classes < 0) return false;
   for (int g : {(int)MHD_SYNC_EEDGE, (int)MHD_SYNC_JEDGE})
@@ -2254,6 +2283,7 @@ static int upload_phys(Solve *S, const mhd_desc *desc, cudaStream_t st) {
     std::vector<DevPhysOp> other;
     for (int t = 0; t < n; ++t) {
       const mhd_phys_op &o = ops[t];
+      if (!group_field(q < kMaxGroups ? q : (int)MHD_SYNC_EEDGE, o.dst.field)) S->T->own_fields = false;
       bool ok1 = false, ok2 = true;
       const int64_t dc = S->code(table_dof(q, o.dst), &ok1);
       if (!ok1) return fail(MHD_ERR_ARG, "physical operation %d of table %d: destination out of range", t, q);
@@ -2574,7 +2604,7 @@ static int add_solve(mhd_batch *b, const mhd_desc *desc, bool periodic, int *slo
       if ((rc = upload_aliases(S, desc->edge_aliases, st))) return bail(rc);
       if ((rc = upload_phys(S, desc, st))) return bail(rc);
       if ((rc = upload_singular(S, desc->singular, st)) || (rc = alloc_singular_geo(S, st))) return bail(rc);
-      S->T->hall_late = hall_inside(S, desc);
+      S->T->hall_late = !S->T->own_fields || hall_inside(S, desc);
       S->T->sync_joined = joined_syncs(S, desc);
       S->T->alias_all = alias_owners(S, desc);
       if (S->consts.resistive) {

@@ -2835,9 +2835,9 @@ __global__ void __launch_bounds__(kVecThreads) k_res_cross(Dir D, const ResCG *c
   });
 }
 
-void launch_res_cross(const Dir &D, int op, cudaStream_t st, const ResCG *cg, int use_p) {
+void launch_res_cross(const Dir &D, int op, cudaStream_t st, const ResCG *cg, int use_p, bool full) {
   grids<float>();
-  t_full = false;
+  t_full = full;
   switch (op) {
     case RES_X_SETUP: launch_dependent(k_res_cross<RES_X_SETUP>, g_grid_tiles, kVecThreads, st, D, cg, use_p); break;
     case RES_X_DEMOTE_R: launch_dependent(k_res_cross<RES_X_DEMOTE_R>, g_grid_tiles, kVecThreads, st, D, cg, use_p); break;

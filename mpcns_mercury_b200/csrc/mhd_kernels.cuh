@@ -88,9 +88,10 @@ int res_dot_grid();
 // Mixed-precision implicit substep: moves its vectors between every masked
 // solve of the FP32 directory D and its FP64 companion (DevSolve::companion;
 // RES_X_SETUP also hands over the step's dt) (k_res_cross, FP32 translation
-// unit).  cg, use_p: the states and the direction of the CG whose solution is taken.
+// unit).  cg, use_p: the states and the direction of the CG whose solution is taken;
+// full: as in launch_step_kernel.
 enum ResCrossOp { RES_X_SETUP = 0, RES_X_DEMOTE_R, RES_X_ADD_X, RES_X_DEMOTE_X };
-void launch_res_cross(const Dir &D, int op, cudaStream_t st, const ResCG *cg = nullptr, int use_p = 0);
+void launch_res_cross(const Dir &D, int op, cudaStream_t st, const ResCG *cg, int use_p, bool full);
 // The ends of a substep whose decisions stay on the device.  launch_res_begin
 // masks the resistive solves that take this step (and their companions; mixed:
 // the CG runs on these) and sets up their CG states.  launch_res_end after the

@@ -267,3 +267,31 @@ def test_owner_copy_of_a_ghost_face_in_the_substep(precision):
         for f in ("E_XI", "E_ETA", "E_ZETA"):  # E_res's array: its further copies go to ghosts
             got[-1][f] = got[-1][f][G:-G, G:-G, G:-G]
     same(*got)
+
+
+@PRECISIONS
+def test_operation_on_another_groups_field(precision):
+    """Sync(Ehall) sets a density that the fluid pass reads: the step's graph runs
+    the passes in the row of the step that is launched kernel by kernel."""
+    from mpcns_mercury_b200 import capi
+
+    got = []
+    for eager in (False, True):
+        t = Tables(precision)
+        t.add_set("EHALL", dof("U_H", 3, 2, 4), 0)
+        t.add_copy("EEDGE", "owner", dof("PV_H", 4, 3, 2, 3), dof("PV_NA", 4, 3, 2, 3))
+        batch, slot = t.start()
+        if eager:
+            batch.request(slot, 3)
+            ms, names, n = (ctypes.c_float * 100)(), (ctypes.c_char_p * 100)(), ctypes.c_int()
+            capi.check(capi.lib().mhd_batch_step_profiled(batch.b, 3, 100, ms, names, ctypes.byref(n)), "step_profiled")
+            order = [names[q].decode() for q in range(n.value)]
+            assert order.index("k_fluid") > order.index("k_add_hall")
+        else:
+            batch.request(slot, 3)
+            batch.run(3)
+        info = batch.poll()[slot]
+        assert info.status == 0 and info.step == 3
+        got.append(fields(batch, slot))
+        batch.close()
+    same(*got)

@@ -72,6 +72,6 @@ def test_static_fields_are_not_stored_by_a_step(static):
 def test_fluid_pass_is_launched_in_full():
     with open(os.path.join(CSRC, "mhd_ctx.cu")) as f:
         s = re.sub(r"//[^\n]*", "", f.read())
-    assert re.search(r"b->after_flip \|\| k == SK_FLUID\)", body(s, "void launch(mhd_batch *b"))
+    assert re.search(r"b->after_flip \|\| k == SK_FLUID\b", body(s, "void launch(mhd_batch *b"))
     direct = re.findall(r"launch_step_kernel\(SK_FLUID[^;]*;", s)
     assert direct and all(c.rstrip(";").endswith(", true)") for c in direct)
