@@ -439,6 +439,7 @@ void drop_graphs(mhd_batch *b);
 // layer (mhd_sync); otherwise the layers the step reads (kHaloDepth).
 void enqueue_sync(mhd_batch *b, int mode, int g, int *nk, bool full = false) {
   sync_pre(b, mode, g, nk);
+  for (int p = kNumPhases - 1; full && p >= kPhFullFirst; --p) sync1(b, mode, copy_op(g, p), nk);
   sync1(b, mode, copy_op(g, full ? kPhHaloFull : kPhHalo), nk);
   sync_post(b, mode, g, nk);
   sync1(b, mode, copy_op(g, kPhOwner), nk);
@@ -909,6 +910,27 @@ std::vector<char> step_halo_mask(const Encoded &h, const Encoded *owner, const E
   return keep;
 }
 
+// The halo copies read the values from before the sync.  On a block with fewer
+// cells along an axis than ghost layers a copy may read a ghost that another one
+// writes: it runs ahead of that one (never inside a step, whose copies go two
+// layers deep).  Per copy: how many copies must follow it one after the other.
+std::vector<uint8_t> full_levels(const Encoded &h) {
+  const size_t n = h.dst.size();
+  CodeSet by_dst(n);
+  for (size_t t = 0; t < n; ++t) by_dst.add(h.dst[t], (int64_t)t);
+  std::vector<uint8_t> level(n, 0);
+  for (size_t t = 0; t < n; ++t) {
+    int64_t c = h.src[t];
+    while (level[t] < kFullLevels) {
+      const CodeSet::Slot &e = by_dst.slot[by_dst.at(c)];
+      if (e.code != c) break;
+      ++level[t];
+      c = h.src[e.value];
+    }
+  }
+  return level;
+}
+
 // Whether a group's copies of the step may run at once: the kept halo copies h,
 // the owner copies o and the copies from the staging slots u write different
 // positions and none reads what another phase writes (*one); the same of the
@@ -952,6 +974,9 @@ bool reads_no_ghost_write(const Encoded &h, const std::vector<char> &keep, const
 // (per_group 4: the stash copies, then the copies from the staging slots).
 int upload_encoded(Solve *S, const std::vector<Encoded> &enc, cudaStream_t st, int per_group = 2) {
   std::vector<std::vector<int64_t>> seg(kNumPhases * MHD_NUM_GROUPS);
+  bool thin = false;  // a block thinner than its ghost layers
+  for (const Box &bx : S->boxes)
+    for (int a = 0; a < 3; ++a) thin = thin || bx.n[a] < S->nghost;
   mhd::parallel_for(kNumPhases * MHD_NUM_GROUPS, [&](int q) {
     const int g = q / kNumPhases, phase = q % kNumPhases;
     const Encoded &h = enc[per_group * g], &o = enc[per_group * g + 1];
@@ -966,9 +991,22 @@ int upload_encoded(Solve *S, const std::vector<Encoded> &enc, cudaStream_t st, i
         break;
       }
       case kPhOwner: seg[q] = build_segments(o, S->es, -1); break;
-      case kPhHaloFull: seg[q] = build_segments(h, S->es, -1); break;
+      case kPhHaloFull: {
+        if (!thin) {
+          seg[q] = build_segments(h, S->es, -1);
+          break;
+        }
+        const std::vector<uint8_t> level = full_levels(h);
+        std::vector<char> keep(level.size());
+        for (int l = 0; l <= kFullLevels; ++l) {
+          for (size_t t = 0; t < level.size(); ++t) keep[t] = level[t] == l;
+          seg[l == 0 ? q : q - phase + kPhFullFirst + l - 1] = build_segments(h, S->es, -1, &keep);
+        }
+        break;
+      }
       case kPhStash: if (stash) seg[q] = build_segments(*stash, S->es, -1); break;
-      default: if (unstash) seg[q] = build_segments(*unstash, S->es, -1); break;
+      case kPhUnstash: if (unstash) seg[q] = build_segments(*unstash, S->es, -1); break;
+      default: break;  // with kPhHaloFull
     }
   });
   for (int q = 0; q < kNumPhases * MHD_NUM_GROUPS; ++q) {

@@ -221,9 +221,11 @@ struct DevAlias {
 constexpr int kMaxGroups = MHD_NUM_GROUPS;
 // Copy phases of a group: 0 halo copies to the step's depth, 1 owner copies,
 // 2 every halo copy, 3 staging <- sources the halo phase overwrites, 4
-// destinations <- staging.
-constexpr int kNumPhases = 5;
-enum CopyPhase : int { kPhHalo = 0, kPhOwner = 1, kPhHaloFull = 2, kPhStash = 3, kPhUnstash = 4 };
+// destinations <- staging, 5 and on: halo copies that run ahead of phase 2, the
+// last of these phases first (full_levels).
+constexpr int kFullLevels = 3;
+constexpr int kNumPhases = 5 + kFullLevels;
+enum CopyPhase : int { kPhHalo = 0, kPhOwner = 1, kPhHaloFull = 2, kPhStash = 3, kPhUnstash = 4, kPhFullFirst = 5 };
 
 // Physical boundary operations (mhd_phys_op) of one solve: per group, and
 // the step's wall EMF as table kMaxGroups.  MHD_PHYS_SET operations are one
