@@ -595,9 +595,13 @@ __device__ __forceinline__ Num<R> num_limiter(const ConstsT<R> &c, R rhoH, R rho
   d.ne_eff = sqrt(ne_true * ne_true + c.ne_hall_floor * c.ne_hall_floor);
   if constexpr (sizeof(R) == 4) {
     const R it = R(1.0) / ne_true, ie = R(1.0) / d.ne_eff;
-    const bool some = ne_true > R(0.0);
-    d.chiH = some ? d.nH * it : R(1.0);
-    d.chiNa = some ? d.nNa * it : R(0.0);
+    d.chiH = d.nH * it;
+    d.chiNa = d.nNa * it;
+    if (!(ne_true >= R(1.2e-38))) {  // no normal number: its reciprocal may overflow, the quotients are at most 1
+      const bool some = ne_true > R(0.0);
+      d.chiH = some ? d.nH / ne_true : R(1.0);
+      d.chiNa = some ? d.nNa / ne_true : R(0.0);
+    }
     d.wH = d.nH * ie;
     d.wNa = d.nNa * ie;
     return d;
