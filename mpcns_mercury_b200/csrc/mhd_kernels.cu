@@ -1285,25 +1285,32 @@ __global__ void __launch_bounds__(kVecThreads, 3) k_jcell(Dir D) {
   });
 }
 
-// Quotients by one divisor b > 0.  FP32: by its reciprocal.  FP64: the quotient
+// Quotients by one divisor b >= 1e-12.  FP32: by its reciprocal.  FP64: the quotient
 // that IEEE division rounds to, from the correctly rounded reciprocal y = RN(1/b)
 // and one residual, q = RN(a y), RN(q + RN(a - b q) y) (Markstein, "Computation
 // of elementary functions on the IBM RISC System/6000 processor", 1990): exact
-// while nothing under- or overflows, so values outside [1e-280, 1e280] are
-// divided (a zero keeps its sign).
+// while y, the quotient and the residual are normal numbers, so a outside
+// [2^-600, 2^930) and any a by a divisor from 2^332 on (or NaN) is divided (a zero
+// keeps its sign).  The ranges are tested on the upper words: tests of the
+// quotient in FP64 took 6 to 10 % of a step.
 template <class R>
 struct Divisor {
+  static constexpr uint32_t kLow = (1023u - 600u) << 20, kSpan = ((1023u + 930u) << 20) - kLow, kTop = (1023u + 332u) << 20;
   R b, y;
-  __device__ __forceinline__ explicit Divisor(R d) : b(d) {
-    if constexpr (sizeof(R) == 4) y = R(1.0) / d;
-    else y = __drcp_rn(d);
+  uint32_t span;  // FP64: the range's width, 0 where everything is divided
+  __device__ __forceinline__ Divisor(R d, R recip) : b(d), y(recip), span(0) {
+    if constexpr (sizeof(R) == 8) span = (uint32_t)__double2hiint(d) < kTop ? kSpan : 0u;
   }
-  __device__ __forceinline__ Divisor(R d, R recip) : b(d), y(recip) {}
+  __device__ __forceinline__ explicit Divisor(R d) : Divisor(d, reciprocal(d)) {}
+  __device__ __forceinline__ static R reciprocal(R d) {
+    if constexpr (sizeof(R) == 4) return R(1.0) / d;
+    else return __drcp_rn(d);
+  }
   __device__ __forceinline__ R operator()(R a) const {
     if constexpr (sizeof(R) == 4) return a * y;
     else {
-      const R q = a * y, m = fabs(a);
-      if (m >= R(1e-280) && m <= R(1e280)) return fma(fma(-b, q, a), y, q);
+      const R q = a * y;
+      if (((uint32_t)__double2hiint(a) & 0x7fffffffu) - kLow < span) return fma(fma(-b, q, a), y, q);
       return a == R(0.0) ? q : a / b;
     }
   }
