@@ -194,6 +194,9 @@ struct Solve {
   Tables *T = nullptr;
   double res_rtol = 0.0;
   int res_max_it = 0;
+  // substeps that the solve can still take part in: the steps requested and not
+  // queued yet, 0 once one that was queued after that request went without it
+  int64_t res_left = 0, res_request = 0;  // (res_request: the batch's count of requests then)
   int res_direct = 0;  // mixed precision: FP64 CG while the last substep took at most this many iterations
   // mixed precision with the implicit resistive substep: slot of the FP64
   // companion solve (same blocks and tables) in the batch's companion batch
@@ -292,6 +295,7 @@ struct mhd_batch {
   cudaEvent_t cg_done = nullptr;
   bool cg_pending = false;
   std::vector<Solve *> cg_solves;
+  int64_t requests = 0, cg_requests = 0;  // mhd_batch_request calls, and how many ahead of the last substep
   double res_ms = 0.0;
   int64_t res_steps = 0;
   int kernels_per_step = 0;
@@ -1684,7 +1688,10 @@ int fold_cg(mhd_batch *b) {
     Solve *S = b->cg_solves[s];
     if (!S) continue;
     const ResCG &h = b->precision == kMixed ? b->shadow->hcg[S->shadow_slot] : b->hcg[s];
-    if (!h.ran) continue;
+    if (!h.ran) {  // done, or stopped by its status
+      if (S->res_request <= b->cg_requests) S->res_left = 0;
+      continue;
+    }
     any = true;
     take_cg(S, h);
   }
@@ -1725,6 +1732,7 @@ int res_step_device(mhd_batch *b) {
     if (b->slots[s] && b->slots[s]->consts.resistive) b->cg_solves[s] = b->slots[s];
   CUDA_TRY(cudaEventRecord(b->cg_done, b->stream));
   b->cg_pending = true;
+  b->cg_requests = b->requests;
   if (mixed) launch_res_cross(b->dir(1), RES_X_DEMOTE_X, b->stream, c->res.cg, c->res.use_p, b->n_foreign > 0);
   else launch(b, 1, SK_RES_VEC, &nk, nullptr, RES_E_FROM_CG);
   res_finish(b, &nk);
@@ -3305,6 +3313,8 @@ int mhd_batch_request(mhd_batch *b, int slot, int64_t nsteps) {
   if (nsteps < 0) return fail(MHD_ERR_ARG, "nsteps %lld", (long long)nsteps);
   if (nsteps > 0 && !b->slots[slot]->prepared) return fail(MHD_ERR_STATE, "steps requested before prepare");
   const long long n = nsteps;
+  b->slots[slot]->res_left = n;
+  b->slots[slot]->res_request = ++b->requests;
   return set_state_field(b, slot, offsetof(SolveState, remaining), &n, sizeof n);
 }
 
@@ -3364,11 +3374,17 @@ int mhd_batch_run(mhd_batch *b, int nsteps) {
     CUDA_TRY(cudaGraphLaunch(b->graph_a, b->stream));
     if ((rc = fold_cg(b))) return rc;  // the previous step's
     fold_substep_time(b, false);
-    bool device = !b->cg_host_loop;
-    if (b->precision == kMixed)
-      for (const Solve *S : b->slots) device = device && !(S && S->consts.resistive && !runs_direct(S));
+    bool device = !b->cg_host_loop, any = false;
+    for (Solve *S : b->slots) {
+      if (!S || !S->consts.resistive) continue;
+      if (b->precision == kMixed) device = device && runs_direct(S);
+      any = any || S->res_left > 0;
+      if (S->res_left > 0) --S->res_left;
+    }
     const int p = b->res_ev_next;
-    if (device) {
+    if (!any) {
+      // no resistive solve has steps left: the others go on without a substep
+    } else if (device) {
       CUDA_TRY(cudaEventRecord(b->res_ev[p][0], b->stream));
       if ((rc = res_step_device(b))) return rc;
       CUDA_TRY(cudaEventRecord(b->res_ev[p][1], b->stream));
