@@ -353,7 +353,9 @@ int mhd_kernels_per_step(mhd_ctx *ctx);
 /* Raw device pointer of one field component array of a block, with the box
  * layout: element (i,j,k) at base[(i+G)*si + (j+G)*sj + (k+G)].  The
  * elements are double, except in mixed precision (mhd_desc.precision = 1),
- * where every field other than MHD_JAC and MHD_JD* holds float. */
+ * where every field other than MHD_JAC and MHD_JD* holds float.  For reading:
+ * a caller that writes a field through it calls mhd_prepare before the next
+ * step, as after an upload (the step keeps values derived from the state). */
 int mhd_device_view(mhd_ctx *ctx, int field, int block, int comp, double **base, int32_t *G, int64_t *si,
                     int64_t *sj, int32_t ext[3]);
 

@@ -2983,6 +2983,7 @@ int mhd_batch_sync(mhd_batch *b, int slot, int group) {
     if (db) launch(b, 1, SK_RES_COPYB, nk, nullptr, RES_DB_FROM_B);
     enqueue_sync(b, 1, group, nk, true);
     if (db) launch(b, 1, SK_RES_COPYB, nk, nullptr, RES_B_FROM_DB);
+    if (group == MHD_SYNC_UCELL && b->slots[slot]->prepared) launch(b, 1, SK_FLUX_TERMS, nk);
   });
 }
 

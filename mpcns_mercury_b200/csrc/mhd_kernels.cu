@@ -1964,6 +1964,38 @@ __global__ void __launch_bounds__(kVecThreads) k_face_normals(Dir D) {
   });
 }
 
+// A cell's terms of the Rusanov flux (FluidCell) from its density as it stands in
+// U, |u|^2 and the pressure.
+template <class R>
+__device__ __forceinline__ void flux_terms(const ConstsT<R> &c, R rho, R u2, R p, R &re, R &cs) {
+  if constexpr (sizeof(R) == 4) re = p * c.inv_g1 + R(0.5) * rho * u2;
+  else re = p / (c.gamma - R(1.0)) + R(0.5) * rho * u2;
+  cs = sqrt(dmax(R(0.0), c.gamma * p / dmax(rho, R(1e-30))));
+}
+
+// The flux terms again after an explicit Sync(U) between steps: it may give ghosts
+// on rotated seams other densities than the step's sync left there, and the
+// next step's fluxes take these with the primitive variables as they are.
+template <class R>
+__global__ void __launch_bounds__(kVecThreads) k_flux_terms(Dir D) {
+  for_vec_items<R, kAlloc>(D, [&](const DevSolve &S, const auto &B, const VItem &it) {
+    constexpr int N = group_size(kAlloc, sizeof(R));
+    const ConstsT<R> &c = consts_of<R>(S);
+    const uint32_t o = it.o;
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const int pv0 = s ? cPVN : cPVH;
+      const auto rho = B.lv(s ? cUN : cUH, o), u = B.lv(pv0, o), v = B.lv(pv0 + 1, o), w = B.lv(pv0 + 2, o), p = B.lv(pv0 + 3, o);
+      Vec<R, N> re, cs;
+#pragma unroll
+      for (int e = 0; e < N; ++e)
+        flux_terms(c, rho.v[e], u.v[e] * u.v[e] + v.v[e] * v.v[e] + w.v[e] * w.v[e], p.v[e], re.v[e], cs.v[e]);
+      B.st(cFT + 2 * s, it, re, it.klo, it.khi);
+      B.st(cFT + 2 * s + 1, it, cs, it.klo, it.khi);
+    }
+  });
+}
+
 // calc_PV + calc_Uplus (Z4_Mercury/src/physics/MercurySolver_Tools.cpp:159-301) on the allocated
 // cell range the step keeps, the fluid fluxes' cell terms, the contravariant
 // velocities UCON and the next step's Hall cell field there, and the next
@@ -2014,15 +2046,9 @@ __global__ void __launch_bounds__(kVecThreads, kPvCtas) k_pv_uplus(Dir D, int en
           if (eint < R(0.0)) eint = R(0.0);
           const R p = dmax((c.gamma - R(1.0)) * eint, R(1e-12));
           pr.v[e] = p;
-          // the Rusanov flux's terms of the cell (fluid_cell)
-          if constexpr (sizeof(R) == 4) {
-            T.v[e] = by(p) * c.inv_coeff[s];
-            re.v[e] = p * c.inv_g1 + R(0.5) * r0.v[e] * u2;
-          } else {
-            T.v[e] = p / (rh * coeff);
-            re.v[e] = p / (c.gamma - R(1.0)) + R(0.5) * r0.v[e] * u2;
-          }
-          cs.v[e] = sqrt(dmax(R(0.0), c.gamma * p / dmax(r0.v[e], R(1e-30))));
+          if constexpr (sizeof(R) == 4) T.v[e] = by(p) * c.inv_coeff[s];
+          else T.v[e] = p / (rh * coeff);
+          flux_terms(c, r0.v[e], u2, p, re.v[e], cs.v[e]);
           vel[s][0].v[e] = u;
           vel[s][1].v[e] = v;
           vel[s][2].v[e] = w;
@@ -2629,6 +2655,7 @@ static const void *kernel_fn(StepKernel k) {
     case SK_PV_UPLUS: return (const void *)k_pv_uplus<R>;
     case SK_SYNC: return (const void *)k_sync<R, kMaxSyncOps>;
     case SK_FACE_NORMALS: return (const void *)k_face_normals<R>;
+    case SK_FLUX_TERMS: return (const void *)k_flux_terms<R>;
     case SK_DIVB: return (const void *)k_div_b<R>;
     case SK_RES_SEED: return (const void *)k_res_seed<R>;
     case SK_RES_W: return (const void *)k_res_w<R>;
@@ -2652,7 +2679,7 @@ static int kernel_threads(StepKernel k) {
     case SK_FACE_EMF: case SK_EDGE_EMF: case SK_ADD_HALL: case SK_BFACE: case SK_BCELL_JEDGE:
     case SK_JCELL: case SK_PV_UPLUS: case SK_FACE_NORMALS: case SK_DIVB: case SK_RES_SEED: case SK_RES_W:
     case SK_RES_VEC: case SK_RES_DB: case SK_RES_DJ: case SK_RES_Q: case SK_RES_BUPDATE: case SK_RES_CG:
-    case SK_RES_PUPD_E:
+    case SK_RES_PUPD_E: case SK_FLUX_TERMS:
       return kVecThreads;
     default: return kTileThreads;
   }
@@ -2723,6 +2750,7 @@ static void launch_as(StepKernel k, const Dir &D, cudaStream_t st, const SyncOps
       else launch_dependent(k_sync<R, kMaxSyncOps>, G, kTileThreads, st, D, *ops);
       break;
     case SK_FACE_NORMALS: k_face_normals<R><<<G, kVecThreads, 0, st>>>(D); break;
+    case SK_FLUX_TERMS: launch_dependent(k_flux_terms<R>, G, kVecThreads, st, D); break;
     case SK_DIVB: k_div_b<R><<<G, kVecThreads, 0, st>>>(D); break;
     case SK_RES_SEED: k_res_seed<R><<<G, kVecThreads, 0, st>>>(D); break;
     case SK_RES_W: k_res_w<R><<<G, kVecThreads, 0, st>>>(D); break;
@@ -2951,7 +2979,7 @@ const char *step_kernel_name(StepKernel k) {
                                 "k_res_seed", "k_res_w",    "k_res_vec",     "k_res_db",   "k_res_dj",
                                 "k_res_q",    "k_res_dot",  "k_res_sum",     "k_res_copyb", "k_res_bupdate",
                                 "k_res_cg",   "k_res_pupd_e", "k_phys",      "k_sing_setup", "k_sing_emf",
-                                "k_sing_j",   "k_res_clearb"};
+                                "k_sing_j",   "k_res_clearb", "k_flux_terms"};
   static_assert(sizeof(names) / sizeof(names[0]) == SK_COUNT, "a name per kernel");
   return (k >= 0 && k < SK_COUNT) ? names[k] : "?";
 }

@@ -15,7 +15,8 @@ enum StepKernel {
   // grids with physical boundaries and singular edges
   SK_PHYS, SK_SING_SETUP, SK_SING_EMF, SK_SING_J,
   // implicit resistive substep on grids with physical boundaries: zero the ghost faces of dB
-  SK_RES_CLEARB, SK_COUNT
+  SK_RES_CLEARB,
+  SK_FLUX_TERMS, SK_COUNT
 };
 
 // One launch of k_sync runs up to kMaxSyncOps independent sync operations: a copy
