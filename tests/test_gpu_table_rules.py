@@ -295,3 +295,71 @@ def test_operation_on_another_groups_field(precision):
         got.append(fields(batch, slot))
         batch.close()
     same(*got)
+
+
+def test_owner_copies_of_the_substep_that_are_not_there_already():
+    """Sync(dB) with an owner copy between faces of different edges: its owner copies run, the rest is left out."""
+    got = []
+    for ordered in (False, True):
+        t = Tables(resistive=True)
+        t.add_copy("DB", "owner", dof("B_XI", 2, 2, 3), dof("B_XI", 3, 2, 3))
+        t.k.res_rtol = t.d.constants.res_rtol = 1e-3
+        if ordered:
+            t.ordered("DB")
+        got.append(t.run())
+    same(*got)
+
+
+def _shell_run(rule, ordered):
+    """Three steps of a small shell with one entry that breaks `rule` of the joined syncs."""
+    from mpcns_mercury_b200 import capi
+    from mpcns_mercury_b200 import magnetosphere as M
+    from mpcns_mercury_b200.capi import Batch, MhdCopy, MhdPhysOp, SolveDesc
+
+    case = M.ShellCase(na=6, nr=5)
+    k = M.constants(case)
+    topo = M.topology(case)
+    t = Tables.__new__(Tables)
+    t.keep, t.desc = [], SolveDesc(case.cells, G, k, topology=topo)
+    t.d = t.desc.desc
+    hall, edge = t.group("EHALL"), t.group("EEDGE")
+    if rule == "staged source set by its group":
+        t.add_set("EHALL", hall.stash[0].src, 11)
+    elif rule == "staged source set by the wall":
+        op = MhdPhysOp()
+        op.kind, op.arg, op.dst, op.src = 0, 11, edge.stash[0].src, edge.stash[0].src
+        t.d.wall, t.d.n_wall = t._array(MhdPhysOp, [t.d.wall[q] for q in range(t.d.n_wall)] + [op]), t.d.n_wall + 1
+    elif rule == "a slot of two groups":
+        rows = [MhdCopy(c.dst, c.src, c.sign) for c in (edge.stash[q] for q in range(2 * edge.n_stash))]
+        rows[0].dst.i = rows[edge.n_stash].src.i = hall.stash[0].dst.i
+        edge.stash = t._array(MhdCopy, rows)
+    else:  # an owned edge staged: E there takes its Hall EMF behind the staging of the joined order
+        n = edge.n_stash
+        rows = [edge.stash[q] for q in range(2 * n)]
+        slot = MhdCopy(rows[0].dst, edge.owner[0].src, 1.0)
+        slot.dst.i = t.d.n_staging
+        back = MhdCopy(edge.halo[0].dst, slot.dst, 1.0)
+        edge.stash, edge.n_stash = t._array(MhdCopy, rows[:n] + [slot] + rows[n:] + [back]), n + 1
+        t.set_copies("EEDGE", "halo", t.copies("EEDGE", "halo")[1:])
+        t.d.n_staging += 1
+    if ordered:
+        t.ordered("JEDGE")
+    batch = Batch(1, 0)
+    slot = batch.add(t.desc)
+    M.set_up(batch, case, slot=slot, k=k)
+    batch.prepare(slot)
+    batch.request(slot, 3)
+    batch.run(3)
+    info = batch.poll()[slot]
+    assert info.status == 0 and info.step == 3
+    out = [batch.download(slot, f, (-G,) * 3, tuple(v + 1 + G for v in n), block=b) for f in FIELDS for b, n in enumerate(case.cells)]
+    batch.close()
+    capi.lib().mhd_topology_destroy(ctypes.c_void_p(topo.value))
+    return out
+
+
+@pytest.mark.parametrize("rule", ["staged source set by its group", "staged source set by the wall", "a slot of two groups",
+                                  "an owned edge staged"])
+def test_rules_of_the_joined_syncs(rule):
+    for a, b in zip(_shell_run(rule, False), _shell_run(rule, True)):
+        assert np.array_equal(a, b, equal_nan=True)
