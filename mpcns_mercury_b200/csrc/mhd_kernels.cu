@@ -373,13 +373,13 @@ struct VV : V<R> {
   // A field that a pass of the step or of the substep writes.  These passes start
   // while their predecessor may still write it, and the wait
   // (wait_for_predecessors) orders ordinary loads only.  An ordinary load does not
-  // pass a store that could be to its address, so k_bcell_jedge, k_pv_uplus,
-  // k_res_db, k_res_pupd_e and k_res_bupdate load all they need ahead of their
-  // first store (on the 96^3 mixed box 0.038 ms instead of 0.041 and 0.076
-  // instead of 0.081, a step of the 8^3 FP64 box 48 us instead of 50); the EMF
-  // passes, k_bface and k_res_cg are no faster that way.  With every launch in
-  // full and read-only loads instead, a step takes 63 us on the 8^3 FP64 box,
-  // 95 (73) on 32^3, 164 (138) on 64^3 mixed.
+  // pass a store that could be to its address, so k_edge_emf, k_bcell_jedge,
+  // k_pv_uplus, k_res_db, k_res_pupd_e, k_res_bupdate and in FP64 k_face_emf load
+  // all they need ahead of their first store (k_bcell_jedge on the 96^3 mixed box
+  // 0.038 ms instead of 0.041, k_pv_uplus 0.076 instead of 0.081, a step of the
+  // 8^3 FP64 box 48 us instead of 50); k_bface and k_res_cg are no faster that
+  // way.  With every launch in full and read-only loads instead, a step takes
+  // 63 us on the 8^3 FP64 box, 95 (73) on 32^3, 164 (139) on 64^3 mixed.
   __device__ __forceinline__ Vc lv(int comp, uint32_t o) const { return *(const Vc *)((const char *)c(comp) + o); }
   __device__ __forceinline__ R ld(int comp, uint32_t bo) const { return *(const R *)((const char *)c(comp) + bo); }
   // lv of a static field of the implicit substep: an FP64 companion reads the
@@ -638,7 +638,17 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(R) == 8 ? 2 : 3) k_face_em
   for_vec_items<R, kExt>(D, [&](const DevSolve &S, const VV<R> &B, const VItem &it) {
     const int i = it.i, j = it.j;
     const uint32_t o = it.o, di = B.di, dj = B.dj;
-    if (uniform(consts_of<R>(S).ambipolar)) {
+    // Behind every load where the registers allow it (FP64; lv): a step of the 32^3
+    // FP64 box takes 73 us, 77 with stores in between; in FP32 one fewer CTA fits.
+    constexpr bool kLate = sizeof(R) == 8;
+    const bool ambi = uniform(consts_of<R>(S).ambipolar) != 0;
+    Vec<R> pnode, dpe[3];
+    auto put_pe = [&] {
+      B.st(cPEN, it, pnode, 0, B.n2 + 1, i >= 0 && j >= 0 && i <= B.n0 && j <= B.n1);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) B.st(cDPE + q, it, dpe[q], 0, B.n2, i >= 0 && j >= 0 && i < B.n0 && j < B.n1);
+    };
+    if (ambi) {
       auto pe = [&](uint32_t q) { return B.lv(cPVH + 3, q) + B.lv(cPVN + 3, q); };
       auto pe1 = [&](uint32_t q) { return B.ld(cPVH + 3, q) + B.ld(cPVN + 3, q); };
       constexpr uint32_t es = sizeof(R);
@@ -654,16 +664,16 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(R) == 8 ? 2 : 3) k_face_em
       sum = sum + pjm;
       sum = sum + pkm;
       sum = sum + p0;
-      B.st(cPEN, it, R(0.125) * sum, 0, B.n2 + 1, i >= 0 && j >= 0 && i <= B.n0 && j <= B.n1);
+      pnode = R(0.125) * sum;
       {
         // grad p_e term of the ion momentum sources of an owned cell, the
         // same for both species (AddSourceToRHS_Fluid, FluidRHS.cpp:206-527)
         const Vec<R> gi = pe(o + di) - pim, gj = pe(o + dj) - pjm, gk = vup(p0, pe1(o + 16u)) - pkm;
 #pragma unroll
         for (int q = 0; q < 3; ++q)
-          B.st(cDPE + q, it, R(0.5) * (B.fixed(cAMB + q, o) * gi + B.fixed(cAMB + 3 + q, o) * gj + B.fixed(cAMB + 6 + q, o) * gk), 0,
-               B.n2, i >= 0 && j >= 0 && i < B.n0 && j < B.n1);
+          dpe[q] = R(0.5) * (B.fixed(cAMB + q, o) * gi + B.fixed(cAMB + 3 + q, o) * gj + B.fixed(cAMB + 6 + q, o) * gk);
       }
+      if (!kLate) put_pe();
     }
     // induced and total B averaged to the cells (cell_beta_ind, cell_beta_tot)
     auto ind = [&](int a, uint32_t q, uint32_t d) { return R(0.5) * (B.lv(cBX + a, q) + B.lv(cBX + a, q + d)); };
@@ -691,25 +701,32 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(R) == 8 ? 2 : 3) k_face_em
     };
     const bool ri = i < B.n0 + 1, rj = j < B.n1 + 1;  // in the range of the other families
     const int k1 = B.n2 + 1;
+    Vec<R> xe, xz, yx, yz;  // the fluxes: face family, component
+    auto put_x = [&] {
+      B.st(cEFX, it, vset(R(0.0)), -1, k1, rj);
+      B.st(cEFX + 1, it, xz, -1, k1, rj);
+      B.st(cEFX + 2, it, -xe, -1, k1, rj);
+    };
+    auto put_y = [&] {
+      B.st(cEFY, it, -yz, -1, k1, ri);
+      B.st(cEFY + 1, it, vset(R(0.0)), -1, k1, ri);
+      B.st(cEFY + 2, it, yx, -1, k1, ri);
+    };
     {
       const Vec<R> bff = B.lv(cBX, o) + B.fixed(cBAX, o);
       const uint32_t q = o - di;
       const Vec<R> ufL = B.lv(cUC, q);
-      const Vec<R> Ge = flux(1, 0, tot(1, q, dj), ind(1, q, dj), ufL, B.lv(cUC + 1, q), bff);
-      const Vec<R> Gz = flux(2, 0, tot_k(q), ind_k(q), ufL, B.lv(cUC + 2, q), bff);
-      B.st(cEFX, it, vset(R(0.0)), -1, k1, rj);
-      B.st(cEFX + 1, it, Gz, -1, k1, rj);
-      B.st(cEFX + 2, it, -Ge, -1, k1, rj);
+      xe = flux(1, 0, tot(1, q, dj), ind(1, q, dj), ufL, B.lv(cUC + 1, q), bff);
+      xz = flux(2, 0, tot_k(q), ind_k(q), ufL, B.lv(cUC + 2, q), bff);
+      if (!kLate) put_x();
     }
     {
       const Vec<R> bff = B.lv(cBY, o) + B.fixed(cBAY, o);
       const uint32_t q = o - dj;
       const Vec<R> ufL = B.lv(cUC + 1, q);
-      const Vec<R> Gx = flux(0, 1, tot(0, q, di), ind(0, q, di), ufL, B.lv(cUC, q), bff);
-      const Vec<R> Gz = flux(2, 1, tot_k(q), ind_k(q), ufL, B.lv(cUC + 2, q), bff);
-      B.st(cEFY, it, -Gz, -1, k1, ri);
-      B.st(cEFY + 1, it, vset(R(0.0)), -1, k1, ri);
-      B.st(cEFY + 2, it, Gx, -1, k1, ri);
+      yx = flux(0, 1, tot(0, q, di), ind(0, q, di), ufL, B.lv(cUC, q), bff);
+      yz = flux(2, 1, tot_k(q), ind_k(q), ufL, B.lv(cUC + 2, q), bff);
+      if (!kLate) put_y();
     }
     {
       const Vec<R> bff = B.lv(cBZ, o) + B.fixed(cBAZ, o);
@@ -721,6 +738,11 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(R) == 8 ? 2 : 3) k_face_em
       const Vec<R> ufL = vdown(u[2], B.ld(cUC + 2, q));
       const Vec<R> Gx = flux(0, 2, totL(0, di), indL(0, di), ufL, vdown(u[0], B.ld(cUC, q)), bff);
       const Vec<R> Ge = flux(1, 2, totL(1, dj), indL(1, dj), ufL, vdown(u[1], B.ld(cUC + 1, q)), bff);
+      if (kLate) {
+        put_x();
+        put_y();
+        if (ambi) put_pe();
+      }
       B.st(cEFZ, it, Ge, -1, k1 + 1, ri && rj);
       B.st(cEFZ + 1, it, -Gx, -1, k1 + 1, ri && rj);
       B.st(cEFZ + 2, it, vset(R(0.0)), -1, k1 + 1, ri && rj);
@@ -836,16 +858,8 @@ __global__ void __launch_bounds__(kVecThreads, 3) k_edge_emf(Dir D) {
       if (ambi) e = e - pc * (B.upper(pn, cPEN, o) - pn) / ne_of(rho_ij(cUH), rho_ij(cUN));
       E[2] = add_artificial(B, c, 2, o, e);
     }
-    // E_Hall of family ax, and E: with it inside the block, without on its faces
-    const bool late = S.hall_late != 0;
-    auto put = [&](int ax, const Vec<R> &h, int hi, bool owned, bool face, bool kfaces) {
-      B.st(cHX + ax, it, h, 0, hi, owned);
-      B.st(cEX + ax, it, vmap<R>([&](int e) {
-             const bool f = face || (kfaces && (it.k + e == 0 || it.k + e == B.n2));
-             return f ? E[ax].v[e] : E[ax].v[e] + h.v[e];
-           }), 0, hi, owned);
-    };
     const R Cwh = R(0.1);
+    Vec<R> h[3];  // E_Hall
     // over the four cells at an edge, in the reference's order: lower row and
     // lower k first
     auto mean_k = [&](int comp, uint32_t d) {
@@ -870,23 +884,33 @@ __global__ void __launch_bounds__(kVecThreads, 3) k_edge_emf(Dir D) {
       const Vec<R> Ecen = mean_k(cEHC, dj) * B.fixed(cDRX, o) + mean_k(cEHC + 1, dj) * B.fixed(cDRX + 1, o) +
                           mean_k(cEHC + 2, dj) * B.fixed(cDRX + 2, o);
       const Vec<R> by = B.lv(cBY, o);
-      put(0, tail(0, Ecen, max_k(cHB, dj), B.lv(cBZ, o) - B.lv(cBZ, o - dj), by - B.lower(by, cBY, o)), B.n2 + 1, it.i < B.n0,
-          late || it.j == 0 || it.j == B.n1, true);
+      h[0] = tail(0, Ecen, max_k(cHB, dj), B.lv(cBZ, o) - B.lv(cBZ, o - dj), by - B.lower(by, cBY, o));
     }
     {
       const Vec<R> Ecen = mean_k(cEHC, di) * B.fixed(cDRY, o) + mean_k(cEHC + 1, di) * B.fixed(cDRY + 1, o) +
                           mean_k(cEHC + 2, di) * B.fixed(cDRY + 2, o);
       const Vec<R> bx = B.lv(cBX, o);
-      put(1, tail(1, Ecen, max_k(cHB, di), bx - B.lower(bx, cBX, o), B.lv(cBZ, o) - B.lv(cBZ, o - di)), B.n2 + 1, it.j < B.n1,
-          late || it.i == 0 || it.i == B.n0, true);
+      h[1] = tail(1, Ecen, max_k(cHB, di), bx - B.lower(bx, cBX, o), B.lv(cBZ, o) - B.lv(cBZ, o - di));
     }
     {
       const Vec<R> Ecen =
           mean_ij(cEHC) * B.fixed(cDRZ, o) + mean_ij(cEHC + 1) * B.fixed(cDRZ + 1, o) + mean_ij(cEHC + 2) * B.fixed(cDRZ + 2, o);
       const Vec<R> be = vmax(vmax(B.lv(cHB, o - di - dj), B.lv(cHB, o - di)), vmax(B.lv(cHB, o - dj), B.lv(cHB, o)));
-      put(2, tail(2, Ecen, be, B.lv(cBY, o) - B.lv(cBY, o - di), B.lv(cBX, o) - B.lv(cBX, o - dj)), B.n2, true,
-          late || it.i == 0 || it.i == B.n0 || it.j == 0 || it.j == B.n1, false);
+      h[2] = tail(2, Ecen, be, B.lv(cBY, o) - B.lv(cBY, o - di), B.lv(cBX, o) - B.lv(cBX, o - dj));
     }
+    // E_Hall of family ax, and E: with it inside the block, without on its faces
+    // (the stores behind every load: lv)
+    const bool late = S.hall_late != 0;
+    auto put = [&](int ax, int hi, bool owned, bool face, bool kfaces) {
+      B.st(cHX + ax, it, h[ax], 0, hi, owned);
+      B.st(cEX + ax, it, vmap<R>([&](int e) {
+             const bool f = face || (kfaces && (it.k + e == 0 || it.k + e == B.n2));
+             return f ? E[ax].v[e] : E[ax].v[e] + h[ax].v[e];
+           }), 0, hi, owned);
+    };
+    put(0, B.n2 + 1, it.i < B.n0, late || it.j == 0 || it.j == B.n1, true);
+    put(1, B.n2 + 1, it.j < B.n1, late || it.i == 0 || it.i == B.n0, true);
+    put(2, B.n2, true, late || it.i == 0 || it.i == B.n0 || it.j == 0 || it.j == B.n1, false);
   });
 }
 
