@@ -296,8 +296,8 @@ def roofline(prof, cells, peak, peak_kind, precision=0, traffic_key=None):
     return {"kernel": top, "bound": "hbm", "achieved": round(achieved, 2), "peak": peak, "unit": "GB/s",
             "frac": round(achieved / peak, 4), "peak_source": peak_kind,
             "algo_bytes_per_launch": int(algo_bytes), "launch_ms": round(ms, 5),
-            "traffic": traffic, "traffic_note": ("ncu DRAM bytes per owned cell of a captured launch (8-solve "
-                                                 "ensemble) x this launch's owned cells") if per_cell else None,
+            "traffic": traffic, "traffic_note": ("ncu DRAM bytes per owned cell of a captured launch "
+                                                 "(profiles/dram_bytes.json) x this launch's owned cells") if per_cell else None,
             "share_of_step": round(ms / sum(prof.values()), 4)}
 
 

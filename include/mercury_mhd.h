@@ -43,7 +43,7 @@ enum mhd_status {
                            at its next step, the batch's other solves go on */
   MHD_ERR_SOLVE = 6,    /* implicit solve did not converge */
   MHD_ERR_STATE = 7,    /* call out of order (e.g. step before prepare) */
-  MHD_ERR_TIMEOUT = 8   /* a wait inside a kernel ran into its bound: the solve stops */
+  MHD_ERR_TIMEOUT = 8   /* reserved: no kernel waits, so none returns it */
 };
 
 /* Field identifiers: the reference's catalog names
@@ -498,7 +498,7 @@ int mhd_batch_prepare(mhd_batch *batch, int slot, double time, int64_t step);
  * captured anew).  The choice does not change results: every variant
  * computes each face flux and cell update with the same operations.
  * Variant 6 is variant 0's tile with more resident work items in mixed
- * precision. */
+ * precision; in FP64 it is variant 0. */
 #define MHD_NUM_FLUID_TILES 7
 int mhd_fluid_tile_shape(int variant, int32_t shape[4]);
 int mhd_batch_fluid_tile(mhd_batch *batch, int variant);

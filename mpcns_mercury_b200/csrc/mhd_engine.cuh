@@ -18,7 +18,8 @@ namespace mhd {
 // The fluid kernel's tile variants: cells along k, j, i of one work item (256
 // cells, two items per tile, one per ion species), and a rank of its register
 // budget (fluid_ctas).  The batch runs one of them (mhd_batch_fluid_tile),
-// picked by timing (mhd_batch_time_fluid_tiles); variant 0 is the default:
+// picked by timing (mhd_batch_time_fluid_tiles; in FP64 variants 0 and 6 are one
+// kernel); variant 0 is the default:
 // 16 x 4 x 4 wastes fewer lanes than wider tiles on k extents that are not
 // multiples of 32.
 struct FluidTile {

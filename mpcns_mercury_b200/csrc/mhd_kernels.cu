@@ -263,7 +263,7 @@ __device__ __forceinline__ void for_items(const Dir &D, F &&f) {
 
 // ------------------------------------------------------------------ vector items
 // The step's stencil passes take 16 bytes of consecutive k positions (4 FP32 or
-// 2 FP64 values, aligned: block rows start on 64-byte boundaries) per thread and
+// 2 FP64 values, aligned: rows are padded to 8 elements) per thread and
 // array, element by element with the operations of the scalar form.
 template <class R, int M = 16 / (int)sizeof(R)>
 struct alignas(M * sizeof(R)) Vec {
@@ -1444,9 +1444,10 @@ __global__ void __launch_bounds__(kVecThreads) k_div_b(Dir D) {
 // SolveImplicitResistiveDiffusion_ (Z4_Mercury/src/implicit/Mercury_ImplicitResistive.cpp:475-575):
 // (I + dt eta alpha C^T beta C) E = eta J(B*) on the owned edges with eta > 0.
 // The operator is self-adjoint in the inner product weighted by
-// W = 1 / (eta alpha), so CG runs in that inner product; the edge, face and J
-// fields of the explicit step are the operator's scratch (E: E_res, B: dB,
-// J: dJ), with the step's own E / B / J sync and alias tables.
+// W = 1 / (eta alpha), so CG runs in that inner product; the edge and J fields
+// of the explicit step are the operator's scratch (E: E_res, J: dJ), dB has
+// arrays of its own (RES_BSTAR), with the E and J sync and alias tables and
+// Sync(dB)'s.
 
 // Owned-range test of an edge of family a at (i, j, k).
 __device__ __forceinline__ bool edge_owned(int a, int i, int j, int k, int n0, int n1, int n2) {
@@ -1877,11 +1878,8 @@ __global__ void __launch_bounds__(kVecThreads) k_res_bupdate(Dir D) {
   });
 }
 
-// Static per-face terms of the CFL time step and the Rusanov wave speed, once
-// per solve (run by mhd_prepare): |a| = sqrt(ax ax + ay ay + az az) and
-// a / |a| of the face area vectors JD, the operations and order
 // Per-solve static terms, evaluated once at prepare with the reference's
-// expressions: the face normals and |JD| that Compute_Timestep
+// expressions: the face normals a / |a| and |a| of the area vectors JD that Compute_Timestep
 // (Timestep.cpp:15-16,78-93) and calc_Jac_radius_GCL (FluidRHS.cpp:5-14) apply
 // every step (owned faces and one more layer), the ambipolar gradient
 // coefficients (owned cells), the contravariant-velocity coefficients (the
