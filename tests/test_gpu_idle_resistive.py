@@ -48,7 +48,7 @@ def test_idle_resistive_solves(precision):
 
     def per_step(batch, slot, steps=300):
         best = float("inf")
-        for _ in range(5):
+        for _ in range(15):
             batch.request(slot, steps)
             batch.poll()
             t = time.perf_counter()
